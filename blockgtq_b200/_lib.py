@@ -24,6 +24,7 @@ ENC_NO_TCGEN05 = 128
 DEC_K_MIXED, DEC_V_NIBBLE, DEC_PROGRAMMATIC, DEC_GENERIC = 1, 2, 4, 8
 PF_NO_TCGEN05 = 16
 COMBINE_PROGRAMMATIC = 1
+STEP_Q_ROTATED = 1
 
 
 class HeadDesc(C.Structure):
@@ -44,6 +45,25 @@ class HeadDesc(C.Structure):
 
 class DecodePlan(C.Structure):
     _fields_ = [("opaque", C.c_uint8 * 4096)]
+
+
+class LayerStep(C.Structure):
+    """Mirror of ``BgtqLayerStep``."""
+    _fields_ = [
+        ("plan", C.c_void_p), ("desc", C.c_void_p), ("rot_k", C.c_void_p), ("rot_v", C.c_void_p), ("v_rot", C.c_void_p),
+        ("k_packed", C.c_void_p), ("kp_sb", C.c_int64), ("kp_sh", C.c_int64), ("kp_st", C.c_int64),
+        ("k_norms", C.c_void_p), ("kn_sb", C.c_int64), ("kn_sh", C.c_int64), ("kn_st", C.c_int64),
+        ("v_packed", C.c_void_p), ("vp_sb", C.c_int64), ("vp_sh", C.c_int64), ("vp_st", C.c_int64),
+        ("v_norms", C.c_void_p), ("vn_sb", C.c_int64), ("vn_sh", C.c_int64), ("vn_st", C.c_int64),
+        ("q_rot", C.c_void_p), ("part_o", C.c_void_p), ("part_lse", C.c_void_p),
+        ("out", C.c_void_p), ("o_sb", C.c_int64), ("o_sh", C.c_int64),
+        ("k_buf", C.c_void_p), ("v_buf", C.c_void_p), ("kb_sb", C.c_int64), ("kb_sh", C.c_int64),
+        ("buf_o", C.c_void_p), ("buf_lse", C.c_void_p), ("pos_dev", C.c_void_p), ("status", C.c_void_p),
+        ("n_batch", C.c_int32), ("n_q", C.c_int32), ("n_kv", C.c_int32), ("t_capacity", C.c_int32),
+        ("kp_row_bytes", C.c_int32), ("kn_count", C.c_int32), ("n_splits", C.c_int32), ("pos_add", C.c_int32),
+        ("enc_flags", C.c_int32), ("combine_flags", C.c_int32), ("flags", C.c_int32), ("n_sink", C.c_int32),
+        ("window", C.c_int32), ("scale", C.c_float),
+    ]
 
 
 _i32, _i64, _f32, _vp = C.c_int32, C.c_int64, C.c_float, C.c_void_p
@@ -74,6 +94,13 @@ _SIGNATURES = {
                                     _vp, _i64, _i64, _vp, _i64, _i64, _i32, _i32, _i32,
                                     _vp, _i64, _i64, _i64, _i32, _vp, _i64, _i64, _i64, _i32,
                                     _vp, _i64, _i64, _i64, _vp, _i64, _i64, _i64, _i32, _vp, _i32, _vp, _vp]),
+    "bgtq_layer_step_size": (C.c_int, []),
+    "bgtq_layer_step": (C.c_int, [_vp, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _vp, _i64, _vp]),
+    "bgtq_attend_scratch_bytes": (C.c_int64, [_i32, _i32, _i32]),
+    "bgtq_attend": (C.c_int, [_vp, _vp, _vp, _vp, _i64, _i64,
+                              _vp, _i64, _i64, _i64, _vp, _i64, _i64, _i64,
+                              _vp, _i64, _i64, _i64, _vp, _i64, _i64, _i64,
+                              _i32, _i32, _i32, _i32, _i32, _i32, _f32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "bgtq_rotate_q": (C.c_int, [_vp, _vp, _vp, _i64, _i64, _vp, _i32, _i32, _i32, _vp]),
     "bgtq_decode_plan": (C.c_int, [_vp, _i32, _i32, _vp]),
     "bgtq_decode_default_splits": (C.c_int, [_i32, _i32, _i32]),
@@ -139,6 +166,8 @@ def lib():
     if handle.bgtq_desc_size() != C.sizeof(HeadDesc):
         raise RuntimeError(f"BgtqHeadDesc size mismatch: library {handle.bgtq_desc_size()} vs binding "
                            f"{C.sizeof(HeadDesc)}")
+    if handle.bgtq_layer_step_size() != C.sizeof(LayerStep):
+        raise RuntimeError("BgtqLayerStep size mismatch between the library and the binding")
     _lib = handle
     return _lib
 
@@ -153,7 +182,11 @@ def ptr(t):
 
 
 def stream_ptr(device=None):
-    return torch.cuda.current_stream(device).cuda_stream
+    # (the raw handle: building a Stream object for it costs a microsecond of every call)
+    if device is not None and type(device) is not torch.device:
+        device = torch.device(device)
+    index = None if device is None else device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def require_cuda(t: torch.Tensor, name: str):

@@ -16,7 +16,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .layer import HD, combine, decode, make_decode_plan
+from .layer import HD, attend, make_decode_plan
 
 _cache = {}
 
@@ -54,10 +54,10 @@ class _AdHocLayer:
 
 
 def _layer_for(segments, codebook_flat, v_lut, v_bits, n_kv, device):
-    segs = tuple(tuple(int(x) for x in s) for s in segments)
-    key = (segs, codebook_flat.data_ptr(), v_lut.data_ptr(), int(v_bits), n_kv, str(device))
+    key = (tuple(map(tuple, segments)), codebook_flat.data_ptr(), v_lut.data_ptr(), int(v_bits), n_kv, device)
     lt = _cache.get(key)
     if lt is None:
+        segs = tuple(tuple(int(x) for x in s) for s in segments)
         raw = [s for s in segs if s[0] > 4 and s[2] > 0]
         nopack = (min(s[1] for s in raw), sum(s[2] for s in raw)) if raw else (HD, 0)
         lt = _AdHocLayer(segs, codebook_flat, v_lut, v_bits, n_kv, nopack, device)
@@ -98,21 +98,29 @@ def fused_blockgtq_decode_attention(
         scale = 1.0 / math.sqrt(D)
     if q_pack_perm is not None:
         q = q[:, :, :, q_pack_perm]
-    q2 = q.reshape(B, n_q, D).to(torch.float16).contiguous()
     if v_norms.dim() == 4:
         v_norms = v_norms[..., 0]
+    if k_norms.dtype != torch.float16:
+        k_norms = k_norms.to(torch.float16)
     lt = _layer_for(segments, codebook_flat, v_lut, vb_codebook, n_kv, q.device)
     flags = (_lib.DEC_K_MIXED if k_nibble else 0) | (_lib.DEC_V_NIBBLE if v_nibble else 0)
-    part_o, part_lse = decode(lt, q2, k_packed, k_norms.to(torch.float16), v_codes, v_norms, 0, T,
-                              n_splits=max(1, int(t_splits)), scale=scale, flags=flags)
-    rot = None
-    if v_rotation is not None:
-        rot = v_rotation.to(torch.float32).contiguous()
-        rot = rot.unsqueeze(0).expand(n_kv, -1, -1).contiguous() if rot.dim() == 2 else rot
-    out, _o32, lse = combine(part_o, part_lse, n_kv, v_rot=rot, want_lse=return_lse)
-    if return_lse:
-        return out.unsqueeze(2), lse
-    return out.unsqueeze(2)
+    out, _o32, lse = attend(lt, q.reshape(B, n_q, D), k_packed, k_norms, v_codes, v_norms, 0, T, rotate=False,
+                            n_splits=max(1, int(t_splits)), scale=scale, flags=flags, v_rot=_rotation(v_rotation, n_kv),
+                            want_lse=return_lse)
+    out = out.unsqueeze(2)
+    return (out, lse) if return_lse else out
+
+
+def _rotation(v_rotation, n_kv):
+    """The V rotation argument (one matrix for all heads, or one per head) as (n_kv, 128, 128) fp32."""
+    if v_rotation is None:
+        return None
+    rot = v_rotation
+    if rot.dtype != torch.float32 or not rot.is_contiguous():
+        rot = rot.to(torch.float32).contiguous()
+    if rot.dim() == 2 and n_kv > 1:
+        rot = rot.unsqueeze(0).expand(n_kv, -1, -1).contiguous()
+    return rot
 
 
 @torch.no_grad()
@@ -141,10 +149,7 @@ def fused_blockgtq_prefill_attention(
         v_norms = v_norms[..., 0]
     lt = _layer_for(segments, codebook_flat, v_lut, vb_codebook, n_kv, q.device)
     flags = (_lib.DEC_K_MIXED if k_nibble else 0) | (_lib.DEC_V_NIBBLE if v_nibble else 0)
-    rot = None
-    if v_rotation is not None:
-        rot = v_rotation.to(torch.float32).contiguous()
-        rot = rot.unsqueeze(0).expand(n_kv, -1, -1).contiguous() if rot.dim() == 2 else rot
+    rot = _rotation(v_rotation, n_kv)
     q16 = q.to(torch.float16)
     if q16.stride(3) != 1:
         q16 = q16.contiguous()

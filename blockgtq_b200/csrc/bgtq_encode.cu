@@ -648,3 +648,23 @@ extern "C" __attribute__((visibility("default"))) int bgtq_step_prepare_ring(
                              vp_st, v_norms, vn_sb, vn_sh, vn_st, flags, pos_dev, t_capacity, status, stream, nullptr, nullptr, 0, k_buf, v_buf, kb_sb, kb_sh,
                              n_sink, window);
 }
+
+// Rotation only: the query items of the kernel above, without rows to append.  (One CTA per four query heads reads a
+// head's rotation once for four rows; a CTA per row that walked its own segments took 4.7 us for 32 rows, this 3.5.)
+int bgtq::launch_rotate_q(const BgtqHeadDesc* desc, const float* rot_k, const void* q, int64_t q_sb, int64_t q_sh, void* q_rot,
+                          int32_t n_batch, int32_t n_q, int32_t n_kv, bool programmatic, cudaStream_t stream) {
+    if (!desc || !rot_k || !q || !q_rot || n_batch < 1 || n_kv < 1 || n_q < n_kv || n_q % n_kv) return BGTQ_E_BADARG;
+    PrepParams P = {};
+    P.e.desc = desc; P.e.rot_k = rot_k; P.e.n_batch = n_batch; P.e.n_kv = n_kv; P.e.n_tok = 1;
+    P.q = static_cast<const __half*>(q); P.q_sb = q_sb; P.q_sh = q_sh; P.q_rot = static_cast<__half*>(q_rot);
+    P.n_q = n_q; P.do_rot = 1; P.rot_group = (n_q / n_kv) % 4 == 0 ? 4 : 1;
+    const int64_t items = (int64_t)n_batch * n_q / P.rot_group;
+    if (items > 0x7fffffffLL) return BGTQ_E_TOOBIG;
+    return launch_kernel(prep_kernel, dim3((unsigned)items), dim3(512), 0, stream, programmatic, P) == cudaSuccess ? BGTQ_OK
+                                                                                                              : BGTQ_E_LAUNCH;
+}
+
+extern "C" __attribute__((visibility("default"))) int bgtq_rotate_q(const BgtqHeadDesc* desc, const float* rot_k, const void* q, int64_t q_sb, int64_t q_sh,
+                             void* q_rot, int32_t n_batch, int32_t n_q, int32_t n_kv, void* stream) {
+    return launch_rotate_q(desc, rot_k, q, q_sb, q_sh, q_rot, n_batch, n_q, n_kv, false, static_cast<cudaStream_t>(stream));
+}

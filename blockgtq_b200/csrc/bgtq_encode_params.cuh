@@ -56,4 +56,8 @@ int launch_encode_tc(const EncParams& P, cudaStream_t stream);
 int launch_encode_t5w(const EncParams& P, cudaStream_t stream);
 int encode_t5w_max_row_bytes();
 
+// Query rotation alone (the query items of the step-preparation kernel), optionally as a programmatic dependent.
+int launch_rotate_q(const BgtqHeadDesc* desc, const float* rot_k, const void* q, int64_t q_sb, int64_t q_sh, void* q_rot,
+                    int32_t n_batch, int32_t n_q, int32_t n_kv, bool programmatic, cudaStream_t stream);
+
 }  // namespace bgtq

@@ -1,31 +1,8 @@
-// Small kernels around the fused decode: query rotation, split-KV combine
-// (kernel c) and attention over the fp16 sink / recent-window tokens (kernel d).
+// Small kernels around the fused decode: split-KV combine (kernel c) and attention over the fp16 sink / recent-window tokens (kernel d).
 #include "bgtq_common.cuh"
 
 namespace bgtq {
 namespace {
-
-// ---------------------------------------------------------------------------
-// q_rot[p] = fp16( sum_j q[head_perm[j]] * rot_k[j][p] ), fp32 accumulate.
-// The rotation is block diagonal, so only the inputs of p's own segment count.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) rotate_q_kernel(const BgtqHeadDesc* desc, const float* rot_k,
-                                                        const __half* q, int64_t q_sb, int64_t q_sh,
-                                                        __half* q_rot, int n_q, int n_kv) {
-    __shared__ float qs[kHD];
-    const int p = threadIdx.x, hq = blockIdx.x, b = blockIdx.y;
-    const int h = hq / (n_q / n_kv);
-    const BgtqHeadDesc& d = desc[h];
-    qs[p] = __half2float(q[b * q_sb + hq * q_sh + d.head_perm[p]]);
-    __syncthreads();
-    const int g = d.group_of[p];
-    const int js = d.seg_start[g], je = js + d.seg_len[g];
-    const float* W = rot_k + (size_t)h * kHD * kHD + p;
-    float acc = 0.f;
-#pragma unroll 8
-    for (int j = js; j < je; ++j) acc = fmaf(qs[j], __ldg(W + (size_t)j * kHD), acc);
-    q_rot[((size_t)b * n_q + hq) * kHD + p] = __float2half_rn(acc);
-}
 
 // Optional last step of the combine on a sequence-sharded cache: the row's fp32 result and LSE go straight
 // into this rank's slot of EVERY rank's exchange buffer (plain peer stores over NVLink), and the last CTA of
@@ -620,15 +597,6 @@ extern "C" __attribute__((visibility("default"))) int bgtq_desc_size(void) { ret
 extern "C" __attribute__((visibility("default"))) const char* bgtq_error_string(int code) {
     const int i = -code;
     return (i >= 0 && i < (int)(sizeof(kErrNames) / sizeof(kErrNames[0]))) ? kErrNames[i] : "unknown error";
-}
-
-extern "C" __attribute__((visibility("default"))) int bgtq_rotate_q(const BgtqHeadDesc* desc, const float* rot_k, const void* q, int64_t q_sb, int64_t q_sh,
-                             void* q_rot, int32_t n_batch, int32_t n_q, int32_t n_kv, void* stream) {
-    if (!desc || !rot_k || !q || !q_rot || n_batch < 1 || n_kv < 1 || n_q < n_kv || n_q % n_kv) return BGTQ_E_BADARG;
-    if (n_batch > 65535) return BGTQ_E_TOOBIG;
-    rotate_q_kernel<<<dim3(n_q, n_batch), 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        desc, rot_k, static_cast<const __half*>(q), q_sb, q_sh, static_cast<__half*>(q_rot), n_q, n_kv);
-    return cudaGetLastError() == cudaSuccess ? BGTQ_OK : BGTQ_E_LAUNCH;
 }
 
 extern "C" __attribute__((visibility("default"))) int bgtq_combine(const float* part_o, const float* part_lse, int32_t n_splits, const float* v_rot,

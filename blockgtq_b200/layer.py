@@ -167,10 +167,10 @@ class LayerTables:
 
 def _strides3(t: torch.Tensor):
     """(batch, head, token) element strides of a (B, H, T, X) tensor with unit last stride."""
-    if t.dim() != 4 or t.stride(3) != 1:
-        raise ValueError(f"expected a (B, H, T, X) tensor with contiguous last dim, got {tuple(t.shape)} "
-                         f"strides {t.stride()}")
-    return t.stride(0), t.stride(1), t.stride(2)
+    st = t.stride()
+    if len(st) != 4 or st[3] != 1:
+        raise ValueError(f"expected a (B, H, T, X) tensor with contiguous last dim, got {tuple(t.shape)} strides {st}")
+    return st[:3]
 
 
 def encode(layer: LayerTables, k, v, t0, k_packed, k_norms, v_packed, v_norms, *, flags=0,
@@ -370,6 +370,37 @@ def decode(layer: LayerTables, q_rot, k_packed, k_norms, v_packed, v_norms, t_be
         _lib.stream_ptr(q_rot.device)), "bgtq_decode")
     _lib.count_launch()
     return part_o, part_lse
+
+
+def attend(layer, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, *, rotate, n_splits=None, scale=None, flags=0,
+           v_rot=None, buf_o=None, buf_lse=None, want_f32=False, want_lse=False, status=None):
+    """Query rotation (``rotate``: q is in the original basis), split-KV decode over rows [t_begin, t_end) and combine
+    in one library call.  q (B, n_q, 128) fp16 -> (out fp16 (B, n_q, 128), f32 copy | None, LSE | None)."""
+    _lib.require_cuda(q, "q")
+    B, n_q, _ = q.shape
+    if k_norms.dtype != torch.float16 or v_norms.dtype != torch.float16:
+        raise TypeError("cache norms must be float16")
+    q_sb, q_sh, q_sd = q.stride()
+    if q.dtype != torch.float16 or q_sd != 1 or not (rotate or q.is_contiguous()):
+        q = q.to(torch.float16).contiguous()
+        q_sb, q_sh = n_q * HD, HD
+    if n_splits is None:
+        n_splits = default_splits(B, layer.n_kv, t_end - t_begin)
+    dev = q.device
+    scratch = torch.empty(B * n_q * (n_splits * (HD + 1) + HD // 2), dtype=torch.float32, device=dev)
+    out = torch.empty(B, n_q, HD, dtype=torch.float16, device=dev)
+    o32 = torch.empty(B, n_q, HD, dtype=torch.float32, device=dev) if want_f32 else None
+    lse = torch.empty(B, n_q, dtype=torch.float32, device=dev) if want_lse else None
+    _lib.check(_lib.lib().bgtq_attend(
+        C.addressof(layer.plan(flags | _lib.DEC_PROGRAMMATIC)), _lib.ptr(layer.desc_dev), _lib.ptr(layer.rot_k) if rotate else None,
+        q.data_ptr(), q_sb, q_sh,
+        k_packed.data_ptr(), *_strides3(k_packed), k_norms.data_ptr(), *_strides3(k_norms),
+        v_packed.data_ptr(), *_strides3(v_packed), v_norms.data_ptr(), *v_norms.stride(),
+        B, n_q, layer.n_kv, t_begin, t_end, n_splits, 1.0 / math.sqrt(HD) if scale is None else scale,
+        _lib.ptr(v_rot), _lib.ptr(buf_o), _lib.ptr(buf_lse), scratch.data_ptr(), out.data_ptr(), _lib.ptr(o32), _lib.ptr(lse),
+        _lib.ptr(status), _lib.stream_ptr(dev)), "bgtq_attend")
+    _lib.count_launch(3 if rotate else 2)
+    return out, o32, lse
 
 
 def prefill_attention(layer: LayerTables, q_rot, k_packed, k_norms, v_packed, v_norms, n_tokens, *,

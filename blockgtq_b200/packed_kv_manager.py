@@ -15,17 +15,16 @@ Extensions beyond the reference class (all off by default):
 """
 from __future__ import annotations
 
-import os
-
+import ctypes as C
 import math
+import os
 
 import torch
 
 from . import _lib
 from .calib import packed_v_bytes
-from .layer import (HD, LayerTables, buffer_attn, combine, combine_ranks, decode, decode_grid_size, decode_partition,
-                    default_splits, encode, rotate_q,
-                    step_prepare)
+from .layer import (HD, LayerTables, attend, buffer_attn, combine, decode, decode_grid_size, decode_partition, default_splits,
+                    encode, rotate_q, step_prepare)
 from .quantizer import BlockGTQQuantizer, build_batched_encode_args
 
 __all__ = ["BlockGTQKVManager", "decode_step"]
@@ -57,7 +56,7 @@ class BlockGTQKVManager:
         self._max_k_packed_bytes = 0
         self._max_n_groups = 0
         self._k_packed = self._k_norms = self._v_packed = self._v_norms = None
-        self._part_dev = self._part_key = None
+        self._part_dev = self._part_key = self._part_len = None
         # three-region policy
         self.n_sink, self.recent_window, self.block_size = int(n_sink), int(recent_window), int(block_size)
         self._buffered = self.n_sink > 0 or self.recent_window > 0
@@ -72,14 +71,15 @@ class BlockGTQKVManager:
         self._exchange = None                 # sequence sharding: see sharding.SequenceShard
         self._enc_flags = (_lib.ENC_K_MIXED if k_mixed else 0) | (_lib.ENC_V_NIBBLE if v_nibble else 0)
         self._dec_flags = (_lib.DEC_K_MIXED if k_mixed else 0) | (_lib.DEC_V_NIBBLE if v_nibble else 0)
-        # single-token decode steps are captured once per layer and replayed (the reference graphs only
-        # its T=1 encode, packed_kv_manager.py:182-257); needs the plain (unbuffered) cache
-        # (with fp16 regions the captured step needs one-token blocks, the policy's default)
+        # single-token decode steps take the position from the device and keep their arrays, so that they can be
+        # captured (the reference graphs only its T=1 encode, packed_kv_manager.py:182-257); with fp16 regions that
+        # needs one-token blocks, the policy's default
         graphable = (not self._buffered) or (self.block_size == 1 and self.recent_window >= 1)
         self._use_graph = graphable if use_cuda_graph is None else bool(use_cuda_graph)
         if self._use_graph and not graphable:
             raise ValueError("CUDA-graph replay with fp16 sink/recent buffers needs block_size == 1 and a window")
-        self._graphs = [dict() for _ in range(n_layers)]      # per layer: {rope fused or not: CUDA graph}
+        self._graphs = [dict() for _ in range(n_layers)]      # sequence sharding, per layer: {rope fused or not: CUDA graph}
+        self._steps = [None] * n_layers                       # per layer: the constant arguments of bgtq_layer_step
         self._g_qkv = self._g_out = self._pos = None
 
     @property
@@ -141,8 +141,7 @@ class BlockGTQKVManager:
         self._n_splits = default_splits(self.B, self.n_kv, self.max_T) if dev.type == "cuda" else 1
         # item ranges of the step's decode launches (one table for every layer: same shape, same length),
         # refreshed when the cache length changes the way the kernel cuts it into items
-        self._part_key = None
-        self._part_dev = None
+        self._part_key = self._part_len = self._part_dev = None
         if dev.type == "cuda":
             self._part_cta = decode_grid_size(self.B, self.n_kv, self._n_splits)
             self._part_host = torch.empty(self._part_cta + 5, dtype=torch.int32)
@@ -164,6 +163,7 @@ class BlockGTQKVManager:
         self._g_qkv = torch.zeros(self.n_layers, self.B, self.n_q + 2 * self.n_kv, 1, self.hd, dtype=torch.float16,
                                   device=dev)
         self._g_out = torch.zeros(self.n_layers, self.B, self.n_q, self.hd, dtype=torch.float16, device=dev)
+        self._g_out4 = list(self._g_out.unsqueeze(3).unbind(0))      # per layer (B, n_q, 1, hd)
         self._pos = torch.zeros(1, dtype=torch.int32, device=dev)
         self._g_rope = torch.zeros(2, self.B, self.hd, dtype=torch.float16, device=dev)     # cos, sin of the step
         self._buf_o = torch.zeros(self.B, self.n_q, self.hd, dtype=torch.float32, device=dev)
@@ -320,8 +320,9 @@ class BlockGTQKVManager:
         length only through the number of items per (batch, head) pair and their size, which change every few
         hundred tokens; a table made for another length is ignored by the kernel, so this is about balance
         only."""
-        if self._part_dev is None or torch.cuda.is_current_stream_capturing():
+        if self._part_len == self._seq_len or self._part_dev is None or torch.cuda.is_current_stream_capturing():
             return      # (inside a caller's capture the table is refreshed by increment_seq_len, outside it)
+        self._part_len = self._seq_len
         n_tok = max(0, min(self.max_T, self._seq_len + self._step_decode_pos_add()))
         units = (n_tok + 31) // 32
         c_units = max(1, -(-units // self._n_splits))
@@ -332,54 +333,82 @@ class BlockGTQKVManager:
         decode_partition(self.B, self.n_kv, n_tok, self._n_splits, self._part_cta, out=self._part_host)
         self._part_dev.copy_(self._part_host)      # stream ordered: lands before the next step's launches
 
-    def _layer_step(self, li: int, rope: bool = False):
-        """rotate_q -> append K,V at *pos -> decode over [0, *pos + 1) -> combine, all on static buffers."""
-        lt = self._layers[li]
-        gq, gk, gv = self.static_inputs(li)
+    def _step_args(self, li: int) -> "_lib.LayerStep":
+        """The constant arguments of layer ``li``'s step (every array of it lives as long as the manager)."""
+        s = self._steps[li]
         baked = all(self.quantizers[li][h]._q_perm_baked for h in range(self.n_kv))
-        # the three kernels are chained as programmatic dependents: each sets up its static tables while
-        # the one before it drains, and waits on the device before touching the step's data
-        pd = self.programmatic
+        if s is not None and s.key == (baked, self.programmatic):
+            return s
+        lt, pd = self._layers[li], self.programmatic
+        kp, kn, vp, vn = self._k_packed[li], self._k_norms[li], self._v_packed[li], self._v_norms[li]
+        plan = lt.plan(self._dec_flags | (_lib.DEC_PROGRAMMATIC if pd else 0))
+        s = _lib.LayerStep(
+            plan=C.addressof(plan), desc=lt.desc_dev.data_ptr(), rot_k=lt.rot_k.data_ptr(), rot_v=lt.rot_v.data_ptr(),
+            v_rot=lt.v_rot.data_ptr(), q_rot=self._q_rot.data_ptr(), part_o=self._part_o.data_ptr(),
+            part_lse=self._part_lse.data_ptr(), out=self._g_out[li].data_ptr(), o_sb=self._g_out.stride(1),
+            o_sh=self._g_out.stride(2), pos_dev=self._pos.data_ptr(), status=self._status.data_ptr(), n_batch=self.B, n_q=self.n_q,
+            n_kv=self.n_kv, t_capacity=self.max_T, kp_row_bytes=kp.shape[3], kn_count=kn.shape[3], n_splits=self._n_splits,
+            pos_add=self._step_decode_pos_add(),
+            enc_flags=self._enc_flags | _lib.ENC_K_NORMS_F16 | (_lib.ENC_PROGRAMMATIC if pd else 0),
+            combine_flags=_lib.COMBINE_PROGRAMMATIC if pd else 0, flags=_lib.STEP_Q_ROTATED if baked else 0, scale=self.scale)
+        for name, t in (("k_packed", kp), ("k_norms", kn), ("v_packed", vp), ("v_norms", vn)):
+            setattr(s, name, t.data_ptr())
+            for suffix, stride in zip(("sb", "sh", "st"), t.stride()):
+                setattr(s, f"{name[0]}{name[2]}_{suffix}", stride)
+        if self._buffered:
+            kb, vb = self._k_buf[li], self._v_buf[li]
+            s.k_buf, s.v_buf, s.kb_sb, s.kb_sh = kb.data_ptr(), vb.data_ptr(), kb.stride(0), kb.stride(1)
+            s.buf_o, s.buf_lse, s.n_sink, s.window = self._buf_o.data_ptr(), self._buf_lse.data_ptr(), self.n_sink, self.recent_window
+        s.key, s.addr, s.n_launch = (baked, pd), C.addressof(s), 4 if self._buffered else 3
+        self._steps[li] = s
+        return s
+
+    def _launch_step(self, li: int, q, k, v, rope=None):
+        """rotate_q + append K,V at *pos -> decode over [0, *pos + 1) -> (fp16 regions) -> combine into
+        ``static_outputs()[li]``, one library call; q/k/v (B, heads, 1, hd) fp16 with unit last stride."""
+        s = self._step_args(li)
+        qs, ks, vs = q.stride(), k.stride(), v.stride()
+        cos = sin = None
+        r_sb = 0
+        if rope is not None:
+            cos, sin = rope
+            r_sb = cos.stride(0)
+        _lib.check(_lib.lib().bgtq_layer_step(
+            s.addr, q.data_ptr(), qs[0], qs[1], k.data_ptr(), ks[0], ks[1], v.data_ptr(), vs[0], vs[1],
+            None if cos is None else cos.data_ptr(), None if sin is None else sin.data_ptr(), r_sb,
+            _lib.stream_ptr(self._pos.device)), "bgtq_layer_step")
+        _lib.count_launch(s.n_launch)
+
+    def _layer_step(self, li: int, rope: bool = False):
+        """One layer's step on the static buffers."""
+        gq, gk, gv = self.static_inputs(li)
         ex = self._exchange
-        q_rot = self._q_rot
+        if ex is None:
+            self._launch_step(li, gq, gk, gv, (self._g_rope[0], self._g_rope[1]) if rope else None)
+            return
+        # sequence sharding.  The kernels are chained as programmatic dependents: each sets up its static tables while
+        # the one before it drains, and waits on the device before touching the step's data
+        lt, pd = self._layers[li], self.programmatic
+        baked = all(self.quantizers[li][h]._q_perm_baked for h in range(self.n_kv))
         if baked:                   # queries arrive in the packed-K basis already: stage them without allocating
             self._q_rot.copy_(gq[:, :, 0])
-        if self._buffered:          # three regions, everything derived from the device-side token count
-            ns, win = self.n_sink, self.recent_window
-            step_prepare(lt, None if baked else gq, gk, gv, 0, self._k_packed[li], self._k_norms[li],
-                         self._v_packed[li], self._v_norms[li], q_rot=self._q_rot, pos_dev=self._pos,
-                         flags=self._enc_flags | (_lib.ENC_PROGRAMMATIC if pd else 0), status=self._status,
-                         ring=(self._k_buf[li], self._v_buf[li], ns, win))
-            decode(lt, q_rot, self._k_packed[li], self._k_norms[li], self._v_packed[li], self._v_norms[li],
-                   0, self.max_T, n_splits=self._n_splits, scale=self.scale, status=self._status,
-                   part_o=self._part_o, part_lse=self._part_lse, pos_dev=self._pos, pos_add=-(ns + win),
-                   flags=self._dec_flags | (_lib.DEC_PROGRAMMATIC if pd else 0))
-            buffer_attn(gq, self._k_buf[li], self._v_buf[li], self.n_kv, self.scale, sink_cap=ns, ring_size=win + 1,
-                        pos_dev=self._pos, out=(self._buf_o, self._buf_lse))
-            combine(self._part_o, self._part_lse, self.n_kv, v_rot=lt.v_rot, buf_o=self._buf_o, buf_lse=self._buf_lse,
-                    out=self._g_out[li], programmatic=pd)
-            return
-        if ex is None or ex.is_owner:
+        if ex.is_owner:
             step_prepare(lt, None if baked else gq, gk, gv, 0, self._k_packed[li], self._k_norms[li],
                          self._v_packed[li], self._v_norms[li], q_rot=self._q_rot, pos_dev=self._pos,
                          flags=self._enc_flags | (_lib.ENC_PROGRAMMATIC if pd else 0), status=self._status,
                          rope=(self._g_rope[0], self._g_rope[1]) if rope else None)
         elif not baked:                           # this rank does not hold the tail: nothing to append
             rotate_q(lt, gq[:, :, 0], out=self._q_rot)
-        decode(lt, q_rot, self._k_packed[li], self._k_norms[li], self._v_packed[li], self._v_norms[li],
+        decode(lt, self._q_rot, self._k_packed[li], self._k_norms[li], self._v_packed[li], self._v_norms[li],
                0, self.max_T, n_splits=self._n_splits, scale=self.scale, status=self._status,
-               part_o=self._part_o, part_lse=self._part_lse, pos_dev=self._pos,
-               pos_add=1 if (ex is None or ex.is_owner) else 0,
+               part_o=self._part_o, part_lse=self._part_lse, pos_dev=self._pos, pos_add=self._step_decode_pos_add(),
                flags=self._dec_flags | (_lib.DEC_PROGRAMMATIC if pd else 0))
-        if ex is None:
-            combine(self._part_o, self._part_lse, self.n_kv, v_rot=lt.v_rot, out=self._g_out[li], programmatic=pd)
-        elif ex.transport == "p2p":     # combine + peer stores in one launch, then the bounded wait + merge
+        if ex.transport == "p2p":       # combine + peer stores in one launch, then the bounded wait + merge
             ex.combine_publish(self._part_o, self._part_lse, self.n_kv, lt.v_rot, programmatic=pd)
-            ex.exchange_and_merge(self._g_out[li])
         else:       # local result straight into the message, one all-gather, merge of the messages
             combine(self._part_o, self._part_lse, self.n_kv, v_rot=lt.v_rot, out=self._g_out[li], programmatic=pd,
                     o32_out=ex.msg_o, lse_out=ex.msg_lse)
-            ex.exchange_and_merge(self._g_out[li])
+        ex.exchange_and_merge(self._g_out[li])
 
     def layer_step(self, layer_idx: int, rope: bool = False):
         """Launch one layer's decode step (append the token in ``static_inputs(layer_idx)`` at the current
@@ -397,11 +426,35 @@ class BlockGTQKVManager:
         self._sync_pos()
         self._layer_step(layer_idx, rope)
 
-    def _replay_layer(self, li: int, q, k_new, v_new, rope=None) -> torch.Tensor:
+    def _call_layer(self, li: int, q, k_new, v_new, rope=None) -> torch.Tensor:
+        """One layer's step on the caller's tensors: (B, n_q, 1, hd) fp16.  The kernels read them in place; inputs of
+        another type or with a strided last dim go through the static buffers."""
         self._ensure_storage()
         if self._seq_len + 1 > self.max_T:
             raise ValueError("cache overflow")
         self._sync_pos()
+        if self._exchange is not None:
+            return self._replay_layer(li, q, k_new, v_new, rope)
+        f16, B, hd = torch.float16, self.B, self.hd
+        if (q.dtype != f16 or k_new.dtype != f16 or v_new.dtype != f16 or q.shape != (B, self.n_q, 1, hd)
+                or k_new.shape != (B, self.n_kv, 1, hd) or v_new.shape != k_new.shape or q.stride(3) != 1 or k_new.stride(3) != 1
+                or v_new.stride(3) != 1 or k_new.device != self._pos.device or v_new.device != self._pos.device):
+            q, k_new, v_new = self._stage(li, q, k_new, v_new)
+        if rope is not None:
+            cos, sin = rope
+            if (cos.dtype == f16 and sin.dtype == f16 and cos.numel() == B * hd and cos.stride(-1) == 1 and sin.stride(-1) == 1
+                    and cos.shape[0] == B and sin.shape == cos.shape and sin.stride(0) == cos.stride(0)):
+                rope = (cos, sin)
+            else:
+                rope = self._stage_rope(cos, sin)
+        elif self._step_args(li).flags & _lib.STEP_Q_ROTATED and not q.is_contiguous():
+            q, k_new, v_new = self._stage(li, q.contiguous(), k_new, v_new)
+        self._launch_step(li, q, k_new, v_new, rope)
+        return self._g_out4[li]
+
+    @torch.no_grad()
+    def _stage(self, li: int, q, k_new, v_new):
+        """Copy a step's inputs into the static buffers; returns those."""
         gq, gk, gv = self.static_inputs(li)
         if q.data_ptr() != gq.data_ptr():
             gq.copy_(q.reshape(gq.shape))
@@ -409,10 +462,20 @@ class BlockGTQKVManager:
             gk.copy_(k_new)
         if v_new.data_ptr() != gv.data_ptr():
             gv.copy_(v_new)
+        return gq, gk, gv
+
+    @torch.no_grad()
+    def _stage_rope(self, cos, sin):
+        self._g_rope[0].copy_(cos.reshape(self.B, self.hd))
+        self._g_rope[1].copy_(sin.reshape(self.B, self.hd))
+        return self._g_rope[0], self._g_rope[1]
+
+    def _replay_layer(self, li: int, q, k_new, v_new, rope=None) -> torch.Tensor:
+        """Sequence sharding: the layer's launches and its collective are captured once and replayed."""
+        self._stage(li, q, k_new, v_new)
         use_rope = rope is not None
         if use_rope:
-            self._g_rope[0].copy_(rope[0].reshape(self.B, self.hd))
-            self._g_rope[1].copy_(rope[1].reshape(self.B, self.hd))
+            self._stage_rope(*rope)
         g = self._graphs[li].get(use_rope)
         if g is None:
             self._layer_step(li, use_rope)            # eager once: sets kernel attributes, validates shapes
@@ -423,23 +486,25 @@ class BlockGTQKVManager:
             self._graphs[li][use_rope] = g
         else:
             g.replay()
-            _lib.count_launch(4 if self._buffered else
-                              ((4 if self._exchange.transport == "p2p" else 5) if self._exchange else 3))
-        return self._g_out[li]
+            _lib.count_launch(4 if self._exchange.transport == "p2p" else 5)
+        return self._g_out4[li]
 
     # -- decode ----------------------------------------------------------------------------
-    @torch.no_grad()
     def append_and_attend(self, layer_idx: int, q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor,
                           n_splits: int = None, rope=None) -> torch.Tensor:
         """Quantise and append (B, n_kv, S, hd) K/V, then attend the (B, n_q, 1, hd) query over the
         whole cache.  Returns (B, n_q, 1, hd) fp16 (packed_kv_manager.py:268-348).
         ``rope=(cos, sin)`` (fp16, (B, [1,] hd), single-token steps): q and k_new are pre-RoPE and the append
         kernel applies the rotary embedding itself (an extension; the reference's callers rotate first)."""
-        t, S = self.seq_len, k_new.shape[2]
-        if self._use_graph and S == 1 and n_splits is None and q.is_cuda:
-            return self._replay_layer(layer_idx, q, k_new, v_new, rope).unsqueeze(2)
+        if self._use_graph and k_new.shape[2] == 1 and n_splits is None and q.is_cuda:
+            return self._call_layer(layer_idx, q, k_new, v_new, rope)
         if rope is not None:
-            raise NotImplementedError("fused RoPE is available on the single-token graph path only")
+            raise NotImplementedError("fused RoPE is available on the single-token step path only")
+        return self._append_and_attend(layer_idx, q, k_new, v_new, n_splits)
+
+    @torch.no_grad()
+    def _append_and_attend(self, layer_idx: int, q, k_new, v_new, n_splits):
+        t, S = self.seq_len, k_new.shape[2]
         defer = self._buffered and S == 1
         f0, f1 = self._append_tokens(layer_idx, k_new, v_new, t, defer_flush=defer)
         out, _, _ = self.attend(layer_idx, q, t + S, n_splits=n_splits, flushed=f0 if defer else None)
@@ -466,15 +531,12 @@ class BlockGTQKVManager:
         lo = max(0, min(lo, n_packed))
         hi = max(lo, min(hi, n_packed))
         baked = all(self.quantizers[li][h]._q_perm_baked for h in range(self.n_kv))
-        q_rot = q.contiguous() if baked else rotate_q(lt, q)
-        part_o, part_lse = decode(lt, q_rot, self._k_packed[li], self._k_norms[li], self._v_packed[li],
-                                  self._v_norms[li], lo, hi, n_splits=n_splits, scale=self.scale,
-                                  status=self._status, flags=self._dec_flags)
         buf_o = buf_lse = None
         if self._buffered and with_buffers:
             buf_o, buf_lse = self._buffer_partial(li, q, n_sink_tok, n_packed, n_recent)
-        return combine(part_o, part_lse, self.n_kv, v_rot=lt.v_rot, buf_o=buf_o, buf_lse=buf_lse,
-                       want_f32=want_partial, want_lse=want_partial)
+        return attend(lt, q, self._k_packed[li], self._k_norms[li], self._v_packed[li], self._v_norms[li], lo, hi, rotate=not baked,
+                      n_splits=n_splits, scale=self.scale, flags=self._dec_flags, v_rot=lt.v_rot, buf_o=buf_o, buf_lse=buf_lse,
+                      want_f32=want_partial, want_lse=want_partial, status=self._status)
 
     def _buffer_partial(self, li, q, n_sink_tok, n_packed, n_recent):
         """(O, LSE) of the fp16 region: sink slots [0, n_sink_tok) + ring slots of the recent tokens."""

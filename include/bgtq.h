@@ -388,6 +388,58 @@ int bgtq_combine(const float* part_o, const float* part_lse, int32_t n_splits,
                  void* out, int64_t o_sb, int64_t o_sh,
                  float* out_f32, float* lse_out, int32_t flags, void* stream);
 
+/* ---- whole steps ------------------------------------------------------------
+ * The launches of one layer's decode step in one call: bgtq_step_prepare (its ring form when k_buf is set, its
+ * rotary form when rope tables are passed) -> bgtq_decode over rows [0, *pos_dev + pos_add) -> with k_buf
+ * bgtq_buffer_attn_pos -> bgtq_combine.  Replaces the body of append_and_attend
+ * (blockgtq/packed_kv_manager.py:268-348) for a step whose arrays stay where they are: everything constant over
+ * the steps is filled in once (host memory, plain values; the plan and every pointer must outlive its use), and
+ * a call passes only the step's rows.  Arguments as for those functions.  No allocation, no synchronisation. */
+#define BGTQ_STEP_Q_ROTATED 1     /* queries arrive in the packed-K basis, rows contiguous over the heads: no rotation */
+typedef struct BgtqLayerStep {
+    const BgtqDecodePlan* plan;
+    const BgtqHeadDesc* desc;
+    const float* rot_k;
+    const float* rot_v;
+    const float* v_rot;
+    uint8_t* k_packed; int64_t kp_sb, kp_sh, kp_st;
+    void* k_norms;     int64_t kn_sb, kn_sh, kn_st;       /* fp16 */
+    uint8_t* v_packed; int64_t vp_sb, vp_sh, vp_st;
+    void* v_norms;     int64_t vn_sb, vn_sh, vn_st;
+    void* q_rot;                                          /* (n_batch, n_q, 128) fp16 */
+    float* part_o;
+    float* part_lse;
+    void* out;         int64_t o_sb, o_sh;                /* fp16 */
+    void* k_buf;                                          /* fp16 sink + ring, or NULL */
+    void* v_buf;       int64_t kb_sb, kb_sh;
+    float* buf_o;
+    float* buf_lse;
+    const int32_t* pos_dev;
+    int32_t* status;
+    int32_t n_batch, n_q, n_kv, t_capacity, kp_row_bytes, kn_count, n_splits, pos_add;
+    int32_t enc_flags, combine_flags, flags, n_sink, window;
+    float scale;
+} BgtqLayerStep;
+int bgtq_layer_step_size(void);
+int bgtq_layer_step(const BgtqLayerStep* step, const void* q, int64_t q_sb, int64_t q_sh,
+                    const void* k, int64_t k_sb, int64_t k_sh, const void* v, int64_t v_sb, int64_t v_sh,
+                    const void* rope_cos, const void* rope_sin, int64_t rope_sb, void* stream);
+
+/* Attention of one query token per (batch, head) over cached rows [t_begin, t_end) in one call: query rotation
+ * (rot_k may be NULL: q is in the packed-K basis and contiguous) -> bgtq_decode -> bgtq_combine into the
+ * contiguous out (n_batch, n_q, 128) fp16 and the optional out_f32 / lse_out.  scratch: device memory of
+ * bgtq_attend_scratch_bytes(n_batch, n_q, n_splits) bytes, 16-byte aligned. */
+int64_t bgtq_attend_scratch_bytes(int32_t n_batch, int32_t n_q, int32_t n_splits);
+int bgtq_attend(const BgtqDecodePlan* plan, const BgtqHeadDesc* desc, const float* rot_k,
+                const void* q, int64_t q_sb, int64_t q_sh,
+                const uint8_t* k_packed, int64_t kp_sb, int64_t kp_sh, int64_t kp_st,
+                const void* k_norms, int64_t kn_sb, int64_t kn_sh, int64_t kn_st,
+                const uint8_t* v_packed, int64_t vp_sb, int64_t vp_sh, int64_t vp_st,
+                const void* v_norms, int64_t vn_sb, int64_t vn_sh, int64_t vn_st,
+                int32_t n_batch, int32_t n_q, int32_t n_kv, int32_t t_begin, int32_t t_end,
+                int32_t n_splits, float scale, const float* v_rot, const float* buf_o, const float* buf_lse,
+                void* scratch, void* out, float* out_f32, float* lse_out, int32_t* status, void* stream);
+
 /* Prefill attention: s_q query positions per (batch, query head) against the packed cache, causal.
  *
  * Replaces _packed_prefill_kernel / fused_blockgtq_prefill_attention
