@@ -94,6 +94,7 @@ _SIGNATURES = {
                                     _vp, _i64, _i64, _vp, _i64, _i64, _i32, _i32, _i32,
                                     _vp, _i64, _i64, _i64, _i32, _vp, _i64, _i64, _i64, _i32,
                                     _vp, _i64, _i64, _i64, _vp, _i64, _i64, _i64, _i32, _vp, _i32, _vp, _vp]),
+    "bgtq_rotate_q_rows": (C.c_int, [_vp, _vp, _vp, _i64, _i64, _i64, _vp, _i32, _i32, _i32, _i32, _vp]),
     "bgtq_layer_step_size": (C.c_int, []),
     "bgtq_layer_step": (C.c_int, [_vp, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _vp, _i64, _vp]),
     "bgtq_attend_scratch_bytes": (C.c_int64, [_i32, _i32, _i32]),
@@ -133,6 +134,10 @@ _SIGNATURES = {
     "bgtq_prefill_attention": (C.c_int, [_vp, _vp, _i64, _i64, _i64, _vp, _i64, _i64, _i64, _vp, _i64, _i64, _i64,
                                          _vp, _i64, _i64, _i64, _vp, _i64, _i64, _i64, _i32, _i32, _i32, _i32, _i32,
                                          _i32, _i32, C.c_float, _i32, _vp, _vp]),
+    "bgtq_prefill_workspace_bytes": (C.c_int64, [_i32] * 8),
+    "bgtq_prefill": (C.c_int, [_vp, _vp, _i64, _i64, _i64, _vp, _i64, _i64, _i64, _vp, _i64, _i64, _i64,
+                               _vp, _i64, _i64, _i64, _vp, _i64, _i64, _i64, _i32, _i32, _i32, _i32, _i32,
+                               _i32, _i32, _f32, _i32, _vp, _vp, _i64, _vp, _vp]),
     "bgtq_combine_publish": (C.c_int, [_vp, _vp, _i32, _vp, _i32, _i32, _i32, _vp, _i64, _i64, _vp, _i32, _i32, _vp, _vp,
                                       _i32, _vp]),
     "bgtq_exchange_publish": (C.c_int, [_vp, _i64, _vp, _i64, _i64, _vp, _i32, _i32, _vp, _vp, _vp]),

@@ -15,8 +15,10 @@
 #include "bgtq_prefill_common.cuh"
 
 namespace bgtq {
-// the tcgen05 form (bgtq_prefill_t5.cu); returns false when the shape does not fit it
-bool launch_prefill_t5(const PfParams& P, int n_batch, cudaStream_t stream, cudaError_t* err);
+// the tcgen05 form (bgtq_prefill_t5.cu)
+int64_t prefill_t5_workspace(int n_batch, int n_q, int n_kv, int s_q, int n_tok, int q_pos_offset, bool causal, bool rot);
+cudaError_t launch_prefill_t5(const PfParams& P, int n_batch, const float* v_rot, uint8_t* ws, __half* out16, float* out32,
+                              cudaStream_t stream);
 namespace {
 
 constexpr int kPfRows = 256;      // query rows per CTA
@@ -307,13 +309,13 @@ __global__ void __launch_bounds__(kPfWarps * 32, 1) prefill_kernel(const PfParam
 
 using namespace bgtq;
 
-extern "C" __attribute__((visibility("default"))) int bgtq_prefill_attention(
-    const BgtqHeadDesc* desc, const void* q_rot, int64_t q_sb, int64_t q_sh, int64_t q_ss, const uint8_t* k_packed,
-    int64_t kp_sb, int64_t kp_sh, int64_t kp_st, const void* k_norms, int64_t kn_sb, int64_t kn_sh, int64_t kn_st,
-    const uint8_t* v_packed, int64_t vp_sb, int64_t vp_sh, int64_t vp_st, const void* v_norms, int64_t vn_sb,
-    int64_t vn_sh, int64_t vn_st, int32_t n_batch, int32_t n_q, int32_t n_kv, int32_t s_q, int32_t n_tokens,
-    int32_t q_pos_offset, int32_t causal, float scale, int32_t flags, float* out_rot, void* stream) {
-    if (!desc || !q_rot || !k_packed || !k_norms || !v_packed || !v_norms || !out_rot) return BGTQ_E_BADARG;
+// Argument checks and launch parameters shared by the entry points (everything but the outputs).
+static int pf_params(PfParams& P, const BgtqHeadDesc* desc, const void* q_rot, int64_t q_sb, int64_t q_sh, int64_t q_ss,
+                     const uint8_t* k_packed, int64_t kp_sb, int64_t kp_sh, int64_t kp_st, const void* k_norms, int64_t kn_sb,
+                     int64_t kn_sh, int64_t kn_st, const uint8_t* v_packed, int64_t vp_sb, int64_t vp_sh, int64_t vp_st,
+                     const void* v_norms, int64_t vn_sb, int64_t vn_sh, int64_t vn_st, int32_t n_batch, int32_t n_q, int32_t n_kv,
+                     int32_t s_q, int32_t n_tokens, int32_t q_pos_offset, int32_t causal, float scale, int32_t flags) {
+    if (!desc || !q_rot || !k_packed || !k_norms || !v_packed || !v_norms) return BGTQ_E_BADARG;
     if (n_batch < 1 || n_kv < 1 || n_q < n_kv || n_q % n_kv || s_q < 1 || n_tokens < 0 || q_pos_offset < 0)
         return BGTQ_E_BADARG;
     const int gqa = n_q / n_kv;
@@ -321,13 +323,11 @@ extern "C" __attribute__((visibility("default"))) int bgtq_prefill_attention(
     if (kp_st < 1 || kp_st > 160 || vp_st < 1 || vp_st > 128 || kn_st < 1 || kn_st > 16 || vn_st < 1 || vn_st > 8)
         return BGTQ_E_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(q_rot) & 3u) || (q_sb & 1) || (q_sh & 1) || (q_ss & 1) ||
-        (reinterpret_cast<uintptr_t>(out_rot) & 7u) || (reinterpret_cast<uintptr_t>(k_norms) & 1u) ||
-        (reinterpret_cast<uintptr_t>(v_norms) & 1u))
+        (reinterpret_cast<uintptr_t>(k_norms) & 1u) || (reinterpret_cast<uintptr_t>(v_norms) & 1u))
         return BGTQ_E_ALIGN;
-    const int bq = kPfRows / gqa;
-    const int64_t q_blocks = ((int64_t)s_q + bq - 1) / bq;
-    if (q_blocks > 0x7FFFFFFF || n_kv > 65535 || n_batch > 65535) return BGTQ_E_TOOBIG;
-    PfParams P;
+    if (((int64_t)s_q * gqa + kPfRows - 1) / kPfRows * 16 > 0x7FFFFFFF || (int64_t)s_q * gqa > 0x7FFFFFFF - kPfRows || n_kv > 65535 ||
+        n_batch > 65535)
+        return BGTQ_E_TOOBIG;
     P.desc = desc;
     P.q = static_cast<const __half*>(q_rot);
     P.q_sb = q_sb; P.q_sh = q_sh; P.q_ss = q_ss;
@@ -340,23 +340,80 @@ extern "C" __attribute__((visibility("default"))) int bgtq_prefill_attention(
     P.n_q = n_q; P.n_kv = n_kv; P.gqa = gqa; P.s_q = s_q; P.n_tok = n_tokens;
     P.q_pos_offset = q_pos_offset; P.causal = causal ? 1 : 0; P.flags = flags;
     P.scale_log2 = scale * 1.4426950408889634f;
-    P.out = out_rot;
-    P.status = nullptr;
-    if (!(flags & BGTQ_PF_NO_TCGEN05)) {     // the tensor-memory form, when the shape fits it
-        cudaError_t e = cudaSuccess;
-        if (launch_prefill_t5(P, n_batch, static_cast<cudaStream_t>(stream), &e)) {
-            if (e != cudaSuccess) {
-                cudaGetLastError();
-                return BGTQ_E_LAUNCH;
-            }
-            return BGTQ_OK;
-        }
+    P.out = nullptr;
+    return BGTQ_OK;
+}
+
+extern "C" __attribute__((visibility("default"))) int64_t bgtq_prefill_workspace_bytes(int32_t n_batch, int32_t n_q, int32_t n_kv,
+                                                                                      int32_t s_q, int32_t n_tokens,
+                                                                                      int32_t q_pos_offset, int32_t causal,
+                                                                                      int32_t with_rotation) {
+    if (n_batch < 1 || n_kv < 1 || n_q < n_kv || n_q % n_kv || s_q < 1 || n_tokens < 0 || q_pos_offset < 0) return 0;
+    return prefill_t5_workspace(n_batch, n_q, n_kv, s_q, n_tokens, q_pos_offset, causal != 0, with_rotation != 0);
+}
+
+extern "C" __attribute__((visibility("default"))) int bgtq_prefill(
+    const BgtqHeadDesc* desc, const void* q_rot, int64_t q_sb, int64_t q_sh, int64_t q_ss, const uint8_t* k_packed,
+    int64_t kp_sb, int64_t kp_sh, int64_t kp_st, const void* k_norms, int64_t kn_sb, int64_t kn_sh, int64_t kn_st,
+    const uint8_t* v_packed, int64_t vp_sb, int64_t vp_sh, int64_t vp_st, const void* v_norms, int64_t vn_sb,
+    int64_t vn_sh, int64_t vn_st, int32_t n_batch, int32_t n_q, int32_t n_kv, int32_t s_q, int32_t n_tokens,
+    int32_t q_pos_offset, int32_t causal, float scale, int32_t flags, const float* v_rot, void* workspace, int64_t workspace_bytes,
+    void* out, void* stream) {
+    PfParams P;
+    const int rc = pf_params(P, desc, q_rot, q_sb, q_sh, q_ss, k_packed, kp_sb, kp_sh, kp_st, k_norms, kn_sb, kn_sh, kn_st, v_packed,
+                             vp_sb, vp_sh, vp_st, v_norms, vn_sb, vn_sh, vn_st, n_batch, n_q, n_kv, s_q, n_tokens, q_pos_offset, causal,
+                             scale, flags);
+    if (rc != BGTQ_OK) return rc;
+    if (!out || !workspace ||
+        workspace_bytes < prefill_t5_workspace(n_batch, n_q, n_kv, s_q, n_tokens, q_pos_offset, causal != 0, v_rot != nullptr))
+        return BGTQ_E_BADARG;
+    if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(workspace)) & 15u) return BGTQ_E_ALIGN;
+    if (launch_prefill_t5(P, n_batch, v_rot, static_cast<uint8_t*>(workspace), static_cast<__half*>(out), nullptr,
+                          static_cast<cudaStream_t>(stream)) != cudaSuccess) {
+        cudaGetLastError();
+        return BGTQ_E_LAUNCH;
     }
+    return BGTQ_OK;
+}
+
+extern "C" __attribute__((visibility("default"))) int bgtq_prefill_attention(
+    const BgtqHeadDesc* desc, const void* q_rot, int64_t q_sb, int64_t q_sh, int64_t q_ss, const uint8_t* k_packed,
+    int64_t kp_sb, int64_t kp_sh, int64_t kp_st, const void* k_norms, int64_t kn_sb, int64_t kn_sh, int64_t kn_st,
+    const uint8_t* v_packed, int64_t vp_sb, int64_t vp_sh, int64_t vp_st, const void* v_norms, int64_t vn_sb,
+    int64_t vn_sh, int64_t vn_st, int32_t n_batch, int32_t n_q, int32_t n_kv, int32_t s_q, int32_t n_tokens,
+    int32_t q_pos_offset, int32_t causal, float scale, int32_t flags, float* out_rot, void* stream) {
+    PfParams P;
+    const int rc = pf_params(P, desc, q_rot, q_sb, q_sh, q_ss, k_packed, kp_sb, kp_sh, kp_st, k_norms, kn_sb, kn_sh, kn_st, v_packed,
+                             vp_sb, vp_sh, vp_st, v_norms, vn_sb, vn_sh, vn_st, n_batch, n_q, n_kv, s_q, n_tokens, q_pos_offset, causal,
+                             scale, flags);
+    if (rc != BGTQ_OK) return rc;
+    if (!out_rot) return BGTQ_E_BADARG;
+    if (reinterpret_cast<uintptr_t>(out_rot) & 7u) return BGTQ_E_ALIGN;
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (!(flags & BGTQ_PF_NO_TCGEN05) && !(reinterpret_cast<uintptr_t>(out_rot) & 15u)) {
+        // the caller of this form has no workspace to give: take it from the stream's pool for the launch
+        void* ws = nullptr;
+        const int64_t n = prefill_t5_workspace(n_batch, n_q, n_kv, s_q, n_tokens, q_pos_offset, causal != 0, false);
+        cudaError_t e = cudaMallocAsync(&ws, (size_t)(n > 16 ? n : 16), st);
+        if (e == cudaSuccess) {
+            e = launch_prefill_t5(P, n_batch, nullptr, static_cast<uint8_t*>(ws), nullptr, out_rot, st);
+            const cudaError_t f = cudaFreeAsync(ws, st);
+            if (e == cudaSuccess) e = f;
+        }
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return BGTQ_E_LAUNCH;
+        }
+        return BGTQ_OK;
+    }
+    P.out = out_rot;
+    const int bq = kPfRows / P.gqa;
+    const int64_t q_blocks = ((int64_t)s_q + bq - 1) / bq;
     const int smem = (int)sizeof(PfSmem);
     if (cudaFuncSetAttribute(prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
         cudaGetLastError();
         return BGTQ_E_LAUNCH;
     }
-    prefill_kernel<<<dim3((unsigned)q_blocks, n_kv, n_batch), kPfWarps * 32, smem, static_cast<cudaStream_t>(stream)>>>(P);
+    prefill_kernel<<<dim3((unsigned)q_blocks, n_kv, n_batch), kPfWarps * 32, smem, st>>>(P);
     return cudaGetLastError() == cudaSuccess ? BGTQ_OK : BGTQ_E_LAUNCH;
 }

@@ -1,4 +1,4 @@
-// Shared by the two prefill-attention kernels (mma.sync and tcgen05): launch parameters, the per-head list of
+// Shared by the two forms of the prefill attention (mma.sync and tcgen05): launch parameters, the per-head list of
 // dequantisation tasks (8 consecutive codes of one width) and the dequantisers themselves.
 #pragma once
 #include "bgtq_common.cuh"
@@ -18,7 +18,6 @@ struct PfParams {
     int32_t n_q, n_kv, gqa, s_q, n_tok, q_pos_offset, causal, flags;
     float scale_log2;
     float* out;
-    int32_t* status;                         // tcgen05 kernel: set to 1 when a bounded wait gave up
 };
 
 // Dequantisation tasks of one head.  ktask.x: first code | count << 8 | stored bits << 12 | segment << 16 |

@@ -247,11 +247,25 @@ def rotate_q(layer: LayerTables, q: torch.Tensor, out: torch.Tensor = None) -> t
 
 
 def rotate_q_bulk(layer: LayerTables, q: torch.Tensor) -> torch.Tensor:
-    """Many positions at once: q (B, n_q, S, 128) fp16 -> same shape in the packed-K basis, as one
-    gather + fp32 GEMM per KV head group (the per-row kernel behind :func:`rotate_q` is meant for the
-    handful of rows of a decode step)."""
+    """Many positions at once: q (B, n_q, S, 128) -> same shape, fp16, in the packed-K basis (the per-row kernel
+    behind :func:`rotate_q` is meant for the handful of rows of a decode step).  fp16 queries go through the
+    tensor cores; queries of another type are rotated in fp32 first and rounded once."""
     _lib.require_cuda(q, "q")
     B, n_q, S, D = q.shape
+    if q.dtype == torch.float16:
+        st = q.stride()
+        if st[3] != 1 or (q.data_ptr() | 2 * (st[0] | st[1] | st[2])) & 15:
+            q = q.contiguous()
+            if q.data_ptr() & 15:
+                q = q.clone()
+            st = q.stride()
+        out = torch.empty(B, n_q, S, D, dtype=torch.float16, device=q.device)
+        if out.numel():
+            _lib.check(_lib.lib().bgtq_rotate_q_rows(_lib.ptr(layer.desc_dev), _lib.ptr(layer.rot_k), q.data_ptr(), *st[:3],
+                                                     out.data_ptr(), B, n_q, layer.n_kv, S, _lib.stream_ptr(q.device)),
+                       "bgtq_rotate_q_rows")
+            _lib.count_launch()
+        return out
     gqa = n_q // layer.n_kv
     qg = q.reshape(B, layer.n_kv, gqa * S, D).float()
     idx = layer.head_perm.view(1, layer.n_kv, 1, D).expand(B, layer.n_kv, gqa * S, D)
@@ -403,11 +417,14 @@ def attend(layer, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, *, ro
     return out, o32, lse
 
 
+_PREFILL_WORKSPACE = 2 << 30        # bytes of dequantised operand tiles per launch
+
+
 def prefill_attention(layer: LayerTables, q_rot, k_packed, k_norms, v_packed, v_norms, n_tokens, *,
                       q_pos_offset=0, causal=True, scale=None, flags=0, v_rot=None):
     """Attention of q_rot (B, n_q, S_q, 128) fp16 (packed-K basis) over the first ``n_tokens`` cache rows;
     query i has absolute position ``q_pos_offset + i`` and, when ``causal``, sees tokens up to it.
-    ``v_rot`` (n_kv, 128, 128) fp32 = R finishes V's rotation with one batched fp32 GEMM.
+    ``v_rot`` (n_kv, 128, 128) fp32 = R finishes V's rotation.
     Returns (B, n_q, S_q, 128) fp16.  ``_lib.PF_NO_TCGEN05`` in ``flags`` (or the environment variable
     ``BGTQ_PF_NO_TCGEN05``) keeps the products on mma.sync instead of tcgen05 / tensor memory."""
     _lib.require_cuda(q_rot, "q_rot")
@@ -420,20 +437,44 @@ def prefill_attention(layer: LayerTables, q_rot, k_packed, k_norms, v_packed, v_
         raise TypeError("cache norms must be float16")
     if scale is None:
         scale = 1.0 / math.sqrt(HD)
-    out_rot = torch.empty(B, n_q, S_q, HD, dtype=torch.float32, device=q_rot.device)
-    kps, kns, vps = _strides3(k_packed), _strides3(k_norms), _strides3(v_packed)
-    vns = (v_norms.stride(0), v_norms.stride(1), v_norms.stride(2))
-    _lib.check(_lib.lib().bgtq_prefill_attention(
-        _lib.ptr(layer.desc_dev), _lib.ptr(q_rot), q_rot.stride(0), q_rot.stride(1), q_rot.stride(2),
-        _lib.ptr(k_packed), *kps, _lib.ptr(k_norms), *kns, _lib.ptr(v_packed), *vps, _lib.ptr(v_norms), *vns,
-        B, n_q, layer.n_kv, S_q, int(n_tokens), int(q_pos_offset), 1 if causal else 0, float(scale), int(flags),
-        _lib.ptr(out_rot), _lib.stream_ptr(q_rot.device)), "bgtq_prefill_attention")
-    _lib.count_launch()
-    if v_rot is None:
-        return out_rot.to(torch.float16)
-    gqa = n_q // layer.n_kv
-    o = torch.matmul(out_rot.view(B, layer.n_kv, gqa * S_q, HD), v_rot.view(1, layer.n_kv, HD, HD))
-    return o.view(B, n_q, S_q, HD).to(torch.float16)
+    dev = q_rot.device
+    qs, kps, kns, vps = q_rot.stride()[:3], _strides3(k_packed), _strides3(k_norms), _strides3(v_packed)
+    vns = v_norms.stride()[:3]
+    L, causal = _lib.lib(), 1 if causal else 0
+    n_tokens, q_pos_offset = int(n_tokens), int(q_pos_offset)
+    if flags & _lib.PF_NO_TCGEN05:
+        out_rot = torch.empty(B, n_q, S_q, HD, dtype=torch.float32, device=dev)
+        _lib.check(L.bgtq_prefill_attention(
+            _lib.ptr(layer.desc_dev), _lib.ptr(q_rot), *qs, _lib.ptr(k_packed), *kps, _lib.ptr(k_norms), *kns,
+            _lib.ptr(v_packed), *vps, _lib.ptr(v_norms), *vns, B, n_q, layer.n_kv, S_q, n_tokens, q_pos_offset, causal,
+            float(scale), int(flags), _lib.ptr(out_rot), _lib.stream_ptr(dev)), "bgtq_prefill_attention")
+        _lib.count_launch()
+        if v_rot is None:
+            return out_rot.to(torch.float16)
+        gqa = n_q // layer.n_kv
+        o = torch.matmul(out_rot.view(B, layer.n_kv, gqa * S_q, HD), v_rot.view(1, layer.n_kv, HD, HD))
+        return o.view(B, n_q, S_q, HD).to(torch.float16)
+    out = torch.empty(B, n_q, S_q, HD, dtype=torch.float16, device=dev)
+
+    def ws_bytes(n):
+        return L.bgtq_prefill_workspace_bytes(n, n_q, layer.n_kv, S_q, n_tokens, q_pos_offset, causal, v_rot is not None)
+
+    # as many batch entries per launch as keep the dequantised tiles within the bound (one at least)
+    nb = B
+    while nb > 1 and ws_bytes(nb) > _PREFILL_WORKSPACE:
+        nb = (nb + 1) // 2
+    size = max(ws_bytes(nb), ws_bytes(B % nb) if B % nb else 0)
+    ws = torch.empty(max(size, 16), dtype=torch.uint8, device=dev)
+    for b in range(0, B, nb):
+        n = min(nb, B - b)
+        sl = slice(b, b + n)
+        _lib.check(L.bgtq_prefill(
+            _lib.ptr(layer.desc_dev), q_rot[sl].data_ptr(), *qs, k_packed[sl].data_ptr(), *kps, k_norms[sl].data_ptr(), *kns,
+            v_packed[sl].data_ptr(), *vps, v_norms[sl].data_ptr(), *vns, n, n_q, layer.n_kv, S_q, n_tokens, q_pos_offset, causal,
+            float(scale), int(flags), _lib.ptr(v_rot), ws.data_ptr(), ws.numel(), out[sl].data_ptr(), _lib.stream_ptr(dev)),
+            "bgtq_prefill")
+        _lib.count_launch(2)
+    return out
 
 
 def combine_ranks(gathered, n_batch, n_q, *, out=None):

@@ -154,6 +154,12 @@ int bgtq_rotate_q(const BgtqHeadDesc* desc, const float* rot_k,
                   const void* q, int64_t q_sb, int64_t q_sh,
                   void* q_rot, int32_t n_batch, int32_t n_q, int32_t n_kv, void* stream);
 
+/* The same for n_pos query positions per (batch, query head): position i of (b, hq) at q + b*q_sb + hq*q_sh +
+ * i*q_ss (16-byte aligned rows) -> q_rot (n_batch, n_q, n_pos, 128) fp16 contiguous.  tcgen05; its bounded waits
+ * report through bgtq_prefill_tcgen05_status(). */
+int bgtq_rotate_q_rows(const BgtqHeadDesc* desc, const float* rot_k, const void* q, int64_t q_sb, int64_t q_sh, int64_t q_ss,
+                       void* q_rot, int32_t n_batch, int32_t n_q, int32_t n_kv, int32_t n_pos, void* stream);
+
 /* One decode step's preparation in a single latency-oriented launch: the query
  * rotation of bgtq_rotate_q and the append of ONE new token per (batch, KV head)
  * of bgtq_encode (same arguments, n_tok = 1, no code outputs).  q / q_rot may be
@@ -452,10 +458,12 @@ int bgtq_attend(const BgtqDecodePlan* plan, const BgtqHeadDesc* desc, const floa
  * out_rot: (n_batch, n_q, s_q, 128) fp32 contiguous, softmax-normalised and still in V's rotated basis:
  * multiply each KV head's rows by its R (one plain GEMM) to finish.  A query with no visible token
  * yields zeros.  n_q / n_kv <= 16.
- * Two kernels: the products run on tcgen05 with accumulators in tensor memory when n_q / n_kv divides 128
- * (bgtq_prefill_t5.cu), else, or with BGTQ_PF_NO_TCGEN05 in flags, on mma.sync (bgtq_prefill.cu).  The tcgen05
- * kernel bounds its waits; bgtq_prefill_tcgen05_status() returns 1 (sticky, per process) if one ever gave up,
- * in which case that launch's output is invalid. */
+ * The products run on tcgen05 with accumulators in tensor memory (bgtq_prefill_t5.cu), or, with
+ * BGTQ_PF_NO_TCGEN05 in flags, on mma.sync (bgtq_prefill.cu).  The tcgen05 form dequantises the cache once into
+ * a workspace, which this entry point takes from the stream's memory pool for the launch (cudaMallocAsync);
+ * bgtq_prefill below takes the caller's and is the one to call repeatedly.  The tcgen05 form bounds its waits;
+ * bgtq_prefill_tcgen05_status() returns 1 (sticky, per process) if one ever gave up, in which case that
+ * launch's output is invalid. */
 #define BGTQ_PF_NO_TCGEN05 16
 int bgtq_prefill_tcgen05_status(void);
 int bgtq_prefill_attention(const BgtqHeadDesc* desc, const void* q_rot, int64_t q_sb, int64_t q_sh, int64_t q_ss,
@@ -466,6 +474,22 @@ int bgtq_prefill_attention(const BgtqHeadDesc* desc, const void* q_rot, int64_t 
                 int32_t n_batch, int32_t n_q, int32_t n_kv, int32_t s_q, int32_t n_tokens,
                 int32_t q_pos_offset, int32_t causal, float scale, int32_t flags,
                 float* out_rot, void* stream);
+
+/* The same (tcgen05 form) with the caller's workspace and the finished output: out (n_batch, n_q, s_q, 128) fp16
+ * contiguous, 16-byte aligned, multiplied by v_rot (n_kv, 128, 128) fp32 = R when that is not NULL.  workspace:
+ * device memory of bgtq_prefill_workspace_bytes(...) bytes for the same shape (768 bytes per cached token and KV
+ * head, rounded up to 128 tokens, plus partial outputs when the launch has so few query rows that the cache is cut
+ * among several CTAs), 16-byte aligned; its contents mean nothing after the launch. */
+int64_t bgtq_prefill_workspace_bytes(int32_t n_batch, int32_t n_q, int32_t n_kv, int32_t s_q, int32_t n_tokens,
+                int32_t q_pos_offset, int32_t causal, int32_t with_rotation);
+int bgtq_prefill(const BgtqHeadDesc* desc, const void* q_rot, int64_t q_sb, int64_t q_sh, int64_t q_ss,
+                const uint8_t* k_packed, int64_t kp_sb, int64_t kp_sh, int64_t kp_st,
+                const void* k_norms, int64_t kn_sb, int64_t kn_sh, int64_t kn_st,
+                const uint8_t* v_packed, int64_t vp_sb, int64_t vp_sh, int64_t vp_st,
+                const void* v_norms, int64_t vn_sb, int64_t vn_sh, int64_t vn_st,
+                int32_t n_batch, int32_t n_q, int32_t n_kv, int32_t s_q, int32_t n_tokens,
+                int32_t q_pos_offset, int32_t causal, float scale, int32_t flags,
+                const float* v_rot, void* workspace, int64_t workspace_bytes, void* out, void* stream);
 
 /* Final merge of per-rank results after an all-gather (sequence-sharded cache: every rank ran
  * bgtq_decode + bgtq_combine over its own token chunk with out_f32 / lse_out pointing into one message
