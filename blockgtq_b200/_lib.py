@@ -97,6 +97,7 @@ _SIGNATURES = {
     "bgtq_rotate_q_rows": (C.c_int, [_vp, _vp, _vp, _i64, _i64, _i64, _vp, _i32, _i32, _i32, _i32, _vp]),
     "bgtq_layer_step_size": (C.c_int, []),
     "bgtq_layer_step": (C.c_int, [_vp, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _vp, _i64, _vp]),
+    "bgtq_layer_encode": (C.c_int, [_vp, _vp, _i64, _i64, _i64, _vp, _i64, _i64, _i64, _i32, _i32, _i32, _vp]),
     "bgtq_attend_scratch_bytes": (C.c_int64, [_i32, _i32, _i32]),
     "bgtq_attend": (C.c_int, [_vp, _vp, _vp, _vp, _i64, _i64,
                               _vp, _i64, _i64, _i64, _vp, _i64, _i64, _i64,

@@ -1,0 +1,764 @@
+// Bulk (prefill) encoder: rotation on tcgen05, then one pass of a thread over its half of a row.
+//
+//   * a CTA of 16 warps works on tiles of 128 rows of one (KV head, K or V); the rotation W is staged once as
+//     hi = fp16(W), lo = fp16((W - hi) * 2^10) in the tensor cores' operand layout;
+//   * the warps form two groups of eight, which run out of phase, each on its own tiles: rows arrive by cp.async a
+//     tile ahead (V: straight into the operand's swizzled layout; K: and move on into packed order), two warps issue 8
+//     tcgen05.mma each (x . hi and x . lo into 2 x 128 tensor-memory columns), and meanwhile all warps sum the rows' group
+//     norms;
+//   * then thread (row, half) takes its half of the row's columns eight at a time straight from tensor memory (tcgen05.ld of
+//     one lane): the row is the thread's own, so everything that depends on the column (segment, bin grid, code width,
+//     byte position) is uniform over the warp, codes never leave registers, two values share an instruction where they can
+//     (f32x2), and whole 32-bit words of the packed row go to a staging image of the tile that leaves as coalesced words.
+// Bound: instruction issue and its latencies with 16 warps per SM (all registers and shared memory are taken): 1 048 576 K and
+// as many V rows take 452 us (K rows alone 286, V rows 165), where the bytes alone would take 100.  The form before gave a
+// quad of lanes four rows and four columns each, loaded three tables per element and passed the codes through shared memory
+// to a packing pass: 204 warp instructions per row and 753 us.  Tried and slower: rolled loops (smaller code, less overlap
+// of the table lookups: 589 us).
+// The sums that decide a code (group norms, products) keep the order they had: the packed bytes are bit for bit the same.
+// Every wait is bounded; tensor memory is released on every path out of the kernel.
+#include "bgtq_common.cuh"
+#include "bgtq_encode_params.cuh"
+#include "bgtq_tcgen05.cuh"
+
+namespace bgtq {
+// Sticky error word of this kernel: set when a wait for the tensor cores ran out.
+__device__ int g_enc5_status = 0;
+
+namespace {
+
+constexpr int kThreads = 512;
+constexpr int kGroup = 256;                     // threads of a group
+constexpr int kTileRows = 128;                  // = tensor-memory lanes
+constexpr int kTile = kTileRows * kHD * 2;      // bytes of a row tile
+constexpr int kMaxTasks = 40;           // 128 / 4 + one remainder per segment
+constexpr int kLevelOff = kTileRows * (kHD + 4) + 16;       // past the widest staged rows
+static_assert(kLevelOff + 2 * BGTQ_MAX_SEGMENTS * kTileRows * 4 <= kTile, "staged rows and level sums fit the operand tile");
+constexpr float kLoScale = 1024.0f;
+constexpr uint32_t kTmemCols = 512;             // per group: hi accumulator 128 columns + lo accumulator 128 columns
+constexpr int kSeg = BGTQ_MAX_SEGMENTS;
+constexpr int kLutLd = BGTQ_N_BINS + 4;
+
+// Up to eight consecutive codes of one segment, at most 32 bits: first column | count << 8 | stored bits << 12 | segment << 16
+// | bytes << 20.
+// A K row's tasks follow each other in its bytes; half 0 of a row takes tasks [0, split), half 1 the rest.  (A V row is
+// cut in the middle.)
+struct E5Smem {
+    __align__(128) uint8_t w_hi[kTile];
+    __align__(128) uint8_t w_lo[kTile];
+    // Row tiles of each group, in the tensor cores' 128-byte-swizzle layout: 16-byte chunk c of row r at
+    // (c / 8) * 16384 + r * 128 + ((c % 8) ^ (r % 8)) * 16.  V: two operand tiles, used in turn.  K: [0] = rows as they come,
+    // [1] = operand, columns in packed order.  After the product the operand tile holds the staged packed rows.
+    __align__(1024) uint8_t buf[2][2][kTile];
+    // per group: the two partial sums of squares of a (segment, row), replaced by its group norm and by 1 / norm (or 1
+    // where the norm is below the floor)
+    float part[2][2][kSeg][kTileRows];
+    float vbound[16][32], vcent[16][32];            // one copy per lane: conflict-free lookups
+    float kcent[512];
+    uint8_t code_lut[kSeg][kLutLd];                 // entry 256 = entry 255; V: [0] = boundaries below the bin
+    float2 grid[kSeg];                              // in units of 256 bins.  K: {offset, 1 / range}; V: [0] = {1 / range, offset / range}
+    __align__(16) uint8_t norm_ctl[2][16];          // K, per half and 16-byte chunk: pairs to sum (bits 0..3), segments that end behind a pair (4..7)
+    uint32_t tasks[kMaxTasks];
+    int32_t n_tasks, split, split_byte, row_bytes, data_bytes, n_seg, v_search, v_sb, v_nb;
+    int32_t seg_start[kSeg], seg_len[kSeg], seg_bw[kSeg], seg_lut_off[kSeg];
+    __align__(16) uint16_t to[kHD];                 // K: operand offset (row 0) of an input column, its packed position's place
+    __align__(8) uint64_t mma_bar[2];
+    uint32_t tmem_base;
+};
+static_assert(sizeof(E5Smem) > 114 * 1024 && sizeof(E5Smem) <= 227 * 1024, "exactly one CTA per SM (it takes all tensor memory)");
+
+// Entries trunc(clamp(256 v, 0, 255)) of a byte table for two values already saturated to [0, 1]: adding 2^23 with rounding
+// toward zero leaves the truncated bin in the low bits.  `table` = the table's shared address - 0x4B000000 (the bits of
+// 2^23).  v = 1 reads entry 256, a copy of entry 255.
+__device__ __forceinline__ void bin_addr2(float v0, float v1, uint32_t table, uint32_t& a0, uint32_t& a1) {
+    float b0, b1;
+    unpack_f2(fma_rz_f2(pack_f2(v0, v1), pack_f2(256.0f, 256.0f), pack_f2(8388608.0f, 8388608.0f)), b0, b1);
+    a0 = __float_as_uint(b0) + table;
+    a1 = __float_as_uint(b1) + table;
+}
+__device__ __forceinline__ uint32_t bin_of(float v) { return min(__float_as_uint(__fmaf_rz(v, 256.0f, 8388608.0f)) - 0x4B000000u, 255u); }
+__device__ __forceinline__ uint32_t lds8(uint32_t addr) {
+    uint32_t v;
+    asm("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ float lds_f(uint32_t addr) {
+    float v;
+    asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+    return v;
+}
+// eight fp32 columns of this thread's tensor-memory lane (no wait)
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+    uint32_t* r = reinterpret_cast<uint32_t*>(v);
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ void group_sync(int grp) { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(kGroup) : "memory"); }
+
+// eight codes, LSB first, `m` = 2^(stored bits); what does not fit 32 bits is zero
+__device__ __forceinline__ uint32_t squeeze8(const uint32_t (&c)[8], uint32_t m) {
+    uint32_t w = c[7];
+#pragma unroll
+    for (int e = 6; e >= 0; --e) w = w * m + c[e];
+    return w;
+}
+
+// A thread's part of a packed row on its way into the staging image: bytes are appended, whole words stored.  Staged rows
+// start on word boundaries, so that the position inside a word is the same for every row and all control is uniform.
+struct ByteStream {
+    uint32_t addr;      // shared address of the word being filled
+    uint32_t acc, pos;  // its bits so far
+    uint32_t skip;      // bits of the first word that belong to the row's other half
+    __device__ __forceinline__ void open(uint32_t row_addr, uint32_t byte) {
+        addr = row_addr + (byte & ~3u);
+        pos = skip = (byte & 3u) * 8u;
+        acc = 0u;
+    }
+    __device__ __forceinline__ void bytes(uint32_t lo, uint32_t hi) {
+#pragma unroll 1
+        for (uint32_t b = lo; b < hi; b += 8u) asm volatile("st.shared.u8 [%0], %1;" ::"r"(addr + (b >> 3)), "r"(acc >> b) : "memory");
+    }
+    __device__ __forceinline__ void put(uint32_t w, uint32_t n_bits) {      // n_bits a multiple of 8, at most 32; w has no bits past them
+        acc |= w << pos;
+        const uint32_t old = pos;
+        pos += n_bits;
+        if (pos >= 32u) {
+            if (skip) {
+                bytes(skip, 32u);
+                skip = 0u;
+            } else {
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(acc) : "memory");
+            }
+            addr += 4u;
+            acc = __funnelshift_rc(w, 0u, 32u - old);       // what did not fit (old = 0: nothing)
+            pos -= 32u;
+        }
+    }
+    __device__ __forceinline__ void close() { bytes(skip, pos); }
+};
+
+// Per-CTA tables: rotation split into the operand layout, bin tables, tasks.  (A few microseconds of every launch: descriptor
+// fields come to shared memory first, all loads at once, and the lists are made by a warp, not by one thread.)
+__device__ void e5_setup(E5Smem& S, const EncParams& P, const BgtqHeadDesc& d, bool is_v, int h) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid < kSeg) {
+        S.seg_start[tid] = d.seg_start[tid];
+        S.seg_len[tid] = d.seg_len[tid];
+        S.seg_bw[tid] = d.seg_bw[tid];
+        S.seg_lut_off[tid] = d.seg_lut_off[tid];
+        if (!is_v) S.grid[tid] = make_float2(d.lut_off[tid], d.lut_inv[tid] * (1.0f / 256.0f));      // (a power of two: exact)
+    }
+    if (tid == 32) {
+        S.n_seg = is_v ? 1 : d.n_seg;
+        S.v_sb = (P.flags & BGTQ_ENC_V_NIBBLE) ? 4 : d.v_bits;
+        S.v_nb = (1 << d.v_bits) - 1;
+    }
+    if (tid < kHD) S.to[d.head_perm[tid]] = (uint16_t)((tid >> 6) * 16384 + ((tid >> 3) & 7) * 16 + (tid & 7) * 2);
+    if (is_v) {
+        S.vbound[tid >> 5][tid & 31] = d.v_bounds[tid >> 5];
+        S.vcent[tid >> 5][tid & 31] = d.v_cents[tid >> 5];
+    } else {
+        *reinterpret_cast<uint32_t*>(&S.code_lut[tid >> 6][4 * (tid & 63)]) = reinterpret_cast<const uint32_t*>(&d.code_lut[0][0])[tid];
+        S.kcent[tid] = d.k_cents[tid];
+    }
+    // operand row n (output position), eight k at a time: W[k][n] is coalesced over n, 16 bytes go to shared memory
+    const float* W = (is_v ? P.rot_v : P.rot_k) + (size_t)h * kHD * kHD;
+#pragma unroll
+    for (int u = 0; u < kHD * kHD / 8 / kThreads; ++u) {
+        const int i = tid + u * kThreads, n = i & (kHD - 1), k8 = i >> 7;
+        __align__(16) __half hi[8], lo[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float w = __ldg(W + (size_t)(8 * k8 + e) * kHD + n);
+            hi[e] = __float2half_rn(w);
+            lo[e] = __float2half_rn((w - __half2float(hi[e])) * kLoScale);
+        }
+        const uint32_t o = (uint32_t)((n >> 3) * 2048 + k8 * 128 + (n & 7) * 16);
+        *reinterpret_cast<uint4*>(S.w_hi + o) = *reinterpret_cast<uint4*>(hi);
+        *reinterpret_cast<uint4*>(S.w_lo + o) = *reinterpret_cast<uint4*>(lo);
+    }
+    __syncthreads();
+    if (is_v) {
+        // V codes count the boundaries below a value.  A monotonic grid of 256 bins finds all but one of them: the table
+        // holds the boundaries in earlier bins, and one comparison with the next boundary settles the rest, as long as no
+        // bin holds two of them (else a halving search does).
+        const int nb = S.v_nb;
+        const float b0 = S.vbound[0][lane], b1 = S.vbound[nb - 1][lane];
+        const float per = (b1 > b0 ? 250.0f / (b1 - b0) : 1.0f) * (1.0f / 256.0f), off = 3.0f / 256.0f - b0 * per;
+        auto v_bin = [&](float y) { return bin_of(__saturatef(fmaf(y, per, off))); };
+        if (tid <= BGTQ_N_BINS) {
+            int below = 0;
+#pragma unroll 1
+            for (int i = 0; i < nb; ++i) below += v_bin(S.vbound[i][lane]) < (uint32_t)min(tid, BGTQ_N_BINS - 1) ? 1 : 0;
+            S.code_lut[0][tid] = (uint8_t)below;
+        }
+        if (warp == 15) {
+            const bool two = lane + 1 < nb && v_bin(S.vbound[lane & 15][lane]) >= v_bin(S.vbound[(lane + 1) & 15][lane]);
+            const bool any = __any_sync(0xffffffffu, two);
+            if (lane == 0) {
+                S.v_search = any ? 1 : 0;
+                S.grid[0] = make_float2(per, off);
+                S.row_bytes = seg_storage_bytes(S.v_sb, kHD);
+            }
+        }
+    } else {
+        if (tid < kSeg) S.code_lut[tid][BGTQ_N_BINS] = S.code_lut[tid][BGTQ_N_BINS - 1];
+        const int n_seg = S.n_seg;
+        if (warp == 0) {        // lane = segment: its tasks behind those of the segments before
+            const bool live = lane < n_seg;
+            const int st = live ? S.seg_start[lane] : 0, len = live ? S.seg_len[lane] : 0, bw = live ? S.seg_bw[lane] : 1;
+            const int sb = (P.flags & BGTQ_ENC_K_MIXED) ? (bw <= 4 ? 4 : 8) : (bw <= 4 ? bw : 8), per = sb == 8 ? 4 : 8;
+            auto n_bytes = [&](int n) { return sb == 3 ? 3 : (n * sb + 7) >> 3; };
+            const int nt = (len + per - 1) / per, bytes = nt > 0 ? (nt - 1) * n_bytes(per) + n_bytes(len - (nt - 1) * per) : 0;
+            int t_at = nt, b_at = bytes;
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                const int tu = __shfl_up_sync(0xffffffffu, t_at, o), bu = __shfl_up_sync(0xffffffffu, b_at, o);
+                if (lane >= o) {
+                    t_at += tu;
+                    b_at += bu;
+                }
+            }
+            if (lane == n_seg - 1) {
+                S.n_tasks = S.split = t_at;
+                S.data_bytes = S.split_byte = b_at;
+            }
+            __syncwarp();
+            t_at -= nt;
+            b_at -= bytes;
+#pragma unroll 1
+            for (int c = 0; c < nt; ++c) {
+                const int first = st + per * c, n = min(per, len - per * c);
+                S.tasks[t_at + c] = (uint32_t)first | (uint32_t)n << 8 | (uint32_t)sb << 12 | (uint32_t)lane << 16 | (uint32_t)n_bytes(n) << 20;
+                // the row is cut before its first task in the upper half of the columns
+                if (first >= kHD / 2 && first - (c > 0 ? per : (st > 0 ? 1 : kHD)) < kHD / 2) {
+                    S.split = t_at + c;
+                    S.split_byte = b_at + c * n_bytes(per);
+                }
+            }
+            if (lane == 0) S.row_bytes = P.kp_row_bytes;
+        } else if (warp == 1) {        // lane = (half, chunk): which of the chunk's pairs the half sums, where segments end
+            const int hf = lane >> 4, c = lane & 15;
+            uint32_t ctl = 0u;
+#pragma unroll 1
+            for (int s = 0; s < n_seg; ++s) {
+                const int p0 = S.seg_start[s] >> 1, p1 = p0 + (S.seg_len[s] >> 1);
+                for (int j = 0; j < 4; ++j) {
+                    const int p = 4 * c + j;
+                    if (p >= p0 && p < p1 && ((p - p0) & 1) == hf) ctl |= 1u << j;
+                    if (p == p1 - 1) ctl |= 16u << j;
+                }
+            }
+            S.norm_ctl[hf][c] = (uint8_t)ctl;
+        }
+    }
+}
+
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+    return v;
+}
+
+// Half a V row: 64 columns of one thread's tensor-memory lane -> its bytes in the staged row; returns the sum of the squared
+// levels.  SEARCH: boundaries by halving (see e5_setup).
+template <bool SEARCH, bool CODES>
+__device__ __forceinline__ float e5_half_v(E5Smem& S, uint32_t lane_base, int hf, float r, uint32_t row_addr, uint8_t* codes) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t lut = smem_u32(S.code_lut[0]) - 0x4B000000u, vb = smem_u32(&S.vbound[0][lane]);
+    constexpr uint32_t kCent = sizeof(S.vbound);          // vcent lies behind vbound
+    const float2 g = S.grid[0];
+    const uint32_t sb = (uint32_t)S.v_sb, mul = 1u << sb;
+    const uint32_t col = lane_base + 64u * hf;
+    const uint64_t r2 = pack_f2(r, r), scale2 = pack_f2(1.0f / kLoScale, 1.0f / kLoScale);
+    uint32_t addr = row_addr + 8u * sb * hf, acc = 0u, pos = 0u;
+    uint64_t csq2 = 0ull;
+    float hi[2][8], lo[2][8];
+    tmem_ld8(col, hi[0]);
+    tmem_ld8(col + kHD, lo[0]);
+#pragma unroll
+    for (int t2 = 0; t2 < 8; t2 += 2) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int ti = t2 + u;
+            tmem_ld_wait();
+            if (ti + 1 < 8) {       // the next columns come while these are worked on
+                tmem_ld8(col + 8u * (ti + 1), hi[u ^ 1]);
+                tmem_ld8(col + kHD + 8u * (ti + 1), lo[u ^ 1]);
+            }
+            uint32_t c[8];
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+                float y[2], cv[2];
+                uint32_t at[2];
+                unpack_f2(mul_f2(fma_f2(pack_f2(lo[u][e], lo[u][e + 1]), scale2, pack_f2(hi[u][e], hi[u][e + 1])), r2), y[0], y[1]);
+                if (!SEARCH) bin_addr2(__saturatef(fmaf(y[0], g.x, g.y)), __saturatef(fmaf(y[1], g.x, g.y)), lut, at[0], at[1]);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    uint32_t cc = 0u;
+                    if (!SEARCH) {
+                        cc = lds8(at[k]);
+                        cc += y[k] > lds_f(vb + 128u * cc) ? 1u : 0u;
+                    } else {
+#pragma unroll
+                        for (int st = 3; st >= 0; --st) cc += y[k] > lds_f(vb + 128u * (cc + (1u << st) - 1u)) ? (1u << st) : 0u;
+                    }
+                    c[e + k] = cc;
+                    cv[k] = lds_f(vb + kCent + 128u * cc);
+                }
+                const uint64_t cv2 = pack_f2(cv[0], cv[1]);
+                csq2 = fma_f2(cv2, cv2, csq2);
+            }
+            if (CODES && codes) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) codes[64 * hf + 8 * ti + e] = (uint8_t)c[e];
+            }
+            const uint32_t w = squeeze8(c, mul);
+            acc |= w << pos;
+            if (pos + 8u * sb >= 32u) {
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(acc) : "memory");
+                addr += 4u;
+                acc = __funnelshift_rc(w, 0u, 32u - pos);
+            }
+            pos = (pos + 8u * sb) & 31u;
+        }
+    }
+    float s0, s1;
+    unpack_f2(csq2, s0, s1);
+    return s0 + s1;
+}
+
+// operand descriptor of a tile in the 128-byte-swizzle layout; k-step ks of 16: see tile_step
+__device__ __forceinline__ uint64_t tile_desc(uint32_t smem_addr) {
+    return (1ull << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61) | (uint64_t)(smem_addr >> 4);
+}
+__device__ __forceinline__ uint32_t tile_step(int ks) { return (uint32_t)(ks >> 2) * (16384u >> 4) + (uint32_t)(ks & 3) * 2u; }
+// acc + x0^2 + x1^2 of two fp16 values, in that order (fp16 -> fp32 is exact: the same bits as converting first)
+__device__ __forceinline__ float square2(float acc, uint32_t w) {
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tfma.rn.f32.f16 %0, l, l, %0;\n\tfma.rn.f32.f16 %0, h, h, %0;\n\t}" : "+f"(acc) : "r"(w));
+    return acc;
+}
+
+// Tiles [lo, hi) of one (head, K or V).  `n_mma`: products this thread's group has issued so far (the barrier's phase).
+template <bool IS_V, bool MIXED, bool CODES>
+__device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int h, const int lo_tile, const int hi_tile, int& n_mma) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int grp = tid >> 8, gt = tid & (kGroup - 1);
+    const int hf = (warp >> 2) & 1, row = (warp & 3) * 32 + lane;      // (a warp reads tensor-memory lanes 32 (warp % 4) .. + 31)
+    const int n_rows = P.n_batch * P.n_tok;                  // the launcher checks that this fits
+    const int t0 = P.pos_dev ? *P.pos_dev : P.t0;
+    const uint32_t acc_hi = S.tmem_base + 256u * grp;
+    const uint32_t lane_base = acc_hi + ((uint32_t)((warp & 3) * 32) << 16);
+    uint64_t* const bar = &S.mma_bar[grp];
+    const int n_seg = S.n_seg, rb = S.row_bytes;
+    constexpr bool mixed = !IS_V && MIXED;
+    const bool f16n = P.flags & BGTQ_ENC_K_NORMS_F16;
+    const __half* const src_base = IS_V ? P.v + h * P.v_sh : P.k + h * P.k_sh;
+    const int64_t s_sb = IS_V ? P.v_sb : P.k_sb, s_ss = IS_V ? P.v_ss : P.k_ss;
+    uint8_t* const out_base = IS_V ? P.vp + h * P.vp_sh : P.kp + h * P.kp_sh;
+    const int64_t o_sb = IS_V ? P.vp_sb : P.kp_sb, o_st = IS_V ? P.vp_st : P.kp_st;
+    const uint32_t magic = ((1u << 24) + (uint32_t)rb - 1u) / (uint32_t)rb;      // x / rb = x * magic >> 24 below 128 rows
+    const int stage_ld = 4 * (((rb + 3) >> 2) | 1);       // bytes between staged rows: an odd number of words
+    const int task_lo = hf ? S.split : 0, task_hi = hf ? S.n_tasks : S.split;
+    uint8_t* const codes_out = IS_V ? P.v_codes : P.k_codes;
+
+    // K: where the elements of the chunks that this lane moves into the operand go (chunks 4 j + lane / 8 of rows = lane mod 8:
+    // eight rows and four chunks per access keep the scattered 2-byte stores two to a bank instead of six)
+    uint32_t koff[IS_V ? 1 : 4][8];
+    uint4 nctl = make_uint4(0u, 0u, 0u, 0u);
+    if constexpr (!IS_V) {
+        nctl = *reinterpret_cast<const uint4*>(S.norm_ctl[hf]);
+        const uint32_t rows = smem_u32(S.buf[grp][1]) + ((gt >> 5) * 16 + (lane & 7)) * 128;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint4 o = *reinterpret_cast<const uint4*>(&S.to[(4 * j + (lane >> 3)) * 8]);
+            const uint32_t w[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+            for (int e = 0; e < 8; ++e) koff[j][e] = rows + (((w[e >> 1] >> (16 * (e & 1))) & 0xFFFFu) ^ ((uint32_t)(lane & 7) << 4));
+        }
+    }
+    // Rows of a tile -> a buffer, asynchronously: thread -> chunk (gt & 15) of rows (gt >> 4) + 16 q; rows past the end are
+    // zero-filled.
+    const int fr = gt >> 4, fc = gt & 15;
+    const uint32_t fetch_off = (uint32_t)((fc >> 3) * 16384 + fr * 128 + (((fc & 7) ^ (fr & 7)) << 4));
+    auto prefetch = [&](int tl, int b0, int s0, uint8_t* to) {
+        const uint32_t dst = smem_u32(to) + fetch_off;
+        auto copy = [](uint32_t d, const __half* s, int bytes) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(s), "r"(bytes) : "memory");
+        };
+        if (s0 + kTileRows <= P.n_tok && (tl + 1) * kTileRows <= n_rows) {
+            const __half* src = src_base + b0 * s_sb + (s0 + fr) * s_ss + fc * 8;
+            const int64_t inc = 16 * s_ss;
+#pragma unroll
+            for (int q = 0; q < 8; ++q, src += inc) copy(dst + q * 2048u, src, 16);
+            return;
+        }
+        int b = b0, s = s0 + fr;
+#pragma unroll 1
+        for (int q = 0; q < 8; ++q) {
+            while (s >= P.n_tok) { s -= P.n_tok; ++b; }
+            const bool valid = tl * kTileRows + fr + 16 * q < n_rows;
+            copy(dst + q * 2048u, valid ? src_base + b * s_sb + s * s_ss + fc * 8 : src_base, valid ? 16 : 0);
+            s += 16;
+        }
+    };
+    // (b0, s0) = first row of tile tl
+    const int step_b = (int)((uint32_t)(2 * kTileRows) / (uint32_t)P.n_tok), step_s = 2 * kTileRows - step_b * P.n_tok;
+    int tl = lo_tile + grp;
+    int b0 = (int)((uint32_t)(tl * kTileRows) / (uint32_t)P.n_tok), s0 = tl * kTileRows - b0 * P.n_tok;
+    if (tl < hi_tile) prefetch(tl, b0, s0, S.buf[grp][0]);
+    for (int it = 0, nb0, ns0; tl < hi_tile; tl += 2, ++it, b0 = nb0, s0 = ns0) {
+        const int n0 = tl * kTileRows, n_valid = n_rows - n0 < kTileRows ? n_rows - n0 : kTileRows;
+        nb0 = b0 + step_b;
+        ns0 = s0 + step_s;
+        if (ns0 >= P.n_tok) { ns0 -= P.n_tok; ++nb0; }
+        uint8_t* const a = S.buf[grp][IS_V ? it & 1 : 1];       // the operand tile
+        // sums of squared levels per (half, segment, row), behind the staged rows in the (by then dead) operand tile
+        auto level = [&](int half, int s, int r) -> float& { return reinterpret_cast<float*>(a + kLevelOff)[(half * kSeg + s) * kTileRows + r]; };
+        // ---- the prefetched rows; K: their columns into packed order ----
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if constexpr (!IS_V) {
+            group_sync(grp);
+            const uint32_t raw = smem_u32(S.buf[grp][0]);
+#pragma unroll
+            for (int rg = 0; rg < 2; ++rg)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int chunk = 4 * j + (lane >> 3), r = (gt >> 5) * 16 + 8 * rg + (lane & 7);
+                    const uint4 v = lds128(raw + (uint32_t)((chunk >> 3) * 16384 + r * 128 + (((chunk & 7) ^ (lane & 7)) << 4)));
+                    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int c = 0; c < 8; ++c)
+                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(koff[j][c] + rg * 1024u), "h"((unsigned short)(w[c >> 1] >> (16 * (c & 1)))) : "memory");
+                }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // these rows -> tensor-core reads
+        tc_fence_before_sync();     // also orders this thread's tensor-memory reads of the previous tile
+        group_sync(grp);
+        // ---- product: one warp issues x . hi, another x . lo ----
+        if ((warp & 7) < 2) {
+            tc_fence_after_sync();
+            const uint32_t lead = elect_one();
+            const uint32_t which = warp & 1;
+            const uint32_t dst = __shfl_sync(0xffffffffu, acc_hi, 0) + which * kHD;
+            const uint64_t xd = tile_desc(smem_u32(a)), w = op_desc(smem_u32(which ? S.w_lo : S.w_hi));
+#pragma unroll
+            for (int ks = 0; ks < kHD / 16; ++ks) mma_ss(dst, xd + tile_step(ks), w + 16u * ks, ks > 0, lead);
+            if (lead) umma_commit(bar);
+            __syncwarp();
+        }
+        if (tl + 2 < hi_tile) prefetch(tl + 2, nb0, ns0, S.buf[grp][IS_V ? (it + 1) & 1 : 0]);     // arrives during this tile's work
+        // ---- group norms: the row's two threads take alternate element pairs of each segment ----
+        {
+            const uint32_t xr = smem_u32(a) + (uint32_t)row * 128u, sw = (uint32_t)(row & 7) << 4;
+            float acc = 0.f;
+            float* part = &S.part[grp][hf][0][row];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {       // four chunks requested together
+                uint4 w[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    w[c] = lds128(xr + (uint32_t)(q >> 1) * 16384u + (((uint32_t)(4 * (q & 1) + c) << 4) ^ sw));
+                const uint32_t ctl = IS_V ? (hf ? 0x0A0A0A0Au : 0x05050505u) : q == 0 ? nctl.x : q == 1 ? nctl.y : q == 2 ? nctl.z : nctl.w;
+                if (ctl == 0x05050505u) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc = square2(square2(acc, w[c].x), w[c].z);
+                } else if (IS_V || ctl == 0x0A0A0A0Au) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc = square2(square2(acc, w[c].y), w[c].w);
+                } else {
+                    auto pair = [&](uint32_t bit, uint32_t v) {
+                        if (ctl & bit) acc = square2(acc, v);
+                        if (ctl & (bit << 4)) {
+                            *part = acc;
+                            part += kTileRows;
+                            acc = 0.f;
+                        }
+                    };
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        pair(1u << (8 * c), w[c].x);
+                        pair(2u << (8 * c), w[c].y);
+                        pair(4u << (8 * c), w[c].z);
+                        pair(8u << (8 * c), w[c].w);
+                    }
+                }
+            }
+            if (IS_V) *part = acc;
+        }
+        const int n = n0 + row;
+        int b = b0, t = s0 + row;                   // this thread's row
+        while (t >= P.n_tok) { t -= P.n_tok; ++b; }
+        group_sync(grp);
+        // half hf finishes segments 2 hf, 2 hf + 1, 2 hf + 4, 2 hf + 5 (norm rows are written two values at a time)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int s = 2 * hf + (u & 1) + 4 * (u >> 1);
+            if (s >= n_seg) continue;
+            const float nr = sqrtf((S.part[grp][0][s][row] + S.part[grp][1][s][row]) + 1e-30f);
+            S.part[grp][0][s][row] = nr;
+            S.part[grp][1][s][row] = nr > (IS_V ? 1e-8f : 1e-10f) ? 1.0f / nr : 1.0f;
+        }
+        if (!bar_and(3 + grp, kGroup, mbar_wait_bounded(bar, n_mma++ & 1))) {      // same verdict for the whole group
+            if (gt == 0) atomicExch(&g_enc5_status, kStatusWaitTimeout);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            return false;
+        }
+        tc_fence_after_sync();
+        // ---- quantise and pack this thread's half of its row ----
+        const uint32_t row_addr = smem_u32(a) + (uint32_t)(row * stage_ld);
+        uint8_t* const cd = CODES && codes_out && n < n_rows ? codes_out + (((size_t)b * P.n_kv + h) * P.n_tok + t) * kHD : nullptr;
+        float csq = 0.f;
+        ByteStream out;
+        if (IS_V) {
+            const float r = S.part[grp][1][0][row];
+            csq = S.v_search ? e5_half_v<true, CODES>(S, lane_base, hf, r, row_addr, cd) : e5_half_v<false, CODES>(S, lane_base, hf, r, row_addr, cd);
+            level(hf, 0, row) = csq;
+        } else {
+            out.open(row_addr, hf ? (uint32_t)S.split_byte : 0u);
+            // (a last short task near column 128 loads from column 120: no read past the accumulators)
+            auto load_of = [](uint32_t task) { return min(task & 0xFFu, (uint32_t)kHD - 8u); };
+            int seg_now = -1;
+            const uint32_t lut0 = smem_u32(S.code_lut[0]) - 0x4B000000u;
+            const uint64_t scale2 = pack_f2(1.0f / kLoScale, 1.0f / kLoScale);
+            // Two tasks at a time: their table lookups overlap.  An odd count repeats the last task and packs it once.
+            float hi[2][8], lo[2][8];
+            auto fetch = [&](int ti, int u, uint32_t& tk) {
+                tk = S.tasks[min(ti, task_hi - 1)];
+                tmem_ld8(lane_base + load_of(tk), hi[u]);
+                tmem_ld8(lane_base + kHD + load_of(tk), lo[u]);
+            };
+            uint32_t next[2] = {0u, 0u};
+            if (task_lo < task_hi) {
+                fetch(task_lo, 0, next[0]);
+                fetch(task_lo + 1, 1, next[1]);
+            }
+            for (int ti = task_lo; ti < task_hi; ti += 2) {
+                const uint32_t cur[2] = {next[0], next[1]};
+                uint32_t c[2][8];
+                __syncwarp();
+                tmem_ld_wait();
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const uint32_t off = (cur[u] & 0xFFu) - load_of(cur[u]);      // 0, 2, 4 or 6
+                    if (off) {
+                        if (off & 2u) {
+#pragma unroll
+                            for (int e = 0; e < 6; ++e) { hi[u][e] = hi[u][e + 2]; lo[u][e] = lo[u][e + 2]; }
+                        }
+                        if (off & 4u) {
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) { hi[u][e] = hi[u][e + 4]; lo[u][e] = lo[u][e + 4]; }
+                        }
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int seg = (cur[u] >> 16) & 0xF;
+                    const float r = S.part[grp][1][seg][row];
+                    const float2 g = S.grid[seg];
+                    const uint32_t lut = lut0 + (uint32_t)(seg * kLutLd);
+                    const uint64_t r2 = pack_f2(r, r), off2 = pack_f2(-g.x, -g.x);
+#pragma unroll
+                    for (int e = 0; e < 8; e += 2) {
+                        const uint64_t x2 = fma_f2(pack_f2(lo[u][e], lo[u][e + 1]), scale2, pack_f2(hi[u][e], hi[u][e + 1]));
+                        float y0, y1;
+                        unpack_f2(fma_f2(x2, r2, off2), y0, y1);
+                        uint32_t a0, a1;
+                        bin_addr2(__saturatef(y0 * g.y), __saturatef(y1 * g.y), lut, a0, a1);
+                        c[u][e] = lds8(a0);
+                        c[u][e + 1] = lds8(a1);
+                    }
+                }
+                if (ti + 2 < task_hi) {       // the next tasks' columns come while this pair is packed
+                    fetch(ti + 2, 0, next[0]);
+                    fetch(ti + 3, 1, next[1]);
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int cnt = (cur[u] >> 8) & 0xF, sb = (cur[u] >> 12) & 0xF, seg = (cur[u] >> 16) & 0xF, nb = (cur[u] >> 20) & 0xF;
+                    if (ti + u >= task_hi) break;
+                    if (cnt < 8) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) c[u][e] = e < cnt ? c[u][e] : 0u;
+                    }
+                    if (mixed) {        // squared norm of the chosen levels, per segment
+                        if (seg != seg_now) {
+                            if (seg_now >= 0) level(hf, seg_now, row) = csq;
+                            csq = 0.f;
+                            seg_now = seg;
+                        }
+                        const uint32_t cent = smem_u32(S.kcent + S.seg_lut_off[seg]);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const float cv = e < cnt ? lds_f(cent + 4u * c[u][e]) : 0.f;
+                            csq = fmaf(cv, cv, csq);
+                        }
+                    }
+                    if (CODES && cd) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            if (e < cnt) cd[(cur[u] & 0xFFu) + e] = (uint8_t)c[u][e];
+                    }
+                    out.put(squeeze8(c[u], 1u << sb), 8u * nb);
+                }
+            }
+            if (mixed && seg_now >= 0) level(hf, seg_now, row) = csq;
+            if (hf)
+#pragma unroll 1
+                for (int p = S.data_bytes; p < rb; p += 4) out.put(0u, 8u * min(4, rb - p));      // rows of a head with fewer bytes than the widest
+            out.close();
+        }
+        tc_fence_before_sync();
+        group_sync(grp);
+        // ---- norms out ----
+        if (n < n_rows) {
+            if (!IS_V) {
+                const size_t o = b * P.kn_sb + h * P.kn_sh + (size_t)(t0 + t) * P.kn_st;
+                const int mid = S.split < S.n_tasks ? (int)(S.tasks[S.split] & 0xFFu) : kHD;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int s = 2 * hf + (u & 1) + 4 * (u >> 1);
+                    if (s >= P.kn_count) continue;
+                    float val = s < n_seg ? S.part[grp][0][s][row] : 0.f;
+                    if (mixed && s < n_seg) {       // (a segment on both sides of the split has two sums)
+                        const float q = (S.seg_start[s] < mid ? level(0, s, row) : 0.f) +
+                                        (S.seg_start[s] + S.seg_len[s] > mid ? level(1, s, row) : 0.f);
+                        val = val / fmaxf(sqrtf(q), 1e-10f);
+                    }
+                    if (f16n) static_cast<__half*>(P.kn)[o + s] = __float2half_rn(val);
+                    else static_cast<float*>(P.kn)[o + s] = val;
+                }
+            } else if (hf == 0) {
+                const float cnorm = sqrtf((level(0, 0, row) + level(1, 0, row)) + 1e-20f);
+                P.vn[b * P.vn_sb + h * P.vn_sh + (size_t)(t0 + t) * P.vn_st] =
+                    __float2half_rn(S.part[grp][0][0][row] / (cnorm > 1e-10f ? cnorm : 1.0f));
+            }
+        }
+        // ---- rows out: where the tile's rows are one run of bytes in the cache, as its aligned words ----
+        if (o_st == rb && s0 + n_valid <= P.n_tok) {
+            uint8_t* const dst0 = out_base + b0 * o_sb + (int64_t)(t0 + s0) * o_st;
+            const int total = n_valid * rb, head = min((int)((4u - (uint32_t)(reinterpret_cast<uintptr_t>(dst0) & 3u)) & 3u), total);
+            const int words = (total - head) >> 2, tail = total - head - 4 * words;
+            const uint32_t stage = smem_u32(a);
+            auto row_of = [&](int x) { return (int)(((uint32_t)x * magic) >> 24); };     // x / rb, exact below 128 rows
+            if (head == 0 && (rb & 3) == 0) {
+                for (int i = gt; i < words; i += kGroup) {
+                    const int r = row_of(4 * i);
+                    *reinterpret_cast<uint32_t*>(dst0 + 4 * i) = lds32(stage + (uint32_t)(r * (stage_ld - rb) + 4 * i));
+                }
+                continue;
+            }
+            if (gt < head) dst0[gt] = a[gt];                                                   // (inside row 0: rb >= 4)
+            if (gt < tail) {
+                const int x = total - tail + gt, r = row_of(x);
+                dst0[x] = a[r * stage_ld + x - r * rb];
+            }
+            for (int i = gt; i < words; i += kGroup) {
+                const int x = head + 4 * i, r = row_of(x), p = x - r * rb;
+                const uint32_t at = stage + (uint32_t)(r * stage_ld + (p & ~3));
+                uint32_t w = lds32(at);
+                if (p & 3) w = __funnelshift_r(w, lds32(at + 4), (uint32_t)(p & 3) * 8u);
+                const int left = rb - p;            // bytes of this row from here
+                if (left < 4) w = (w & ((1u << (8 * left)) - 1u)) | lds32(stage + (uint32_t)((r + 1) * stage_ld)) << (8 * left);
+                *reinterpret_cast<uint32_t*>(dst0 + x) = w;
+            }
+        } else {
+            for (int i = gt; i < n_valid * rb; i += kGroup) {
+                const int r = i / rb, p = i - r * rb;
+                const int nn = n0 + r, bb = (int)((uint32_t)nn / (uint32_t)P.n_tok), tt = nn - bb * P.n_tok;
+                out_base[bb * o_sb + (int64_t)(t0 + tt) * o_st + p] = a[r * stage_ld + p];
+            }
+        }
+    }
+    return true;
+}
+
+// One CTA per SM.  The tiles of all (KV head, K or V) form one list, a K tile kUnitsK units long and a V tile kUnitsV (what
+// they take: a K row's columns move into packed order first); CTA i works on the tiles that begin in its share of the units,
+// and loads the tables again where its share crosses into the next (head, role).
+constexpr int kUnitsK = 13, kUnitsV = 7;
+template <bool MIXED, bool CODES>
+__global__ void __launch_bounds__(kThreads, 1) encode_t5_kernel(const EncParams P, const int units_k, const int units_v) {
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    E5Smem& S = *reinterpret_cast<E5Smem*>(smem_raw);
+    const int tid = threadIdx.x;
+    if (tid == 0) {
+        mbar_init(&S.mma_bar[0], 2);
+        mbar_init(&S.mma_bar[1], 2);
+        mbar_fence_init();
+    }
+    if (tid < 32) tmem_alloc(&S.tmem_base, kTmemCols);
+    grid_launch_dependents();
+    const int n_tiles = (P.n_batch * P.n_tok + kTileRows - 1) / kTileRows;
+    const int64_t len_k = (int64_t)units_k * n_tiles, len_v = (int64_t)units_v * n_tiles, len = len_k + len_v, all = len * P.n_kv;
+    const int64_t u0 = all * blockIdx.x / gridDim.x, u1 = all * (blockIdx.x + 1) / gridDim.x;
+    bool waited = false, in_range = true;
+    int n_mma = 0;
+    for (int64_t u = u0; u < u1 && in_range;) {
+        const int h = (int)(u / len);
+        const bool is_v = u - h * len >= len_k;
+        const int64_t base = h * len + (is_v ? len_k : 0), end = base + (is_v ? len_v : len_k);
+        const int w = is_v ? units_v : units_k;
+        const int lo = (int)((u - base + w - 1) / w), hi = (int)((min(u1, end) - base + w - 1) / w);
+        u = end;
+        if (lo >= hi) continue;
+        e5_setup(S, P, P.desc[h], is_v, h);
+        if (!waited) {
+            grid_dependency_wait();       // the rows, and what this launch overwrites, belong to earlier work in the stream
+            waited = true;
+            if (P.pos_dev) in_range = enc_range_ok(P, *P.pos_dev, P.n_tok);      // (uniform over the launch: else nothing is stored)
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");          // W operand: generic stores -> tensor-core reads
+        tc_fence_before_sync();
+        __syncthreads();
+        tc_fence_after_sync();
+        if (!in_range) break;
+        const bool ok = is_v ? e5_role<true, MIXED, CODES>(S, P, h, lo, hi, n_mma) : e5_role<false, MIXED, CODES>(S, P, h, lo, hi, n_mma);
+        if (!__syncthreads_and(ok ? 1 : 0)) break;      // (also: everyone is done with this range's tables)
+    }
+    if (!waited) grid_dependency_wait();
+    tc_fence_before_sync();
+    __syncthreads();
+    if (tid < 32) tmem_dealloc(S.tmem_base, kTmemCols);
+}
+
+}  // namespace
+
+// The launcher's caller checks: every input row 16-byte aligned and n_tok >= 16 (as for the warp-MMA bulk path).
+int launch_encode_t5(const EncParams& P, cudaStream_t stream) {
+    const int64_t n_rows = (int64_t)P.n_batch * P.n_tok;
+    if (n_rows > (1LL << 30)) return BGTQ_E_TOOBIG;
+    const bool do_k = !(P.flags & BGTQ_ENC_SKIP_K), do_v = !(P.flags & BGTQ_ENC_SKIP_V);
+    if (!do_k && !do_v) return BGTQ_OK;
+    const int n_tiles = (int)((n_rows + kTileRows - 1) / kTileRows);
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int64_t all = (int64_t)n_tiles * P.n_kv * ((do_k ? 1 : 0) + (do_v ? 1 : 0));
+    const bool few = all <= sms;                // one tile per CTA
+    const int units_k = do_k ? (few ? 1 : kUnitsK) : 0, units_v = do_v ? (few ? 1 : kUnitsV) : 0;
+    const int smem = (int)sizeof(E5Smem);
+    const bool mixed = P.flags & BGTQ_ENC_K_MIXED, codes = P.k_codes != nullptr || P.v_codes != nullptr;
+    auto kern = mixed ? (codes ? encode_t5_kernel<true, true> : encode_t5_kernel<true, false>)
+                      : (codes ? encode_t5_kernel<false, true> : encode_t5_kernel<false, false>);
+    // the attribute is per device: set it on every launch (cheap, and legal under stream capture)
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return BGTQ_E_LAUNCH;
+    }
+    return launch_kernel(kern, dim3((unsigned)(few ? all : sms)), dim3(kThreads), smem, stream, true, P, units_k,
+                         units_v) == cudaSuccess ? BGTQ_OK : BGTQ_E_LAUNCH;
+}
+
+}  // namespace bgtq
+
+extern "C" __attribute__((visibility("default"))) int bgtq_encode_tcgen05_status(void) {
+    int v = 0;
+    if (cudaMemcpyFromSymbol(&v, bgtq::g_enc5_status, sizeof(v)) != cudaSuccess) {
+        cudaGetLastError();
+        return BGTQ_E_LAUNCH;
+    }
+    return v;
+}

@@ -323,8 +323,6 @@ constexpr int kWarpMma = 16, kWarpCopy = 17;
 constexpr int kSlots = 5;
 constexpr uint32_t kTmemCols = 512;     // S (and P) of block m: columns [128 m, 128 m + 128); O of block m: [256 + 128 m, 384 + 128 m)
 constexpr uint32_t kColS = 0, kColO = 256;
-// instruction descriptor: D fp32, A and B fp16, both K-major, M = N = 128
-constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 constexpr float kLazyLog2 = 8.0f;       // a row rescales O only when its maximum grew by more than 2^8
 
 struct AtSmem {
@@ -353,54 +351,6 @@ __device__ __forceinline__ float at_exp2(float x) {      // hardware 2^x; ex2(-i
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-__device__ __forceinline__ uint64_t pack_f2(float lo, float hi) {
-    uint64_t d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-    return d;
-}
-__device__ __forceinline__ void unpack_f2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ uint64_t fma_f2(uint64_t a, uint64_t b, uint64_t c) {       // two fp32 FMAs in one instruction
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-// Products are issued by a whole warp with one elected lane enabled, so that descriptors and addresses live in uniform
-// registers: issued from inside a one-lane branch, with a descriptor built per product, they cost 95 cycles each against
-// the 64 that the tensor pipe takes.
-__device__ __forceinline__ uint32_t elect_one() {
-    uint32_t e;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
-    return e;
-}
-// operand descriptor (see umma_desc); k-step ks is 16 ks further (256 bytes in units of 16)
-__device__ __forceinline__ uint64_t op_desc(uint32_t smem_addr) {
-    return ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(2048u >> 4) << 32) | (1ull << 46) | (uint64_t)(smem_addr >> 4);
-}
-// D(tmem, 128 x 128 fp32) (+)= A . B^T, A and B 128 x 16 fp16 in shared memory; executed by the lane with `leader` set
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate, uint32_t leader) {
-    asm volatile(
-        "{\n\t.reg .pred p, e;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.ne.b32 e, %5, 0;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(kIdesc), "r"(accumulate), "r"(leader)
-        : "memory");
-}
-// the same with A in tensor memory
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t accumulate, uint32_t leader) {
-    asm volatile(
-        "{\n\t.reg .pred p, e;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.ne.b32 e, %5, 0;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(kIdesc), "r"(accumulate), "r"(leader)
-        : "memory");
 }
 // 16 consecutive 32-bit columns of this thread's tensor-memory lane from registers
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {

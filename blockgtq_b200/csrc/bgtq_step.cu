@@ -56,6 +56,16 @@ extern "C" __attribute__((visibility("default"))) int bgtq_layer_step(
                         s->n_batch, s->n_q, s->n_kv, s->out, s->o_sb, s->o_sh, nullptr, nullptr, s->combine_flags, stream);
 }
 
+extern "C" __attribute__((visibility("default"))) int bgtq_layer_encode(const BgtqLayerStep* s, const void* k, int64_t k_sb, int64_t k_sh,
+                                                                        int64_t k_ss, const void* v, int64_t v_sb, int64_t v_sh,
+                                                                        int64_t v_ss, int32_t n_tok, int32_t t0, int32_t flags, void* stream) {
+    if (!s) return BGTQ_E_BADARG;
+    return bgtq_encode(s->desc, s->rot_k, s->rot_v, k, k_sb, k_sh, k_ss, v, v_sb, v_sh, v_ss, s->n_batch, s->n_kv, n_tok, t0, s->k_packed,
+                       s->kp_sb, s->kp_sh, s->kp_st, s->kp_row_bytes, s->k_norms, s->kn_sb, s->kn_sh, s->kn_st, s->kn_count, s->v_packed,
+                       s->vp_sb, s->vp_sh, s->vp_st, s->v_norms, s->vn_sb, s->vn_sh, s->vn_st, nullptr, nullptr,
+                       (s->enc_flags & ~BGTQ_ENC_PROGRAMMATIC) | flags, nullptr, s->t_capacity, nullptr, stream);
+}
+
 extern "C" __attribute__((visibility("default"))) int64_t bgtq_attend_scratch_bytes(int32_t n_batch, int32_t n_q, int32_t n_splits) {
     if (n_batch < 1 || n_q < 1 || n_splits < 1) return 0;
     const int64_t rows = (int64_t)n_batch * n_q;

@@ -1,5 +1,5 @@
 // Thin wrappers around the tcgen05 (fifth-generation tensor core) and tensor-memory PTX used by the
-// bulk encoders: allocation, shared-memory matrix descriptors, MMA issue/commit, tensor-memory loads.
+// bulk encoder and the prefill attention: allocation, shared-memory matrix descriptors, MMA issue/commit, tensor-memory loads.
 #pragma once
 #include "bgtq_common.cuh"
 
@@ -16,24 +16,39 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t base, uint32_t cols) {    
 }
 __device__ __forceinline__ void tc_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// shared-memory matrix descriptor: no swizzle, K-major, 128 B between the two k chunks of a step, 2048 B between 8-row groups
-__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
-    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(2048u >> 4) << 32) |
-           (1ull << 46);
+// instruction descriptor: D fp32, A and B fp16, both K-major, M = N = 128
+constexpr uint32_t kIdesc128 = (1u << 4) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+// Products are issued by a whole warp with one elected lane enabled, so that descriptors and addresses live in uniform
+// registers: issued from inside a one-lane branch, with a descriptor built per product, they cost 95 cycles each against
+// the 64 that the tensor pipe takes.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e;
 }
-// The same with the distance between 8-row groups given by the caller (8 k-chunks of 128 B per group when the
-// operand is 64 elements deep: 1024).
-__device__ __forceinline__ uint64_t umma_desc_sbo(uint32_t smem_addr, uint32_t sbo_bytes) {
-    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(sbo_bytes >> 4) << 32) |
-           (1ull << 46);
+// shared-memory operand descriptor: no swizzle, K-major, 128 B between the two k chunks of a step, 2048 B between 8-row
+// groups; k-step ks is 16 ks further (256 bytes in units of 16)
+__device__ __forceinline__ uint64_t op_desc(uint32_t smem_addr) {
+    return ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(2048u >> 4) << 32) | (1ull << 46) | (uint64_t)(smem_addr >> 4);
 }
-// D(tmem, 128 x 128 fp32) (+)= A(smem, 128 x 16 fp16) . B(smem, 128 x 16 fp16)^T      (one thread)
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// D(tmem, 128 x 128 fp32) (+)= A . B^T, A and B 128 x 16 fp16 in shared memory; executed by the lane with `leader` set
+__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate, uint32_t leader) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, e;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "setp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(kIdesc128), "r"(accumulate), "r"(leader)
+        : "memory");
+}
+// the same with A in tensor memory
+__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t accumulate, uint32_t leader) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(kIdesc128), "r"(accumulate), "r"(leader)
         : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {                          // one thread
@@ -69,16 +84,6 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&v)[32]) 
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// 16 lanes x 16 fp32 columns in the register layout of two m16n8 accumulator tiles: lane offset of the
-// address selects lanes [l, l + 16); thread t gets rows t/4 and t/4 + 8, columns 2(t%4), 2(t%4) + 1 of
-// columns [c, c + 8) in v[0..3] and of [c + 8, c + 16) in v[4..7].
-__device__ __forceinline__ void tmem_ld_16x16(uint32_t taddr, float (&v)[8]) {
-    uint32_t* r = reinterpret_cast<uint32_t*>(v);
-    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr)
-                 : "memory");
-}
 // Named barrier over `count` threads that also ANDs a per-thread flag (whole warps only).
 __device__ __forceinline__ bool bar_and(uint32_t id, uint32_t count, bool flag) {
     uint32_t out;
@@ -91,6 +96,34 @@ __device__ __forceinline__ bool bar_and(uint32_t id, uint32_t count, bool flag) 
         : "r"((uint32_t)flag), "r"(id), "r"(count)
         : "memory");
     return out != 0;
+}
+
+// ---- two fp32 operations in one instruction ------------------------------------
+__device__ __forceinline__ uint64_t pack_f2(float lo, float hi) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ void unpack_f2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma_f2(uint64_t a, uint64_t b, uint64_t c) {       // two fp32 FMAs in one instruction
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul_f2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t fma_rz_f2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rz.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
 }
 
 }  // namespace bgtq

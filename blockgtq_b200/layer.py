@@ -180,21 +180,15 @@ def encode(layer: LayerTables, k, v, t0, k_packed, k_norms, v_packed, v_norms, *
     ``v_packed`` (B, n_kv, T, bytes) u8 and ``v_norms`` (B, n_kv, T) f16.  Either side may be None.
     Bulk row counts (>= 128 rows) run the tcgen05 / tensor-memory encoder; ``_lib.ENC_NO_TCGEN05`` in ``flags``
     (or the environment variable ``BGTQ_ENC_NO_TCGEN05``) keeps them on the warp-MMA one."""
-    L = _lib.lib()
     ref = k if k is not None else v
     _lib.require_cuda(ref, "k/v")
     B, H, S, D = ref.shape
     if H != layer.n_kv or D != HD:
         raise ValueError("shape does not match the layer tables")
-    if k is None:
-        flags |= _lib.ENC_SKIP_K
-    if v is None:
-        flags |= _lib.ENC_SKIP_V
-    if os.environ.get("BGTQ_ENC_NO_TCGEN05"):
-        flags |= _lib.ENC_NO_TCGEN05
-    ks = _strides3(k) if k is not None else (0, 0, 0)
-    vs = _strides3(v) if v is not None else (0, 0, 0)
+    kps = kns = vps = vns = ks = vs = (0, 0, 0)
+    kp_bytes = kn_count = 1
     if k is not None:
+        ks = _strides3(k)
         if k.dtype != torch.float16 or k_packed.dtype != torch.uint8:
             raise TypeError("k must be float16 and k_packed uint8")
         if k_norms.dtype == torch.float16:
@@ -206,26 +200,35 @@ def encode(layer: LayerTables, k, v, t0, k_packed, k_norms, v_packed, v_norms, *
             raise ValueError("cache overflow")
         kp_bytes, kn_count = k_packed.shape[3], k_norms.shape[3]
     else:
-        kps = kns = (0, 0, 0)
-        kp_bytes = kn_count = 1
+        flags |= _lib.ENC_SKIP_K
     if v is not None:
+        vs = _strides3(v)
         if v.dtype != torch.float16 or v_packed.dtype != torch.uint8 or v_norms.dtype != torch.float16:
             raise TypeError("v must be float16, v_packed uint8, v_norms float16")
         vps = _strides3(v_packed)
         need = HD // 2 if flags & _lib.ENC_V_NIBBLE else layer.vpb
         if v_packed.shape[3] < need:
             raise ValueError("v_packed rows are too short")
-        vns = (v_norms.stride(0), v_norms.stride(1), v_norms.stride(2))
+        vns = v_norms.stride()[:3]
     else:
-        vps = vns = (0, 0, 0)
-    _lib.check(L.bgtq_encode(
-        _lib.ptr(layer.desc_dev), _lib.ptr(layer.rot_k), _lib.ptr(layer.rot_v),
-        _lib.ptr(k), *ks, _lib.ptr(v), *vs, B, H, S, int(t0),
-        _lib.ptr(k_packed), *kps, kp_bytes, _lib.ptr(k_norms), *kns, kn_count,
-        _lib.ptr(v_packed), *vps, _lib.ptr(v_norms), *vns,
-        _lib.ptr(k_codes), _lib.ptr(v_codes), flags, _lib.ptr(pos_dev),
-        int((k_packed if k is not None else v_packed).shape[2]), _lib.ptr(status),
-        _lib.stream_ptr(ref.device)), "bgtq_encode")
+        flags |= _lib.ENC_SKIP_V
+    _encode_rows(layer, k, ks, v, vs, B, S, int(t0), k_packed, kps, kp_bytes, k_norms, kns, kn_count, v_packed, vps, v_norms, vns,
+                 (k_packed if k is not None else v_packed).shape[2], flags, k_codes, v_codes, pos_dev, status)
+
+
+def _no_tcgen05() -> int:
+    return _lib.ENC_NO_TCGEN05 if os.environ.get("BGTQ_ENC_NO_TCGEN05") else 0
+
+
+def _encode_rows(layer, k, ks, v, vs, B, S, t0, kp, kps, kp_bytes, kn, kns, kn_count, vp, vps, vn, vns, capacity, flags,
+                 k_codes=None, v_codes=None, pos_dev=None, status=None):
+    """The library call behind :func:`encode`: tensors with their (batch, head, token) strides, nothing checked."""
+    ptr = _lib.ptr
+    _lib.check(_lib.lib().bgtq_encode(
+        ptr(layer.desc_dev), ptr(layer.rot_k), ptr(layer.rot_v), ptr(k), *ks, ptr(v), *vs, B, layer.n_kv, S, t0,
+        ptr(kp), *kps, kp_bytes, ptr(kn), *kns, kn_count, ptr(vp), *vps, ptr(vn), *vns,
+        ptr(k_codes), ptr(v_codes), flags | _no_tcgen05(), ptr(pos_dev), capacity, ptr(status),
+        _lib.stream_ptr((k if k is not None else v).device)), "bgtq_encode")
     _lib.count_launch()
 
 

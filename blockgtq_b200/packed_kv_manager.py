@@ -24,7 +24,7 @@ import torch
 from . import _lib
 from .calib import packed_v_bytes
 from .layer import (HD, LayerTables, attend, buffer_attn, combine, decode, decode_grid_size, decode_partition, default_splits,
-                    encode, rotate_q, step_prepare)
+                    encode, rotate_q, step_prepare, _no_tcgen05)
 from .quantizer import BlockGTQQuantizer, build_batched_encode_args
 
 __all__ = ["BlockGTQKVManager", "decode_step"]
@@ -193,10 +193,21 @@ class BlockGTQKVManager:
         """Encode (B, n_kv, S, hd) fp16 into packed rows [t_start, t_end): one launch, written in place
         (packed_kv_manager.py:138-180)."""
         self._ensure_storage()
-        li = layer_idx
-        assert k.shape[2] == t_end - t_start
-        encode(self._layers[li], k.to(torch.float16), v.to(torch.float16), t_start,
-               self._k_packed[li], self._k_norms[li], self._v_packed[li], self._v_norms[li], flags=self._enc_flags)
+        n = k.shape[2]
+        assert n == t_end - t_start
+        if k.dtype != torch.float16:
+            k = k.to(torch.float16)
+        if v.dtype != torch.float16:
+            v = v.to(torch.float16)
+        _lib.require_cuda(k, "k/v")
+        ks, vs = k.stride(), v.stride()
+        if k.shape != (self.B, self.n_kv, n, self.hd) or v.shape != k.shape or ks[3] != 1 or vs[3] != 1 or t_end > self.max_T:
+            li = layer_idx          # (another batch size, or an error to report)
+            return encode(self._layers[li], k, v, t_start, self._k_packed[li], self._k_norms[li], self._v_packed[li],
+                          self._v_norms[li], flags=self._enc_flags)
+        _lib.check(_lib.lib().bgtq_layer_encode(self._step_args(layer_idx).addr, k.data_ptr(), *ks[:3], v.data_ptr(), *vs[:3], n,
+                                                int(t_start), _no_tcgen05(), _lib.stream_ptr(k.device)), "bgtq_layer_encode")
+        _lib.count_launch()
 
     def init_from_cache(self, past_key_value):
         """Bulk-encode an HF cache after prefill (packed_kv_manager.py:259-266).  Accepts the
@@ -612,6 +623,8 @@ class BlockGTQKVManager:
 
 
 def _layer_kv(pkv, li):
+    if isinstance(pkv, (list, tuple)):
+        return pkv[li][0], pkv[li][1]
     if hasattr(pkv, "key_cache"):
         return pkv.key_cache[li], pkv.value_cache[li]
     if hasattr(pkv, "layers"):

@@ -13,7 +13,7 @@ from typing import Optional
 import torch
 
 from . import _lib, calib
-from .layer import LayerTables, encode as _encode
+from .layer import LayerTables, _encode_rows, encode as _encode
 
 HD = _lib.HD
 
@@ -346,60 +346,61 @@ def build_batched_encode_args(quantizers: list, device="cuda") -> dict:
     }
 
 
-def _flat4(x: torch.Tensor):
-    """(n_kv, N, hd) -> (1, n_kv, N, hd) view for the encoder's (B, H, S, D) grid."""
+def _rows3(x: torch.Tensor):
+    """(n_kv, N, hd) fp16 contiguous."""
     if x.dim() != 3 or x.shape[2] != HD:
         raise ValueError("expected (n_kv, N, 128)")
-    return x.to(torch.float16).contiguous().unsqueeze(0)
+    _lib.require_cuda(x, "k/v")
+    return x if x.dtype == torch.float16 and x.is_contiguous() else x.detach().to(torch.float16).contiguous()
 
 
-@torch.no_grad()
+def _compress_k(k_flat, args, row_bytes: int, flags: int):
+    """One launch over all heads: (packed (n_kv, N, row_bytes) u8, norms (n_kv, N, max_ng) f32)."""
+    lt = args["_layer"]
+    k = _rows3(k_flat)
+    n_kv, n, _ = k.shape
+    if n_kv != lt.n_kv:
+        raise ValueError("shape does not match the layer tables")
+    kp = torch.empty(n_kv, n, row_bytes, dtype=torch.uint8, device=k.device)
+    kn = torch.empty(n_kv, n, lt.max_ng, dtype=torch.float32, device=k.device)
+    _encode_rows(lt, k, (0, n * HD, HD), None, (0, 0, 0), 1, n, 0, kp, (0, n * row_bytes, row_bytes), row_bytes, kn,
+                 (0, n * lt.max_ng, lt.max_ng), lt.max_ng, None, (0, 0, 0), None, (0, 0, 0), n, flags | _lib.ENC_SKIP_V)
+    return kp, kn
+
+
+def _compress_v(v_flat, args, row_bytes: int, flags: int):
+    lt = args["_layer"]
+    v = _rows3(v_flat)
+    n_kv, n, _ = v.shape
+    if n_kv != lt.n_kv:
+        raise ValueError("shape does not match the layer tables")
+    vp = torch.empty(n_kv, n, row_bytes, dtype=torch.uint8, device=v.device)
+    vn = torch.empty(n_kv, n, dtype=torch.float16, device=v.device)
+    _encode_rows(lt, None, (0, 0, 0), v, (0, n * HD, HD), 1, n, 0, None, (0, 0, 0), 1, None, (0, 0, 0), 1, vp,
+                 (0, n * row_bytes, row_bytes), vn, (0, n, 1), n, flags | _lib.ENC_SKIP_K)
+    return vp, vn
+
+
 def compress_k_packed_batched(k_flat, args, block_n: int = 32):
     """(n_kv, N, hd) fp16 -> (packed (n_kv, N, max_tpb) u8, norms (n_kv, N, max_ng) f32)
     (quantizer.py:2104-2172)."""
-    lt = args["_layer"]
-    n_kv, n, _ = k_flat.shape
-    kp = torch.empty(1, n_kv, n, lt.max_tpb, dtype=torch.uint8, device=k_flat.device)
-    kn = torch.empty(1, n_kv, n, lt.max_ng, dtype=torch.float32, device=k_flat.device)
-    _encode(lt, _flat4(k_flat), None, 0, kp, kn, None, None)
-    return kp[0], kn[0]
+    return _compress_k(k_flat, args, args["_layer"].max_tpb, 0)
 
 
-@torch.no_grad()
 def compress_v_packed_batched(v_flat, args, block_n: int = 32):
     """(n_kv, N, hd) fp16 -> (packed (n_kv, N, vpb) u8, norms (n_kv, N) f16) (quantizer.py:1979-2029)."""
-    lt = args["_layer"]
-    n_kv, n, _ = v_flat.shape
-    vp = torch.empty(1, n_kv, n, lt.vpb, dtype=torch.uint8, device=v_flat.device)
-    vn = torch.empty(1, n_kv, n, dtype=torch.float16, device=v_flat.device)
-    _encode(lt, None, _flat4(v_flat), 0, None, None, vp, vn)
-    return vp[0], vn[0]
+    return _compress_v(v_flat, args, args["_layer"].vpb, 0)
 
 
-@torch.no_grad()
 def compress_k_mixed_batched(k_flat, args, block_n: int = 32, norm_correct: bool = True):
     """-> (k_mixed (n_kv, N, max_mixed_bytes) u8: nibble pairs then raw bytes, norms f32)
     (quantizer.py:1843-1976)."""
-    lt = args["_layer"]
-    n_kv, n, _ = k_flat.shape
-    kp = torch.empty(1, n_kv, n, lt.max_mixed_bytes, dtype=torch.uint8, device=k_flat.device)
-    kn = torch.empty(1, n_kv, n, lt.max_ng, dtype=torch.float32, device=k_flat.device)
-    if norm_correct:
-        _encode(lt, _flat4(k_flat), None, 0, kp, kn, None, None, flags=_lib.ENC_K_MIXED)
-    else:
-        # layout from the mixed mode, norms from the plain mode
-        _encode(lt, _flat4(k_flat), None, 0, kp, kn.clone(), None, None, flags=_lib.ENC_K_MIXED)
-        tmp = torch.empty(1, n_kv, n, lt.max_tpb, dtype=torch.uint8, device=k_flat.device)
-        _encode(lt, _flat4(k_flat), None, 0, tmp, kn, None, None)
-    return kp[0], kn[0]
+    kp, kn = _compress_k(k_flat, args, args["_layer"].max_mixed_bytes, _lib.ENC_K_MIXED)
+    if not norm_correct:        # layout from the mixed mode, norms from the plain mode
+        kn = compress_k_packed_batched(k_flat, args)[1]
+    return kp, kn
 
 
-@torch.no_grad()
 def compress_v_nibble4_batched(v_flat, args, block_n: int = 32):
     """-> (nibble4 (n_kv, N, hd/2) u8, norms (n_kv, N) f16) (quantizer.py:2032-2101)."""
-    lt = args["_layer"]
-    n_kv, n, _ = v_flat.shape
-    vp = torch.empty(1, n_kv, n, HD // 2, dtype=torch.uint8, device=v_flat.device)
-    vn = torch.empty(1, n_kv, n, dtype=torch.float16, device=v_flat.device)
-    _encode(lt, None, _flat4(v_flat), 0, None, None, vp, vn, flags=_lib.ENC_V_NIBBLE)
-    return vp[0], vn[0]
+    return _compress_v(v_flat, args, HD // 2, _lib.ENC_V_NIBBLE)

@@ -431,6 +431,11 @@ int bgtq_layer_step(const BgtqLayerStep* step, const void* q, int64_t q_sb, int6
                     const void* k, int64_t k_sb, int64_t k_sh, const void* v, int64_t v_sb, int64_t v_sh,
                     const void* rope_cos, const void* rope_sin, int64_t rope_sb, void* stream);
 
+/* bgtq_encode of n_tok tokens into rows [t0, t0 + n_tok) of the same layer's cache; flags: further BGTQ_ENC_* bits. */
+int bgtq_layer_encode(const BgtqLayerStep* step, const void* k, int64_t k_sb, int64_t k_sh, int64_t k_ss,
+                      const void* v, int64_t v_sb, int64_t v_sh, int64_t v_ss, int32_t n_tok, int32_t t0,
+                      int32_t flags, void* stream);
+
 /* Attention of one query token per (batch, head) over cached rows [t_begin, t_end) in one call: query rotation
  * (rot_k may be NULL: q is in the packed-K basis and contiguous) -> bgtq_decode -> bgtq_combine into the
  * contiguous out (n_batch, n_q, 128) fp16 and the optional out_f32 / lse_out.  scratch: device memory of
