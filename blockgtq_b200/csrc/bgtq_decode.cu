@@ -44,18 +44,13 @@ static int decode_impl(
 
     // Tiles of 16 warps x 32 tokens, two stages; rows too wide for that (padded strides, the nibble layout with
     // large tables) fall back to 16 tokens per warp.
-    int nu = 2;
-    size_t smem = 0;
-    for (;; --nu) {
-        if (nu == 0) return BGTQ_E_TOOBIG;
-        const StageLayout sl = stage_layout(kDecWarps * 16u * nu, P.kp_st, P.kn_st, P.vp_st, P.vn_st);
-        P.off_kn = sl.off_kn; P.off_v = sl.off_v; P.off_vn = sl.off_vn;
-        P.stage_bytes = sl.stage_bytes;
-        P.stage_off = kOffStagesMin + P.plan.lut_bytes;
-        const uint32_t region = kDecStages * P.stage_bytes > kMergeBytes ? kDecStages * P.stage_bytes : kMergeBytes;
-        smem = (size_t)P.stage_off + region;
-        if (smem <= 227 * 1024) break;
-    }
+    const int nu = decode_nu(P.plan.lut_bytes, P.kp_st, P.kn_st, P.vp_st, P.vn_st);
+    if (nu == 0) return BGTQ_E_TOOBIG;
+    const StageLayout sl = stage_layout(kDecWarps * 16u * nu, P.kp_st, P.kn_st, P.vp_st, P.vn_st);
+    P.off_kn = sl.off_kn; P.off_v = sl.off_v; P.off_vn = sl.off_vn;
+    P.stage_bytes = sl.stage_bytes;
+    P.stage_off = kOffStagesMin + P.plan.lut_bytes;
+    const size_t smem = decode_smem(P.plan.lut_bytes, sl.stage_bytes);
 
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -70,8 +65,8 @@ static int decode_impl(
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool pdl = (P.plan.flags & BGTQ_DEC_PROGRAMMATIC) != 0;
     cudaError_t e;
-    // the kernel specialised for this layer's heads, when the plan carries one (it exists for the wide tile only)
-    bool jit = P.plan.jit_kernel != nullptr && nu == 2 && !(P.plan.flags & BGTQ_DEC_GENERIC);
+    // the kernel specialised for this layer's heads, when the plan carries one for this tile width
+    bool jit = P.plan.jit_kernel != nullptr && nu == decode_jit_nu(P.plan) && !(P.plan.flags & BGTQ_DEC_GENERIC);
     if (jit && P.plan.row_st[0] > 0) {
         // compiled for fixed row strides and for arrays whose every (batch, head) slice and first row start on a
         // 16-byte boundary: any other launch takes the general kernel

@@ -104,7 +104,7 @@ std::string make_prelude(const DecPlanDev& pl) {
     char buf[512];
     std::string s;
     s += "#define BGTQ_JIT 1\n#define BGTQ_HEAD_DIM 128\n";
-    snprintf(buf, sizeof(buf), "#define BGTQ_JIT_VB %d\n#define BGTQ_JIT_NU 2\n", pl.v_sbits);
+    snprintf(buf, sizeof(buf), "#define BGTQ_JIT_VB %d\n#define BGTQ_JIT_NU %d\n", pl.v_sbits, decode_jit_nu(pl));
     s += buf;
     if (pl.row_st[0] > 0) {       // row strides fixed at compile time (and 16-byte aligned slices promised at launch)
         snprintf(buf, sizeof(buf), "#define BGTQ_JIT_STRIDES 1\n#define BGTQ_JIT_KP_ST %du\n#define BGTQ_JIT_KN_ST %du\n"
@@ -258,7 +258,7 @@ extern "C" __attribute__((visibility("default"))) int bgtq_decode_plan_specializ
 }
 
 namespace bgtq {
-// Launch the specialised kernel recorded in the plan (tiles of 16 warps x 32 tokens only).
+// Launch the specialised kernel recorded in the plan.
 cudaError_t launch_decode_jit(const DecParams& P, dim3 grid, size_t smem, cudaStream_t stream, bool programmatic) {
     const void* fn = P.plan.jit_kernel;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -958,6 +958,25 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
 }
 
 #ifndef BGTQ_JIT
+// Shared memory of a launch, and the 16-token row tiles per warp that fit (2, else 1; 0: none does).
+inline size_t decode_smem(uint32_t lut_bytes, uint32_t stage_bytes) {
+    const uint32_t stages = kDecStages * stage_bytes;
+    return (size_t)kOffStagesMin + lut_bytes + (stages > kMergeBytes ? stages : kMergeBytes);
+}
+inline int decode_nu(uint32_t lut_bytes, uint32_t kp_st, uint32_t kn_st, uint32_t vp_st, uint32_t vn_st) {
+    for (int nu = 2; nu > 0; --nu)
+        if (decode_smem(lut_bytes, stage_layout(kDecWarps * 16u * nu, kp_st, kn_st, vp_st, vn_st).stage_bytes) <= 227 * 1024) return nu;
+    return 0;
+}
+// The tile a plan's specialised kernel is compiled for: what its row strides let fit, or the wide one without them.
+// (Nibble rows of four and more bits only fit the narrow one: a layer step of 4 x 4100 tokens x 8 heads of them took
+// 34.3 us with the general kernel and takes 27.7 with the specialised one.)
+inline int decode_jit_nu(const DecPlanDev& pl) {
+    if (pl.row_st[0] <= 0) return 2;
+    const int nu = decode_nu(pl.lut_bytes, pl.row_st[0], pl.row_st[1], pl.row_st[2], pl.row_st[3]);
+    return nu ? nu : 2;
+}
+
 // Launch one instantiation; defined once per stored V width in its own translation unit.
 template <int VB>
 cudaError_t launch_decode(const DecParams& P, int nu, dim3 grid, size_t smem, cudaStream_t stream, bool programmatic) {

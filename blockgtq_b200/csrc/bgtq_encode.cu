@@ -290,7 +290,7 @@ __device__ __forceinline__ float rope_element(const __half* row, int dim, const 
     return __half2float(__hadd_rn(__hmul_rn(x, cs[dim]), __hmul_rn(xr, sn[dim])));
 }
 
-__global__ void __launch_bounds__(512) prep_kernel(const PrepParams P) {
+__global__ void __launch_bounds__(512, 2) prep_kernel(const PrepParams P) {
     __shared__ float xs[kHD];
     __shared__ float xn[kHD];
     __shared__ float part[4][kHD];
@@ -336,8 +336,35 @@ __global__ void __launch_bounds__(512) prep_kernel(const PrepParams P) {
     const int g_p = d.group_of[p];
     const float lut_off_p = d.lut_off[g_p], lut_inv_p = d.lut_inv[g_p];
     const int cent_off_p = d.seg_lut_off[g_p];
+    // ... and what the tail of a K row looks up: the segment that this warp sums, and which codes make byte p of the
+    // packed row: mode (0: none, 1: bit stream, 2: raw, 3: nibble pair) | width << 2 | first code << 5 | codes << 13 | byte of
+    // the stream << 21 (one register: two CTAs have to fit an SM)
+    const int n_seg = d.n_seg;
+    const int w_seg = warp < n_seg ? d.seg_start[warp & 7] | d.seg_len[warp & 7] << 8 : 0;
+    const bool mixed = E.flags & BGTQ_ENC_K_MIXED;
+    uint32_t byte_of = 0u;
+    if (kind == 1 && c == 0) {
+        if (mixed) {
+            const int nib = d.nopack_start / 2;
+            if (p < nib) byte_of = 3u | (uint32_t)(2 * p) << 5;
+            else if (p < nib + d.nopack_len) byte_of = 2u | (uint32_t)(d.nopack_start + (p - nib)) << 5;
+        } else {
+            for (int s = 0; s < n_seg; ++s) {
+                const int bw = d.seg_bw[s], len = d.seg_len[s], t = p - d.seg_pack_off[s];
+                if (t >= 0 && t < seg_storage_bytes(bw, len))
+                    byte_of = bw >= 5 ? 2u | (uint32_t)(d.seg_start[s] + t) << 5
+                                      : 1u | (uint32_t)bw << 2 | (uint32_t)d.seg_start[s] << 5 | (uint32_t)len << 13 | (uint32_t)t << 21;
+            }
+        }
+    }
     grid_launch_dependents();
     grid_dependency_wait();       // inputs and the slot position come from earlier work in the stream
+    // A plain append's input does not depend on the position: both are on their way before either is looked at.
+    const __half* cs = P.rope_cos ? P.rope_cos + b * P.rope_sb : nullptr;
+    const __half* sn = P.rope_cos ? P.rope_sin + b * P.rope_sb : nullptr;
+    float x_early = 0.f;
+    if (P.k_buf == nullptr && c == 0 && kind != 0)
+        x_early = kind == 1 ? rope_element(E.k + b * E.k_sb + h * E.k_sh, perm_p, cs, sn) : __half2float(E.v[b * E.v_sb + h * E.v_sh + p]);
     int t0 = E.pos_dev ? *E.pos_dev : E.t0;
     if (P.k_buf != nullptr && kind != 0) {
         // three-region mode: the step's token enters the sink (first n_sink tokens) or its ring slot, copied by
@@ -369,8 +396,6 @@ __global__ void __launch_bounds__(512) prep_kernel(const PrepParams P) {
         if (E.pos_dev && !enc_range_ok(E, t0, 1)) return;
     }
 
-    const __half* cs = P.rope_cos ? P.rope_cos + b * P.rope_sb : nullptr;
-    const __half* sn = P.rope_cos ? P.rope_sin + b * P.rope_sb : nullptr;
     if (kind == 0 && P.rot_group == 4) {
         __shared__ float xg[4][kHD];
         __shared__ float pg[4][4][kHD];
@@ -394,6 +419,7 @@ __global__ void __launch_bounds__(512) prep_kernel(const PrepParams P) {
     int g = 0;
     if (c == 0) {
         if (kind == 0) x = rope_element(P.q + b * P.q_sb + hq * P.q_sh, perm_p, cs, sn);
+        else if (P.k_buf == nullptr) x = x_early;
         else if (kind == 1) x = rope_element(k_src, perm_p, cs, sn);
         else x = __half2float(v_src[p]);
         xs[p] = x;
@@ -402,9 +428,9 @@ __global__ void __launch_bounds__(512) prep_kernel(const PrepParams P) {
     __syncthreads();
     float raw_v = 0.f;
     if (kind == 1) {            // group norms: warp s reduces segment s
-        if (warp < d.n_seg) {
+        if (warp < n_seg) {
             float acc = 0.f;
-            for (int i = d.seg_start[warp] + lane; i < d.seg_start[warp] + d.seg_len[warp]; i += 32) acc = fmaf(xs[i], xs[i], acc);
+            for (int i = (w_seg & 0xFF) + lane; i < (w_seg & 0xFF) + (w_seg >> 8); i += 32) acc = fmaf(xs[i], xs[i], acc);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
             if (lane == 0) gn[warp] = sqrtf(acc + 1e-30f);
@@ -438,7 +464,6 @@ __global__ void __launch_bounds__(512) prep_kernel(const PrepParams P) {
         return;
     }
     if (kind == 1) {
-        const bool mixed = E.flags & BGTQ_ENC_K_MIXED;
         float c2 = 0.f;
         if (c == 0) {
             float u = (y - lut_off_p) * lut_inv_p;
@@ -451,37 +476,29 @@ __global__ void __launch_bounds__(512) prep_kernel(const PrepParams P) {
             xs[p] = c2;
         }
         __syncthreads();
-        if (mixed && warp < d.n_seg) {
+        if (mixed && warp < n_seg) {
             float acc = 0.f;
-            for (int i = d.seg_start[warp] + lane; i < d.seg_start[warp] + d.seg_len[warp]; i += 32) acc += xs[i];
+            for (int i = (w_seg & 0xFF) + lane; i < (w_seg & 0xFF) + (w_seg >> 8); i += 32) acc += xs[i];
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
             if (lane == 0) gc[warp] = fmaxf(sqrtf(acc), 1e-10f);
         }
-        __syncthreads();
+        if (mixed) __syncthreads();
         if (c != 0) return;
         if (p < E.kn_count) {
-            float val = p < d.n_seg ? gn[p] : 0.f;
-            if (mixed && p < d.n_seg) val = val / gc[p];
+            float val = p < n_seg ? gn[p] : 0.f;
+            if (mixed && p < n_seg) val = val / gc[p];
             const size_t o = b * E.kn_sb + h * E.kn_sh + (size_t)t0 * E.kn_st + p;
             if (E.flags & BGTQ_ENC_K_NORMS_F16) static_cast<__half*>(E.kn)[o] = __float2half_rn(val);
             else static_cast<float*>(E.kn)[o] = val;
         }
         if (p < E.kp_row_bytes) {
             uint32_t byte = 0;
-            if (mixed) {
-                const int nib = d.nopack_start / 2;
-                if (p < nib) byte = (codes[2 * p] & 15u) | ((codes[2 * p + 1] & 15u) << 4);
-                else if (p < nib + d.nopack_len) byte = codes[d.nopack_start + (p - nib)];
-            } else {
-                for (int s = 0; s < d.n_seg; ++s) {
-                    const int bw = d.seg_bw[s], nb = seg_storage_bytes(bw, d.seg_len[s]);
-                    if (p >= d.seg_pack_off[s] && p < d.seg_pack_off[s] + nb) {
-                        const int st = p - d.seg_pack_off[s];
-                        byte = bw >= 5 ? codes[d.seg_start[s] + st] : pack_byte(&codes[d.seg_start[s]], d.seg_len[s], bw, st);
-                    }
-                }
-            }
+            const uint32_t mode = byte_of & 3u;
+            const uint8_t* cd = &codes[(byte_of >> 5) & 0xFFu];
+            if (mode == 1u) byte = pack_byte(cd, (int)(byte_of >> 13) & 0xFF, (int)(byte_of >> 2) & 7, (int)(byte_of >> 21));
+            else if (mode == 2u) byte = cd[0];
+            else if (mode == 3u) byte = (cd[0] & 15u) | ((cd[1] & 15u) << 4);
             E.kp[b * E.kp_sb + h * E.kp_sh + (size_t)t0 * E.kp_st + p] = (uint8_t)byte;
         }
         return;

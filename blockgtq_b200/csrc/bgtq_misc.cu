@@ -24,6 +24,7 @@ struct PublishArgs {
 // rows than SMs the CTAs queue up instead, so that variant reads the entries where it uses them and fits
 // three CTAs per SM, whose latency chains overlap.
 // ---------------------------------------------------------------------------
+constexpr int kCombineChunk = 256;
 template <bool kPrefetch>
 __global__ void __launch_bounds__(512, kPrefetch ? 1 : 3) combine_kernel(const float* part_o, const float* part_lse, int n_splits,
                                                        const float* v_rot, const float* buf_o, const float* buf_lse,
@@ -53,61 +54,57 @@ __global__ void __launch_bounds__(512, kPrefetch ? 1 : 3) combine_kernel(const f
     const float* po = rank_stride ? part_o + row * kHD + d : part_o + row * n_splits * kHD + d;
     const int64_t sl = rank_stride ? rank_stride : 1, so = rank_stride ? rank_stride : kHD;
     // The slot count only sets the granularity of the decode launch's work split: most slots hold no partial
-    // (LSE = -inf).  The block finds the maximum and the live slots together (each thread looks at one slot per
-    // 512), keeps them in slot order, and only then walks the live ones: no thread scans the whole row alone.
-    __shared__ float s_red[16];
-    __shared__ int s_cnt[16];
-    __shared__ int s_slot[512];
-    __shared__ float s_w[512];
+    // (LSE = -inf).  Every warp looks at all slots itself (eight per lane at most), lists the live ones in order in its own
+    // part of shared memory and walks its quarter's share of them: no barrier between the partials' LSEs and the partials,
+    // which this launch's latency consists of.
     const int warp = tid >> 5, lane = tid & 31;
-    float mx = -INFINITY;
-    for (int s = tid; s < n_splits; s += 512) mx = fmaxf(mx, lse[s * sl]);
+    __shared__ float2 s_list[16][kCombineChunk];          // (weight, slot)
+    float mx = -INFINITY, num = 0.f, den = 0.f;
+    for (int base = 0; base < n_splits; base += kCombineChunk) {       // (one chunk but for more than 256 slots)
+        float l[kCombineChunk / 32];
+        float top = mx;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) s_red[warp] = mx;
-    __syncthreads();
-    mx = s_red[0];
+        for (int i = 0; i < kCombineChunk / 32; ++i) {
+            const int s = base + 32 * i + lane;
+            l[i] = s < n_splits ? lse[s * sl] : -INFINITY;
+        }
 #pragma unroll
-    for (int i = 1; i < 16; ++i) mx = fmaxf(mx, s_red[i]);
-    float num = 0.f, den = 0.f;
-    if (mx > -INFINITY) {
-        for (int base = 0; base < n_splits; base += 512) {
-            const int s = base + tid;
-            const float l = s < n_splits ? lse[s * sl] : -INFINITY;
-            const bool live = l > -INFINITY;
+        for (int i = 0; i < kCombineChunk / 32; ++i) top = fmaxf(top, l[i]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        if (top == -INFINITY) continue;
+        if (mx > -INFINITY && top > mx) {
+            const float f = expf(mx - top);
+            num *= f;
+            den *= f;
+        }
+        mx = top;
+        int total = 0;
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < kCombineChunk / 32; ++i) {
+            const bool live = l[i] > -INFINITY;
             const unsigned bal = __ballot_sync(0xffffffffu, live);
-            __syncthreads();                               // the previous chunk's list has been consumed
-            if (lane == 0) s_cnt[warp] = __popc(bal);
-            __syncthreads();
-            int off = 0, total = 0;
+            if (live) s_list[warp][total + __popc(bal & ((1u << lane) - 1u))] = make_float2(expf(l[i] - mx), __int_as_float(base + 32 * i + lane));
+            total += __popc(bal);
+        }
+        __syncwarp();
+        // quarter c of the live slots, four of its partials requested before the first is used (a slot past the end
+        // contributes exact zeros)
+        for (int i0 = c; i0 < total; i0 += 16) {
+            float a[4], x[4];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int n = s_cnt[i];
-                off += i < warp ? n : 0;
-                total += n;
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + 4 * u;
+                const bool ok = i < total;
+                const float2 e = s_list[warp][ok ? i : i0];
+                a[u] = ok ? e.x : 0.f;
+                x[u] = ok ? po[(int64_t)__float_as_int(e.y) * so] : 0.f;
             }
-            if (live) {
-                const int pos = off + __popc(bal & ((1u << lane) - 1u));
-                s_slot[pos] = s;
-                s_w[pos] = expf(l - mx);
-            }
-            __syncthreads();
-            // quarter c of the live slots, four of its partials requested before the first is used (a slot past
-            // the end contributes exact zeros)
-            for (int i0 = c; i0 < total; i0 += 16) {
-                float a[4], x[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int i = i0 + 4 * u;
-                    const bool ok = i < total;
-                    a[u] = ok ? s_w[i] : 0.f;
-                    x[u] = ok ? po[(int64_t)s_slot[i] * so] : 0.f;
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    den += a[u];
-                    num = fmaf(a[u], x[u], num);
-                }
+            for (int u = 0; u < 4; ++u) {
+                den += a[u];
+                num = fmaf(a[u], x[u], num);
             }
         }
     }

@@ -348,9 +348,9 @@ class BlockGTQKVManager:
         """The constant arguments of layer ``li``'s step (every array of it lives as long as the manager)."""
         s = self._steps[li]
         baked = all(self.quantizers[li][h]._q_perm_baked for h in range(self.n_kv))
-        if s is not None and s.key == (baked, self.programmatic):
-            return s
         lt, pd = self._layers[li], self.programmatic
+        if s is not None and s.key == (lt, baked, pd):
+            return s
         kp, kn, vp, vn = self._k_packed[li], self._k_norms[li], self._v_packed[li], self._v_norms[li]
         plan = lt.plan(self._dec_flags | (_lib.DEC_PROGRAMMATIC if pd else 0))
         s = _lib.LayerStep(
@@ -370,7 +370,7 @@ class BlockGTQKVManager:
             kb, vb = self._k_buf[li], self._v_buf[li]
             s.k_buf, s.v_buf, s.kb_sb, s.kb_sh = kb.data_ptr(), vb.data_ptr(), kb.stride(0), kb.stride(1)
             s.buf_o, s.buf_lse, s.n_sink, s.window = self._buf_o.data_ptr(), self._buf_lse.data_ptr(), self.n_sink, self.recent_window
-        s.key, s.addr, s.n_launch = (baked, pd), C.addressof(s), 4 if self._buffered else 3
+        s.key, s.addr, s.n_launch = (lt, baked, pd), C.addressof(s), 4 if self._buffered else 3
         self._steps[li] = s
         return s
 
