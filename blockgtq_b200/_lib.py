@@ -8,6 +8,8 @@ stream provider.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 import torch
@@ -148,6 +150,7 @@ _SIGNATURES = {
 }
 
 _lib = None
+native = None         # the extension module of csrc/bgtq_native.cpp, once lib() has loaded it
 launches = 0          # kernels enqueued through this binding (read by the benchmark)
 
 
@@ -157,7 +160,7 @@ def exported_symbols():
 
 def lib():
     """Load (building first if the sources are newer) and type the library."""
-    global _lib
+    global _lib, native
     if _lib is not None:
         return _lib
     path = _build.LIB
@@ -174,8 +177,30 @@ def lib():
                            f"{C.sizeof(HeadDesc)}")
     if handle.bgtq_layer_step_size() != C.sizeof(LayerStep):
         raise RuntimeError("BgtqLayerStep size mismatch between the library and the binding")
+    loader = importlib.machinery.ExtensionFileLoader("_native", _build.NATIVE)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_native", loader))
+    loader.exec_module(module)
+    module.bind(*[C.cast(getattr(handle, name), C.c_void_p).value for name in (
+        "bgtq_layer_step", "bgtq_layer_encode", "bgtq_attend", "bgtq_decode_default_splits", "bgtq_encode", "bgtq_rotate_q_rows",
+        "bgtq_prefill", "bgtq_prefill_workspace_bytes")])
+    native = module
     _lib = handle
     return _lib
+
+
+def host():
+    """The extension module with the frequent calls; its functions return None for calls they leave to Python."""
+    if native is None:
+        lib()
+    return native
+
+
+def done(result, what: str, n: int = 1):
+    """Result of a :func:`host` call that was taken: raises for an error code, counts its launches."""
+    if type(result) is int and result != OK:
+        check(result, what)
+    count_launch(n)
+    return result
 
 
 def check(code: int, what: str):

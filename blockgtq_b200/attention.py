@@ -104,10 +104,9 @@ def fused_blockgtq_decode_attention(
         k_norms = k_norms.to(torch.float16)
     lt = _layer_for(segments, codebook_flat, v_lut, vb_codebook, n_kv, q.device)
     flags = (_lib.DEC_K_MIXED if k_nibble else 0) | (_lib.DEC_V_NIBBLE if v_nibble else 0)
-    out, _o32, lse = attend(lt, q.reshape(B, n_q, D), k_packed, k_norms, v_codes, v_norms, 0, T, rotate=False,
+    out, _o32, lse = attend(lt, q, k_packed, k_norms, v_codes, v_norms, 0, T, rotate=False,
                             n_splits=max(1, int(t_splits)), scale=scale, flags=flags, v_rot=_rotation(v_rotation, n_kv),
                             want_lse=return_lse)
-    out = out.unsqueeze(2)
     return (out, lse) if return_lse else out
 
 

@@ -3,6 +3,8 @@
 Compiles every ``csrc/*.cu`` for sm_100a with nvcc and links one shared
 library, ``blockgtq_b200/libbgtq.so``, exporting the C ABI of ``include/bgtq.h``.
 nvcc cross-compiles without a GPU.  The library links only the CUDA runtime.
+``csrc/bgtq_native.cpp``, the host side of the frequent calls, becomes the extension
+module ``blockgtq_b200/_native.so`` (g++ against torch and Python).
 """
 from __future__ import annotations
 
@@ -15,6 +17,8 @@ import sys
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.environ.get("BGTQ_LIB") or os.path.join(PKG, "libbgtq.so")
+NATIVE_SRC = os.path.join(CSRC, "bgtq_native.cpp")
+NATIVE = os.path.join(PKG, "_native.so")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "--use_fast_math=false", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
 
@@ -31,11 +35,14 @@ def sources() -> list:
 
 
 def needs_build() -> bool:
-    if not os.path.exists(LIB):
+    if not os.path.exists(LIB) or not os.path.exists(NATIVE):
+        return True
+    header = os.path.join(os.path.dirname(PKG), "include", "bgtq.h")
+    if os.path.getmtime(NATIVE) < max(os.path.getmtime(NATIVE_SRC), os.path.getmtime(header)):
         return True
     t = os.path.getmtime(LIB)
     deps = sources() + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(CSRC, "*.cuh")) + \
-        [os.path.join(os.path.dirname(PKG), "include", "bgtq.h")]
+        [header]
     return any(os.path.getmtime(d) > t for d in deps)
 
 
@@ -58,10 +65,26 @@ def _embed_jit_sources(objdir: str) -> str:
     return out
 
 
+def _native_cmd(out: str) -> list:
+    import sysconfig
+
+    import torch
+    base = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    cxx = os.environ.get("CXX") or shutil.which("g++") or "g++"
+    inc = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
+           os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    return [cxx, "-shared", "-fPIC", "-O2", "-std=c++17", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *[x for d in inc for x in ("-isystem", d)], NATIVE_SRC, "-o", out, "-L", os.path.join(base, "lib"),
+            "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not needs_build():
         return LIB
     nvcc = _nvcc()
+    native_cmd = _native_cmd(NATIVE + ".tmp")
+    native = subprocess.Popen(native_cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT)
     objdir = os.path.join(PKG, "build")
     os.makedirs(objdir, exist_ok=True)
     jit_inc = _embed_jit_sources(objdir)
@@ -86,6 +109,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if r.returncode != 0:
         raise RuntimeError("link failed: " + r.stdout.decode())
     os.replace(tmp, LIB)
+    out = native.communicate()[0].decode()
+    if native.returncode != 0:
+        raise RuntimeError("building the host extension failed: " + " ".join(native_cmd) + "\n" + out)
+    os.replace(NATIVE + ".tmp", NATIVE)
     return LIB
 
 

@@ -120,6 +120,7 @@ class LayerTables:
         self.max_ng = max(t.n_groups for t in k_tables)
         self.max_mixed_bytes = max(t.pack_meta["nopack_start"] // 2 + t.pack_meta["nopack_len"] for t in k_tables)
         self.head_perm = torch.stack([t.head_perm for t in k_tables]).long().to(self.device)   # (n_kv, 128)
+        self.addrs = (self.desc_dev.data_ptr(), self.rot_k.data_ptr(), self.rot_v.data_ptr())
         self._plans = {}
         self._partition = None
         self._row_strides = {}
@@ -180,6 +181,11 @@ def encode(layer: LayerTables, k, v, t0, k_packed, k_norms, v_packed, v_norms, *
     ``v_packed`` (B, n_kv, T, bytes) u8 and ``v_norms`` (B, n_kv, T) f16.  Either side may be None.
     Bulk row counts (>= 128 rows) run the tcgen05 / tensor-memory encoder; ``_lib.ENC_NO_TCGEN05`` in ``flags``
     (or the environment variable ``BGTQ_ENC_NO_TCGEN05``) keeps them on the warp-MMA one."""
+    if k_codes is None and v_codes is None and pos_dev is None and status is None and type(t0) is int:
+        r = _lib.host().encode(*layer.addrs, layer.n_kv, layer.vpb, k, v, t0, k_packed, k_norms, v_packed, v_norms, flags | _no_tcgen05())
+        if r is not None:
+            _lib.done(r, "bgtq_encode")
+            return
     ref = k if k is not None else v
     _lib.require_cuda(ref, "k/v")
     B, H, S, D = ref.shape
@@ -253,6 +259,9 @@ def rotate_q_bulk(layer: LayerTables, q: torch.Tensor) -> torch.Tensor:
     """Many positions at once: q (B, n_q, S, 128) -> same shape, fp16, in the packed-K basis (the per-row kernel
     behind :func:`rotate_q` is meant for the handful of rows of a decode step).  fp16 queries go through the
     tensor cores; queries of another type are rotated in fp32 first and rounded once."""
+    r = _lib.host().rotate_rows(layer.desc_dev.data_ptr(), layer.rot_k.data_ptr(), layer.n_kv, q)
+    if r is not None:
+        return _lib.done(r, "bgtq_rotate_q_rows")
     _lib.require_cuda(q, "q")
     B, n_q, S, D = q.shape
     if q.dtype == torch.float16:
@@ -392,34 +401,31 @@ def decode(layer: LayerTables, q_rot, k_packed, k_norms, v_packed, v_norms, t_be
 def attend(layer, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, *, rotate, n_splits=None, scale=None, flags=0,
            v_rot=None, buf_o=None, buf_lse=None, want_f32=False, want_lse=False, status=None):
     """Query rotation (``rotate``: q is in the original basis), split-KV decode over rows [t_begin, t_end) and combine
-    in one library call.  q (B, n_q, 128) fp16 -> (out fp16 (B, n_q, 128), f32 copy | None, LSE | None)."""
-    _lib.require_cuda(q, "q")
-    B, n_q, _ = q.shape
-    if k_norms.dtype != torch.float16 or v_norms.dtype != torch.float16:
-        raise TypeError("cache norms must be float16")
-    q_sb, q_sh, q_sd = q.stride()
-    if q.dtype != torch.float16 or q_sd != 1 or not (rotate or q.is_contiguous()):
-        q = q.to(torch.float16).contiguous()
-        q_sb, q_sh = n_q * HD, HD
-    if n_splits is None:
-        n_splits = default_splits(B, layer.n_kv, t_end - t_begin)
-    dev = q.device
-    scratch = torch.empty(B * n_q * (n_splits * (HD + 1) + HD // 2), dtype=torch.float32, device=dev)
-    out = torch.empty(B, n_q, HD, dtype=torch.float16, device=dev)
-    o32 = torch.empty(B, n_q, HD, dtype=torch.float32, device=dev) if want_f32 else None
-    lse = torch.empty(B, n_q, dtype=torch.float32, device=dev) if want_lse else None
-    _lib.check(_lib.lib().bgtq_attend(
-        C.addressof(layer.plan(flags | _lib.DEC_PROGRAMMATIC)), _lib.ptr(layer.desc_dev), _lib.ptr(layer.rot_k) if rotate else None,
-        q.data_ptr(), q_sb, q_sh,
-        k_packed.data_ptr(), *_strides3(k_packed), k_norms.data_ptr(), *_strides3(k_norms),
-        v_packed.data_ptr(), *_strides3(v_packed), v_norms.data_ptr(), *v_norms.stride(),
-        B, n_q, layer.n_kv, t_begin, t_end, n_splits, 1.0 / math.sqrt(HD) if scale is None else scale,
-        _lib.ptr(v_rot), _lib.ptr(buf_o), _lib.ptr(buf_lse), scratch.data_ptr(), out.data_ptr(), _lib.ptr(o32), _lib.ptr(lse),
-        _lib.ptr(status), _lib.stream_ptr(dev)), "bgtq_attend")
-    _lib.count_launch(3 if rotate else 2)
-    return out, o32, lse
+    in one library call.  q (B, n_q, [1,] 128) -> (out fp16 of q's shape, f32 copy (B, n_q, 128) | None, LSE | None)."""
+    plan, ptr = layer.plan(flags | _lib.DEC_PROGRAMMATIC), _lib.ptr
+
+    def call():
+        return _lib.host().attend(
+            C.addressof(plan), ptr(layer.desc_dev), ptr(layer.rot_k) if rotate else None, q, k_packed, k_norms, v_packed, v_norms,
+            t_begin, t_end, n_splits or 0, _SCALE if scale is None else scale, None if v_rot is None else ptr(v_rot), buf_o, buf_lse,
+            want_f32, want_lse, None if status is None else ptr(status), layer.n_kv)
+
+    r = call()
+    if r is None:           # another type or layout, or an argument to complain about
+        _lib.require_cuda(q, "q")
+        if k_norms.dtype != torch.float16 or v_norms.dtype != torch.float16:
+            raise TypeError("cache norms must be float16")
+        for t in (k_packed, k_norms, v_packed):
+            _strides3(t)
+        with torch.cuda.device(q.device):
+            q = q.to(torch.float16).contiguous()
+            r = call()
+        if r is None:
+            raise ValueError("query, cache and layer do not match")
+    return _lib.done(r, "bgtq_attend", 3 if rotate else 2)
 
 
+_SCALE = 1.0 / math.sqrt(HD)
 _PREFILL_WORKSPACE = 2 << 30        # bytes of dequantised operand tiles per launch
 
 
@@ -430,9 +436,15 @@ def prefill_attention(layer: LayerTables, q_rot, k_packed, k_norms, v_packed, v_
     ``v_rot`` (n_kv, 128, 128) fp32 = R finishes V's rotation.
     Returns (B, n_q, S_q, 128) fp16.  ``_lib.PF_NO_TCGEN05`` in ``flags`` (or the environment variable
     ``BGTQ_PF_NO_TCGEN05``) keeps the products on mma.sync instead of tcgen05 / tensor memory."""
-    _lib.require_cuda(q_rot, "q_rot")
     if os.environ.get("BGTQ_PF_NO_TCGEN05"):
         flags |= _lib.PF_NO_TCGEN05
+    if not flags & _lib.PF_NO_TCGEN05:
+        r = _lib.host().prefill(layer.desc_dev.data_ptr(), layer.n_kv, q_rot, k_packed, k_norms, v_packed, v_norms, int(n_tokens),
+                                int(q_pos_offset), bool(causal), _SCALE if scale is None else scale, int(flags),
+                                None if v_rot is None else v_rot.data_ptr(), _PREFILL_WORKSPACE)
+        if r is not None:
+            return _lib.done(r, "bgtq_prefill", 2)
+    _lib.require_cuda(q_rot, "q_rot")
     B, n_q, S_q, D = q_rot.shape
     if D != HD or q_rot.dtype != torch.float16 or q_rot.stride(3) != 1:
         raise ValueError("q_rot must be float16 (B, n_q, S_q, 128) with contiguous rows")

@@ -165,6 +165,7 @@ class BlockGTQKVManager:
         self._g_out = torch.zeros(self.n_layers, self.B, self.n_q, self.hd, dtype=torch.float16, device=dev)
         self._g_out4 = list(self._g_out.unsqueeze(3).unbind(0))      # per layer (B, n_q, 1, hd)
         self._pos = torch.zeros(1, dtype=torch.int32, device=dev)
+        self._dev_index = self._pos.get_device()
         self._g_rope = torch.zeros(2, self.B, self.hd, dtype=torch.float16, device=dev)     # cos, sin of the step
         self._buf_o = torch.zeros(self.B, self.n_q, self.hd, dtype=torch.float32, device=dev)
         self._buf_lse = torch.zeros(self.B, self.n_q, dtype=torch.float32, device=dev)
@@ -200,14 +201,12 @@ class BlockGTQKVManager:
         if v.dtype != torch.float16:
             v = v.to(torch.float16)
         _lib.require_cuda(k, "k/v")
-        ks, vs = k.stride(), v.stride()
-        if k.shape != (self.B, self.n_kv, n, self.hd) or v.shape != k.shape or ks[3] != 1 or vs[3] != 1 or t_end > self.max_T:
+        r = _lib.host().layer_encode(self._step_args(layer_idx).addr, self._dev_index, k, v, int(t_start), _no_tcgen05())
+        if r is None:
             li = layer_idx          # (another batch size, or an error to report)
             return encode(self._layers[li], k, v, t_start, self._k_packed[li], self._k_norms[li], self._v_packed[li],
                           self._v_norms[li], flags=self._enc_flags)
-        _lib.check(_lib.lib().bgtq_layer_encode(self._step_args(layer_idx).addr, k.data_ptr(), *ks[:3], v.data_ptr(), *vs[:3], n,
-                                                int(t_start), _no_tcgen05(), _lib.stream_ptr(k.device)), "bgtq_layer_encode")
-        _lib.count_launch()
+        _lib.done(r, "bgtq_layer_encode")
 
     def init_from_cache(self, past_key_value):
         """Bulk-encode an HF cache after prefill (packed_kv_manager.py:259-266).  Accepts the
@@ -446,21 +445,18 @@ class BlockGTQKVManager:
         self._sync_pos()
         if self._exchange is not None:
             return self._replay_layer(li, q, k_new, v_new, rope)
-        f16, B, hd = torch.float16, self.B, self.hd
-        if (q.dtype != f16 or k_new.dtype != f16 or v_new.dtype != f16 or q.shape != (B, self.n_q, 1, hd)
-                or k_new.shape != (B, self.n_kv, 1, hd) or v_new.shape != k_new.shape or q.stride(3) != 1 or k_new.stride(3) != 1
-                or v_new.stride(3) != 1 or k_new.device != self._pos.device or v_new.device != self._pos.device):
+        s = self._step_args(li)
+        cos, sin = (None, None) if rope is None else rope
+        r = _lib.host().layer_step(s.addr, self._dev_index, q, k_new, v_new, cos, sin)
+        if r is None:               # inputs of another type or layout go through the static buffers
+            if s.flags & _lib.STEP_Q_ROTATED:
+                q = q.contiguous()
             q, k_new, v_new = self._stage(li, q, k_new, v_new)
-        if rope is not None:
-            cos, sin = rope
-            if (cos.dtype == f16 and sin.dtype == f16 and cos.numel() == B * hd and cos.stride(-1) == 1 and sin.stride(-1) == 1
-                    and cos.shape[0] == B and sin.shape == cos.shape and sin.stride(0) == cos.stride(0)):
-                rope = (cos, sin)
-            else:
-                rope = self._stage_rope(cos, sin)
-        elif self._step_args(li).flags & _lib.STEP_Q_ROTATED and not q.is_contiguous():
-            q, k_new, v_new = self._stage(li, q.contiguous(), k_new, v_new)
-        self._launch_step(li, q, k_new, v_new, rope)
+            if rope is not None:
+                cos, sin = self._stage_rope(cos, sin)
+            self._launch_step(li, q, k_new, v_new, None if rope is None else (cos, sin))
+        else:
+            _lib.done(r, "bgtq_layer_step", s.n_launch)
         return self._g_out4[li]
 
     @torch.no_grad()

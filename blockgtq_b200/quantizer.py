@@ -13,7 +13,7 @@ from typing import Optional
 import torch
 
 from . import _lib, calib
-from .layer import LayerTables, _encode_rows, encode as _encode
+from .layer import LayerTables, _encode_rows, _no_tcgen05, encode as _encode
 
 HD = _lib.HD
 
@@ -357,6 +357,9 @@ def _rows3(x: torch.Tensor):
 def _compress_k(k_flat, args, row_bytes: int, flags: int):
     """One launch over all heads: (packed (n_kv, N, row_bytes) u8, norms (n_kv, N, max_ng) f32)."""
     lt = args["_layer"]
+    r = _lib.host().compress(lt.addrs[0], lt.addrs[1], lt.n_kv, k_flat, row_bytes, lt.max_ng, flags | _no_tcgen05())
+    if r is not None:
+        return _lib.done(r, "bgtq_encode")
     k = _rows3(k_flat)
     n_kv, n, _ = k.shape
     if n_kv != lt.n_kv:
@@ -370,6 +373,9 @@ def _compress_k(k_flat, args, row_bytes: int, flags: int):
 
 def _compress_v(v_flat, args, row_bytes: int, flags: int):
     lt = args["_layer"]
+    r = _lib.host().compress(lt.addrs[0], lt.addrs[2], lt.n_kv, v_flat, row_bytes, 0, flags | _no_tcgen05())
+    if r is not None:
+        return _lib.done(r, "bgtq_encode")
     v = _rows3(v_flat)
     n_kv, n, _ = v.shape
     if n_kv != lt.n_kv:
