@@ -78,7 +78,7 @@ static int decode_impl(
               al16(P.kp, P.kp_sb, P.kp_sh, P.kp_st) && al16(P.kn, P.kn_sb, P.kn_sh, P.kn_st) &&
               al16(P.vp, P.vp_sb, P.vp_sh, P.vp_st) && al16(P.vn, P.vn_sb, P.vn_sh, P.vn_st);
     }
-    if (jit) e = launch_decode_jit(P, grid, smem, st, pdl);
+    if (jit) e = launch_decode_jit(P, grid, smem + decode_jit_quad_bytes(P.plan), st, pdl);
     else switch (P.plan.v_sbits) {
         case 1: e = launch_decode_vb1(P, nu, grid, smem, st, pdl); break;
         case 2: e = launch_decode_vb2(P, nu, grid, smem, st, pdl); break;

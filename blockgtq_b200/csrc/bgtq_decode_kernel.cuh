@@ -65,6 +65,7 @@ constexpr uint32_t kOffStagesMin = kOffMisc + kLutAlign;     // + lut_bytes = P.
 static_assert(kOffMisc % 128 == 0, "layout");
 // two regions the tree merge alternates between: 8 slots (first level) and 4 (second); later levels fit in them
 constexpr uint32_t kMergeBytes = (kDecWarps / 2 + kDecWarps / 4) * kMergeSlot * 16;
+constexpr uint32_t kQuadBytes = 256u * 16u * 8u;      // V quad table of the specialised kernel
 #define BGTQ_INF __int_as_float(0x7f800000)
 
 struct DecParams {
@@ -317,6 +318,24 @@ __device__ __forceinline__ uint32_t field_to(uint32_t x, uint32_t to, uint32_t p
     return pos < to ? x << (to - pos) : x >> (pos - to);
 }
 // PW = index of the 32-bit word of the token's norm row that `nw` holds (norms 2 PW and 2 PW + 1), -1: none yet.
+// V quad table of the specialised kernel: two dims of two tokens, 2-bit codes -> two fp16x2 in one 64-bit lookup, where its
+// 32 KB fit besides the stages.  256 entries, 16 replicas (lane mod 16: a half-warp's lookups never collide), made from the
+// pair table of the image when a head's tables arrive.  Half the shifts, masks and loads of the pair table at the same
+// shared-memory wavefronts: the loop is bound by its instructions and their latencies (32 x 16384 tokens x 8 heads, K2V2,
+// a layer step: 228.9 -> 219.1 us; 131072 tokens of one sequence 63.0 -> 60.3).  It needs no alignment: its offset is the
+// load's immediate.  (The same for 2-bit K segments took 8 x 32768 tokens from 39.9 to 41.0 us: not done.)
+constexpr bool kQuadV = BGTQ_JIT_QUAD_V;
+constexpr uint32_t kQuadOff = BGTQ_JIT_QUAD_OFF;
+// `pairs`: absolute shared address of the pair table, entries 1 << esh apart; thread t of 512 writes eight replicas of
+// entry t / 2 = codes of token A (2 dims), then token B.
+__device__ __forceinline__ void make_v_quads(uint8_t* smem, uint32_t pairs, uint32_t esh) {
+    const uint32_t e = threadIdx.x >> 1;
+    const uint32_t w0 = ld32(smem, pairs + (((e & 3u) | ((e >> 4) & 3u) << 2) << esh));
+    const uint32_t w1 = ld32(smem, pairs + ((((e >> 2) & 3u) | (e >> 6) << 2) << esh));
+    uint4* const to = reinterpret_cast<uint4*>(smem + kQuadOff + e * 128u + (threadIdx.x & 1u) * 64u);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) to[r] = make_uint4(w0, w1, w0, w1);
+}
 template <class HeadT, int SG, int NU, int PW>
 __device__ __forceinline__ void k_segment_c(float (&S)[NU][4], const uint8_t* sm, const KLane& kl, uint32_t (&nw)[2 * NU]) {
     constexpr jit::SegC c = HeadT::seg[SG];
@@ -512,6 +531,13 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
         if (!mbar_wait_bounded(lutbar, lut_uses & 1u)) ok = false;
         ++lut_uses;
     };
+    // the head's tables have landed; the quad table made from them (the caller's next barrier publishes it)
+    auto tables_ready = [&](const DecHeadPlan& hp) {
+        wait_tables();
+#ifdef BGTQ_JIT
+        if (kQuadV) make_v_quads(smem, lut_abs + hp.v_tbl, VCfg<VB>::REP_SHIFT + 2);
+#endif
+    };
     const int n_cta = (int)gridDim.x, cta = (int)blockIdx.x;
     load_tables(min(P.n_kv - 1, (int)(((int64_t)cta * P.n_kv) / n_cta)));   // the head this CTA most likely starts in
     bool tables_pending = true;
@@ -638,6 +664,10 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
             if (warp == 0)
                 for (int it = first; it < held; ++it) issue_tile(R, it, g_it + it);
             if (!dep_waited) {
+                if (tables_pending) {       // (behind the preceding launch)
+                    tables_ready(hp);
+                    tables_pending = false;
+                }
                 grid_dependency_wait();
                 dep_waited = true;
                 if (warp == 0)
@@ -658,7 +688,7 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
             qfrag[s * 32 + lane] = v;
         }
         if (tables_pending) {
-            wait_tables();
+            tables_ready(hp);
             tables_pending = false;
         }
         __syncthreads();
@@ -790,6 +820,22 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
                     load_v16<VB, kWordRowsV>(sm, base, bit + 72u * vp_st, gD);
 #pragma unroll
                     for (int g = 0; g < (int)G; ++g) {
+#ifdef BGTQ_JIT
+                        if constexpr (kQuadV) {     // byte i of z: dims 4 i + {0, 1} (even k-tiles) / + {2, 3} (odd) of both tokens
+                            constexpr uint32_t L = 0x0F0F0F0Fu;
+                            const uint32_t zab[2] = {(gA[g] & L) | ((gB[g] & L) << 4), ((gA[g] >> 4) & L) | (gB[g] & ~L)};
+                            const uint32_t zcd[2] = {(gC[g] & L) | ((gD[g] & L) << 4), ((gC[g] >> 4) & L) | (gD[g] & ~L)};
+                            const uint32_t rep8 = ((uint32_t)lane & 15u) << 3;
+#pragma unroll
+                            for (int k = 0; k < PER; ++k) {
+                                const uint2 ab = *reinterpret_cast<const uint2*>(sm + kQuadOff + ((field_to(zab[k & 1], 7, 8 * (k >> 1)) & 0x7F80u) | rep8));
+                                const uint2 cd = *reinterpret_cast<const uint2*>(sm + kQuadOff + ((field_to(zcd[k & 1], 7, 8 * (k >> 1)) & 0x7F80u) | rep8));
+                                const uint32_t a[4] = {ab.x, ab.y, cd.x, cd.y};
+                                mma_16816(O[g * PER + k], a, pf[u]);
+                            }
+                            continue;
+                        }
+#endif
                         const uint32_t xab = (gA[g] & M) | ((gB[g] & M) << VB), yab = ((gA[g] >> VB) & M) | (gB[g] & (M << VB));
                         const uint32_t xcd = (gC[g] & M) | ((gD[g] & M) << VB), ycd = ((gC[g] >> VB) & M) | (gD[g] & (M << VB));
 #pragma unroll
@@ -975,6 +1021,13 @@ inline int decode_jit_nu(const DecPlanDev& pl) {
     if (pl.row_st[0] <= 0) return 2;
     const int nu = decode_nu(pl.lut_bytes, pl.row_st[0], pl.row_st[1], pl.row_st[2], pl.row_st[3]);
     return nu ? nu : 2;
+}
+
+// Bytes of the V quad table of a plan's specialised kernel: for 2-bit V, where it fits besides the wide tile's stages.
+inline uint32_t decode_jit_quad_bytes(const DecPlanDev& pl) {
+    if (pl.v_sbits != 2 || pl.row_st[0] <= 0 || decode_jit_nu(pl) != 2) return 0;
+    const uint32_t stage = stage_layout(kDecWarps * 32u, pl.row_st[0], pl.row_st[1], pl.row_st[2], pl.row_st[3]).stage_bytes;
+    return decode_smem(pl.lut_bytes, stage) + kQuadBytes <= 227 * 1024 ? kQuadBytes : 0u;
 }
 
 // Launch one instantiation; defined once per stored V width in its own translation unit.

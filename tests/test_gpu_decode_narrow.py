@@ -24,3 +24,23 @@ def test_specialised_narrow_tile_matches_general(T):
     go, gl = decode(lt, q, *cache, 0, T, n_splits=5, flags=mgr._dec_flags | _lib.DEC_GENERIC)
     live = torch.isfinite(gl)
     assert live.any() and torch.equal(pl, gl) and torch.equal(po[live], go[live])
+
+
+@pytest.mark.parametrize("T", [1, 31, 512, 513, 3000])
+def test_specialised_2bit_values_match_general(T):
+    """2-bit values: the specialised kernel's 64-bit lookups (two dims of two tokens) against the general kernel's pairs."""
+    from blockgtq_b200 import BlockGTQKVManager, _lib
+    from blockgtq_b200.layer import decode
+    from helpers import HD, synth_head
+    gen = torch.Generator().manual_seed(T)
+    B, n_kv, gqa = 2, 3, 4
+    mgr = BlockGTQKVManager(1, n_kv * gqa, n_kv, HD, max_seq_len=3008, batch_size=B, k_avg_bits=2.0, v_bits=2, device=DEV)
+    cal = [synth_head(gen, 256, gqa) for _ in range(n_kv)]
+    mgr.calibrate(0, torch.stack([c[0] for c in cal]).float(), torch.stack([c[1] for c in cal]).float())
+    mgr.init_from_cache([tuple(torch.randn(B, n_kv, T, HD, generator=gen).half().to(DEV) for _ in range(2))])
+    q = torch.randn(B, n_kv * gqa, HD, generator=gen).half().to(DEV)
+    lt, cache = mgr._layers[0], (mgr._k_packed[0], mgr._k_norms[0], mgr._v_packed[0], mgr._v_norms[0])
+    po, pl = decode(lt, q, *cache, 0, T, n_splits=3, flags=mgr._dec_flags)
+    go, gl = decode(lt, q, *cache, 0, T, n_splits=3, flags=mgr._dec_flags | _lib.DEC_GENERIC)
+    live = torch.isfinite(gl)
+    assert live.any() and torch.equal(pl, gl) and torch.equal(po[live], go[live])
