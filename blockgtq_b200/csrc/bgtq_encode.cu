@@ -263,6 +263,10 @@ __global__ void __launch_bounds__(128) encode_kernel(const EncParams P) {
 // query heads of one KV head: quarter c of the CTA fetches row c, every thread applies its 32 rotation entries
 // to all four rows, and quarter c adds up and stores row c.  Same sums in the same order as one row per CTA,
 // a quarter of the rotation reads and of the CTAs.
+// kFourRows (more CTAs than fit the GPU at once, batch a multiple of four): a K or V item is the rows of four consecutive
+// batch entries of one KV head, quarter c taking row c in the same way: 32 sequences x (32 query, 8 KV) heads are 384 CTAs
+// instead of 768, and 25 MB of rotations read instead of 50.  (A kernel of its own: its registers cost the one-row form
+// half a microsecond.)
 // ---------------------------------------------------------------------------
 struct PrepParams {
     EncParams e;            // n_tok == 1
@@ -290,6 +294,37 @@ __device__ __forceinline__ float rope_element(const __half* row, int dim, const 
     return __half2float(__hadd_rn(__hmul_rn(x, cs[dim]), __hmul_rn(xr, sn[dim])));
 }
 
+// Thread p of 128: norm p and byte p of an appended K row (`byte_of`: see prep_kernel), the norm and byte p of a V row.
+__device__ __forceinline__ void prep_store_k(const EncParams& E, int b, int h, int t0, int p, int n_seg, bool mixed, const float* gn,
+                                             const float* gc, const uint8_t* codes, uint32_t byte_of) {
+    if (p < E.kn_count) {
+        float val = p < n_seg ? gn[p] : 0.f;
+        if (mixed && p < n_seg) val = val / gc[p];
+        const size_t o = b * E.kn_sb + h * E.kn_sh + (size_t)t0 * E.kn_st + p;
+        if (E.flags & BGTQ_ENC_K_NORMS_F16) static_cast<__half*>(E.kn)[o] = __float2half_rn(val);
+        else static_cast<float*>(E.kn)[o] = val;
+    }
+    if (p < E.kp_row_bytes) {
+        uint32_t byte = 0;
+        const uint32_t mode = byte_of & 3u;
+        const uint8_t* cd = &codes[(byte_of >> 5) & 0xFFu];
+        if (mode == 1u) byte = pack_byte(cd, (int)(byte_of >> 13) & 0xFF, (int)(byte_of >> 2) & 7, (int)(byte_of >> 21));
+        else if (mode == 2u) byte = cd[0];
+        else if (mode == 3u) byte = (cd[0] & 15u) | ((cd[1] & 15u) << 4);
+        E.kp[b * E.kp_sb + h * E.kp_sh + (size_t)t0 * E.kp_st + p] = (uint8_t)byte;
+    }
+}
+__device__ __forceinline__ void prep_store_v(const EncParams& E, int b, int h, int t0, int p, float raw, const float* c2,
+                                             const uint8_t* codes, int vb) {
+    if (p == 0) {
+        const float cnorm = sqrtf(c2[0] + c2[1] + c2[2] + c2[3] + 1e-20f);
+        E.vn[b * E.vn_sb + h * E.vn_sh + (size_t)t0 * E.vn_st] = __float2half_rn(raw / (cnorm > 1e-10f ? cnorm : 1.0f));
+    }
+    if (p < seg_storage_bytes(vb, kHD))
+        E.vp[b * E.vp_sb + h * E.vp_sh + (size_t)t0 * E.vp_st + p] = (uint8_t)pack_byte(codes, kHD, vb, p);
+}
+
+template <bool kFourRows>
 __global__ void __launch_bounds__(512, 2) prep_kernel(const PrepParams P) {
     __shared__ float xs[kHD];
     __shared__ float xn[kHD];
@@ -301,7 +336,7 @@ __global__ void __launch_bounds__(512, 2) prep_kernel(const PrepParams P) {
     const EncParams& E = P.e;
     const int tid = threadIdx.x, p = tid & 127, c = tid >> 7, warp = tid >> 5, lane = tid & 31;
     const int n_rot = P.do_rot ? E.n_batch * P.n_q / P.rot_group : 0;
-    const int n_rows = E.n_batch * E.n_kv;
+    const int n_rows = E.n_batch * E.n_kv / (kFourRows ? 4 : 1);      // K (V) items
     int item = blockIdx.x, kind;   // 0 rotate, 1 K, 2 V
     int b, h, hq = 0;
     bool skip = false;
@@ -312,7 +347,8 @@ __global__ void __launch_bounds__(512, 2) prep_kernel(const PrepParams P) {
         item -= n_rot;
         kind = 1 + item / n_rows;
         item %= n_rows;
-        b = item / E.n_kv; h = item % E.n_kv;
+        b = item / E.n_kv; h = item - b * E.n_kv;
+        if (kFourRows) b = 4 * b + c;
         skip = (kind == 1 && (E.flags & BGTQ_ENC_SKIP_K)) || (kind == 2 && (E.flags & BGTQ_ENC_SKIP_V));
         if (skip && P.k_buf == nullptr) return;
     }
@@ -343,7 +379,7 @@ __global__ void __launch_bounds__(512, 2) prep_kernel(const PrepParams P) {
     const int w_seg = warp < n_seg ? d.seg_start[warp & 7] | d.seg_len[warp & 7] << 8 : 0;
     const bool mixed = E.flags & BGTQ_ENC_K_MIXED;
     uint32_t byte_of = 0u;
-    if (kind == 1 && c == 0) {
+    if (kind == 1 && (c == 0 || kFourRows)) {
         if (mixed) {
             const int nib = d.nopack_start / 2;
             if (p < nib) byte_of = 3u | (uint32_t)(2 * p) << 5;
@@ -363,13 +399,14 @@ __global__ void __launch_bounds__(512, 2) prep_kernel(const PrepParams P) {
     const __half* cs = P.rope_cos ? P.rope_cos + b * P.rope_sb : nullptr;
     const __half* sn = P.rope_cos ? P.rope_sin + b * P.rope_sb : nullptr;
     float x_early = 0.f;
-    if (P.k_buf == nullptr && c == 0 && kind != 0)
+    if (P.k_buf == nullptr && (c == 0 || kFourRows) && kind != 0)
         x_early = kind == 1 ? rope_element(E.k + b * E.k_sb + h * E.k_sh, perm_p, cs, sn) : __half2float(E.v[b * E.v_sb + h * E.v_sh + p]);
     int t0 = E.pos_dev ? *E.pos_dev : E.t0;
     if (P.k_buf != nullptr && kind != 0) {
         // three-region mode: the step's token enters the sink (first n_sink tokens) or its ring slot, copied by
-        // the last quarter of the CTA; the token this CTA encodes below sits in another slot of the ring
-        if (c == 3) {
+        // the last quarter of the CTA (four rows: each quarter its own); the token this CTA encodes below sits in another
+        // slot of the ring
+        if (c == 3 || kFourRows) {
             const int ring = P.window + 1;
             const int slot = t0 < P.n_sink ? t0 : P.n_sink + (t0 - P.n_sink) % ring;
             const __half* src = kind == 1 ? E.k + b * E.k_sb + h * E.k_sh : E.v + b * E.v_sb + h * E.v_sh;
@@ -413,6 +450,90 @@ __global__ void __launch_bounds__(512, 2) prep_kernel(const PrepParams P) {
         __syncthreads();
         const float yq = (pg[c][0][p] + pg[c][1][p]) + (pg[c][2][p] + pg[c][3][p]);
         P.q_rot[((size_t)b * P.n_q + hq + c) * kHD + p] = __float2half_rn(yq);
+        return;
+    }
+    if (kFourRows && kind != 0) {        // quarter c: the row of batch entry b; the sums of the one-row form in its order
+        __shared__ float xg[4][kHD];
+        __shared__ float pg[4][4][kHD];
+        __shared__ float gn4[4][BGTQ_MAX_SEGMENTS], gc4[4][BGTQ_MAX_SEGMENTS];
+        __shared__ uint8_t codes4[4][kHD];
+        const int w4 = warp & 3;
+        const float x4 = P.k_buf == nullptr ? x_early : kind == 1 ? rope_element(k_src, perm_p, cs, sn) : __half2float(v_src[p]);
+        xg[c][p] = x4;
+        __syncthreads();
+        if (kind == 1) {
+            for (int s = w4; s < n_seg; s += 4) {
+                float acc = 0.f;
+                const int st = d.seg_start[s], en = st + d.seg_len[s];
+                for (int i = st + lane; i < en; i += 32) acc = fmaf(xg[c][i], xg[c][i], acc);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                if (lane == 0) gn4[c][s] = sqrtf(acc + 1e-30f);
+            }
+        } else {
+            float acc = x4 * x4;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (lane == 0) gn4[c][w4] = acc;
+        }
+        __syncthreads();
+        float raw = 0.f;
+        if (kind == 1) {
+            const float nr = gn4[c][g_p];
+            xg[c][p] = x4 / (nr > 1e-10f ? nr : 1.0f);
+        } else {
+            raw = sqrtf(gn4[c][0] + gn4[c][1] + gn4[c][2] + gn4[c][3] + 1e-30f);
+            xg[c][p] = x4 / (raw > 1e-8f ? raw : 1.0f);
+        }
+        __syncthreads();
+        {
+            float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+                a0 = fmaf(xg[0][32 * c + i], w[i], a0);
+                a1 = fmaf(xg[1][32 * c + i], w[i], a1);
+                a2 = fmaf(xg[2][32 * c + i], w[i], a2);
+                a3 = fmaf(xg[3][32 * c + i], w[i], a3);
+            }
+            pg[0][c][p] = a0; pg[1][c][p] = a1; pg[2][c][p] = a2; pg[3][c][p] = a3;
+        }
+        __syncthreads();
+        const float y4 = (pg[c][0][p] + pg[c][1][p]) + (pg[c][2][p] + pg[c][3][p]);
+        if (kind == 1) {
+            float u = (y4 - lut_off_p) * lut_inv_p;
+            u = fminf(fmaxf(u, 0.f), 255.f);
+            const uint8_t cd = s_lut[g_p][(int)u];
+            codes4[c][p] = cd;
+            const float cv = s_cent[cent_off_p + cd];
+            xg[c][p] = cv * cv;
+            if (E.k_codes) E.k_codes[((size_t)b * E.n_kv + h) * kHD + p] = cd;
+            __syncthreads();
+            if (mixed) {
+                for (int s = w4; s < n_seg; s += 4) {
+                    float acc = 0.f;
+                    const int st = d.seg_start[s], en = st + d.seg_len[s];
+                    for (int i = st + lane; i < en; i += 32) acc += xg[c][i];
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                    if (lane == 0) gc4[c][s] = fmaxf(sqrtf(acc), 1e-10f);
+                }
+                __syncthreads();
+            }
+            prep_store_k(E, b, h, t0, p, n_seg, mixed, gn4[c], gc4[c], codes4[c], byte_of);
+        } else {
+            const int nb = (1 << d.v_bits) - 1;
+            int cd = 0;
+            for (int i = 0; i < nb; ++i) cd += y4 > s_vb[i] ? 1 : 0;
+            codes4[c][p] = (uint8_t)cd;
+            if (E.v_codes) E.v_codes[((size_t)b * E.n_kv + h) * kHD + p] = (uint8_t)cd;
+            const float cv = s_vc[cd];
+            float c2 = cv * cv;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) c2 += __shfl_xor_sync(0xffffffffu, c2, o);
+            if (lane == 0) gc4[c][w4] = c2;
+            __syncthreads();
+            prep_store_v(E, b, h, t0, p, raw, gc4[c], codes4[c], (E.flags & BGTQ_ENC_V_NIBBLE) ? 4 : d.v_bits);
+        }
         return;
     }
     float x = 0.f;
@@ -459,7 +580,7 @@ __global__ void __launch_bounds__(512, 2) prep_kernel(const PrepParams P) {
     __syncthreads();
     if (c != 0 && kind != 2) { if (kind == 0) return; }
     const float y = (part[0][p] + part[1][p]) + (part[2][p] + part[3][p]);
-    if (kind == 0) {
+    if (kFourRows || kind == 0) {
         if (c == 0) P.q_rot[((size_t)b * P.n_q + hq) * kHD + p] = __float2half_rn(y);
         return;
     }
@@ -485,22 +606,7 @@ __global__ void __launch_bounds__(512, 2) prep_kernel(const PrepParams P) {
         }
         if (mixed) __syncthreads();
         if (c != 0) return;
-        if (p < E.kn_count) {
-            float val = p < n_seg ? gn[p] : 0.f;
-            if (mixed && p < n_seg) val = val / gc[p];
-            const size_t o = b * E.kn_sb + h * E.kn_sh + (size_t)t0 * E.kn_st + p;
-            if (E.flags & BGTQ_ENC_K_NORMS_F16) static_cast<__half*>(E.kn)[o] = __float2half_rn(val);
-            else static_cast<float*>(E.kn)[o] = val;
-        }
-        if (p < E.kp_row_bytes) {
-            uint32_t byte = 0;
-            const uint32_t mode = byte_of & 3u;
-            const uint8_t* cd = &codes[(byte_of >> 5) & 0xFFu];
-            if (mode == 1u) byte = pack_byte(cd, (int)(byte_of >> 13) & 0xFF, (int)(byte_of >> 2) & 7, (int)(byte_of >> 21));
-            else if (mode == 2u) byte = cd[0];
-            else if (mode == 3u) byte = (cd[0] & 15u) | ((cd[1] & 15u) << 4);
-            E.kp[b * E.kp_sb + h * E.kp_sh + (size_t)t0 * E.kp_st + p] = (uint8_t)byte;
-        }
+        prep_store_k(E, b, h, t0, p, n_seg, mixed, gn, gc, codes, byte_of);
         return;
     }
     // ---- V ----
@@ -519,13 +625,7 @@ __global__ void __launch_bounds__(512, 2) prep_kernel(const PrepParams P) {
     }
     __syncthreads();
     if (c != 0) return;
-    if (p == 0) {
-        const float cnorm = sqrtf(gn[0] + gn[1] + gn[2] + gn[3] + 1e-20f);
-        E.vn[b * E.vn_sb + h * E.vn_sh + (size_t)t0 * E.vn_st] = __float2half_rn(raw_v / (cnorm > 1e-10f ? cnorm : 1.0f));
-    }
-    const int vb = (E.flags & BGTQ_ENC_V_NIBBLE) ? 4 : d.v_bits;
-    if (p < seg_storage_bytes(vb, kHD))
-        E.vp[b * E.vp_sb + h * E.vp_sh + (size_t)t0 * E.vp_st + p] = (uint8_t)pack_byte(&codes[0], kHD, vb, p);
+    prep_store_v(E, b, h, t0, p, raw_v, gn, codes, (E.flags & BGTQ_ENC_V_NIBBLE) ? 4 : d.v_bits);
 }
 
 }  // namespace
@@ -617,10 +717,15 @@ static int step_prepare_impl(
     P.rope_sb = rope_sb;
     P.k_buf = static_cast<__half*>(k_buf); P.v_buf = static_cast<__half*>(v_buf);
     P.kb_sb = kb_sb; P.kb_sh = kb_sh; P.n_sink = n_sink; P.window = window;
-    const int64_t items = (int64_t)(do_rot ? n_batch * n_q / P.rot_group : 0) + 2LL * n_batch * n_kv;
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // four rows per CTA once the one-row CTAs no longer fit the GPU at once (two per SM)
+    const int64_t q_items = do_rot ? (int64_t)n_batch * n_q / P.rot_group : 0;
+    const bool four = n_batch % 4 == 0 && q_items + 2LL * n_batch * n_kv > 2LL * sms;
+    const int64_t items = q_items + 2LL * n_batch * n_kv / (four ? 4 : 1);
     if (items > 0x7fffffffLL) return BGTQ_E_TOOBIG;
-    return launch_kernel(prep_kernel, dim3((unsigned)items), dim3(512), 0, static_cast<cudaStream_t>(stream),
-                         (flags & BGTQ_ENC_PROGRAMMATIC) != 0, P) == cudaSuccess ? BGTQ_OK : BGTQ_E_LAUNCH;
+    return launch_kernel(four ? prep_kernel<true> : prep_kernel<false>, dim3((unsigned)items), dim3(512), 0,
+                         static_cast<cudaStream_t>(stream), (flags & BGTQ_ENC_PROGRAMMATIC) != 0, P) == cudaSuccess ? BGTQ_OK : BGTQ_E_LAUNCH;
 }
 
 extern "C" __attribute__((visibility("default"))) int bgtq_step_prepare(
@@ -676,7 +781,7 @@ int bgtq::launch_rotate_q(const BgtqHeadDesc* desc, const float* rot_k, const vo
     P.n_q = n_q; P.do_rot = 1; P.rot_group = (n_q / n_kv) % 4 == 0 ? 4 : 1;
     const int64_t items = (int64_t)n_batch * n_q / P.rot_group;
     if (items > 0x7fffffffLL) return BGTQ_E_TOOBIG;
-    return launch_kernel(prep_kernel, dim3((unsigned)items), dim3(512), 0, stream, programmatic, P) == cudaSuccess ? BGTQ_OK
+    return launch_kernel(prep_kernel<false>, dim3((unsigned)items), dim3(512), 0, stream, programmatic, P) == cudaSuccess ? BGTQ_OK
                                                                                                               : BGTQ_E_LAUNCH;
 }
 

@@ -305,6 +305,8 @@ __global__ void __launch_bounds__(kBufThreads) buffer_attn_kernel(const __half* 
     // shared memory: sc_cap logits / probabilities, 16 floats of scratch, the query (128 floats), 3 x 128 partial outputs
     extern __shared__ __align__(16) float sc[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    grid_launch_dependents();
+    grid_dependency_wait();       // the rows and the position come from earlier work in the stream
     if (pos_dev) {      // region sizes from the device-side token count (one-token blocks, window = ring_size - 1)
         const int avail = *pos_dev + 1;                // tokens including the one appended this step
         const int a0 = max(0, avail - 1 - sink_cap), a1 = max(0, avail - sink_cap);
@@ -419,6 +421,8 @@ __global__ void __launch_bounds__(kBufThreads) buffer_attn_group_kernel(const __
     uint8_t* const vs = smem_rows + (size_t)cap_rows * kBufRowLd;
     float* const sc = reinterpret_cast<float*>(smem_rows + 2 * (size_t)cap_rows * kBufRowLd);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    grid_launch_dependents();
+    grid_dependency_wait();       // the rows and the position come from earlier work in the stream
     if (pos_dev) {      // region sizes from the device-side token count (one-token blocks, window = ring_size - 1)
         const int avail = *pos_dev + 1;                // tokens including the one appended this step
         const int a0 = max(0, avail - 1 - sink_cap), a1 = max(0, avail - sink_cap);
@@ -690,18 +694,17 @@ extern "C" __attribute__((visibility("default"))) int bgtq_buffer_attn_pos(const
             cudaGetLastError();
             return BGTQ_E_LAUNCH;
         }
-        kern<<<dim3(n_kv, n_batch), kBufThreads, smem_group, static_cast<cudaStream_t>(stream)>>>(
-            static_cast<const __half*>(q), q_sb, q_sh, static_cast<const __half*>(k_buf), static_cast<const __half*>(v_buf),
-            kb_sb, kb_sh, n_sink_tokens, n_ring_tokens, sink_cap, ring_first, ring_size > 0 ? ring_size : 1, n_q, scale,
-            buf_o, buf_lse, pos_dev, sc_cap, cap_rows);
-        return cudaGetLastError() == cudaSuccess ? BGTQ_OK : BGTQ_E_LAUNCH;
+        return launch_kernel(kern, dim3(n_kv, n_batch), dim3(kBufThreads), smem_group, static_cast<cudaStream_t>(stream), true,
+                             static_cast<const __half*>(q), q_sb, q_sh, static_cast<const __half*>(k_buf),
+                             static_cast<const __half*>(v_buf), kb_sb, kb_sh, n_sink_tokens, n_ring_tokens, sink_cap, ring_first,
+                             ring_size > 0 ? ring_size : 1, n_q, scale, buf_o, buf_lse, pos_dev, sc_cap, cap_rows) == cudaSuccess
+                   ? BGTQ_OK : BGTQ_E_LAUNCH;
     }
     const size_t smem = (size_t)(sc_cap + 16 + 4 * kHD) * sizeof(float);
-    buffer_attn_kernel<<<dim3(n_q, n_batch), kBufThreads, smem, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __half*>(q), q_sb, q_sh, static_cast<const __half*>(k_buf),
-        static_cast<const __half*>(v_buf), kb_sb, kb_sh, n_sink_tokens, n_ring_tokens, sink_cap, ring_first,
-        ring_size > 0 ? ring_size : 1, n_q, n_kv, scale, buf_o, buf_lse, pos_dev, sc_cap);
-    return cudaGetLastError() == cudaSuccess ? BGTQ_OK : BGTQ_E_LAUNCH;
+    return launch_kernel(buffer_attn_kernel, dim3(n_q, n_batch), dim3(kBufThreads), smem, static_cast<cudaStream_t>(stream), true,
+                         static_cast<const __half*>(q), q_sb, q_sh, static_cast<const __half*>(k_buf), static_cast<const __half*>(v_buf),
+                         kb_sb, kb_sh, n_sink_tokens, n_ring_tokens, sink_cap, ring_first, ring_size > 0 ? ring_size : 1, n_q, n_kv, scale,
+                         buf_o, buf_lse, pos_dev, sc_cap) == cudaSuccess ? BGTQ_OK : BGTQ_E_LAUNCH;
 }
 
 // ---------------------------------------------------------------------------
