@@ -44,8 +44,9 @@ static int decode_impl(
 
     // Tiles of 16 warps x 32 tokens, two stages; rows too wide for that (padded strides, the nibble layout with
     // large tables) fall back to 16 tokens per warp.
-    const int nu = decode_nu(P.plan.lut_bytes, P.kp_st, P.kn_st, P.vp_st, P.vn_st);
+    int nu = decode_nu(P.plan.lut_bytes, P.kp_st, P.kn_st, P.vp_st, P.vn_st);
     if (nu == 0) return BGTQ_E_TOOBIG;
+    if (P.plan.flags & BGTQ_DEC_NARROW) nu = 1;
     const StageLayout sl = stage_layout(kDecWarps * 16u * nu, P.kp_st, P.kn_st, P.vp_st, P.vn_st);
     P.off_kn = sl.off_kn; P.off_v = sl.off_v; P.off_vn = sl.off_vn;
     P.stage_bytes = sl.stage_bytes;

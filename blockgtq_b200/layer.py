@@ -11,6 +11,7 @@ from __future__ import annotations
 import os
 
 import ctypes as C
+import functools
 import math
 
 import numpy as np
@@ -426,6 +427,19 @@ def attend(layer, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, *, ro
 
 
 _SCALE = 1.0 / math.sqrt(HD)
+
+
+@functools.lru_cache(maxsize=None)
+def _sm_count(index: int) -> int:
+    return torch.cuda.get_device_properties(index).multi_processor_count
+
+
+def tile_flags(n_batch: int, n_kv: int, n_tokens: int, device) -> int:
+    """``DEC_NARROW`` while every SM's share of the tokens fits one narrow tile (16 warps x 16 tokens): twice the warps
+    work on half the chain each.  One layer of 8 heads x 500 tokens: 14.8 -> 12.4 us; with longer shares the wide tile, which
+    loads each query fragment for twice the tokens, is faster."""
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    return _lib.DEC_NARROW if n_batch * n_kv * n_tokens <= 256 * _sm_count(index) else 0
 _PREFILL_WORKSPACE = 2 << 30        # bytes of dequantised operand tiles per launch
 
 

@@ -24,7 +24,7 @@ import torch
 from . import _lib
 from .calib import packed_v_bytes
 from .layer import (HD, LayerTables, attend, buffer_attn, combine, decode, decode_grid_size, decode_partition, default_splits,
-                    encode, rotate_q, step_prepare, _no_tcgen05)
+                    encode, rotate_q, step_prepare, tile_flags, _no_tcgen05)
 from .quantizer import BlockGTQQuantizer, build_batched_encode_args
 
 __all__ = ["BlockGTQKVManager", "decode_step"]
@@ -156,6 +156,8 @@ class BlockGTQKVManager:
                     # query), and the position is advanced between steps: the decode may start streaming early.
                     if not os.environ.get("BGTQ_DEC_NO_EARLY_FETCH"):
                         lt.set_early_fetch(1)
+        if dev.type == "cuda":      # by capacity: one kernel for the cache's whole life, captured graphs included
+            self._dec_flags |= tile_flags(self.B, self.n_kv, self.max_T, dev)
         self._prepare_decode_plans()
         self._q_rot = torch.empty(self.B, self.n_q, self.hd, dtype=torch.float16, device=dev)
         self._part_o = torch.empty(self.B, self.n_q, self._n_splits, self.hd, dtype=torch.float32, device=dev)

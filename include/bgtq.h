@@ -225,6 +225,9 @@ int bgtq_step_prepare_ring(const BgtqHeadDesc* desc, const float* rot_k, const f
 #define BGTQ_DEC_V_NIBBLE 2       /* v_packed rows are 4-bit nibbles */
 #define BGTQ_DEC_PROGRAMMATIC 4   /* launch bgtq_decode as a programmatic dependent of the preceding kernel */
 #define BGTQ_DEC_GENERIC 8        /* always launch the general kernel, even if the plan holds a specialised one */
+#define BGTQ_DEC_NARROW 32        /* 16 tokens per warp instead of 32: shorter chains while a CTA gets at most 256 tokens
+                                   * (n_batch * n_kv * tokens <= 256 * SMs), less work per load beyond; same results up to
+                                   * the order of sums */
 
 /* Opaque launch plan of the decode kernel for the KV heads of one layer (host
  * memory, plain bytes, copyable).  Built once per layer from the HOST copy of

@@ -40,7 +40,10 @@ def test_specialised_2bit_values_match_general(T):
     mgr.init_from_cache([tuple(torch.randn(B, n_kv, T, HD, generator=gen).half().to(DEV) for _ in range(2))])
     q = torch.randn(B, n_kv * gqa, HD, generator=gen).half().to(DEV)
     lt, cache = mgr._layers[0], (mgr._k_packed[0], mgr._k_norms[0], mgr._v_packed[0], mgr._v_norms[0])
-    po, pl = decode(lt, q, *cache, 0, T, n_splits=3, flags=mgr._dec_flags)
-    go, gl = decode(lt, q, *cache, 0, T, n_splits=3, flags=mgr._dec_flags | _lib.DEC_GENERIC)
+    wide = mgr._dec_flags & ~_lib.DEC_NARROW
+    po, pl = decode(lt, q, *cache, 0, T, n_splits=3, flags=wide)
+    go, gl = decode(lt, q, *cache, 0, T, n_splits=3, flags=wide | _lib.DEC_GENERIC)
+    no, nl = decode(lt, q, *cache, 0, T, n_splits=3, flags=wide | _lib.DEC_NARROW)          # the other tile: other sums
     live = torch.isfinite(gl)
     assert live.any() and torch.equal(pl, gl) and torch.equal(po[live], go[live])
+    assert torch.equal(torch.isfinite(nl), live) and (no[live] - go[live]).abs().max() < 1e-3 and (nl[live] - gl[live]).abs().max() < 1e-3
