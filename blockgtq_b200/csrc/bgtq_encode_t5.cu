@@ -342,7 +342,10 @@ __device__ __forceinline__ float square2(float acc, uint32_t w) {
 }
 
 // Tiles [lo, hi) of one (head, K or V).  `n_mma`: products this thread's group has issued so far (the barrier's phase).
-template <bool IS_V, bool MIXED, bool CODES>
+// ONE: the CTA's only tile.  Its time is that of one pass over code that no instruction cache holds yet, so the code is kept
+// short where nothing is lost by it: no next tile's loads, the two row groups of the column move in a loop (777 tokens of a
+// layer: 12.0 -> 10.8 us; in the many-tile form the loop costs 1 %, and shorter loops in the epilogue cost 20 % in either).
+template <bool IS_V, bool MIXED, bool CODES, bool ONE>
 __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int h, const int lo_tile, const int hi_tile, int& n_mma) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int grp = tid >> 8, gt = tid & (kGroup - 1);
@@ -422,7 +425,7 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
         if constexpr (!IS_V) {
             group_sync(grp);
             const uint32_t raw = smem_u32(S.buf[grp][0]);
-#pragma unroll
+#pragma unroll (ONE ? 1 : 2)
             for (int rg = 0; rg < 2; ++rg)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -449,7 +452,7 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
             if (lead) umma_commit(bar);
             __syncwarp();
         }
-        if (tl + 2 < hi_tile) prefetch(tl + 2, nb0, ns0, S.buf[grp][IS_V ? (it + 1) & 1 : 0]);     // arrives during this tile's work
+        if (!ONE && tl + 2 < hi_tile) prefetch(tl + 2, nb0, ns0, S.buf[grp][IS_V ? (it + 1) & 1 : 0]);     // arrives during this tile's work
         // ---- group norms: the row's two threads take alternate element pairs of each segment ----
         {
             const uint32_t xr = smem_u32(a) + (uint32_t)row * 128u, sw = (uint32_t)(row & 7) << 4;
@@ -680,7 +683,7 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
 // they take: a K row's columns move into packed order first); CTA i works on the tiles that begin in its share of the units,
 // and loads the tables again where its share crosses into the next (head, role).
 constexpr int kUnitsK = 13, kUnitsV = 7;
-template <bool MIXED, bool CODES>
+template <bool MIXED, bool CODES, bool ONE>
 __global__ void __launch_bounds__(kThreads, 1) encode_t5_kernel(const EncParams P, const int units_k, const int units_v) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     E5Smem& S = *reinterpret_cast<E5Smem*>(smem_raw);
@@ -716,8 +719,8 @@ __global__ void __launch_bounds__(kThreads, 1) encode_t5_kernel(const EncParams 
         __syncthreads();
         tc_fence_after_sync();
         if (!in_range) break;
-        const bool ok = is_v ? e5_role<true, MIXED, CODES>(S, P, h, lo, hi, n_mma) : e5_role<false, MIXED, CODES>(S, P, h, lo, hi, n_mma);
-        if (!__syncthreads_and(ok ? 1 : 0)) break;      // (also: everyone is done with this range's tables)
+        const bool ok = is_v ? e5_role<true, MIXED, CODES, ONE>(S, P, h, lo, hi, n_mma) : e5_role<false, MIXED, CODES, ONE>(S, P, h, lo, hi, n_mma);
+        if (!__syncthreads_and(ok ? 1 : 0) || ONE) break;      // (also: everyone is done with this range's tables)
     }
     if (!waited) grid_dependency_wait();
     tc_fence_before_sync();
@@ -737,12 +740,12 @@ int launch_encode_t5(const EncParams& P, cudaStream_t stream) {
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t all = (int64_t)n_tiles * P.n_kv * ((do_k ? 1 : 0) + (do_v ? 1 : 0));
-    const bool few = all <= sms;                // one tile per CTA
+    const bool few = all <= sms;                // one tile per CTA (the code written out for it: ONE)
     const int units_k = do_k ? (few ? 1 : kUnitsK) : 0, units_v = do_v ? (few ? 1 : kUnitsV) : 0;
     const int smem = (int)sizeof(E5Smem);
     const bool mixed = P.flags & BGTQ_ENC_K_MIXED, codes = P.k_codes != nullptr || P.v_codes != nullptr;
-    auto kern = mixed ? (codes ? encode_t5_kernel<true, true> : encode_t5_kernel<true, false>)
-                      : (codes ? encode_t5_kernel<false, true> : encode_t5_kernel<false, false>);
+    auto kern = mixed ? (codes ? encode_t5_kernel<true, true, false> : few ? encode_t5_kernel<true, false, true> : encode_t5_kernel<true, false, false>)
+                      : (codes ? encode_t5_kernel<false, true, false> : few ? encode_t5_kernel<false, false, true> : encode_t5_kernel<false, false, false>);
     // the attribute is per device: set it on every launch (cheap, and legal under stream capture)
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
         cudaGetLastError();

@@ -44,3 +44,31 @@ def test_rows_do_not_depend_on_their_tile(case, B, T, t0, pad, mixed):
     for a, b in zip(whole[2:], other[2:]):
         assert ((a.float() - b.float()).abs() <= 2e-3 * b.float().abs()).float().mean().item() > 0.999
     assert _lib.lib().bgtq_encode_tcgen05_status() == 0
+
+
+@pytest.mark.parametrize("case", ["a3_1to8", "u3"])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_one_tile_per_cta_and_more(case, mixed):
+    """The build for launches whose CTAs have one tile each gives the bytes of the one for more tiles."""
+    from blockgtq_b200 import _lib
+    from blockgtq_b200.layer import LayerTables, encode
+    from helpers import HD, tables_for
+    tabs = [tables_for(case, h) for h in range(2)]
+    lt = LayerTables([t[0] for t in tabs], [t[1] for t in tabs], DEV)
+    tiles = torch.cuda.get_device_properties(0).multi_processor_count // 4      # x 2 heads x (K, V): the most with one per CTA
+    n = 128 * tiles + 1
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    k, v = (torch.randn(1, 2, n, HD, generator=gen, device=DEV).half() * s for s in (3.0, 1.0))
+    flags = _lib.ENC_K_MIXED | _lib.ENC_V_NIBBLE if mixed else 0
+    kb, vb = (lt.max_mixed_bytes, HD // 2) if mixed else (lt.max_tpb, lt.vpb)
+
+    def run(parts):
+        out = [torch.zeros(1, 2, n, w, dtype=torch.uint8, device=DEV) for w in (kb, vb)]
+        out += [torch.zeros(1, 2, n, lt.max_ng, dtype=torch.float16, device=DEV), torch.zeros(1, 2, n, dtype=torch.float16, device=DEV)]
+        for lo, hi in parts:
+            encode(lt, k[:, :, lo:hi], v[:, :, lo:hi], lo, out[0], out[2], out[1], out[3], flags=flags)
+        return out
+
+    for a, b in zip(run([(0, n)]), run([(0, n - 1), (n - 200, n)])):
+        assert torch.equal(a, b)
+    assert _lib.lib().bgtq_encode_tcgen05_status() == 0
