@@ -2,16 +2,18 @@
 // The kernel itself lives in bgtq_decode_kernel.cuh (one translation unit per stored V width), the
 // plan / table-image builders in bgtq_decode_plan.cu.
 #include "bgtq_decode_kernel.cuh"
+#include "bgtq_encode_params.cuh"
 
 using namespace bgtq;
 
-static int decode_impl(
+// early_fetch false: the plan's early fetch stays off for this launch.
+int bgtq::launch_decode_plan(
     const BgtqDecodePlan* plan_host, const void* q_rot, const uint8_t* k_packed,
     int64_t kp_sb, int64_t kp_sh, int64_t kp_st, const void* k_norms, int64_t kn_sb, int64_t kn_sh, int64_t kn_st,
     const uint8_t* v_packed, int64_t vp_sb, int64_t vp_sh, int64_t vp_st, const void* v_norms, int64_t vn_sb,
     int64_t vn_sh, int64_t vn_st, int32_t n_batch, int32_t n_q, int32_t n_kv, int32_t t_begin, int32_t t_end,
     int32_t n_splits, float scale, float* part_o, float* part_lse, int32_t* status, const int32_t* pos_dev,
-    int32_t pos_add, void* stream) {
+    int32_t pos_add, bool early_fetch, void* stream) {
     if (!plan_host || !q_rot || !k_packed || !k_norms || !v_packed || !v_norms || !part_o || !part_lse)
         return BGTQ_E_BADARG;
     if (n_batch < 1 || n_kv < 1 || n_q < n_kv || n_q % n_kv || n_splits < 1 || t_end < t_begin || t_begin < 0)
@@ -20,6 +22,7 @@ static int decode_impl(
     memcpy(&P.plan, plan_host, sizeof(DecPlanDev));
     if (P.plan.n_heads != n_kv) return BGTQ_E_BADARG;
     if (!P.plan.image) return BGTQ_E_BADARG;          // bgtq_decode_plan_set_image has not been called
+    if (!early_fetch) P.plan.early_fresh = 0;
     const int gqa = n_q / n_kv;
     if (gqa > 8) return BGTQ_E_UNSUPPORTED;
     if (kp_st < 1 || kp_st > 160 || vp_st < 1 || vp_st > 128 || kn_st < 1 || kn_st > 16 || vn_st < 1 || vn_st > 8)
@@ -102,9 +105,9 @@ extern "C" __attribute__((visibility("default"))) int bgtq_decode(
     int32_t n_splits, float scale, float* part_o, float* part_lse, int32_t* status, const int32_t* pos_dev,
     int32_t pos_add, void* stream) {
     (void)desc;      // the kernel reads its tables from the plan's image
-    return decode_impl(plan_host, q_rot, k_packed, kp_sb, kp_sh, kp_st, k_norms, kn_sb, kn_sh, kn_st, v_packed,
-                       vp_sb, vp_sh, vp_st, v_norms, vn_sb, vn_sh, vn_st, n_batch, n_q, n_kv, t_begin, t_end, n_splits,
-                       scale, part_o, part_lse, status, pos_dev, pos_add, stream);
+    return launch_decode_plan(plan_host, q_rot, k_packed, kp_sb, kp_sh, kp_st, k_norms, kn_sb, kn_sh, kn_st, v_packed,
+                              vp_sb, vp_sh, vp_st, v_norms, vn_sb, vn_sh, vn_st, n_batch, n_q, n_kv, t_begin, t_end, n_splits,
+                              scale, part_o, part_lse, status, pos_dev, pos_add, true, stream);
 }
 
 // ---------------------------------------------------------------------------

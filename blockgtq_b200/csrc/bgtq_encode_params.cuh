@@ -1,4 +1,4 @@
-// Launch parameters and helpers shared by the encoder kernels.
+// Launch parameters and helpers shared by the encoder kernels, and the launches that bgtq_step.cu puts together.
 #pragma once
 #include "bgtq_common.cuh"
 
@@ -57,5 +57,13 @@ int launch_encode_t5(const EncParams& P, cudaStream_t stream);
 // Query rotation alone (the query items of the step-preparation kernel), optionally as a programmatic dependent.
 int launch_rotate_q(const BgtqHeadDesc* desc, const float* rot_k, const void* q, int64_t q_sb, int64_t q_sh, void* q_rot,
                     int32_t n_batch, int32_t n_q, int32_t n_kv, bool programmatic, cudaStream_t stream);
+
+// bgtq_decode with the plan's early fetch as it is or off for this launch (bgtq_decode.cu).
+int launch_decode_plan(const BgtqDecodePlan* plan_host, const void* q_rot, const uint8_t* k_packed, int64_t kp_sb, int64_t kp_sh,
+                       int64_t kp_st, const void* k_norms, int64_t kn_sb, int64_t kn_sh, int64_t kn_st, const uint8_t* v_packed,
+                       int64_t vp_sb, int64_t vp_sh, int64_t vp_st, const void* v_norms, int64_t vn_sb, int64_t vn_sh, int64_t vn_st,
+                       int32_t n_batch, int32_t n_q, int32_t n_kv, int32_t t_begin, int32_t t_end, int32_t n_splits, float scale,
+                       float* part_o, float* part_lse, int32_t* status, const int32_t* pos_dev, int32_t pos_add, bool early_fetch,
+                       void* stream);
 
 }  // namespace bgtq

@@ -93,9 +93,12 @@ extern "C" __attribute__((visibility("default"))) int bgtq_attend(
     } else if (q_sh != kHD || (n_batch > 1 && q_sb != (int64_t)n_q * kHD)) {
         return BGTQ_E_UNSUPPORTED;
     }
-    const int rc = bgtq_decode(plan, desc, q_dec, k_packed, kp_sb, kp_sh, kp_st, k_norms, kn_sb, kn_sh, kn_st, v_packed, vp_sb, vp_sh,
-                               vp_st, v_norms, vn_sb, vn_sh, vn_st, n_batch, n_q, n_kv, t_begin, t_end, n_splits, scale, part_o,
-                               part_lse, status, nullptr, 0, stream);
+    // No early fetch here, whatever the plan says: what is in front of this call may be a bulk encode of the very rows
+    // that are attended, and it lets its dependents start while it runs.  (A layer step is different: there the launch in
+    // front of the decode is its own append.)
+    const int rc = launch_decode_plan(plan, q_dec, k_packed, kp_sb, kp_sh, kp_st, k_norms, kn_sb, kn_sh, kn_st, v_packed, vp_sb, vp_sh,
+                                      vp_st, v_norms, vn_sb, vn_sh, vn_st, n_batch, n_q, n_kv, t_begin, t_end, n_splits, scale, part_o,
+                                      part_lse, status, nullptr, 0, false, stream);
     if (rc != BGTQ_OK) return rc;
     return bgtq_combine(part_o, part_lse, n_splits, v_rot, buf_o, buf_lse, n_batch, n_q, n_kv, out, (int64_t)n_q * kHD, kHD, out_f32,
                         lse_out, BGTQ_COMBINE_PROGRAMMATIC, stream);

@@ -83,7 +83,7 @@ const char* bgtq_error_string(int code);       /* host pointer to a static strin
 #define BGTQ_ENC_SKIP_K 8
 #define BGTQ_ENC_SKIP_V 16
 #define BGTQ_ENC_FORCE_SIMT 32  /* always use the small-batch fp32 kernel (>= 64 rows normally use tensor cores) */
-#define BGTQ_ENC_PROGRAMMATIC 64  /* bgtq_step_prepare only: programmatic dependent launch, see below */
+#define BGTQ_ENC_PROGRAMMATIC 64  /* bgtq_step_prepare*: programmatic dependent launch, see below (bgtq_encode ignores it) */
 #define BGTQ_ENC_NO_TCGEN05 128   /* bulk encode: keep the rotation on mma.sync (bulk row counts of >= 128 rows and packed
                                    * K rows of <= 120 bytes normally use tcgen05.mma with tensor-memory accumulators) */
 
@@ -94,7 +94,12 @@ const char* bgtq_error_string(int code);       /* host pointer to a static strin
  * and wait on the device for that kernel to complete before they touch any
  * per-call input or output.  Results are identical; the launch latency and the
  * set-up of each kernel of a decode step overlap the previous kernel's tail.
- * Safe after any kind of preceding work; capturable in a CUDA graph. */
+ * Safe after any kind of preceding work; capturable in a CUDA graph.
+ * Launched this way without being asked: bgtq_encode and bgtq_layer_encode from 128 rows on (tcgen05 form),
+ * bgtq_rotate_q_rows, bgtq_prefill and bgtq_prefill_attention (tcgen05 form), bgtq_buffer_attn and
+ * bgtq_buffer_attn_pos, bgtq_exchange_merge, and the rotation and the combine of bgtq_attend.  A kernel of this
+ * library also lets the launch behind it, if that is a programmatic one, become resident early; ordinary launches
+ * behind it wait for its end as always. */
 
 /* Encode K and V rows of all KV heads of one layer and write them straight
  * into their cache slots.
@@ -276,7 +281,11 @@ int bgtq_jit_set_nvrtc_path(const char* path_host);
  * final: the preceding launch writes nothing but the newest fresh_rows rows (the step's append), the query and
  * buffers the decode does not read.  The kernel then reads pos_dev, cuts its ranges and requests its first tiles
  * right away (tiles that reach into the fresh rows are held back), and only waits before it reads the query and
- * before it writes anything.  0 (default): everything waits.  No counterpart in the reference. */
+ * before it writes anything.  0 (default): everything waits.
+ * A launch that is itself a programmatic dependent starts while the work in front of it still runs (see the list of
+ * them above): behind bgtq_encode of rows that the decode reads, neither that encode nor a programmatic launch between
+ * it and the decode may be the preceding launch.  bgtq_attend, which may well be called there, never fetches early.
+ * No counterpart in the reference. */
 int bgtq_decode_plan_set_early_fetch(BgtqDecodePlan* plan_host, int32_t fresh_rows);
 
 /* Optional item-range table of a launch.  bgtq_decode cuts every (batch, KV head) pair into items and hands
@@ -441,7 +450,8 @@ int bgtq_layer_encode(const BgtqLayerStep* step, const void* k, int64_t k_sb, in
 
 /* Attention of one query token per (batch, head) over cached rows [t_begin, t_end) in one call: query rotation
  * (rot_k may be NULL: q is in the packed-K basis and contiguous) -> bgtq_decode -> bgtq_combine into the
- * contiguous out (n_batch, n_q, 128) fp16 and the optional out_f32 / lse_out.  scratch: device memory of
+ * contiguous out (n_batch, n_q, 128) fp16 and the optional out_f32 / lse_out.  The decode starts without the plan's
+ * early fetch: the rows may come from the work right in front of the call.  scratch: device memory of
  * bgtq_attend_scratch_bytes(n_batch, n_q, n_splits) bytes, 16-byte aligned. */
 int64_t bgtq_attend_scratch_bytes(int32_t n_batch, int32_t n_q, int32_t n_splits);
 int bgtq_attend(const BgtqDecodePlan* plan, const BgtqHeadDesc* desc, const float* rot_k,

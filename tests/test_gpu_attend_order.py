@@ -1,0 +1,96 @@
+"""An attention enqueued right behind the encode that writes its rows reads the new rows, however busy the stream is:
+the launches may start while the encode still runs, and only the rows that they may read by then are read."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _manager(layers, batch, n_kv, gqa, cap, **kw):
+    from blockgtq_b200 import BlockGTQKVManager
+    from helpers import HD, synth_head
+    gen = torch.Generator().manual_seed(n_kv)
+    mgr = BlockGTQKVManager(layers, n_kv * gqa, n_kv, HD, max_seq_len=cap, batch_size=batch, device=DEV, **kw)
+    cal = [synth_head(gen, 256, gqa) for _ in range(n_kv)]
+    for li in range(layers):
+        mgr.calibrate(li, torch.stack([c[0] for c in cal]).float(), torch.stack([c[1] for c in cal]).float())
+    return mgr
+
+
+def _kv(gen, batch, n_kv, n):
+    from helpers import HD
+    return tuple(torch.randn(batch, n_kv, n, HD, generator=gen, device=DEV).half() for _ in range(2))
+
+
+class _Busy:
+    """Ordinary work that keeps the stream occupied while the host enqueues what follows."""
+
+    def __init__(self):
+        self.a = torch.randn(4096, 4096, device=DEV).half()
+        self.out = torch.empty_like(self.a)
+
+    def __call__(self):
+        for _ in range(3):
+            torch.mm(self.a, self.a, out=self.out)
+
+
+# rows of the bulk encode (batch x tokens) from its smallest to several waves of tiles; few heads leave SMs free for the
+# launches behind it, and with the queries already in the packed basis the decode is the launch right behind the encode
+@pytest.mark.parametrize("batch,n_kv,T,baked,window", [(1, 1, 128, False, 0), (1, 8, 800, False, 0), (2, 2, 400, False, 0),
+                                                       (1, 1, 800, True, 0), (1, 8, 128, True, 0), (1, 2, 700, False, 64),
+                                                       (1, 4, 6000, True, 0)])
+def test_attend_behind_a_bulk_encode(batch, n_kv, T, baked, window):
+    from helpers import HD
+    gqa = 4
+    mgr = _manager(1, batch, n_kv, gqa, T + 8, n_sink=4 if window else 0, recent_window=window)
+    for qz in mgr.quantizers[0]:
+        qz._q_perm_baked = baked
+    gen = torch.Generator(device=DEV).manual_seed(T)
+    prompts = [_kv(gen, batch, n_kv, T) for _ in range(2)]
+    q = torch.randn(batch, n_kv * gqa, 1, HD, generator=gen, device=DEV).half()
+    want = []
+    for kv in prompts:
+        mgr.init_from_cache([kv])
+        torch.cuda.synchronize()
+        want.append([t.clone() for t in mgr.attend(0, q, want_partial=True)])
+        torch.cuda.synchronize()
+    assert not torch.equal(want[0][0], want[1][0])
+    busy = _Busy()
+    got = []
+    for i in range(60):
+        busy()
+        mgr.init_from_cache([prompts[i & 1]])
+        got.append(mgr.attend(0, q, want_partial=True))
+    torch.cuda.synchronize()
+    for i, r in enumerate(got):
+        assert all(torch.equal(a, b) for a, b in zip(r, want[i & 1])), i
+    mgr.check_status()
+
+
+@pytest.mark.parametrize("batch,n_kv,t,S", [(1, 1, 0, 128), (1, 2, 600, 130), (2, 8, 37, 64), (1, 4, 3000, 800)])
+def test_append_and_attend_of_several_tokens(batch, n_kv, t, S):
+    from helpers import HD
+    gqa = 2
+    mgr = _manager(1, batch, n_kv, gqa, t + S + 8)
+    gen = torch.Generator(device=DEV).manual_seed(t + S)
+    if t:
+        mgr.init_from_cache([_kv(gen, batch, n_kv, t)])
+    pieces = [_kv(gen, batch, n_kv, S) for _ in range(2)]
+    q = torch.randn(batch, n_kv * gqa, 1, HD, generator=gen, device=DEV).half()
+    want = []
+    for k, v in pieces:
+        mgr._append_tokens(0, k, v, t)
+        torch.cuda.synchronize()
+        want.append(mgr.attend(0, q, t + S)[0].unsqueeze(2))
+        torch.cuda.synchronize()
+    assert not torch.equal(want[0], want[1])
+    busy = _Busy()
+    got = []
+    for i in range(60):
+        busy()
+        got.append(mgr.append_and_attend(0, q, *pieces[i & 1]))
+    torch.cuda.synchronize()
+    for i, r in enumerate(got):
+        assert torch.equal(r, want[i & 1]), i
+    mgr.check_status()
