@@ -282,9 +282,10 @@ int bgtq_jit_set_nvrtc_path(const char* path_host);
  * buffers the decode does not read.  The kernel then reads pos_dev, cuts its ranges and requests its first tiles
  * right away (tiles that reach into the fresh rows are held back), and only waits before it reads the query and
  * before it writes anything.  0 (default): everything waits.
- * A launch that is itself a programmatic dependent starts while the work in front of it still runs (see the list of
- * them above): behind bgtq_encode of rows that the decode reads, neither that encode nor a programmatic launch between
- * it and the decode may be the preceding launch.  bgtq_attend, which may well be called there, never fetches early.
+ * bgtq_step_prepare, its rope and ring forms, bgtq_rotate_q and any ordinary launch keep (1) and (2) as the preceding
+ * launch whatever is in front of them: they let the decode start only when all work before them is complete.  The other
+ * programmatic dependents listed above do not: behind bgtq_encode of rows that the decode reads, neither that encode nor
+ * one of them may be the preceding launch.  bgtq_attend, which may well be called there, never fetches early.
  * No counterpart in the reference. */
 int bgtq_decode_plan_set_early_fetch(BgtqDecodePlan* plan_host, int32_t fresh_rows);
 

@@ -94,3 +94,40 @@ def test_append_and_attend_of_several_tokens(batch, n_kv, t, S):
     for i, r in enumerate(got):
         assert torch.equal(r, want[i & 1]), i
     mgr.check_status()
+
+
+@pytest.mark.parametrize("batch,n_kv,T", [(1, 1, 128), (1, 8, 800), (2, 2, 3000)])
+def test_layer_step_behind_a_bulk_encode(batch, n_kv, T):
+    """The step's decode reads the older rows and the position before its own dependency wait; the rows may come from an
+    encode right in front of the step, the position from the kernel that advanced it."""
+    from helpers import HD
+    gqa = 4
+    mgr = _manager(1, batch, n_kv, gqa, T + 64)
+    mgr._ensure_storage()
+    gen = torch.Generator(device=DEV).manual_seed(T + 1)
+    prompts = [_kv(gen, batch, n_kv, T) for _ in range(2)]
+    steps = [(torch.randn(batch, n_kv * gqa, 1, HD, generator=gen, device=DEV).half(),) + _kv(gen, batch, n_kv, 1) for _ in range(4)]
+
+    def run(i, sync):
+        mgr.seq_len = T
+        mgr._sync_pos()                 # nothing but the encode's launch is left between it and the first step
+        mgr._encode_kv(0, *prompts[i], 0, T)
+        out = []
+        for s in steps:
+            sync()
+            out.append(mgr.append_and_attend(0, *s).clone())
+            sync()
+            mgr.increment_seq_len()
+        return out
+
+    want = [run(i, torch.cuda.synchronize) for i in range(2)]
+    assert not torch.equal(want[0][0], want[1][0])
+    busy = _Busy()
+    got = []
+    for i in range(40):
+        busy()
+        got.append(run(i & 1, lambda: None))
+    torch.cuda.synchronize()
+    for i, r in enumerate(got):
+        assert all(torch.equal(a, b) for a, b in zip(r, want[i & 1])), i
+    mgr.check_status()
