@@ -33,6 +33,9 @@ struct Fns {
 PyObject* none() { Py_RETURN_NONE; }
 PyObject* code(int rc) { return PyLong_FromLong(rc); }
 
+// A Python exception is set: the call ends with it (see `guarded`).
+struct PythonError {};
+
 struct Args {
     PyObject* const* a;
     // a tensor, or null where the argument is None or no tensor (`bad` then)
@@ -43,7 +46,11 @@ struct Args {
     }
     int64_t num(int i) const { return PyLong_AsLongLong(a[i]); }
     template <typename T> T* ptr(int i) const { return a[i] == Py_None ? nullptr : reinterpret_cast<T*>(PyLong_AsUnsignedLongLong(a[i])); }
-    bool truth(int i) const { return a[i] == Py_True; }
+    bool truth(int i) const {
+        const int r = PyObject_IsTrue(a[i]);
+        if (r < 0) throw PythonError();
+        return r != 0;
+    }
 };
 
 void* stream_of(const at::Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
@@ -272,6 +279,7 @@ template <PyObject* (*FN)(PyObject*, PyObject* const*, Py_ssize_t)>
 PyObject* guarded(PyObject* self, PyObject* const* argv, Py_ssize_t n) {
     try {
         return FN(self, argv, n);
+    } catch (const PythonError&) {
     } catch (const c10::OutOfMemoryError& e) {
         PyObject* torch = PyImport_ImportModule("torch");
         PyObject* type = torch ? PyObject_GetAttrString(torch, "OutOfMemoryError") : nullptr;
