@@ -9,6 +9,8 @@
 // The library is not linked: `bind` receives the addresses of its entry points from the ctypes handle.
 #include <Python.h>
 
+#include <cstring>
+
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -44,8 +46,32 @@ struct Args {
         if (a[i] != Py_None) bad = true;
         return nullptr;
     }
-    int64_t num(int i) const { return PyLong_AsLongLong(a[i]); }
-    template <typename T> T* ptr(int i) const { return a[i] == Py_None ? nullptr : reinterpret_cast<T*>(PyLong_AsUnsignedLongLong(a[i])); }
+    // Numbers are taken before the tensors are looked at and while the GIL is held; one that is no number, or does not fit,
+    // ends the call.
+    int64_t num(int i) const {
+        const long long x = PyLong_AsLongLong(a[i]);
+        if (x == -1 && PyErr_Occurred()) throw PythonError();
+        return x;
+    }
+    int i32(int i) const {
+        const int64_t x = num(i);
+        if (x < INT32_MIN || x > INT32_MAX) {
+            PyErr_SetString(PyExc_OverflowError, "argument does not fit 32 bits");
+            throw PythonError();
+        }
+        return (int)x;
+    }
+    float real(int i) const {
+        const double x = PyFloat_AsDouble(a[i]);
+        if (x == -1.0 && PyErr_Occurred()) throw PythonError();
+        return (float)x;
+    }
+    template <typename T> T* ptr(int i) const {
+        if (a[i] == Py_None) return nullptr;
+        const unsigned long long x = PyLong_AsUnsignedLongLong(a[i]);
+        if (x == ~0ull && PyErr_Occurred()) throw PythonError();
+        return reinterpret_cast<T*>(x);
+    }
     bool truth(int i) const {
         const int r = PyObject_IsTrue(a[i]);
         if (r < 0) throw PythonError();
@@ -76,7 +102,7 @@ PyObject* layer_step(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     if (n != 7) return none();
     const Args A{argv};
     const auto* s = A.ptr<const BgtqLayerStep>(0);
-    const int64_t dev = A.num(1);
+    const int dev = A.i32(1);
     bool bad = false;
     const at::Tensor *q = A.tensor(2, bad), *k = A.tensor(3, bad), *v = A.tensor(4, bad), *cs = A.tensor(5, bad), *sn = A.tensor(6, bad);
     if (bad || !is(q, 4, at::kHalf) || !is(k, 4, at::kHalf) || !is(v, 4, at::kHalf)) return none();
@@ -108,7 +134,7 @@ PyObject* layer_encode(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     if (n != 6) return none();
     const Args A{argv};
     const auto* s = A.ptr<const BgtqLayerStep>(0);
-    const int64_t dev = A.num(1), t0 = A.num(4);
+    const int dev = A.i32(1), t0 = A.i32(4), flags = A.i32(5);
     bool bad = false;
     const at::Tensor *k = A.tensor(2, bad), *v = A.tensor(3, bad);
     if (bad || !is(k, 4, at::kHalf) || !is(v, 4, at::kHalf) || k->get_device() != dev || v->get_device() != dev || k->sizes() != v->sizes() ||
@@ -118,7 +144,7 @@ PyObject* layer_encode(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     int rc;
     Py_BEGIN_ALLOW_THREADS
     rc = F.layer_encode(s, k->data_ptr(), k->stride(0), k->stride(1), k->stride(2), v->data_ptr(), v->stride(0), v->stride(1), v->stride(2),
-                        (int)k->size(2), (int)t0, (int)A.num(5), st);
+                        (int)k->size(2), t0, flags, st);
     Py_END_ALLOW_THREADS
     return code(rc);
 }
@@ -127,7 +153,10 @@ PyObject* layer_encode(PyObject*, PyObject* const* argv, Py_ssize_t n) {
 PyObject* encode(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     if (n != 13) return none();
     const Args A{argv};
-    const int64_t n_kv = A.num(3), vpb = A.num(4), t0 = A.num(7), flags = A.num(12);
+    const auto* desc = A.ptr<const BgtqHeadDesc>(0);
+    const auto* rot_k = A.ptr<const float>(1);
+    const auto* rot_v = A.ptr<const float>(2);
+    const int n_kv = A.i32(3), vpb = A.i32(4), t0 = A.i32(7), flags = A.i32(12);
     bool bad = false;
     const at::Tensor *k = A.tensor(5, bad), *v = A.tensor(6, bad), *kp = A.tensor(8, bad), *kn = A.tensor(9, bad), *vp = A.tensor(10, bad),
                      *vn = A.tensor(11, bad);
@@ -137,11 +166,11 @@ PyObject* encode(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     void* const st = stream_of(*k);
     int rc;
     Py_BEGIN_ALLOW_THREADS
-    rc = F.encode(A.ptr<const BgtqHeadDesc>(0), A.ptr<const float>(1), A.ptr<const float>(2), k->data_ptr(), k->stride(0), k->stride(1),
-                  k->stride(2), v->data_ptr(), v->stride(0), v->stride(1), v->stride(2), (int)k->size(0), (int)n_kv, (int)k->size(2), (int)t0,
+    rc = F.encode(desc, rot_k, rot_v, k->data_ptr(), k->stride(0), k->stride(1),
+                  k->stride(2), v->data_ptr(), v->stride(0), v->stride(1), v->stride(2), (int)k->size(0), n_kv, (int)k->size(2), t0,
                   kp->data_ptr<uint8_t>(), kp->stride(0), kp->stride(1), kp->stride(2), (int)kp->size(3), kn->data_ptr(), kn->stride(0),
                   kn->stride(1), kn->stride(2), (int)kn->size(3), vp->data_ptr<uint8_t>(), vp->stride(0), vp->stride(1), vp->stride(2),
-                  vn->data_ptr(), vn->stride(0), vn->stride(1), vn->stride(2), nullptr, nullptr, (int)(flags | BGTQ_ENC_K_NORMS_F16), nullptr,
+                  vn->data_ptr(), vn->stride(0), vn->stride(1), vn->stride(2), nullptr, nullptr, flags | BGTQ_ENC_K_NORMS_F16, nullptr,
                   (int)kp->size(2), nullptr, st);
     Py_END_ALLOW_THREADS
     return code(rc);
@@ -152,7 +181,10 @@ PyObject* encode(PyObject*, PyObject* const* argv, Py_ssize_t n) {
 PyObject* compress(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     if (n != 7) return none();
     const Args A{argv};
-    const int64_t n_kv = A.num(2), rb = A.num(4), ng = A.num(5);
+    const auto* desc = A.ptr<const BgtqHeadDesc>(0);
+    const auto* rot = A.ptr<const float>(1);
+    const int64_t n_kv = A.i32(2), rb = A.i32(4), ng = A.i32(5);
+    const int flags = A.i32(6);
     bool bad = false;
     const at::Tensor* x = A.tensor(3, bad);
     if (bad || !is(x, 3, at::kHalf) || !x->is_contiguous() || x->size(0) != n_kv || x->size(2) != kHD) return none();
@@ -160,9 +192,6 @@ PyObject* compress(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     at::Tensor packed = empty({n_kv, N, rb}, at::kByte, *x);
     at::Tensor norms = ng ? empty({n_kv, N, ng}, at::kFloat, *x) : empty({n_kv, N}, at::kHalf, *x);
     void* const st = stream_of(*x);
-    const int flags = (int)A.num(6);
-    const auto* desc = A.ptr<const BgtqHeadDesc>(0);
-    const auto* rot = A.ptr<const float>(1);
     int rc;
     Py_BEGIN_ALLOW_THREADS
     rc = ng ? F.encode(desc, rot, nullptr, x->data_ptr(), 0, N * kHD, kHD, nullptr, 0, 0, 0, 1, (int)n_kv, (int)N, 0, packed.data_ptr<uint8_t>(), 0,
@@ -182,35 +211,36 @@ PyObject* compress(PyObject*, PyObject* const* argv, Py_ssize_t n) {
 PyObject* attend(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     if (n != 19) return none();
     const Args A{argv};
+    const auto* plan = A.ptr<const BgtqDecodePlan>(0);
+    const auto* desc = A.ptr<const BgtqHeadDesc>(1);
+    const auto* rot_k = A.ptr<const float>(2);
+    const int t0 = A.i32(8), t1 = A.i32(9), n_kv = A.i32(18);
+    int ns = A.i32(10);
+    const float scale = A.real(11);
+    const auto* v_rot = A.ptr<const float>(12);
+    const bool want32 = A.truth(15), want_lse = A.truth(16);
+    auto* status = A.ptr<int32_t>(17);
     bool bad = false;
     const at::Tensor *q = A.tensor(3, bad), *kp = A.tensor(4, bad), *kn = A.tensor(5, bad), *vp = A.tensor(6, bad), *vn = A.tensor(7, bad),
                      *bo = A.tensor(13, bad), *bl = A.tensor(14, bad);
     const bool four = q && q->dim() == 4;
     if (bad || !is(q, four ? 4 : 3, at::kHalf) || (four && q->size(2) != 1) || q->size(-1) != kHD || !here(*q) || !cache_ok(kp, kn, vp, vn))
         return none();
-    const auto* rot_k = A.ptr<const float>(2);
     if (!rot_k && !q->is_contiguous()) return none();
-    const int64_t B = q->size(0), n_q = q->size(1), t0 = A.num(8), t1 = A.num(9), n_kv = A.num(18);
+    const int64_t B = q->size(0), n_q = q->size(1);
     if (kp->size(0) < B || kp->size(1) != n_kv || t1 > kp->size(2)) return none();
-    int64_t ns = A.num(10);
-    if (ns < 1) ns = F.default_splits((int)B, (int)n_kv, (int)(t1 - t0));
-    const bool want32 = A.truth(15), want_lse = A.truth(16);
+    if (ns < 1) ns = F.default_splits((int)B, n_kv, t1 - t0);
     at::Tensor scratch = empty({B * n_q * (ns * (kHD + 1) + kHD / 2)}, at::kFloat, *q);
     at::Tensor out = four ? empty({B, n_q, 1, kHD}, at::kHalf, *q) : empty({B, n_q, kHD}, at::kHalf, *q);
     at::Tensor o32, lse;
     if (want32) o32 = empty({B, n_q, kHD}, at::kFloat, *q);
     if (want_lse) lse = empty({B, n_q}, at::kFloat, *q);
     void* const st = stream_of(*q);
-    const float scale = (float)PyFloat_AsDouble(argv[11]);
-    const auto* plan = A.ptr<const BgtqDecodePlan>(0);
-    const auto* desc = A.ptr<const BgtqHeadDesc>(1);
-    const auto* v_rot = A.ptr<const float>(12);
-    auto* status = A.ptr<int32_t>(17);
     int rc;
     Py_BEGIN_ALLOW_THREADS
     rc = F.attend(plan, desc, rot_k, q->data_ptr(), q->stride(0), q->stride(1), kp->data_ptr<uint8_t>(), kp->stride(0), kp->stride(1), kp->stride(2),
                   kn->data_ptr(), kn->stride(0), kn->stride(1), kn->stride(2), vp->data_ptr<uint8_t>(), vp->stride(0), vp->stride(1), vp->stride(2),
-                  vn->data_ptr(), vn->stride(0), vn->stride(1), vn->stride(2), (int)B, (int)n_q, (int)n_kv, (int)t0, (int)t1, (int)ns, scale, v_rot,
+                  vn->data_ptr(), vn->stride(0), vn->stride(1), vn->stride(2), (int)B, (int)n_q, n_kv, t0, t1, ns, scale, v_rot,
                   bo ? bo->data_ptr<float>() : nullptr, bl ? bl->data_ptr<float>() : nullptr, scratch.data_ptr(), out.data_ptr(),
                   want32 ? o32.data_ptr<float>() : nullptr, want_lse ? lse.data_ptr<float>() : nullptr, status, st);
     Py_END_ALLOW_THREADS
@@ -222,6 +252,9 @@ PyObject* attend(PyObject*, PyObject* const* argv, Py_ssize_t n) {
 PyObject* rotate_rows(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     if (n != 4) return none();
     const Args A{argv};
+    const auto* desc = A.ptr<const BgtqHeadDesc>(0);
+    const auto* rot_k = A.ptr<const float>(1);
+    const int n_kv = A.i32(2);
     bool bad = false;
     const at::Tensor* q = A.tensor(3, bad);
     if (bad || !is(q, 4, at::kHalf) || q->size(3) != kHD || q->numel() == 0 || !here(*q)) return none();
@@ -230,8 +263,8 @@ PyObject* rotate_rows(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     void* const st = stream_of(*q);
     int rc;
     Py_BEGIN_ALLOW_THREADS
-    rc = F.rotate_rows(A.ptr<const BgtqHeadDesc>(0), A.ptr<const float>(1), q->data_ptr(), q->stride(0), q->stride(1), q->stride(2), out.data_ptr(),
-                       (int)q->size(0), (int)q->size(1), (int)A.num(2), (int)q->size(2), st);
+    rc = F.rotate_rows(desc, rot_k, q->data_ptr(), q->stride(0), q->stride(1), q->stride(2), out.data_ptr(),
+                       (int)q->size(0), (int)q->size(1), n_kv, (int)q->size(2), st);
     Py_END_ALLOW_THREADS
     return rc == BGTQ_OK ? wrap(std::move(out)) : code(rc);
 }
@@ -241,24 +274,24 @@ PyObject* rotate_rows(PyObject*, PyObject* const* argv, Py_ssize_t n) {
 PyObject* prefill(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     if (n != 14) return none();
     const Args A{argv};
+    const auto* desc = A.ptr<const BgtqHeadDesc>(0);
+    const int n_kv = A.i32(1), T = A.i32(7), off = A.i32(8), causal = A.truth(9) ? 1 : 0, flags = A.i32(11);
+    const float scale = A.real(10);
+    const auto* v_rot = A.ptr<const float>(12);
+    const int64_t bound = A.num(13);
     bool bad = false;
     const at::Tensor *q = A.tensor(2, bad), *kp = A.tensor(3, bad), *kn = A.tensor(4, bad), *vp = A.tensor(5, bad), *vn = A.tensor(6, bad);
     if (bad || !is(q, 4, at::kHalf) || q->size(3) != kHD || q->numel() == 0 || !here(*q) || !cache_ok(kp, kn, vp, vn)) return none();
-    const int64_t B = q->size(0), n_q = q->size(1), S = q->size(2), n_kv = A.num(1), T = A.num(7), off = A.num(8);
-    const int causal = A.truth(9) ? 1 : 0;
-    const auto* v_rot = A.ptr<const float>(12);
-    const int64_t ws_bytes = F.prefill_workspace((int)B, (int)n_q, (int)n_kv, (int)S, (int)T, (int)off, causal, v_rot ? 1 : 0);
-    if (B > 1 && ws_bytes > A.num(13)) return none();
+    const int64_t B = q->size(0), n_q = q->size(1), S = q->size(2);
+    const int64_t ws_bytes = F.prefill_workspace((int)B, (int)n_q, n_kv, (int)S, T, off, causal, v_rot ? 1 : 0);
+    if (B > 1 && ws_bytes > bound) return none();
     at::Tensor ws = empty({ws_bytes > 16 ? ws_bytes : 16}, at::kByte, *q), out = empty({B, n_q, S, kHD}, at::kHalf, *q);
     void* const st = stream_of(*q);
-    const float scale = (float)PyFloat_AsDouble(argv[10]);
-    const int flags = (int)A.num(11);
-    const auto* desc = A.ptr<const BgtqHeadDesc>(0);
     int rc;
     Py_BEGIN_ALLOW_THREADS
     rc = F.prefill(desc, q->data_ptr(), q->stride(0), q->stride(1), q->stride(2), kp->data_ptr<uint8_t>(), kp->stride(0), kp->stride(1), kp->stride(2),
                    kn->data_ptr(), kn->stride(0), kn->stride(1), kn->stride(2), vp->data_ptr<uint8_t>(), vp->stride(0), vp->stride(1), vp->stride(2),
-                   vn->data_ptr(), vn->stride(0), vn->stride(1), vn->stride(2), (int)B, (int)n_q, (int)n_kv, (int)S, (int)T, (int)off, causal,
+                   vn->data_ptr(), vn->stride(0), vn->stride(1), vn->stride(2), (int)B, (int)n_q, n_kv, (int)S, T, off, causal,
                    scale, flags, v_rot, ws.data_ptr(), ws.numel(), out.data_ptr(), st);
     Py_END_ALLOW_THREADS
     return rc == BGTQ_OK ? wrap(std::move(out)) : code(rc);
@@ -270,7 +303,10 @@ PyObject* bind(PyObject*, PyObject* const* argv, Py_ssize_t n) {
         PyErr_SetString(PyExc_ValueError, "bind: wrong number of addresses");
         return nullptr;
     }
-    for (Py_ssize_t i = 0; i < n; ++i) reinterpret_cast<void**>(&F)[i] = PyLong_AsVoidPtr(argv[i]);
+    const Args A{argv};
+    void* fns[sizeof(F) / sizeof(void*)];
+    for (Py_ssize_t i = 0; i < n; ++i) fns[i] = A.ptr<void>((int)i);
+    memcpy(&F, fns, sizeof(F));
     return none();
 }
 

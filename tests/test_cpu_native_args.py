@@ -1,0 +1,48 @@
+"""The native calls take their numbers as Python takes them: one that is no number, or does not fit, is an exception."""
+import pytest
+import torch
+
+from blockgtq_b200 import _lib
+
+X3, X4 = torch.zeros(1, 4, 128, dtype=torch.float16), torch.zeros(1, 1, 4, 128, dtype=torch.float16)
+U8, N3 = torch.zeros(1, 1, 4, 48, dtype=torch.uint8), torch.zeros(1, 1, 4, dtype=torch.float16)
+CALLS = {       # function: (arguments, {position: kind of number})
+    "layer_step": ([0, 0, X4, X4, X4, None, None], {0: "ptr", 1: "i32"}),
+    "layer_encode": ([0, 0, X4, X4, 0, 0], {0: "ptr", 1: "i32", 4: "i32", 5: "i32"}),
+    "encode": ([0, 0, 0, 1, 48, X4, X4, 0, U8, X4, U8, N3, 0], {0: "ptr", 1: "ptr", 2: "ptr", 3: "i32", 4: "i32", 7: "i32", 12: "i32"}),
+    "compress": ([0, 0, 1, X3, 48, 0, 0], {0: "ptr", 1: "ptr", 2: "i32", 4: "i32", 5: "i32", 6: "i32"}),
+    "attend": ([0, 0, None, X3, U8, X4, U8, N3, 0, 4, 1, 1.0, None, None, None, False, False, None, 1],
+               {0: "ptr", 1: "ptr", 2: "ptr", 8: "i32", 9: "i32", 10: "i32", 11: "real", 12: "ptr", 15: "truth", 16: "truth", 17: "ptr",
+                18: "i32"}),
+    "rotate_rows": ([0, 0, 1, X4], {0: "ptr", 1: "ptr", 2: "i32"}),
+    "prefill": ([0, 1, X4, U8, X4, U8, N3, 4, 0, True, 1.0, 0, None, 1 << 40],
+                {0: "ptr", 1: "i32", 7: "i32", 8: "i32", 9: "truth", 10: "real", 11: "i32", 12: "ptr", 13: "i64"}),
+}
+
+
+class NoTruth:
+    def __bool__(self):
+        raise ValueError("no truth")
+
+
+@pytest.mark.parametrize("name", list(CALLS))
+def test_bad_numbers_raise(name):
+    fn = getattr(_lib.host(), name)
+    args, numbers = CALLS[name]
+    assert fn(*args) is None                     # CPU tensors: left to the Python wrapper
+    for i, kind in numbers.items():
+        bad = {"truth": [(NoTruth(), ValueError)], "real": [("1.0", TypeError)],
+               "i32": [("3", TypeError), (2.0, TypeError), (1 << 40, OverflowError), (-(1 << 31) - 1, OverflowError)],
+               "i64": [("3", TypeError), (1 << 70, OverflowError)], "ptr": [("3", TypeError), (-1, OverflowError)]}[kind]
+        for value, error in bad:
+            with pytest.raises(error):
+                fn(*args[:i], value, *args[i + 1:])
+    if name == "attend":                          # -1 is a number like any other
+        assert fn(*args[:8], -1, *args[9:]) is None
+
+
+def test_bind_takes_addresses_only():
+    with pytest.raises(TypeError):
+        _lib.host().bind(*["x"] * 8)
+    with pytest.raises(ValueError):
+        _lib.host().bind(0)

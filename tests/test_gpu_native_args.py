@@ -29,3 +29,17 @@ def test_true_flags_of_other_types_ask_for_the_lse(flag):
     out, lse = fused_blockgtq_decode_attention(*args, return_lse=flag, **kw)
     ref = fused_blockgtq_decode_attention(*args, return_lse=True, **kw)
     assert torch.equal(out, ref[0]) and torch.equal(lse, ref[1])
+
+
+def test_ranges_may_be_any_whole_numbers():
+    from blockgtq_b200 import BlockGTQKVManager
+    from helpers import HD, synth_head
+    gen = torch.Generator().manual_seed(4)
+    mgr = BlockGTQKVManager(1, 2, 1, HD, max_seq_len=64, device=DEV)
+    qs, ks = synth_head(gen, 256, 2)
+    mgr.calibrate(0, qs.float(), ks.float())
+    mgr.init_from_cache([tuple(torch.randn(1, 1, 40, HD, generator=gen).half().to(DEV) for _ in range(2))])
+    q = torch.randn(1, 2, 1, HD, generator=gen).half().to(DEV)
+    want = mgr.attend(0, q, token_range=(3, 39), n_splits=2)[0]
+    for lo, hi, n in ((np.int64(3), np.int32(39), np.int64(2)), (3.0, 39.0, 2.0), (torch.tensor(3), torch.tensor(39), torch.tensor(2))):
+        assert torch.equal(mgr.attend(0, q, token_range=(lo, hi), n_splits=n)[0], want)
