@@ -205,7 +205,7 @@ PyObject* compress(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     return Py_BuildValue("(NN)", wrap(std::move(packed)), wrap(std::move(norms)));
 }
 
-// attend(plan, desc, rot_k | None, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, n_splits | 0, scale, v_rot | None,
+// attend(plan, desc, rot_k | None, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, n_splits (0: the library's), scale, v_rot | None,
 //        buf_o | None, buf_lse | None, want_f32, want_lse, status | None, n_kv) -> (out, f32 | None, lse | None) | code | None
 // q (B, n_q, [1,] 128); out has q's rank.
 PyObject* attend(PyObject*, PyObject* const* argv, Py_ssize_t n) {
@@ -220,6 +220,7 @@ PyObject* attend(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     const auto* v_rot = A.ptr<const float>(12);
     const bool want32 = A.truth(15), want_lse = A.truth(16);
     auto* status = A.ptr<int32_t>(17);
+    if (ns < 0) return code(BGTQ_E_BADARG);
     bool bad = false;
     const at::Tensor *q = A.tensor(3, bad), *kp = A.tensor(4, bad), *kn = A.tensor(5, bad), *vp = A.tensor(6, bad), *vn = A.tensor(7, bad),
                      *bo = A.tensor(13, bad), *bl = A.tensor(14, bad);
@@ -229,7 +230,7 @@ PyObject* attend(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     if (!rot_k && !q->is_contiguous()) return none();
     const int64_t B = q->size(0), n_q = q->size(1);
     if (kp->size(0) < B || kp->size(1) != n_kv || t1 > kp->size(2)) return none();
-    if (ns < 1) ns = F.default_splits((int)B, n_kv, t1 - t0);
+    if (ns == 0) ns = F.default_splits((int)B, n_kv, t1 - t0);
     at::Tensor scratch = empty({B * n_q * (ns * (kHD + 1) + kHD / 2)}, at::kFloat, *q);
     at::Tensor out = four ? empty({B, n_q, 1, kHD}, at::kHalf, *q) : empty({B, n_q, kHD}, at::kHalf, *q);
     at::Tensor o32, lse;

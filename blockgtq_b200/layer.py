@@ -404,7 +404,7 @@ def attend(layer, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, *, ro
     """Query rotation (``rotate``: q is in the original basis), split-KV decode over rows [t_begin, t_end) and combine
     in one library call.  q (B, n_q, [1,] 128) -> (out fp16 of q's shape, f32 copy (B, n_q, 128) | None, LSE | None)."""
     plan, ptr = layer.plan(flags | _lib.DEC_PROGRAMMATIC), _lib.ptr
-    t_begin, t_end, n_splits = int(t_begin), int(t_end), 0 if n_splits is None else int(n_splits)
+    t_begin, t_end, n_splits = int(t_begin), int(t_end), 0 if n_splits is None else int(n_splits) or -1       # (0 is refused like -1)
 
     def call():
         return _lib.host().attend(

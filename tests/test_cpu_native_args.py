@@ -37,8 +37,9 @@ def test_bad_numbers_raise(name):
         for value, error in bad:
             with pytest.raises(error):
                 fn(*args[:i], value, *args[i + 1:])
-    if name == "attend":                          # -1 is a number like any other
+    if name == "attend":                          # -1 is a number like any other, but no count of splits
         assert fn(*args[:8], -1, *args[9:]) is None
+        assert fn(*args[:10], -1, *args[11:]) == -1
 
 
 def test_bind_takes_addresses_only():

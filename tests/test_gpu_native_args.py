@@ -43,3 +43,6 @@ def test_ranges_may_be_any_whole_numbers():
     want = mgr.attend(0, q, token_range=(3, 39), n_splits=2)[0]
     for lo, hi, n in ((np.int64(3), np.int32(39), np.int64(2)), (3.0, 39.0, 2.0), (torch.tensor(3), torch.tensor(39), torch.tensor(2))):
         assert torch.equal(mgr.attend(0, q, token_range=(lo, hi), n_splits=n)[0], want)
+    for n in (0, -1):
+        with pytest.raises(RuntimeError, match="bad argument"):
+            mgr.attend(0, q, n_splits=n)
