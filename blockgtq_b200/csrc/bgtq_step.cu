@@ -10,6 +10,11 @@
 
 using namespace bgtq;
 
+// The query rows of (n_batch, n_q) heads lie one behind the other; the stride of a dim of one element says nothing.
+static bool contiguous_rows(int32_t n_batch, int32_t n_q, int64_t q_sb, int64_t q_sh) {
+    return (n_q == 1 || q_sh == kHD) && (n_batch == 1 || q_sb == (int64_t)n_q * kHD);
+}
+
 extern "C" __attribute__((visibility("default"))) int bgtq_layer_step_size(void) { return (int)sizeof(BgtqLayerStep); }
 
 extern "C" __attribute__((visibility("default"))) int bgtq_layer_step(
@@ -21,7 +26,7 @@ extern "C" __attribute__((visibility("default"))) int bgtq_layer_step(
     const void* q_dec = s->q_rot;
     const bool rotate = !(s->flags & BGTQ_STEP_Q_ROTATED);
     if (!rotate) {      // the queries arrive in the packed-K basis: the decode reads them where they are
-        if (q_sh != kHD || (s->n_batch > 1 && q_sb != (int64_t)s->n_q * kHD)) return BGTQ_E_UNSUPPORTED;
+        if (!contiguous_rows(s->n_batch, s->n_q, q_sb, q_sh)) return BGTQ_E_UNSUPPORTED;
         q_dec = q;
     }
     int rc;
@@ -90,7 +95,7 @@ extern "C" __attribute__((visibility("default"))) int bgtq_attend(
         const int rc = launch_rotate_q(desc, rot_k, q, q_sb, q_sh, q_rot, n_batch, n_q, n_kv, true, static_cast<cudaStream_t>(stream));
         if (rc != BGTQ_OK) return rc;
         q_dec = q_rot;
-    } else if (q_sh != kHD || (n_batch > 1 && q_sb != (int64_t)n_q * kHD)) {
+    } else if (!contiguous_rows(n_batch, n_q, q_sb, q_sh)) {
         return BGTQ_E_UNSUPPORTED;
     }
     // No early fetch here, whatever the plan says: what is in front of this call may be a bulk encode of the very rows

@@ -47,3 +47,19 @@ def test_bind_takes_addresses_only():
         _lib.host().bind(*["x"] * 8)
     with pytest.raises(ValueError):
         _lib.host().bind(0)
+
+
+def test_strides_of_single_heads_and_batches_do_not_matter():
+    """Queries in the packed basis have to lie one behind the other; with one head or one batch entry any stride of that
+    dim says so.  (A plan without a table image is refused before anything is launched: -1, where strides are -2.)"""
+    import ctypes as C
+    L, plan = _lib.lib(), _lib.DecodePlan()
+    buf = C.create_string_buffer(1 << 16)
+    a = (C.addressof(buf) + 255) & ~255
+
+    def attend(B, n_q, sb, sh):
+        return L.bgtq_attend(C.addressof(plan), None, None, a, sb, sh, a, 0, 0, 48, a, 0, 0, 2, a, 0, 0, 48, a, 0, 0, 1, B, n_q, 1, 0, 4, 1,
+                             1.0, None, None, None, a, a, None, None, None, None)
+
+    assert attend(1, 4, 7, 128) == attend(1, 1, 7, 4096) == attend(3, 1, 128, 4096) == attend(2, 4, 512, 128) == -1
+    assert attend(1, 4, 512, 4096) == attend(2, 1, 4096, 128) == attend(2, 4, 1024, 128) == -2

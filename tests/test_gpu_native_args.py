@@ -46,3 +46,26 @@ def test_ranges_may_be_any_whole_numbers():
     for n in (0, -1):
         with pytest.raises(RuntimeError, match="bad argument"):
             mgr.attend(0, q, n_splits=n)
+
+
+def test_one_query_head_cut_out_of_a_larger_tensor():
+    """(B, 1, 1, 128) views whose head dim of one has another tensor's stride: one query head per KV head."""
+    from blockgtq_b200 import fused_blockgtq_decode_attention
+    from blockgtq_b200.quantizer import BlockGTQQuantizer
+    from helpers import HD, synth_head
+    gen = torch.Generator().manual_seed(5)
+    qz = BlockGTQQuantizer(HD, avg_bits=3.0, device=torch.device(DEV))
+    qs, ks = synth_head(gen, 256, 1)
+    qz.calibrate(qs.float(), ks.float())
+    qz.init_v_quantizer(v_bits=3, seed=42)
+    ka = qz.build_kernel_args()
+    kp, kn, _ = qz.compress_packed(torch.randn(1, 1, 50, HD, generator=gen).half().to(DEV))
+    vp, vn = qz.compress_v_packed(torch.randn(1, 1, 50, HD, generator=gen).half().to(DEV))
+    q = torch.randn(1, 1, 9, HD, generator=gen).half().to(DEV)[:, :, 4:5]
+    assert q.is_contiguous() and q.stride(1) != HD
+
+    def run(q):
+        return fused_blockgtq_decode_attention(q, kp, kn.half(), ka["codebook_flat"], ka["lut_offset"], ka["norm_group"], ka["segments_b"],
+                                               vp, vn, qz.v_lut, v_bits=3, v_rotation=qz._v_rot)
+
+    assert torch.equal(run(q), run(q.clone()))
