@@ -18,7 +18,8 @@ import torch
 from . import _lib
 from .layer import HD, attend, make_decode_plan, tile_flags
 
-_cache = {}
+_cache = {}           # tables by the full description of the tensors they were made of
+_recent = {}          # the latest tensors seen at an address, with their tables
 
 
 class _AdHocLayer:
@@ -53,17 +54,38 @@ class _AdHocLayer:
         return p[0]
 
 
+def _version(t):
+    return None if t.is_inference() else t._version
+
+
+def _stamp(t):
+    """What a tensor holds, as far as that can be known without reading it: where it lies, how, and how often it was
+    written in place (inference tensors do not count that)."""
+    return t.data_ptr(), t.dtype, t.shape, t.stride(), _version(t)
+
+
 def _layer_for(segments, codebook_flat, v_lut, v_bits, n_kv, device):
-    key = (tuple(map(tuple, segments)), codebook_flat.data_ptr(), v_lut.data_ptr(), int(v_bits), n_kv, device)
-    lt = _cache.get(key)
+    """The tables made of these arguments, kept from call to call (making them reads the tensors back to the host).  The
+    caches keep the tensors they go by alive, so that no other tensor can come to lie at such an address."""
+    rest = (tuple(map(tuple, segments)), int(v_bits), n_kv, device)
+    key = (codebook_flat.data_ptr(), v_lut.data_ptr(), rest)
+    hit = _recent.get(key)          # the very same tensors as in an earlier call: their versions say the rest
+    if hit is not None and hit[0] is codebook_flat and hit[1] is v_lut and (hit[2] is None or hit[2] == codebook_flat._version) and \
+            (hit[3] is None or hit[3] == v_lut._version):
+        return hit[4]
+    full = (_stamp(codebook_flat), _stamp(v_lut), rest)
+    lt = _cache.get(full)
     if lt is None:
         segs = tuple(tuple(int(x) for x in s) for s in segments)
         raw = [s for s in segs if s[0] > 4 and s[2] > 0]
         nopack = (min(s[1] for s in raw), sum(s[2] for s in raw)) if raw else (HD, 0)
         lt = _AdHocLayer(segs, codebook_flat, v_lut, v_bits, n_kv, nopack, device)
+        lt.sources = (codebook_flat, v_lut)
         if len(_cache) > 4096:
             _cache.clear()
-        _cache[key] = lt
+            _recent.clear()
+        _cache[full] = lt
+    _recent[key] = (codebook_flat, v_lut, _version(codebook_flat), _version(v_lut), lt)
     return lt
 
 
