@@ -271,7 +271,7 @@ PyObject* rotate_rows(PyObject*, PyObject* const* argv, Py_ssize_t n) {
 }
 
 // prefill(desc, n_kv, q, k_packed, k_norms, v_packed, v_norms, n_tokens, q_pos_offset, causal, scale, flags, v_rot | None, bound)
-//   -> tensor | code | None; None too when the workspace would be larger than `bound` bytes and the batch has several entries
+//   -> tensor | code | None; None too when the workspace would be larger than `bound` bytes
 PyObject* prefill(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     if (n != 14) return none();
     const Args A{argv};
@@ -285,7 +285,7 @@ PyObject* prefill(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     if (bad || !is(q, 4, at::kHalf) || q->size(3) != kHD || q->numel() == 0 || !here(*q) || !cache_ok(kp, kn, vp, vn)) return none();
     const int64_t B = q->size(0), n_q = q->size(1), S = q->size(2);
     const int64_t ws_bytes = F.prefill_workspace((int)B, (int)n_q, n_kv, (int)S, T, off, causal, v_rot ? 1 : 0);
-    if (B > 1 && ws_bytes > bound) return none();
+    if (ws_bytes > bound) return none();
     at::Tensor ws = empty({ws_bytes > 16 ? ws_bytes : 16}, at::kByte, *q), out = empty({B, n_q, S, kHD}, at::kHalf, *q);
     void* const st = stream_of(*q);
     int rc;

@@ -441,6 +441,8 @@ def tile_flags(n_batch: int, n_kv: int, n_tokens: int, device) -> int:
     loads each query fragment for twice the tokens, is faster."""
     index = device.index if device.index is not None else torch.cuda.current_device()
     return _lib.DEC_NARROW if n_batch * n_kv * n_tokens <= 256 * _sm_count(index) else 0
+
+
 _PREFILL_WORKSPACE = 2 << 30        # bytes of dequantised operand tiles per launch
 
 
@@ -450,58 +452,71 @@ def prefill_attention(layer: LayerTables, q_rot, k_packed, k_norms, v_packed, v_
     query i has absolute position ``q_pos_offset + i`` and, when ``causal``, sees tokens up to it.
     ``v_rot`` (n_kv, 128, 128) fp32 = R finishes V's rotation.
     Returns (B, n_q, S_q, 128) fp16.  ``_lib.PF_NO_TCGEN05`` in ``flags`` (or the environment variable
-    ``BGTQ_PF_NO_TCGEN05``) keeps the products on mma.sync instead of tcgen05 / tensor memory."""
-    if os.environ.get("BGTQ_PF_NO_TCGEN05"):
-        flags |= _lib.PF_NO_TCGEN05
-    if not flags & _lib.PF_NO_TCGEN05:
-        r = _lib.host().prefill(layer.desc_dev.data_ptr(), layer.n_kv, q_rot, k_packed, k_norms, v_packed, v_norms, int(n_tokens),
-                                int(q_pos_offset), bool(causal), _SCALE if scale is None else scale, int(flags),
-                                None if v_rot is None else v_rot.data_ptr(), _PREFILL_WORKSPACE)
-        if r is not None:
-            return _lib.done(r, "bgtq_prefill", 2)
+    ``BGTQ_PF_NO_TCGEN05``) keeps the products on mma.sync instead of tcgen05 / tensor memory.
+
+    The tcgen05 form dequantises the cache into a workspace from torch's allocator, 768 bytes per token and KV head
+    and at most 2 GiB at a time (the batch, then the KV heads, in several launches beyond that).  Where the device
+    has no room for it, the call runs on mma.sync, which reads the packed rows themselves."""
+    scale = _SCALE if scale is None else scale
+    n_tokens, q_pos_offset, causal, flags = int(n_tokens), int(q_pos_offset), bool(causal), int(flags)
+    if not (flags & _lib.PF_NO_TCGEN05 or os.environ.get("BGTQ_PF_NO_TCGEN05")):
+        try:
+            r = _lib.host().prefill(layer.desc_dev.data_ptr(), layer.n_kv, q_rot, k_packed, k_norms, v_packed, v_norms, n_tokens,
+                                    q_pos_offset, causal, scale, flags, None if v_rot is None else v_rot.data_ptr(),
+                                    _PREFILL_WORKSPACE)
+            if r is not None:
+                return _lib.done(r, "bgtq_prefill", 2)
+            return _prefill_parts(layer, q_rot, k_packed, k_norms, v_packed, v_norms, n_tokens, q_pos_offset, causal, scale, flags, v_rot)
+        except torch.OutOfMemoryError:
+            pass
+    qs, kps, kns, vps, vns = _prefill_strides(q_rot, k_packed, k_norms, v_packed, v_norms)
+    B, n_q, S_q, _ = q_rot.shape
+    dev = q_rot.device
+    out_rot = torch.empty(B, n_q, S_q, HD, dtype=torch.float32, device=dev)
+    _lib.check(_lib.lib().bgtq_prefill_attention(
+        _lib.ptr(layer.desc_dev), _lib.ptr(q_rot), *qs, _lib.ptr(k_packed), *kps, _lib.ptr(k_norms), *kns,
+        _lib.ptr(v_packed), *vps, _lib.ptr(v_norms), *vns, B, n_q, layer.n_kv, S_q, n_tokens, q_pos_offset, causal,
+        float(scale), flags | _lib.PF_NO_TCGEN05, _lib.ptr(out_rot), _lib.stream_ptr(dev)), "bgtq_prefill_attention")
+    _lib.count_launch()
+    if v_rot is None:
+        return out_rot.to(torch.float16)
+    gqa = n_q // layer.n_kv
+    o = torch.matmul(out_rot.view(B, layer.n_kv, gqa * S_q, HD), v_rot.view(1, layer.n_kv, HD, HD))
+    return o.view(B, n_q, S_q, HD).to(torch.float16)
+
+
+def _prefill_strides(q_rot, k_packed, k_norms, v_packed, v_norms):
     _lib.require_cuda(q_rot, "q_rot")
-    B, n_q, S_q, D = q_rot.shape
-    if D != HD or q_rot.dtype != torch.float16 or q_rot.stride(3) != 1:
+    if q_rot.dim() != 4 or q_rot.shape[3] != HD or q_rot.dtype != torch.float16 or q_rot.stride(3) != 1:
         raise ValueError("q_rot must be float16 (B, n_q, S_q, 128) with contiguous rows")
     if k_norms.dtype != torch.float16 or v_norms.dtype != torch.float16:
         raise TypeError("cache norms must be float16")
-    if scale is None:
-        scale = 1.0 / math.sqrt(HD)
-    dev = q_rot.device
-    qs, kps, kns, vps = q_rot.stride()[:3], _strides3(k_packed), _strides3(k_norms), _strides3(v_packed)
-    vns = v_norms.stride()[:3]
-    L, causal = _lib.lib(), 1 if causal else 0
-    n_tokens, q_pos_offset = int(n_tokens), int(q_pos_offset)
-    if flags & _lib.PF_NO_TCGEN05:
-        out_rot = torch.empty(B, n_q, S_q, HD, dtype=torch.float32, device=dev)
-        _lib.check(L.bgtq_prefill_attention(
-            _lib.ptr(layer.desc_dev), _lib.ptr(q_rot), *qs, _lib.ptr(k_packed), *kps, _lib.ptr(k_norms), *kns,
-            _lib.ptr(v_packed), *vps, _lib.ptr(v_norms), *vns, B, n_q, layer.n_kv, S_q, n_tokens, q_pos_offset, causal,
-            float(scale), int(flags), _lib.ptr(out_rot), _lib.stream_ptr(dev)), "bgtq_prefill_attention")
-        _lib.count_launch()
-        if v_rot is None:
-            return out_rot.to(torch.float16)
-        gqa = n_q // layer.n_kv
-        o = torch.matmul(out_rot.view(B, layer.n_kv, gqa * S_q, HD), v_rot.view(1, layer.n_kv, HD, HD))
-        return o.view(B, n_q, S_q, HD).to(torch.float16)
+    return q_rot.stride()[:3], _strides3(k_packed), _strides3(k_norms), _strides3(v_packed), v_norms.stride()[:3]
+
+
+def _prefill_parts(layer, q_rot, k_packed, k_norms, v_packed, v_norms, n_tokens, q_pos_offset, causal, scale, flags, v_rot):
+    """The tcgen05 form in as many launches as keep the dequantised tiles within their bound: fewer batch entries per
+    launch first, then (one entry) fewer KV heads; one of each at least."""
+    qs, kps, kns, vps, vns = _prefill_strides(q_rot, k_packed, k_norms, v_packed, v_norms)
+    B, n_q, S_q, _ = q_rot.shape
+    n_kv, gqa, dev, L = layer.n_kv, n_q // layer.n_kv, q_rot.device, _lib.lib()
+
+    def ws_bytes(n, m):
+        return L.bgtq_prefill_workspace_bytes(n, m * gqa, m, S_q, n_tokens, q_pos_offset, causal, v_rot is not None)
+
+    nb, nh = B, n_kv
+    while ws_bytes(nb, nh) > _PREFILL_WORKSPACE and nb * nh > 1:
+        nb, nh = ((nb + 1) // 2, nh) if nb > 1 else (1, (nh + 1) // 2)
+    parts = [(b, min(nb, B - b), h, min(nh, n_kv - h)) for b in range(0, B, nb) for h in range(0, n_kv, nh)]
+    ws = torch.empty(max([16] + [ws_bytes(n, m) for _, n, _, m in parts]), dtype=torch.uint8, device=dev)
     out = torch.empty(B, n_q, S_q, HD, dtype=torch.float16, device=dev)
-
-    def ws_bytes(n):
-        return L.bgtq_prefill_workspace_bytes(n, n_q, layer.n_kv, S_q, n_tokens, q_pos_offset, causal, v_rot is not None)
-
-    # as many batch entries per launch as keep the dequantised tiles within the bound (one at least)
-    nb = B
-    while nb > 1 and ws_bytes(nb) > _PREFILL_WORKSPACE:
-        nb = (nb + 1) // 2
-    size = max(ws_bytes(nb), ws_bytes(B % nb) if B % nb else 0)
-    ws = torch.empty(max(size, 16), dtype=torch.uint8, device=dev)
-    for b in range(0, B, nb):
-        n = min(nb, B - b)
-        sl = slice(b, b + n)
+    for b, n, h, m in parts:        # (with fewer heads than all there is one batch entry: its heads' rows are contiguous)
+        bs, hs, qh = slice(b, b + n), slice(h, h + m), slice(h * gqa, (h + m) * gqa if m < n_kv else n_q)
         _lib.check(L.bgtq_prefill(
-            _lib.ptr(layer.desc_dev), q_rot[sl].data_ptr(), *qs, k_packed[sl].data_ptr(), *kps, k_norms[sl].data_ptr(), *kns,
-            v_packed[sl].data_ptr(), *vps, v_norms[sl].data_ptr(), *vns, n, n_q, layer.n_kv, S_q, n_tokens, q_pos_offset, causal,
-            float(scale), int(flags), _lib.ptr(v_rot), ws.data_ptr(), ws.numel(), out[sl].data_ptr(), _lib.stream_ptr(dev)),
+            layer.desc_dev.data_ptr() + h * C.sizeof(_lib.HeadDesc), q_rot[bs, qh].data_ptr(), *qs, k_packed[bs, hs].data_ptr(), *kps,
+            k_norms[bs, hs].data_ptr(), *kns, v_packed[bs, hs].data_ptr(), *vps, v_norms[bs, hs].data_ptr(), *vns, n,
+            m * gqa if m < n_kv else n_q, m, S_q, n_tokens, q_pos_offset, causal, float(scale), flags,
+            None if v_rot is None else v_rot[hs].data_ptr(), ws.data_ptr(), ws.numel(), out[bs, qh].data_ptr(), _lib.stream_ptr(dev)),
             "bgtq_prefill")
         _lib.count_launch(2)
     return out
