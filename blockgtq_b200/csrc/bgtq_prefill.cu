@@ -391,20 +391,17 @@ extern "C" __attribute__((visibility("default"))) int bgtq_prefill_attention(
     if (reinterpret_cast<uintptr_t>(out_rot) & 7u) return BGTQ_E_ALIGN;
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (!(flags & BGTQ_PF_NO_TCGEN05) && !(reinterpret_cast<uintptr_t>(out_rot) & 15u)) {
-        // the caller of this form has no workspace to give: take it from the stream's pool for the launch
+        // the caller of this form has no workspace to give: take it from the stream's pool for the launch; where the pool
+        // has none, the form below needs none
         void* ws = nullptr;
         const int64_t n = prefill_t5_workspace(n_batch, n_q, n_kv, s_q, n_tokens, q_pos_offset, causal != 0, false);
-        cudaError_t e = cudaMallocAsync(&ws, (size_t)(n > 16 ? n : 16), st);
-        if (e == cudaSuccess) {
-            e = launch_prefill_t5(P, n_batch, nullptr, static_cast<uint8_t*>(ws), nullptr, out_rot, st);
-            const cudaError_t f = cudaFreeAsync(ws, st);
-            if (e == cudaSuccess) e = f;
-        }
-        if (e != cudaSuccess) {
+        if (cudaMallocAsync(&ws, (size_t)(n > 16 ? n : 16), st) == cudaSuccess) {
+            const cudaError_t e = launch_prefill_t5(P, n_batch, nullptr, static_cast<uint8_t*>(ws), nullptr, out_rot, st);
+            if (cudaFreeAsync(ws, st) == cudaSuccess && e == cudaSuccess) return BGTQ_OK;
             cudaGetLastError();
             return BGTQ_E_LAUNCH;
         }
-        return BGTQ_OK;
+        cudaGetLastError();
     }
     P.out = out_rot;
     const int bq = kPfRows / P.gqa;

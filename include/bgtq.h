@@ -8,7 +8,8 @@
  * Conventions
  *   - every pointer is a DEVICE pointer unless the comment says "host";
  *   - the caller owns all memory; no entry point allocates, frees or
- *     synchronises (bgtq_*_noalloc: see its own comment);
+ *     synchronises (but for bgtq_prefill_attention, which takes a workspace
+ *     from the stream's pool, and bgtq_*_noalloc: see their own comments);
  *   - work is enqueued on `stream` (a cudaStream_t passed as void*);
  *   - return value: BGTQ_OK or a negative BGTQ_E_* code; nothing throws;
  *   - strides are in ELEMENTS of the pointed-to type unless stated in bytes;
@@ -479,8 +480,10 @@ int bgtq_attend(const BgtqDecodePlan* plan, const BgtqHeadDesc* desc, const floa
  * yields zeros.  n_q / n_kv <= 16.
  * The products run on tcgen05 with accumulators in tensor memory (bgtq_prefill_t5.cu), or, with
  * BGTQ_PF_NO_TCGEN05 in flags, on mma.sync (bgtq_prefill.cu).  The tcgen05 form dequantises the cache once into
- * a workspace, which this entry point takes from the stream's memory pool for the launch (cudaMallocAsync);
- * bgtq_prefill below takes the caller's and is the one to call repeatedly.  The tcgen05 form bounds its waits;
+ * a workspace of bgtq_prefill_workspace_bytes(..., 0) bytes, which this entry point takes from the stream's memory
+ * pool for the launch and gives back behind it (cudaMallocAsync / cudaFreeAsync); where the pool cannot give it,
+ * the call runs on mma.sync, which needs none.  bgtq_prefill below takes the caller's workspace and is the one to call
+ * repeatedly, or beside another allocator that holds the device's memory.  The tcgen05 form bounds its waits;
  * bgtq_prefill_tcgen05_status() returns 1 (sticky, per process) if one ever gave up, in which case that
  * launch's output is invalid. */
 #define BGTQ_PF_NO_TCGEN05 16
@@ -497,8 +500,8 @@ int bgtq_prefill_attention(const BgtqHeadDesc* desc, const void* q_rot, int64_t 
 /* The same (tcgen05 form) with the caller's workspace and the finished output: out (n_batch, n_q, s_q, 128) fp16
  * contiguous, 16-byte aligned, multiplied by v_rot (n_kv, 128, 128) fp32 = R when that is not NULL.  workspace:
  * device memory of bgtq_prefill_workspace_bytes(...) bytes for the same shape (768 bytes per cached token and KV
- * head, rounded up to 128 tokens, plus partial outputs when the launch has so few query rows that the cache is cut
- * among several CTAs), 16-byte aligned; its contents mean nothing after the launch. */
+ * head, one and a half times those tokens in fp16, rounded up to 128 tokens, plus partial outputs when the launch has so
+ * few query rows that the cache is cut among several CTAs), 16-byte aligned; its contents mean nothing after the launch. */
 int64_t bgtq_prefill_workspace_bytes(int32_t n_batch, int32_t n_q, int32_t n_kv, int32_t s_q, int32_t n_tokens,
                 int32_t q_pos_offset, int32_t causal, int32_t with_rotation);
 int bgtq_prefill(const BgtqHeadDesc* desc, const void* q_rot, int64_t q_sb, int64_t q_sh, int64_t q_ss,

@@ -80,3 +80,40 @@ def test_no_room_for_the_workspace():
         del fill
     again = layer.prefill_attention(lt, q_rot, *cache, T, **args).float()
     assert ((again - want.float()).abs() <= 1e-3 + want.float().abs() * 2.0 ** -10).all()
+
+
+def test_entry_point_without_a_workspace():
+    """bgtq_prefill_attention takes its workspace from the stream's pool; a pool that cannot give it changes the kernel."""
+    from blockgtq_b200 import _lib
+    from helpers import HD
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    B, n_kv, gqa, T, S_q = 1, 2, 3, 60000, 50
+    lt, q_rot, (kp, kn, vp, vn) = _case(B, n_kv, gqa, T, S_q)
+
+    def run(flags):
+        out = torch.full((B, n_kv * gqa, S_q, HD), float("nan"), device=DEV)
+        rc = _lib.lib().bgtq_prefill_attention(
+            lt.desc_dev.data_ptr(), q_rot.data_ptr(), *q_rot.stride()[:3], kp.data_ptr(), *kp.stride()[:3], kn.data_ptr(), *kn.stride()[:3],
+            vp.data_ptr(), *vp.stride()[:3], vn.data_ptr(), *vn.stride()[:3], B, n_kv * gqa, n_kv, S_q, T, T - S_q, 1, 1.0 / HD ** 0.5, flags,
+            out.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        torch.cuda.synchronize()
+        return out
+
+    mma, t5 = run(_lib.PF_NO_TCGEN05), run(0)
+    assert not torch.equal(mma, t5) and ((t5 - mma).abs() <= 1e-3 + mma.abs() * 2.0 ** -10).all()
+    props = rt.cudaMemPoolProps()
+    props.allocType = rt.cudaMemAllocationType.cudaMemAllocationTypePinned
+    props.location.type, props.location.id = rt.cudaMemLocationType.cudaMemLocationTypeDevice, 0
+    props.maxSize = 1 << 20                     # (pools grow in steps of some 32 MB; the workspace takes 92)
+    err, small = rt.cudaMemPoolCreate(props)
+    assert err == rt.cudaError_t.cudaSuccess
+    err, usual = rt.cudaDeviceGetMemPool(0)
+    assert err == rt.cudaError_t.cudaSuccess
+    try:
+        assert rt.cudaDeviceSetMemPool(0, small)[0] == rt.cudaError_t.cudaSuccess
+        assert torch.equal(run(0), mma)
+    finally:
+        rt.cudaDeviceSetMemPool(0, usual)
+        rt.cudaMemPoolDestroy(small)
+    assert torch.equal(run(0), t5)
