@@ -180,6 +180,10 @@ def lib():
     loader = importlib.machinery.ExtensionFileLoader("_native", _build.NATIVE)
     module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_native", loader))
     loader.exec_module(module)
+    built_for = getattr(module, "abi", "another version")
+    if built_for != _build.native_abi():
+        raise RuntimeError(f"{_build.NATIVE} was built for {built_for}, this is {_build.native_abi()}: rebuild it "
+                           "(python -m blockgtq_b200.build --force)")
     module.bind(*[C.cast(getattr(handle, name), C.c_void_p).value for name in (
         "bgtq_layer_step", "bgtq_layer_encode", "bgtq_attend", "bgtq_decode_default_splits", "bgtq_encode", "bgtq_rotate_q_rows",
         "bgtq_prefill", "bgtq_prefill_workspace_bytes")])

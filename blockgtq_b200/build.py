@@ -19,6 +19,7 @@ CSRC = os.path.join(PKG, "csrc")
 LIB = os.environ.get("BGTQ_LIB") or os.path.join(PKG, "libbgtq.so")
 NATIVE_SRC = os.path.join(CSRC, "bgtq_native.cpp")
 NATIVE = os.path.join(PKG, "_native.so")
+NATIVE_STAMP = os.path.join(PKG, "build", "native.abi")         # the versions it was built for
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "--use_fast_math=false", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
 
@@ -34,9 +35,23 @@ def sources() -> list:
     return sorted(glob.glob(os.path.join(CSRC, "*.cu")))
 
 
+def native_abi() -> str:
+    """What the extension module is bound to beyond its sources: torch's internal C++ API and the Python ABI."""
+    import sysconfig
+
+    import torch
+    return f"torch {torch.__version__}, {sysconfig.get_config_var('SOABI')}"
+
+
 def needs_build() -> bool:
     if not os.path.exists(LIB) or not os.path.exists(NATIVE):
         return True
+    try:
+        with open(NATIVE_STAMP) as f:
+            if f.read() != native_abi():
+                return True
+    except OSError:
+        pass            # (the module says it itself when it is loaded)
     header = os.path.join(os.path.dirname(PKG), "include", "bgtq.h")
     if os.path.getmtime(NATIVE) < max(os.path.getmtime(NATIVE_SRC), os.path.getmtime(header)):
         return True
@@ -75,6 +90,7 @@ def _native_cmd(out: str) -> list:
     inc = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
            os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
     return [cxx, "-shared", "-fPIC", "-O2", "-std=c++17", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            f'-DBGTQ_NATIVE_ABI="{native_abi()}"',
             *[x for d in inc for x in ("-isystem", d)], NATIVE_SRC, "-o", out, "-L", os.path.join(base, "lib"),
             "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
 
@@ -113,6 +129,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if native.returncode != 0:
         raise RuntimeError("building the host extension failed: " + " ".join(native_cmd) + "\n" + out)
     os.replace(NATIVE + ".tmp", NATIVE)
+    with open(NATIVE_STAMP, "w") as f:
+        f.write(native_abi())
     return LIB
 
 

@@ -336,4 +336,8 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, 
 
 }  // namespace
 
-extern "C" __attribute__((visibility("default"))) PyObject* PyInit__native(void) { return PyModule_Create(&kModule); }
+extern "C" __attribute__((visibility("default"))) PyObject* PyInit__native(void) {
+    PyObject* m = PyModule_Create(&kModule);
+    if (m && PyModule_AddStringConstant(m, "abi", BGTQ_NATIVE_ABI) != 0) Py_CLEAR(m);
+    return m;
+}
