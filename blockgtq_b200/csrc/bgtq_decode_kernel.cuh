@@ -491,7 +491,9 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
 
     // Everything up to grid_dependency_wait() touches only static tables, so under a programmatic
     // launch it overlaps the tail of the preceding kernel (the step's append / query rotation).
-    grid_launch_dependents();
+    // The launch behind this one (the combine, which reads V's rotation ahead of its own wait) may start once this one has
+    // waited: whatever was enqueued in front of this kernel is complete by then.  (No later than before in effect: its CTAs
+    // find room only as this kernel's end; 438.4 us before, 438.8 so for two layers of 32 sequences of 16384 tokens.)
 
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);                      // [kDecStages]
     uint64_t* lutbar = full + kDecStages;
@@ -558,7 +560,10 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
     // With early fetch (see bgtq_decode_plan_set_early_fetch) the wait moves behind the first tile requests.
     const int early_fresh = P.plan.early_fresh;
     bool dep_waited = early_fresh <= 0;
-    if (dep_waited) grid_dependency_wait();
+    if (dep_waited) {
+        grid_dependency_wait();
+        grid_launch_dependents();
+    }
     // ---- this CTA's range of items ---------------------------------------------------------------------
     // (32-bit unsigned arithmetic: a 64-bit division costs a few hundred cycles of every CTA's start-up, and
     // item counts that need one do not occur: the launch wrapper rejects them)
@@ -669,6 +674,7 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
                     tables_pending = false;
                 }
                 grid_dependency_wait();
+                grid_launch_dependents();
                 dep_waited = true;
                 if (warp == 0)
                     for (int it = held; it < last; ++it) issue_tile(R, it, g_it + it);

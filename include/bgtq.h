@@ -100,7 +100,9 @@ const char* bgtq_error_string(int code);       /* host pointer to a static strin
  * bgtq_rotate_q_rows, bgtq_prefill and bgtq_prefill_attention (tcgen05 form), bgtq_buffer_attn and
  * bgtq_buffer_attn_pos, bgtq_exchange_merge, and the rotation and the combine of bgtq_attend.  A kernel of this
  * library also lets the launch behind it, if that is a programmatic one, become resident early; ordinary launches
- * behind it wait for its end as always. */
+ * behind it wait for its end as always.
+ * Static tables (descriptors, rotations, plan images, item-range tables) are read ahead of the wait: what writes them
+ * belongs in front of the launch that precedes the call. */
 
 /* Encode K and V rows of all KV heads of one layer and write them straight
  * into their cache slots.

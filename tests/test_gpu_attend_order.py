@@ -131,3 +131,42 @@ def test_layer_step_behind_a_bulk_encode(batch, n_kv, T):
     for i, r in enumerate(got):
         assert all(torch.equal(a, b) for a, b in zip(r, want[i & 1])), i
     mgr.check_status()
+
+
+def test_operator_with_a_rotation_made_for_the_call():
+    """The operator's V rotation may be a tensor that the call itself converts: the merge reads it as converted, not as its
+    memory was a moment before."""
+    from blockgtq_b200 import fused_blockgtq_decode_attention
+    from blockgtq_b200.quantizer import BlockGTQQuantizer
+    from helpers import HD, synth_head
+    gen = torch.Generator().manual_seed(6)
+    qz = BlockGTQQuantizer(HD, avg_bits=3.0, device=torch.device(DEV))
+    qs, ks = synth_head(gen, 256, 2)
+    qz.calibrate(qs.float(), ks.float())
+    qz.init_v_quantizer(v_bits=3, seed=42)
+    ka = qz.build_kernel_args()
+    kp, kn, _ = qz.compress_packed(torch.randn(1, 1, 700, HD, generator=gen).half().to(DEV))
+    vp, vn = qz.compress_v_packed(torch.randn(1, 1, 700, HD, generator=gen).half().to(DEV))
+    q = torch.randn(1, 2, 1, HD, generator=gen).half().to(DEV)
+    rots = [torch.linalg.qr(torch.randn(HD, HD, generator=gen))[0].half().to(DEV) for _ in range(2)]
+    kn = kn.half()
+
+    def run(rot):
+        return fused_blockgtq_decode_attention(q, kp, kn, ka["codebook_flat"], ka["lut_offset"], ka["norm_group"], ka["segments_b"],
+                                               vp, vn, qz.v_lut, v_bits=3, v_rotation=rot)
+
+    want = []
+    for r in rots:
+        r32 = r.float()
+        torch.cuda.synchronize()
+        want.append(run(r32).clone())
+        torch.cuda.synchronize()
+    busy = _Busy()
+    got = []
+    for i in range(60):
+        busy()
+        got.append(run(rots[i & 1]))
+        got.append(run(rots[1 - (i & 1)]))
+    torch.cuda.synchronize()
+    for i in range(60):
+        assert torch.equal(got[2 * i], want[i & 1]) and torch.equal(got[2 * i + 1], want[1 - (i & 1)]), i
