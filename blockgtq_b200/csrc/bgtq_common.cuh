@@ -160,9 +160,18 @@ __device__ __forceinline__ float f16_bits_to_float(uint32_t h) {
 // while its predecessor in the stream still runs).  grid_launch_dependents lets the NEXT kernel's blocks
 // become resident early; grid_dependency_wait blocks until the PREVIOUS kernel has completed and its
 // writes are visible.  Both are no-ops for a kernel launched the ordinary way.  Every kernel of a chain
-// executes the wait before it ends, so completion stays transitive along the stream.
+// executes the wait before it ends, so completion stays transitive along the stream.  Data that an earlier launch of the
+// stream may write while this kernel is already resident is read with plain loads, never through the read-only path (__ldg).
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// A plain load that stays behind the wait but not behind the stores in front of it (the compiler takes those for possible
+// writes to the same memory).
+__device__ __forceinline__ uint32_t ld_global_u32(const void* p) {
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
 
 #ifndef BGTQ_JIT
 // Launch with or without the programmatic stream-serialization attribute.

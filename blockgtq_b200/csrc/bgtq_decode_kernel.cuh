@@ -688,9 +688,9 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
             const bool q_ok = g < P.gqa;
             const uint16_t* qrow = P.q_rot + ((size_t)b * P.n_q + (size_t)h * P.gqa + (q_ok ? g : 0)) * kHD;
             uint2 v;
-            v.x = (q_ok && pos < (int)st.end) ? __ldg(reinterpret_cast<const uint32_t*>(qrow + pos)) : 0u;
+            v.x = (q_ok && pos < (int)st.end) ? ld_global_u32(qrow + pos) : 0u;
             v.y = (q_ok && (int)st.c4 + 2 < (int)st.q && pos + 2 < (int)st.end)
-                      ? __ldg(reinterpret_cast<const uint32_t*>(qrow + pos + 2)) : 0u;
+                      ? ld_global_u32(qrow + pos + 2) : 0u;
             qfrag[s * 32 + lane] = v;
         }
         if (tables_pending) {

@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kBufThreads) buffer_attn_kernel(const __half* 
         float s0 = 0.f, s1 = 0.f;
 #pragma unroll 8
         for (int c = 0; c < kHD / 8; ++c) {
-            const uint4 kv = __ldg(kr + c);
+            const uint4 kv = kr[c];
             const float4 qa = *reinterpret_cast<const float4*>(qs + 8 * c), qb = *reinterpret_cast<const float4*>(qs + 8 * c + 4);
             const float2 k0 = __half22float2(*reinterpret_cast<const __half2*>(&kv.x));
             const float2 k1 = __half22float2(*reinterpret_cast<const __half2*>(&kv.y));

@@ -80,7 +80,7 @@ __device__ __forceinline__ void up_stage(uint8_t* dst, const uint8_t* src, int n
     for (int i = tid; i < n_words; i += kUpThreads)
         asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d4 + 4u * i), "l"(s4 + 4 * i) : "memory");
     const int tail = (int)((ph + n_bytes) & 3u);
-    if (tid < tail) dst[4 * n_words + tid] = __ldg(s4 + 4 * n_words + tid);
+    if (tid < tail) dst[4 * n_words + tid] = s4[4 * n_words + tid];
 }
 
 // The 32 (or, for raw-byte codes, 64) bits that start at byte p, from aligned 32-bit loads.  Reads up to 11
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kUpThreads, 1) pf_unpack_kernel(const PfParams
             __align__(16) __half hi[8], lo[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                const float w = __ldg(W + (size_t)(8 * k8 + e) * kHD + n) * kRotScale;
+                const float w = W[(size_t)(8 * k8 + e) * kHD + n] * kRotScale;        // (may have been converted right in front)
                 hi[e] = __float2half_rn(w);
                 lo[e] = __float2half_rn(w - __half2float(hi[e]));
             }
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) pf_attend_kernel(const AtParams
         } else {
             const uint32_t* s32 = reinterpret_cast<const uint32_t*>(src);
             *reinterpret_cast<uint4*>(dst) =
-                g < n_rows ? make_uint4(__ldg(s32), __ldg(s32 + 1), __ldg(s32 + 2), __ldg(s32 + 3)) : make_uint4(0, 0, 0, 0);
+                g < n_rows ? make_uint4(s32[0], s32[1], s32[2], s32[3]) : make_uint4(0, 0, 0, 0);
         }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -717,13 +717,13 @@ __global__ void __launch_bounds__(256) pf_merge_kernel(const float* part, const 
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= n_rows) return;
     float mx = -INFINITY;
-    for (int s = 0; s < n_splits; ++s) mx = fmaxf(mx, __ldg(lse2 + s * n_rows + row));
+    for (int s = 0; s < n_splits; ++s) mx = fmaxf(mx, lse2[s * n_rows + row]);
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     float den = 0.f;
     if (mx > -INFINITY) {
         for (int s = 0; s < n_splits; ++s) {
-            const float w = at_exp2(__ldg(lse2 + s * n_rows + row) - mx);
-            const float4 v = __ldg(reinterpret_cast<const float4*>(part + (s * n_rows + row) * kHD) + lane);
+            const float w = at_exp2(lse2[s * n_rows + row] - mx);
+            const float4 v = reinterpret_cast<const float4*>(part + (s * n_rows + row) * kHD)[lane];
             den += w;
             acc.x = fmaf(w, v.x, acc.x); acc.y = fmaf(w, v.y, acc.y); acc.z = fmaf(w, v.z, acc.z); acc.w = fmaf(w, v.w, acc.w);
         }
