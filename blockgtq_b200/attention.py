@@ -18,19 +18,18 @@ import torch
 from . import _lib
 from .layer import HD, attend, make_decode_plan, tile_flags
 
-_cache = {}           # tables by the full description of the tensors they were made of
+_tables = {}          # tables by contents
+_cache = {}           # the same by the full description of the tensors they were made of, with these tensors
 _recent = {}          # the latest tensors seen at an address, with their tables
 
 
 class _AdHocLayer:
     """Minimal stand-in for LayerTables built from operator arguments."""
 
-    def __init__(self, segments, codebook_flat, v_lut, v_bits, n_kv, nopack, device):
+    def __init__(self, segments, cb, vl, v_bits, n_kv, nopack, device):
         self.n_kv = n_kv
         self.device = device
         self.desc_host = (_lib.HeadDesc * n_kv)()
-        cb = codebook_flat.detach().to(torch.float16).cpu().view(torch.int16).numpy().astype(np.uint16)
-        vl = v_lut.detach().to(torch.float16).cpu().view(torch.int16).numpy().astype(np.uint16)
         for h in range(n_kv):
             d = self.desc_host[h]
             d.n_seg = len(segments)
@@ -74,17 +73,23 @@ def _layer_for(segments, codebook_flat, v_lut, v_bits, n_kv, device):
             (hit[3] is None or hit[3] == v_lut._version):
         return hit[4]
     full = (_stamp(codebook_flat), _stamp(v_lut), rest)
-    lt = _cache.get(full)
-    if lt is None:
-        segs = tuple(tuple(int(x) for x in s) for s in segments)
-        raw = [s for s in segs if s[0] > 4 and s[2] > 0]
-        nopack = (min(s[1] for s in raw), sum(s[2] for s in raw)) if raw else (HD, 0)
-        lt = _AdHocLayer(segs, codebook_flat, v_lut, v_bits, n_kv, nopack, device)
-        lt.sources = (codebook_flat, v_lut)
+    entry = _cache.get(full)
+    if entry is None:
+        cb, vl = (t.detach().to(torch.float16).cpu().view(torch.int16).numpy().astype(np.uint16) for t in (codebook_flat, v_lut))
+        contents = (cb.tobytes(), vl.tobytes(), rest)
+        lt = _tables.get(contents)
+        if lt is None:
+            segs = tuple(tuple(int(x) for x in s) for s in segments)
+            raw = [s for s in segs if s[0] > 4 and s[2] > 0]
+            nopack = (min(s[1] for s in raw), sum(s[2] for s in raw)) if raw else (HD, 0)
+            lt = _AdHocLayer(segs, cb, vl, v_bits, n_kv, nopack, device)
         if len(_cache) > 4096:
+            _tables.clear()
             _cache.clear()
             _recent.clear()
-        _cache[full] = lt
+        _tables[contents] = lt
+        entry = _cache[full] = (lt, codebook_flat, v_lut)
+    lt = entry[0]
     _recent[key] = (codebook_flat, v_lut, _version(codebook_flat), _version(v_lut), lt)
     return lt
 

@@ -18,6 +18,7 @@ def test_tables_follow_the_contents():
         lt = _layer_for(SEGS, cb, lut, 3, 1, torch.device("cpu"))
         assert (_codebook(lt) == i).all(), i
         assert _layer_for(SEGS, cb, lut, 3, 1, torch.device("cpu")) is lt
+        assert _layer_for(SEGS, cb.clone(), lut.clone(), 3, 1, torch.device("cpu")) is lt         # equal contents share them
     cb.mul_(2)                  # written in place
     assert (_codebook(_layer_for(SEGS, cb, lut, 3, 1, torch.device("cpu"))) == 38).all()
     lut[3] = 99.0
