@@ -324,6 +324,8 @@ __device__ __forceinline__ void prep_store_v(const EncParams& E, int b, int h, i
         E.vp[b * E.vp_sb + h * E.vp_sh + (size_t)t0 * E.vp_st + p] = (uint8_t)pack_byte(codes, kHD, vb, p);
 }
 
+// Two CTAs of 512 threads per SM leave a thread 64 registers, 32 of which hold its rotation entries: the one-row form spills
+// 16 bytes (28 read back), the four-row form 48 (116).
 template <bool kFourRows>
 __global__ void __launch_bounds__(512, 2) prep_kernel(const PrepParams P) {
     __shared__ float xs[kHD];

@@ -11,7 +11,9 @@
 //     byte position) is uniform over the warp, codes never leave registers, two values share an instruction where they can
 //     (f32x2), and whole 32-bit words of the packed row go to a staging image of the tile that leaves as coalesced words.
 // Bound: instruction issue and its latencies with 16 warps per SM (all registers and shared memory are taken): 1 048 576 K and
-// as many V rows take 452 us (K rows alone 286, V rows 165), where the bytes alone would take 100.  The form before gave a
+// as many V rows take 452 us (K rows alone 286, V rows 164), where the bytes alone would take 100: 133 warp instructions per
+// row, issue slots and the shared-memory pipe 56 % busy each, tensor pipe 13 %, DRAM 16 %.  K rows cost what V's do not: the
+// move into packed order and a norm per group.  The form before gave a
 // quad of lanes four rows and four columns each, loaded three tables per element and passed the codes through shared memory
 // to a packing pass: 204 warp instructions per row and 753 us.  Tried and slower: rolled loops (smaller code, less overlap
 // of the table lookups: 589 us).

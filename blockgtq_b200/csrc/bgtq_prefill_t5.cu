@@ -26,8 +26,9 @@
 // What bounds attend: the tensor pipe.  A tile costs a CTA 2 x 16 products for S and 2 x 8 for O, 64 cycles each at the
 // nominal rate: 3072 cycles, two thirds of them for S because khat takes two passes (its product of two fp16 numbers
 // has 22 significant bits, all of which the reference's fp32 scaling keeps); the exponentials of the tile take the
-// special-function pipe 2048.  Measured for 16384 causal positions x 32 heads over 8 KV heads: 2.41 ms, 912 TFLOP/s of
-// attention and 1370 TFLOP/s of products, at the power limit; unthrottled a tile takes 4070 cycles.
+// special-function pipe 2048.  Measured for 16384 causal positions x 32 heads over 8 KV heads: 2.41 to 2.50 ms in single
+// launches (about 900 TFLOP/s of attention, 1340 of products; tensor pipe 65 % active, special functions 43 %, issue slots
+// 34 %), 2.72 ms where launches follow each other for seconds, at the power limit; unthrottled a tile takes 4070 cycles.
 // Every wait is bounded: a wait that gives up is recorded in a sticky status word and in shared memory, where the
 // other warps' waits see it; the CTA then drains its copies and products, releases its tensor memory and returns.
 #include "bgtq_prefill_common.cuh"

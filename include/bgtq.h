@@ -85,8 +85,8 @@ const char* bgtq_error_string(int code);       /* host pointer to a static strin
 #define BGTQ_ENC_SKIP_V 16
 #define BGTQ_ENC_FORCE_SIMT 32  /* always use the small-batch fp32 kernel (>= 64 rows normally use tensor cores) */
 #define BGTQ_ENC_PROGRAMMATIC 64  /* bgtq_step_prepare*: programmatic dependent launch, see below (bgtq_encode ignores it) */
-#define BGTQ_ENC_NO_TCGEN05 128   /* bulk encode: keep the rotation on mma.sync (bulk row counts of >= 128 rows and packed
-                                   * K rows of <= 120 bytes normally use tcgen05.mma with tensor-memory accumulators) */
+#define BGTQ_ENC_NO_TCGEN05 128   /* bulk encode: keep the rotation on mma.sync (>= 128 rows normally use tcgen05.mma with
+                                   * tensor-memory accumulators) */
 
 /* Programmatic dependent launch (BGTQ_ENC_PROGRAMMATIC, BGTQ_DEC_PROGRAMMATIC,
  * BGTQ_COMBINE_PROGRAMMATIC).  The kernel is launched with CUDA's programmatic
