@@ -704,6 +704,9 @@ static int step_prepare_impl(
     if (!pos_dev && !k_buf && t_capacity > 0 && t0 >= t_capacity) return BGTQ_E_BADARG;
     const bool do_rot = q != nullptr && q_rot != nullptr;
     if (do_rot && (n_q < n_kv || n_q % n_kv)) return BGTQ_E_BADARG;
+    // Nothing to do: no launch.  (CTAs of a skipped side return at once; a programmatic launch of nothing else would end ahead of
+    // the work in front of it, and what waits for this launch would not wait for that work.)
+    if (!do_rot && !k_buf && (flags & BGTQ_ENC_SKIP_K) && (flags & BGTQ_ENC_SKIP_V)) return BGTQ_OK;
     PrepParams P;
     EncParams& E = P.e;
     E.desc = desc; E.rot_k = rot_k; E.rot_v = rot_v;

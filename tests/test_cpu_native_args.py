@@ -63,3 +63,18 @@ def test_strides_of_single_heads_and_batches_do_not_matter():
 
     assert attend(1, 4, 7, 128) == attend(1, 1, 7, 4096) == attend(3, 1, 128, 4096) == attend(2, 4, 512, 128) == -1
     assert attend(1, 4, 512, 4096) == attend(2, 1, 4096, 128) == attend(2, 4, 1024, 128) == -2
+
+
+def test_a_preparation_with_nothing_to_do_launches_nothing():
+    import ctypes as C
+    L = _lib.lib()
+    buf = C.create_string_buffer(1 << 12)
+    a = (C.addressof(buf) + 255) & ~255
+
+    def prepare(flags, q=None):
+        return L.bgtq_step_prepare(a, a, a, q, 0, 128, q, 1, a, 0, 128, a, 0, 128, 1, 1, 0, a, 0, 0, 48, 48, a, 0, 0, 2, 2, a, 0, 0, 48,
+                                   a, 0, 0, 1, flags | _lib.ENC_PROGRAMMATIC, None, 4, None, None)
+
+    assert prepare(_lib.ENC_SKIP_K | _lib.ENC_SKIP_V) == 0
+    if not torch.cuda.is_available():       # (everything else is launched, and there is nothing to launch on)
+        assert prepare(_lib.ENC_SKIP_K) == prepare(_lib.ENC_SKIP_K | _lib.ENC_SKIP_V, a) == -4

@@ -170,3 +170,41 @@ def test_operator_with_a_rotation_made_for_the_call():
     torch.cuda.synchronize()
     for i in range(60):
         assert torch.equal(got[2 * i], want[i & 1]) and torch.equal(got[2 * i + 1], want[1 - (i & 1)]), i
+
+
+def test_a_preparation_with_nothing_to_do_keeps_the_order():
+    """A step preparation that skips both sides and has no queries still ends behind the work in front of it."""
+    from blockgtq_b200 import _lib
+    from blockgtq_b200.layer import LayerTables, decode, encode, step_prepare
+    from helpers import HD, tables_for
+    n_kv, T = 2, 2000
+    tabs = [tables_for("a3_1to8", h) for h in range(n_kv)]
+    lt = LayerTables([t[0] for t in tabs], [t[1] for t in tabs], DEV)
+    gen = torch.Generator(device=DEV).manual_seed(9)
+    cache = (torch.zeros(1, n_kv, T + 8, lt.max_tpb, dtype=torch.uint8, device=DEV), torch.zeros(1, n_kv, T + 8, lt.max_ng, dtype=torch.float16, device=DEV),
+             torch.zeros(1, n_kv, T + 8, lt.vpb, dtype=torch.uint8, device=DEV), torch.zeros(1, n_kv, T + 8, dtype=torch.float16, device=DEV))
+    prompts = [_kv(gen, 1, n_kv, T) for _ in range(2)]
+    one = _kv(gen, 1, n_kv, 1)
+    q = torch.randn(1, 2 * n_kv, HD, generator=gen, device=DEV).half()
+    n_splits = 8
+
+    def run(i, sync):
+        encode(lt, *prompts[i], 0, *cache)
+        sync()
+        step_prepare(lt, None, *one, T, *cache, flags=_lib.ENC_SKIP_K | _lib.ENC_SKIP_V | _lib.ENC_PROGRAMMATIC)
+        sync()
+        part_o = torch.zeros(1, 2 * n_kv, n_splits, HD, device=DEV) if sync is torch.cuda.synchronize else parts.pop()
+        part_lse = torch.empty(1, 2 * n_kv, n_splits, device=DEV)
+        return decode(lt, q, *cache, 0, T, n_splits=n_splits, flags=_lib.DEC_PROGRAMMATIC, part_o=part_o, part_lse=part_lse)
+
+    want = [run(i, torch.cuda.synchronize) for i in range(2)]
+    assert not torch.equal(want[0][1], want[1][1])
+    parts = [torch.zeros(1, 2 * n_kv, n_splits, HD, device=DEV) for _ in range(60)]        # (nothing ordinary is enqueued in between)
+    busy = _Busy()
+    got = []
+    for i in range(60):
+        busy()
+        got.append(run(i & 1, lambda: None))
+    torch.cuda.synchronize()
+    for i, (o, lse) in enumerate(got):
+        assert torch.equal(o, want[i & 1][0]) and torch.equal(lse, want[i & 1][1]), i
