@@ -379,6 +379,9 @@ class BlockGTQKVManager:
         """rotate_q + append K,V at *pos -> decode over [0, *pos + 1) -> (fp16 regions) -> combine into
         ``static_outputs()[li]``, one library call; q/k/v (B, heads, 1, hd) fp16 with unit last stride."""
         s = self._step_args(li)
+        if s.flags & _lib.STEP_Q_ROTATED and not q.is_contiguous():     # (the static buffer's batch entries hold k and v too)
+            self._q_rot.copy_(q[:, :, 0])
+            q = self._q_rot
         qs, ks, vs = q.stride(), k.stride(), v.stride()
         cos = sin = None
         r_sb = 0
