@@ -256,16 +256,24 @@ def rotate_q(layer: LayerTables, q: torch.Tensor, out: torch.Tensor = None) -> t
     return out
 
 
+def _transformed(t: torch.Tensor) -> bool:
+    """A tensor that torch has to see the operations of: gradients (either mode), vmap and the like, tensor subclasses."""
+    return (t.requires_grad and torch.is_grad_enabled()) or type(t) is not torch.Tensor or torch.autograd.forward_ad._current_level >= 0 or \
+        torch._C._functorch.peek_interpreter_stack() is not None
+
+
 def rotate_q_bulk(layer: LayerTables, q: torch.Tensor) -> torch.Tensor:
     """Many positions at once: q (B, n_q, S, 128) -> same shape, fp16, in the packed-K basis (the per-row kernel
-    behind :func:`rotate_q` is meant for the handful of rows of a decode step).  fp16 queries go through the
-    tensor cores; queries of another type are rotated in fp32 first and rounded once."""
-    r = _lib.host().rotate_rows(layer.desc_dev.data_ptr(), layer.rot_k.data_ptr(), layer.n_kv, q)
-    if r is not None:
-        return _lib.done(r, "bgtq_rotate_q_rows")
-    _lib.require_cuda(q, "q")
+    behind :func:`rotate_q` is meant for the handful of rows of a decode step).  fp16 queries on the GPU go through the
+    tensor cores; queries of another type, on the CPU, or that torch differentiates or maps over, are rotated in fp32 by torch's
+    own operators and rounded once."""
+    fast = q.dtype == torch.float16 and q.is_cuda and not _transformed(q)
+    if fast:
+        r = _lib.host().rotate_rows(layer.desc_dev.data_ptr(), layer.rot_k.data_ptr(), layer.n_kv, q)
+        if r is not None:
+            return _lib.done(r, "bgtq_rotate_q_rows")
     B, n_q, S, D = q.shape
-    if q.dtype == torch.float16:
+    if fast:
         st = q.stride()
         if st[3] != 1 or (q.data_ptr() | 2 * (st[0] | st[1] | st[2])) & 15:
             q = q.contiguous()
