@@ -471,6 +471,10 @@ def prefill_attention(layer: LayerTables, q_rot, k_packed, k_norms, v_packed, v_
     has no room for it, the call runs on mma.sync, which reads the packed rows themselves."""
     scale = _SCALE if scale is None else scale
     n_tokens, q_pos_offset, causal, flags = int(n_tokens), int(q_pos_offset), bool(causal), int(flags)
+    if v_rot is not None:       # the kernels take its address
+        if v_rot.dtype != torch.float32 or v_rot.device != q_rot.device:
+            raise TypeError("v_rot must be float32 on the queries' device")
+        v_rot = v_rot.view(layer.n_kv, HD, HD).contiguous()
     if not (flags & _lib.PF_NO_TCGEN05 or os.environ.get("BGTQ_PF_NO_TCGEN05")):
         try:
             r = _lib.host().prefill(layer.desc_dev.data_ptr(), layer.n_kv, q_rot, k_packed, k_norms, v_packed, v_norms, n_tokens,

@@ -117,3 +117,19 @@ def test_entry_point_without_a_workspace():
         rt.cudaDeviceSetMemPool(0, usual)
         rt.cudaMemPoolDestroy(small)
     assert torch.equal(run(0), t5)
+
+
+def test_rotation_in_any_layout():
+    """V's rotation as a transposed view, as a matrix of its own for one head, as rows of all heads; another type is an error."""
+    from blockgtq_b200 import layer
+    from helpers import HD
+    for n_kv in (1, 3):
+        lt, q_rot, cache = _case(1, n_kv, 2, 300, 40)
+        args = dict(q_pos_offset=260, causal=True)
+        want = layer.prefill_attention(lt, q_rot, *cache, 300, v_rot=lt.v_rot, **args)
+        turned = lt.v_rot.transpose(1, 2).contiguous().transpose(1, 2)
+        for rot in [turned, lt.v_rot.reshape(n_kv * HD, HD)] + ([lt.v_rot[0], turned[0]] if n_kv == 1 else []):
+            assert torch.equal(layer.prefill_attention(lt, q_rot, *cache, 300, v_rot=rot, **args), want)
+        for bad in (lt.v_rot.half(), lt.v_rot[:, :, :64], lt.v_rot.cpu()):
+            with pytest.raises((TypeError, RuntimeError)):
+                layer.prefill_attention(lt, q_rot, *cache, 300, v_rot=bad, **args)
