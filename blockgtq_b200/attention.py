@@ -66,12 +66,14 @@ def _stamp(t):
 def _layer_for(segments, codebook_flat, v_lut, v_bits, n_kv, device):
     """The tables made of these arguments, kept from call to call (making them reads the tensors back to the host).  The
     caches keep the tensors they go by alive, so that no other tensor can come to lie at such an address."""
-    rest = (tuple(map(tuple, segments)), int(v_bits), n_kv, device)
-    key = (codebook_flat.data_ptr(), v_lut.data_ptr(), rest)
-    hit = _recent.get(key)          # the very same tensors as in an earlier call: their versions say the rest
-    if hit is not None and hit[0] is codebook_flat and hit[1] is v_lut and (hit[2] is None or hit[2] == codebook_flat._version) and \
-            (hit[3] is None or hit[3] == v_lut._version):
-        return hit[4]
+    key = (tuple(map(tuple, segments)), codebook_flat.data_ptr(), v_lut.data_ptr(), v_bits, n_kv, device)
+    hit = _recent.get(key)
+    if hit is not None:             # the very same tensors as in an earlier call: their versions say the rest
+        cb, vl, cb_version, vl_version, lt = hit
+        if cb is codebook_flat and vl is v_lut and (cb_version is None or cb_version == cb._version) and \
+                (vl_version is None or vl_version == vl._version):
+            return lt
+    rest = (key[0], v_bits, n_kv, device)
     full = (_stamp(codebook_flat), _stamp(v_lut), rest)
     entry = _cache.get(full)
     if entry is None:

@@ -412,7 +412,7 @@ def attend(layer, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, *, ro
     """Query rotation (``rotate``: q is in the original basis), split-KV decode over rows [t_begin, t_end) and combine
     in one library call.  q (B, n_q, [1,] 128) -> (out fp16 of q's shape, f32 copy (B, n_q, 128) | None, LSE | None)."""
     plan, ptr = layer.plan(flags | _lib.DEC_PROGRAMMATIC), _lib.ptr
-    t_begin, t_end, n_splits = int(t_begin), int(t_end), 0 if n_splits is None else int(n_splits) or -1       # (0 is refused like -1)
+    n_splits = 0 if n_splits is None else n_splits or -1       # (the library's choice; 0 is refused like -1)
 
     def call():
         return _lib.host().attend(
@@ -420,7 +420,11 @@ def attend(layer, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, *, ro
             t_begin, t_end, n_splits, _SCALE if scale is None else scale, None if v_rot is None else ptr(v_rot), buf_o, buf_lse,
             want_f32, want_lse, None if status is None else ptr(status), layer.n_kv)
 
-    r = call()
+    try:
+        r = call()
+    except TypeError:       # (ranges as whole floats, say)
+        t_begin, t_end, n_splits = int(t_begin), int(t_end), int(n_splits)
+        r = call()
     if r is None:           # another type or layout, or an argument to complain about
         _lib.require_cuda(q, "q")
         if k_norms.dtype != torch.float16 or v_norms.dtype != torch.float16:
