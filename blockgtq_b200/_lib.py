@@ -24,6 +24,7 @@ OK = 0
 ENC_K_NORMS_F16, ENC_K_MIXED, ENC_V_NIBBLE, ENC_SKIP_K, ENC_SKIP_V, ENC_FORCE_SIMT, ENC_PROGRAMMATIC = 1, 2, 4, 8, 16, 32, 64
 ENC_NO_TCGEN05 = 128
 DEC_K_MIXED, DEC_V_NIBBLE, DEC_PROGRAMMATIC, DEC_GENERIC, DEC_NARROW = 1, 2, 4, 8, 32
+DEC_CLUSTER_SHIFT = 8
 PF_NO_TCGEN05 = 16
 COMBINE_PROGRAMMATIC = 1
 STEP_Q_ROTATED = 1
@@ -114,6 +115,7 @@ _SIGNATURES = {
     "bgtq_decode_plan_set_partition": (C.c_int, [_vp, _vp]),
     "bgtq_decode_plan_set_early_fetch": (C.c_int, [_vp, _i32]),
     "bgtq_decode_plan_set_row_strides": (C.c_int, [_vp, _i32, _i32, _i32, _i32]),
+    "bgtq_decode_plan_cluster": (C.c_int, [_vp]),
     "bgtq_decode_grid_size": (C.c_int, [_i32, _i32, _i32]),
     "bgtq_decode_partition": (C.c_int, [_i32, _i32, _i32, _i32, _i32, _vp, _i32]),
     "bgtq_decode_plan_specialize": (C.c_int, [_vp, _i32, C.c_char_p, _i64]),

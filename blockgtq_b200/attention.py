@@ -16,7 +16,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .layer import HD, attend, make_decode_plan, tile_flags
+from .layer import HD, attend, cluster_flags, make_decode_plan, tile_flags
 
 _tables = {}          # tables by contents
 _cache = {}           # the same by the full description of the tensors they were made of, with these tensors
@@ -132,7 +132,8 @@ def fused_blockgtq_decode_attention(
     if k_norms.dtype != torch.float16:
         k_norms = k_norms.to(torch.float16)
     lt = _layer_for(segments, codebook_flat, v_lut, vb_codebook, n_kv, q.device)
-    flags = (_lib.DEC_K_MIXED if k_nibble else 0) | (_lib.DEC_V_NIBBLE if v_nibble else 0) | tile_flags(B, n_kv, T, q.device)
+    flags = (_lib.DEC_K_MIXED if k_nibble else 0) | (_lib.DEC_V_NIBBLE if v_nibble else 0) | \
+        (cluster_flags(B, n_kv, T, q.device, grows=True) or tile_flags(B, n_kv, T, q.device))
     out, _o32, lse = attend(lt, q, k_packed, k_norms, v_codes, v_norms, 0, T, rotate=False,
                             n_splits=max(1, int(t_splits)), scale=scale, flags=flags, v_rot=_rotation(v_rotation, n_kv),
                             want_lse=return_lse)

@@ -61,7 +61,7 @@ def needs_build() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
-JIT_SOURCES = ["bgtq_common.cuh", "bgtq_plan.h", "bgtq_decode_kernel.cuh"]
+JIT_SOURCES = ["bgtq_common.cuh", "bgtq_plan.h", "bgtq_decode_params.cuh", "bgtq_decode_cluster.cuh", "bgtq_decode_kernel.cuh"]
 
 
 def _embed_jit_sources(objdir: str) -> str:

@@ -173,6 +173,20 @@ __device__ __forceinline__ uint32_t ld_global_u32(const void* p) {
     return v;
 }
 
+// Byte `t` of a bit-packed run: codes of width bw (1..4) starting at codes[0].
+__device__ __forceinline__ uint32_t enc_pack_byte(const uint8_t* codes, int n, int bw, int t) {
+    const int bit0 = t * 8;
+    uint32_t out = 0;
+    int i = bit0 / bw;
+    for (int pos = i * bw; pos < bit0 + 8; pos += bw, ++i) {
+        if (i >= n) break;
+        const uint32_t c = codes[i] & ((1u << bw) - 1u);
+        const int sh = pos - bit0;
+        out |= sh >= 0 ? (c << sh) : (c >> (-sh));
+    }
+    return out & 0xFFu;
+}
+
 #ifndef BGTQ_JIT
 // Launch with or without the programmatic stream-serialization attribute.
 template <typename... KArgs, typename... Args>

@@ -13,9 +13,9 @@ int bgtq::launch_decode_plan(
     const uint8_t* v_packed, int64_t vp_sb, int64_t vp_sh, int64_t vp_st, const void* v_norms, int64_t vn_sb,
     int64_t vn_sh, int64_t vn_st, int32_t n_batch, int32_t n_q, int32_t n_kv, int32_t t_begin, int32_t t_end,
     int32_t n_splits, float scale, float* part_o, float* part_lse, int32_t* status, const int32_t* pos_dev,
-    int32_t pos_add, bool early_fetch, void* stream) {
-    if (!plan_host || !q_rot || !k_packed || !k_norms || !v_packed || !v_norms || !part_o || !part_lse)
-        return BGTQ_E_BADARG;
+    int32_t pos_add, bool early_fetch, const MergeParams* merge, void* stream) {
+    if (!plan_host || !k_packed || !k_norms || !v_packed || !v_norms) return BGTQ_E_BADARG;
+    if (!q_rot || (merge ? !merge->out : !part_o || !part_lse)) return BGTQ_E_BADARG;
     if (n_batch < 1 || n_kv < 1 || n_q < n_kv || n_q % n_kv || n_splits < 1 || t_end < t_begin || t_begin < 0)
         return BGTQ_E_BADARG;
     DecParams P;
@@ -44,6 +44,7 @@ int bgtq::launch_decode_plan(
     P.scale_log2 = scale * 1.4426950408889634f;
     P.part_o = part_o; P.part_lse = part_lse; P.status = status;
     P.pos_dev = pos_dev; P.pos_add = pos_add;
+    P.m = merge ? *merge : MergeParams{};
 
     // Tiles of 16 warps x 32 tokens, two stages; rows too wide for that (padded strides, the nibble layout with
     // large tables) fall back to 16 tokens per warp.
@@ -54,8 +55,7 @@ int bgtq::launch_decode_plan(
     P.off_kn = sl.off_kn; P.off_v = sl.off_v; P.off_vn = sl.off_vn;
     P.stage_bytes = sl.stage_bytes;
     P.stage_off = kOffStagesMin + P.plan.lut_bytes;
-    const size_t smem = decode_smem(P.plan.lut_bytes, sl.stage_bytes);
-
+    size_t smem = decode_smem(P.plan.lut_bytes, sl.stage_bytes);
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
@@ -65,12 +65,13 @@ int bgtq::launch_decode_plan(
     const int64_t max_items = (int64_t)n_batch * n_kv * n_splits;
     // the kernel cuts the item range among its CTAs in 32-bit arithmetic: (CTA index + 1) * items must fit
     if (max_items * ((int64_t)sms + 1) > 0xFFFFFFFFll) return BGTQ_E_TOOBIG;
-    dim3 grid((unsigned)(max_items < sms ? max_items : sms));
+    const int cluster = merge ? decode_cluster(P.plan) : 0;
+    dim3 grid((unsigned)(merge ? n_batch * n_kv * cluster : max_items < sms ? max_items : sms));
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool pdl = (P.plan.flags & BGTQ_DEC_PROGRAMMATIC) != 0;
     cudaError_t e;
     // the kernel specialised for this layer's heads, when the plan carries one for this tile width
-    bool jit = P.plan.jit_kernel != nullptr && nu == decode_jit_nu(P.plan) && !(P.plan.flags & BGTQ_DEC_GENERIC);
+    bool jit = P.plan.jit_kernel != nullptr && (decode_cluster(P.plan) > 0) == (merge != nullptr) && nu == decode_jit_nu(P.plan) && !(P.plan.flags & BGTQ_DEC_GENERIC);
     if (jit && P.plan.row_st[0] > 0) {
         // compiled for fixed row strides and for arrays whose every (batch, head) slice and first row start on a
         // 16-byte boundary: any other launch takes the general kernel
@@ -82,7 +83,16 @@ int bgtq::launch_decode_plan(
               al16(P.kp, P.kp_sb, P.kp_sh, P.kp_st) && al16(P.kn, P.kn_sb, P.kn_sh, P.kn_st) &&
               al16(P.vp, P.vp_sb, P.vp_sh, P.vp_st) && al16(P.vn, P.vn_sb, P.vn_sh, P.vn_st);
     }
-    if (jit) e = launch_decode_jit(P, grid, smem + decode_jit_quad_bytes(P.plan), st, pdl);
+    if (jit) smem += decode_jit_quad_bytes(P.plan);
+    if (merge) {
+        if (!jit || !cluster) return BGTQ_E_UNSUPPORTED;      // (that form exists in specialised kernels only)
+        const size_t end = (size_t)P.stage_off + decode_jit_quad_bytes(P.plan) + kMergeRowsBytes;
+        P.m.share_off = (uint32_t)(smem > end ? smem : end);
+        P.m.rot_off = P.m.share_off + cluster * kShareBytes;
+        smem = P.m.rot_off + (P.m.v_rot ? kHD * kHD * 4 / cluster : 0);
+        if (smem > 227 * 1024) return BGTQ_E_UNSUPPORTED;
+    }
+    if (jit) e = launch_decode_fn(P.plan.jit_kernel, P, grid, smem, st, pdl, cluster);
     else switch (P.plan.v_sbits) {
         case 1: e = launch_decode_vb1(P, nu, grid, smem, st, pdl); break;
         case 2: e = launch_decode_vb2(P, nu, grid, smem, st, pdl); break;
@@ -107,7 +117,7 @@ extern "C" __attribute__((visibility("default"))) int bgtq_decode(
     (void)desc;      // the kernel reads its tables from the plan's image
     return launch_decode_plan(plan_host, q_rot, k_packed, kp_sb, kp_sh, kp_st, k_norms, kn_sb, kn_sh, kn_st, v_packed,
                               vp_sb, vp_sh, vp_st, v_norms, vn_sb, vn_sh, vn_st, n_batch, n_q, n_kv, t_begin, t_end, n_splits,
-                              scale, part_o, part_lse, status, pos_dev, pos_add, true, stream);
+                              scale, part_o, part_lse, status, pos_dev, pos_add, true, nullptr, stream);
 }
 
 // ---------------------------------------------------------------------------

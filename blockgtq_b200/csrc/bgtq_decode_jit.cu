@@ -1,6 +1,7 @@
 // Run-time specialisation of the decode kernel for the KV heads of one layer.
 //
-// The kernel text (bgtq_common.cuh, bgtq_plan.h, bgtq_decode_kernel.cuh, embedded as strings by the build)
+// The kernel text (bgtq_common.cuh, bgtq_plan.h, bgtq_decode_params.cuh, bgtq_decode_cluster.cuh and bgtq_decode_kernel.cuh,
+// embedded as strings by the build)
 // is compiled with NVRTC behind a generated prelude that spells every head's segment list as compile-time
 // constants, so the K loop of the resulting kernel is straight-line code.  NVRTC is looked up with dlopen
 // (the library does not link it); the cubin is loaded through the CUDA runtime's library API.  Compiled
@@ -26,6 +27,12 @@ const char kSrcCommon[] =
     ;
 const char kSrcPlan[] =
 #include "bgtq_plan.h.str"
+    ;
+const char kSrcParams[] =
+#include "bgtq_decode_params.cuh.str"
+    ;
+const char kSrcCluster[] =
+#include "bgtq_decode_cluster.cuh.str"
     ;
 const char kSrcKernel[] =
 #include "bgtq_decode_kernel.cuh.str"
@@ -104,7 +111,8 @@ std::string make_prelude(const DecPlanDev& pl) {
     char buf[512];
     std::string s;
     s += "#define BGTQ_JIT 1\n#define BGTQ_HEAD_DIM 128\n";
-    snprintf(buf, sizeof(buf), "#define BGTQ_JIT_VB %d\n#define BGTQ_JIT_NU %d\n", pl.v_sbits, decode_jit_nu(pl));
+    snprintf(buf, sizeof(buf), "#define BGTQ_JIT_VB %d\n#define BGTQ_JIT_NU %d\n#define BGTQ_JIT_CLUSTER %d\n", pl.v_sbits, decode_jit_nu(pl),
+             decode_cluster(pl));
     s += buf;
     if (pl.row_st[0] > 0) {       // row strides fixed at compile time (and 16-byte aligned slices promised at launch)
         snprintf(buf, sizeof(buf), "#define BGTQ_JIT_STRIDES 1\n#define BGTQ_JIT_KP_ST %du\n#define BGTQ_JIT_KN_ST %du\n"
@@ -155,7 +163,7 @@ std::string make_prelude(const DecPlanDev& pl) {
 // Compile one prelude to a cubin.  Runs without the lock: NVRTC is thread safe, and callers specialise the
 // layers of a model from several threads.
 int compile(const std::string& prelude, std::vector<char>* cubin, std::string* log) {
-    const std::string src = prelude + kSrcCommon + "\n" + kSrcPlan + "\n" + kSrcKernel + "\n";
+    const std::string src = prelude + kSrcCommon + "\n" + kSrcPlan + "\n" + kSrcParams + "\n" + kSrcCluster + "\n" + kSrcKernel + "\n";
     nvrtcProgram prog = nullptr;
     if (g_nvrtc.CreateProgram(&prog, src.c_str(), "bgtq_decode_jit.cu", 0, nullptr, nullptr) != 0) return BGTQ_E_LAUNCH;
     std::vector<const char*> opts = {"--gpu-architecture=sm_100a", "--std=c++17", "-lineinfo"};
@@ -258,25 +266,3 @@ extern "C" __attribute__((visibility("default"))) int bgtq_decode_plan_specializ
     }
     return BGTQ_OK;
 }
-
-namespace bgtq {
-// Launch the specialised kernel recorded in the plan.
-cudaError_t launch_decode_jit(const DecParams& P, dim3 grid, size_t smem, cudaStream_t stream, bool programmatic) {
-    const void* fn = P.plan.jit_kernel;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(kDecThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = programmatic ? 1 : 0;
-    void* args[1] = {const_cast<DecParams*>(&P)};
-    e = cudaLaunchKernelExC(&cfg, fn, args);
-    return e == cudaSuccess ? cudaGetLastError() : e;
-}
-}  // namespace bgtq

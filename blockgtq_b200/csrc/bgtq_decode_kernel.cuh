@@ -47,46 +47,11 @@
 #ifndef BGTQ_JIT
 #include "bgtq_common.cuh"
 #include "bgtq_plan.h"
+#include "bgtq_decode_params.cuh"
+#include "bgtq_decode_cluster.cuh"
 #endif
 
 namespace bgtq {
-
-constexpr int kDecWarps = 16;
-constexpr int kDecThreads = 32 * kDecWarps;
-constexpr int kDecStages = 2;
-constexpr int kMergeSlot = 9 * 32;   // float4 per warp in the end-of-run merge buffer: 8 of O and (m, l), per lane
-// shared-memory layout (byte offsets from the start of dynamic shared memory)
-// [barriers | query fragments | pad | lookup tables | stages (merge buffer at run end)]
-// The lookup tables start at the first address past kOffMisc whose ABSOLUTE shared-window address is a
-// multiple of kLutAlign (table bases are OR-ed into addresses); the stages follow at a fixed offset that
-// leaves room for the worst-case pad.
-constexpr uint32_t kOffQf = 1024, kOffMisc = kOffQf + kMaxSteps * 32 * 8;
-constexpr uint32_t kOffStagesMin = kOffMisc + kLutAlign;     // + lut_bytes = P.stage_off
-static_assert(kOffMisc % 128 == 0, "layout");
-// two regions the tree merge alternates between: 8 slots (first level) and 4 (second); later levels fit in them
-constexpr uint32_t kMergeBytes = (kDecWarps / 2 + kDecWarps / 4) * kMergeSlot * 16;
-constexpr uint32_t kQuadBytes = 256u * 16u * 8u;      // V quad table of the specialised kernel
-#define BGTQ_INF __int_as_float(0x7f800000)
-
-struct DecParams {
-    const uint16_t* q_rot;  // fp16 bit patterns
-    const uint8_t* kp;
-    const uint8_t* kn;  // byte pointers; strides below are in bytes
-    const uint8_t* vp;
-    const uint8_t* vn;
-    int64_t kp_sb, kp_sh, kn_sb, kn_sh, vp_sb, vp_sh, vn_sb, vn_sh;
-    int32_t kp_st, kn_st, vp_st, vn_st;  // bytes per token
-    int32_t n_batch, n_q, n_kv, gqa;
-    int32_t t_begin, t_end, n_splits;
-    const int32_t* pos_dev;
-    int32_t pos_add;
-    float scale_log2;
-    float* part_o;
-    float* part_lse;
-    int32_t* status;
-    uint32_t stage_off, stage_bytes, off_kn, off_v, off_vn;  // shared-memory layout
-    DecPlanDev plan;
-};
 
 // V unpack parameters per stored width: mask of the even-indexed codes of one
 // 32-bit group, groups per 16 codes, lane replication of the table.
@@ -513,6 +478,7 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
         mbar_fence_init();
     }
     __syncthreads();
+    if constexpr (kMerges) cluster_started();
 
     // ---- lookup tables of one head: bulk copies of the prebuilt image --------------------------------
     int h_loaded = -1;
@@ -541,12 +507,15 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
 #endif
     };
     const int n_cta = (int)gridDim.x, cta = (int)blockIdx.x;
-    load_tables(min(P.n_kv - 1, (int)(((int64_t)cta * P.n_kv) / n_cta)));   // the head this CTA most likely starts in
+    // A pair per cluster (head-major like the items), a share of its tokens per CTA, or a range of items per CTA.
+    const int c_pair = cta / kClusterN, c_rank = cta % kClusterN;
+    load_tables(kMerges ? c_pair / P.n_batch
+                        : min(P.n_kv - 1, (int)(((int64_t)cta * P.n_kv) / n_cta)));   // the head this CTA most likely starts in
     bool tables_pending = true;
     // The item-range table, if the plan carries one, is requested here, ahead of the dependency wait, so that its
     // latency passes behind the start-up work (it is written by a copy ordered before the launch that precedes
     // this one, never by that launch itself).
-    const int32_t* part = P.plan.partition;
+    const int32_t* part = kMerges ? nullptr : P.plan.partition;
     uint32_t pk0 = 0, pk1 = 0, pk2 = 0, pk3 = 0, p_lo = 0, p_hi = 0;
     if (part) {
         pk0 = (uint32_t)__ldg(part);
@@ -570,10 +539,10 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
     const int t_live = P.pos_dev ? min(P.t_end, *P.pos_dev + P.pos_add) : P.t_end;
     const uint32_t n_tok = (uint32_t)max(0, t_live - P.t_begin);
     const uint32_t units = (n_tok + 31u) >> 5;                          // 32-token warp units per pair
-    const uint32_t c_units = max(1u, udiv_fast(units + (uint32_t)P.n_splits - 1u, (uint32_t)P.n_splits));  // units per item
-    const uint32_t n_live = udiv_fast(units + c_units - 1u, c_units);   // non-empty items per pair (<= n_splits)
+    const uint32_t c_units = kMerges ? 1u : max(1u, udiv_fast(units + (uint32_t)P.n_splits - 1u, (uint32_t)P.n_splits));  // units per item
+    const uint32_t n_live = kMerges ? 1u : udiv_fast(units + c_units - 1u, c_units);   // non-empty items per pair (<= n_splits)
     const uint32_t n_items = (uint32_t)(P.n_batch * P.n_kv) * n_live;
-    if (n_items == 0) {     // no tokens at all: every slot of every row is an empty split
+    if (!kMerges && n_items == 0) {     // no tokens at all: every slot of every row is an empty split
         if (!dep_waited) grid_dependency_wait();
         for (int64_t i = (int64_t)cta * kDecThreads + tid; i < (int64_t)P.n_batch * P.n_q * P.n_splits;
              i += (int64_t)n_cta * kDecThreads)
@@ -584,7 +553,10 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
     // Equal item counts, unless the caller's table was made for exactly this launch (the same items per pair,
     // pairs, CTAs and units per item: every CTA sees the same four words, so all take the same branch)
     uint32_t item_lo, item_hi;
-    if (part && pk0 == n_live && pk1 == (uint32_t)(P.n_batch * P.n_kv) && pk2 == (uint32_t)n_cta && pk3 == c_units) {
+    if (kMerges) {
+        item_lo = 0u;
+        item_hi = 1u;
+    } else if (part && pk0 == n_live && pk1 == (uint32_t)(P.n_batch * P.n_kv) && pk2 == (uint32_t)n_cta && pk3 == c_units) {
         item_lo = min(p_lo, n_items);
         item_hi = min(max(p_hi, item_lo), n_items);
     } else {
@@ -613,8 +585,8 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
     // Stream tile `it` of a run into the stage of running tile number `git`.  Called by a whole warp: lanes
     // 0..3 each request one of the four arrays (packed K, K norms, packed V, V norms), so the address
     // arithmetic of a tile takes one lane's worth of time instead of four.
-    auto issue_tile = [&](const Run& R, int it, uint32_t git) {
-        const int st = git % kDecStages;
+    struct TileReq { const uint8_t* src; uint32_t bytes, total, off; };
+    auto tile_req = [&](const Run& R, int it) {
         const int t = R.t0 + it * kTileTok;
         const int nt = min(kTileTok, R.t1 - t);
         const int a = lane & 3;
@@ -622,24 +594,41 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
         const int64_t sb_ = a == 0 ? P.kp_sb : a == 1 ? P.kn_sb : a == 2 ? P.vp_sb : P.vn_sb;
         const int64_t sh_ = a == 0 ? P.kp_sh : a == 1 ? P.kn_sh : a == 2 ? P.vp_sh : P.vn_sh;
         const uint32_t st_ = a == 0 ? kp_st : a == 1 ? kn_st : a == 2 ? vp_st : vn_st;
-        const uint32_t off = a == 0 ? 0u : a == 1 ? off_kn : a == 2 ? off_v : off_vn;
+        TileReq q;
+        q.off = a == 0 ? 0u : a == 1 ? off_kn : a == 2 ? off_v : off_vn;
         const uint8_t* src = base + (size_t)R.b * sb_ + (size_t)R.h * sh_ + (size_t)t * st_;
         const uint32_t ph = kAligned ? 0u : (uint32_t)(reinterpret_cast<uintptr_t>(src) & 15u);
-        const uint32_t z = (ph + (uint32_t)nt * st_ + 15u) & ~15u;
-        uint32_t tot = z + __shfl_xor_sync(0xffffffffu, z, 1);
-        tot += __shfl_xor_sync(0xffffffffu, tot, 2);
+        q.src = src - ph;
+        q.bytes = (ph + (uint32_t)nt * st_ + 15u) & ~15u;
+        q.total = q.bytes + __shfl_xor_sync(0xffffffffu, q.bytes, 1);
+        q.total += __shfl_xor_sync(0xffffffffu, q.total, 2);
+        return q;
+    };
+    auto send_req = [&](const TileReq& q, uint32_t git) {
+        const int st = git % kDecStages;
         if (lane < 4) {
             // the stage was last touched through the generic proxy (its previous tile's readers, or the merge)
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            if (lane == 0) mbar_arrive_expect_tx(&full[st], tot);
-            bulk_g2s_hint(smem + stage_off + (size_t)st * stage_bytes + off, src - ph, z, &full[st], pol);
+            if (lane == 0) mbar_arrive_expect_tx(&full[st], q.total);
+            bulk_g2s_hint(smem + stage_off + (size_t)st * stage_bytes + q.off, q.src, q.bytes, &full[st], pol);
         }
     };
+    auto issue_tile = [&](const Run& R, int it, uint32_t git) { send_req(tile_req(R, it), git); };
     // A run's first tile may already be on its way: the previous run's end requests it before merging its warps.
     bool first_tile_issued = false;
+    Run share;
+    if constexpr (kMerges) {        // shares of whole warp tiles
+        const uint32_t g = (n_tok + kWarpTok - 1u) / kWarpTok;
+        share.h = c_pair / P.n_batch;
+        share.b = c_pair - share.h * P.n_batch;
+        share.s0 = 0;
+        share.cnt = 1;
+        share.t0 = P.t_begin + kWarpTok * (int)(g * (uint32_t)c_rank / (uint32_t)kClusterN);
+        share.t1 = max(share.t0, min(t_live, P.t_begin + kWarpTok * (int)(g * (uint32_t)(c_rank + 1) / (uint32_t)kClusterN)));
+    }
 
     for (uint32_t item = item_lo; item < item_hi;) {
-        const Run R = run_at(item);
+        const Run R = kMerges ? share : run_at(item);
         item += (uint32_t)R.cnt;
         const int h = R.h, b = R.b, s0 = R.s0, cnt = R.cnt, t0 = R.t0, t1 = R.t1;
         const DecHeadPlan& hp = P.plan.head[h];
@@ -669,6 +658,8 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
             if (warp == 0)
                 for (int it = first; it < held; ++it) issue_tile(R, it, g_it + it);
             if (!dep_waited) {
+                TileReq late{};             // the first one held back: nothing but its copies behind the wait (the many-tile form
+                if (kMerges && warp == 0 && held < last) late = tile_req(R, held);      // hardly ever holds one, and keeps its registers)
                 if (tables_pending) {       // (behind the preceding launch)
                     tables_ready(hp);
                     tables_pending = false;
@@ -676,6 +667,7 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
                 grid_dependency_wait();
                 grid_launch_dependents();
                 dep_waited = true;
+                if (kMerges && warp == 0 && held < last) send_req(late, g_it + held++);
                 if (warp == 0)
                     for (int it = held; it < last; ++it) issue_tile(R, it, g_it + it);
             }
@@ -693,6 +685,7 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
                       ? ld_global_u32(qrow + pos + 2) : 0u;
             qfrag[s * 32 + lane] = v;
         }
+        if constexpr (kMerges) merge_prefetch(P, smem, h, c_rank);      // (behind warp 0's requests: its proxy fence would wait for these copies)
         if (tables_pending) {
             tables_ready(hp);
             tables_pending = false;
@@ -879,10 +872,16 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
         }
         // Every tile of the run has been consumed once all warps are here: both stages are idle.
         __syncthreads();
+        if constexpr (kMerges) {
+            cluster_all_started();
+            const int n_live = n_tiles > 1 ? kDecWarps : (t1 - t0 + kWarpTok - 1) / kWarpTok;
+            merge_share(P, smem, smem + stage_off, O, m0, m1, l0, l1, n_live, c_rank);
+            break;
+        }
         // If this CTA has another run, that run's first tile is requested NOW, into the stage it will use (the
         // one the last tile did not), so its DRAM latency passes behind the merge, which then stays inside the
         // other stage.  Otherwise the merge may spread over both.
-        const bool ahead = item < item_hi && kDecStages == 2 && stage_bytes >= kMergeBytes;
+        const bool ahead = !kMerges && item < item_hi && kDecStages == 2 && stage_bytes >= kMergeBytes;
         if (ahead && warp == 0) issue_tile(run_at(item), 0, g_it);
         first_tile_issued = ahead;
         // Merge of the sixteen warps' (O, m, l).  Two tree levels (16 -> 8 -> 4): the upper half of the live warps
@@ -1008,6 +1007,7 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
         }
         __syncthreads();      // the merge buffer is free again before the next run's tiles land in it
     }
+    if constexpr (kMerges) merge_finish(P, smem, smem + stage_off, share.h, share.b, c_rank);
     if (tables_pending) wait_tables();
     if (!dep_waited) grid_dependency_wait();     // (a CTA without items: the launch still completes behind its predecessor)
     if (!ok && P.status && lane == 0) atomicExch(P.status, kStatusWaitTimeout);
@@ -1041,22 +1041,45 @@ inline uint32_t decode_jit_quad_bytes(const DecPlanDev& pl) {
     return decode_smem(pl.lut_bytes, stage) + kQuadBytes <= 227 * 1024 ? kQuadBytes : 0u;
 }
 
+// Launch one of the kernels; cluster > 0: in clusters of that many CTAs.
+inline cudaError_t launch_decode_fn(const void* fn, const DecParams& P, dim3 grid, size_t smem, cudaStream_t stream, bool programmatic,
+                                    int cluster) {
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kDecThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
+    if (programmatic) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 0) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = (unsigned)cluster;
+        attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
+    }
+    void* args[1] = {const_cast<DecParams*>(&P)};
+    e = cudaLaunchKernelExC(&cfg, fn, args);
+    return e == cudaSuccess ? cudaGetLastError() : e;
+}
+
 // Launch one instantiation; defined once per stored V width in its own translation unit.
 template <int VB>
 cudaError_t launch_decode(const DecParams& P, int nu, dim3 grid, size_t smem, cudaStream_t stream, bool programmatic) {
-    auto go = [&](void (*kern)(DecParams)) -> cudaError_t {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        return launch_kernel(kern, grid, dim3(kDecThreads), smem, stream, programmatic, P);
-    };
-    return nu == 2 ? go(decode_kernel<VB, 2>) : go(decode_kernel<VB, 1>);
+    return launch_decode_fn(reinterpret_cast<const void*>(nu == 2 ? decode_kernel<VB, 2> : decode_kernel<VB, 1>), P, grid, smem, stream,
+                            programmatic, 0);
 }
 
 cudaError_t launch_decode_vb1(const DecParams&, int, dim3, size_t, cudaStream_t, bool);
 cudaError_t launch_decode_vb2(const DecParams&, int, dim3, size_t, cudaStream_t, bool);
 cudaError_t launch_decode_vb3(const DecParams&, int, dim3, size_t, cudaStream_t, bool);
 cudaError_t launch_decode_vb4(const DecParams&, int, dim3, size_t, cudaStream_t, bool);
-cudaError_t launch_decode_jit(const DecParams&, dim3, size_t, cudaStream_t, bool);
 #endif
 
 }  // namespace bgtq

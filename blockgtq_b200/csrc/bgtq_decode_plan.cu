@@ -1,10 +1,10 @@
 // Host side of the decode kernel: the launch plan of a layer's KV heads, the
 // prebuilt lookup-table image the kernel copies into shared memory, and the
 // suggested split count.  No GPU work happens here.
+#include <stddef.h>
 #include <string.h>
 
-#include "bgtq_common.cuh"
-#include "bgtq_plan.h"
+#include "bgtq_decode_cluster.cuh"
 
 using namespace bgtq;
 
@@ -122,9 +122,24 @@ extern "C" __attribute__((visibility("default"))) int bgtq_decode_plan(const Bgt
     if (boost == 0 || lut_bytes <= lut_budget) break;
     }
     pl.lut_bytes = (lut_bytes + 127u) / 128u * 128u;
+    if (const int n = decode_cluster(pl)) {      // shares merged in the launch: only where they fit besides tables and stages
+        const uint32_t stages = 2u * (256u * row_bytes + 4u * 64u + 128u);
+        if (n > 16 || (n & (n - 1)) ||
+            kOffStagesMin + pl.lut_bytes + (stages > kMergeRowsBytes ? stages : kMergeRowsBytes) + n * kShareBytes + kHD * kHD * 4u / n > 227u * 1024u)
+            pl.flags &= ~BGTQ_DEC_CLUSTER_MASK;
+    }
     pl.image = nullptr;
     memcpy(out, &pl, sizeof(pl));
     return BGTQ_OK;
+}
+
+extern "C" __attribute__((visibility("default"))) int bgtq_decode_plan_cluster(const BgtqDecodePlan* plan_host) {
+    if (!plan_host) return 0;
+    int32_t flags;
+    const void* kernel;
+    memcpy(&flags, reinterpret_cast<const char*>(plan_host) + offsetof(DecPlanDev, flags), sizeof(flags));
+    memcpy(&kernel, reinterpret_cast<const char*>(plan_host) + offsetof(DecPlanDev, jit_kernel), sizeof(kernel));
+    return kernel && !(flags & BGTQ_DEC_GENERIC) ? (flags & BGTQ_DEC_CLUSTER_MASK) >> BGTQ_DEC_CLUSTER_SHIFT : 0;
 }
 
 extern "C" __attribute__((visibility("default"))) int64_t bgtq_decode_image_bytes(const BgtqDecodePlan* plan_host) {

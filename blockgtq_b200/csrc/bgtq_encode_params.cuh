@@ -34,20 +34,6 @@ __device__ __forceinline__ bool enc_range_ok(const EncParams& P, int t0, int n_t
     return true;
 }
 
-// Byte `t` of a bit-packed run: codes of width bw (1..4) starting at codes[0].
-__device__ __forceinline__ uint32_t enc_pack_byte(const uint8_t* codes, int n, int bw, int t) {
-    const int bit0 = t * 8;
-    uint32_t out = 0;
-    int i = bit0 / bw;
-    for (int pos = i * bw; pos < bit0 + 8; pos += bw, ++i) {
-        if (i >= n) break;
-        const uint32_t c = codes[i] & ((1u << bw) - 1u);
-        const int sh = pos - bit0;
-        out |= sh >= 0 ? (c << sh) : (c >> (-sh));
-    }
-    return out & 0xFFu;
-}
-
 // Tensor-core bulk path (bgtq_encode_tc.cu).  Rows must be 16-byte aligned.
 int launch_encode_tc(const EncParams& P, cudaStream_t stream);
 
@@ -58,12 +44,14 @@ int launch_encode_t5(const EncParams& P, cudaStream_t stream);
 int launch_rotate_q(const BgtqHeadDesc* desc, const float* rot_k, const void* q, int64_t q_sb, int64_t q_sh, void* q_rot,
                     int32_t n_batch, int32_t n_q, int32_t n_kv, bool programmatic, cudaStream_t stream);
 
-// bgtq_decode with the plan's early fetch as it is or off for this launch (bgtq_decode.cu).
+// bgtq_decode with the plan's early fetch as it is or off for this launch; with `merge` (a plan of
+// clusters) the merged rows come out of that launch and part_o and part_lse are null (bgtq_decode.cu).
+struct MergeParams;
 int launch_decode_plan(const BgtqDecodePlan* plan_host, const void* q_rot, const uint8_t* k_packed, int64_t kp_sb, int64_t kp_sh,
                        int64_t kp_st, const void* k_norms, int64_t kn_sb, int64_t kn_sh, int64_t kn_st, const uint8_t* v_packed,
                        int64_t vp_sb, int64_t vp_sh, int64_t vp_st, const void* v_norms, int64_t vn_sb, int64_t vn_sh, int64_t vn_st,
                        int32_t n_batch, int32_t n_q, int32_t n_kv, int32_t t_begin, int32_t t_end, int32_t n_splits, float scale,
                        float* part_o, float* part_lse, int32_t* status, const int32_t* pos_dev, int32_t pos_add, bool early_fetch,
-                       void* stream);
+                       const MergeParams* merge, void* stream);
 
 }  // namespace bgtq

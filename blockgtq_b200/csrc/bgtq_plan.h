@@ -31,6 +31,8 @@
 #pragma once
 #ifndef BGTQ_JIT
 #include <stdint.h>
+
+#include "../../include/bgtq.h"
 #endif
 
 namespace bgtq {
@@ -91,6 +93,10 @@ struct DecPlanDev {
                                // compiled for (bgtq_decode_plan_set_row_strides), or zeros: strides read at run time
     DecHeadPlan head[kMaxPlanHeads];
 };
+
+#ifndef BGTQ_JIT
+inline int decode_cluster(const DecPlanDev& pl) { return (pl.flags & BGTQ_DEC_CLUSTER_MASK) >> BGTQ_DEC_CLUSTER_SHIFT; }
+#endif
 
 // Layout of one stage (a tile of each of the four arrays) in shared memory: byte offsets of the K norms, packed V
 // and V norms behind the packed K, and the stage size.  Each array: one tile of rows + 15 bytes of leading phase

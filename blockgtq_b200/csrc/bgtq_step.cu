@@ -6,6 +6,7 @@
 // change from step to step is filled in once (BgtqLayerStep); a step then costs one call, and the kernels read the
 // caller's query, key and value rows where they lie.
 #include "bgtq_common.cuh"
+#include "bgtq_decode_params.cuh"
 #include "bgtq_encode_params.cuh"
 
 using namespace bgtq;
@@ -48,6 +49,14 @@ extern "C" __attribute__((visibility("default"))) int bgtq_layer_step(
                                s->kn_sb, s->kn_sh, s->kn_st, s->kn_count, s->v_packed, s->vp_sb, s->vp_sh, s->vp_st, s->v_norms,
                                s->vn_sb, s->vn_sh, s->vn_st, s->enc_flags, s->pos_dev, s->t_capacity, s->status, stream);
     if (rc != BGTQ_OK) return rc;
+    if (!ring && bgtq_decode_plan_cluster(s->plan)) {
+        const MergeParams M = {s->v_rot, static_cast<uint16_t*>(s->out), s->o_sb, s->o_sh, nullptr, nullptr, 0, 0};
+        rc = launch_decode_plan(s->plan, q_dec, s->k_packed, s->kp_sb, s->kp_sh, s->kp_st, s->k_norms, s->kn_sb, s->kn_sh, s->kn_st,
+                                s->v_packed, s->vp_sb, s->vp_sh, s->vp_st, s->v_norms, s->vn_sb, s->vn_sh, s->vn_st, s->n_batch, s->n_q,
+                                s->n_kv, 0, s->t_capacity, 1, s->scale, nullptr, nullptr, s->status, s->pos_dev, s->pos_add, true, &M,
+                                stream);
+        if (rc != BGTQ_E_UNSUPPORTED) return rc;
+    }
     rc = bgtq_decode(s->plan, s->desc, q_dec, s->k_packed, s->kp_sb, s->kp_sh, s->kp_st, s->k_norms, s->kn_sb, s->kn_sh, s->kn_st,
                      s->v_packed, s->vp_sb, s->vp_sh, s->vp_st, s->v_norms, s->vn_sb, s->vn_sh, s->vn_st, s->n_batch, s->n_q, s->n_kv,
                      0, s->t_capacity, s->n_splits, s->scale, s->part_o, s->part_lse, s->status, s->pos_dev, s->pos_add, stream);
@@ -101,9 +110,16 @@ extern "C" __attribute__((visibility("default"))) int bgtq_attend(
     // No early fetch here, whatever the plan says: what is in front of this call may be a bulk encode of the very rows
     // that are attended, and it lets its dependents start while it runs.  (A layer step is different: there the launch in
     // front of the decode is its own append.)
+    if (!buf_o && bgtq_decode_plan_cluster(plan)) {
+        const MergeParams M = {v_rot, static_cast<uint16_t*>(out), (int64_t)n_q * kHD, kHD, out_f32, lse_out, 0, 0};
+        const int rc = launch_decode_plan(plan, q_dec, k_packed, kp_sb, kp_sh, kp_st, k_norms, kn_sb, kn_sh, kn_st, v_packed, vp_sb, vp_sh,
+                                          vp_st, v_norms, vn_sb, vn_sh, vn_st, n_batch, n_q, n_kv, t_begin, t_end, 1, scale, nullptr,
+                                          nullptr, status, nullptr, 0, false, &M, stream);
+        if (rc != BGTQ_E_UNSUPPORTED) return rc;
+    }
     const int rc = launch_decode_plan(plan, q_dec, k_packed, kp_sb, kp_sh, kp_st, k_norms, kn_sb, kn_sh, kn_st, v_packed, vp_sb, vp_sh,
                                       vp_st, v_norms, vn_sb, vn_sh, vn_st, n_batch, n_q, n_kv, t_begin, t_end, n_splits, scale, part_o,
-                                      part_lse, status, nullptr, 0, false, stream);
+                                      part_lse, status, nullptr, 0, false, nullptr, stream);
     if (rc != BGTQ_OK) return rc;
     return bgtq_combine(part_o, part_lse, n_splits, v_rot, buf_o, buf_lse, n_batch, n_q, n_kv, out, (int64_t)n_q * kHD, kHD, out_f32,
                         lse_out, BGTQ_COMBINE_PROGRAMMATIC, stream);

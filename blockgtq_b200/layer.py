@@ -436,7 +436,7 @@ def attend(layer, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, *, ro
             r = call()
         if r is None:
             raise ValueError("query, cache and layer do not match")
-    return _lib.done(r, "bgtq_attend", 3 if rotate else 2)
+    return _lib.done(r, "bgtq_attend", (3 if rotate else 2) - (buf_o is None and merges(plan)))
 
 
 _SCALE = 1.0 / math.sqrt(HD)
@@ -457,6 +457,36 @@ def tile_flags(n_batch: int, n_kv: int, n_tokens: int, device) -> int:
     kernel serves the cache's whole life; a short sequence in a large cache runs the wide tile."""
     index = device.index if device.index is not None else torch.cuda.current_device()
     return _lib.DEC_NARROW if n_batch * n_kv * n_tokens <= 256 * _sm_count(index) else 0
+
+
+def merges(plan) -> bool:
+    """Whether the plan's decode merges its shares itself in layer steps and attentions."""
+    return _lib.lib().bgtq_decode_plan_cluster(C.addressof(plan)) > 0
+
+
+def cluster_flags(n_batch: int, n_kv: int, n_tokens: int, device, grows: bool = False) -> int:
+    """Plan flags of the form that merges a pair's shares inside the decode launch (``DEC_CLUSTER_SHIFT``; the narrow tile), for
+    layer steps and attentions over up to ``n_tokens`` rows, or 0 where the decode over all SMs and its merge launch are faster.
+
+    A cluster of C CTAs per (batch, KV head) pair saves the second launch and the partials' way through memory, about 3 us.
+    Against that, pairs * C CTAs share the work instead of one per SM: it is taken while that costs a CTA at most 330 tokens
+    (9 ns each) more than an SM's even share.  C is the largest of 8, 4 and 2 whose clusters all run at once: 14 clusters
+    of 8, 32 of 4 and 72 of 2 do (16 of 8 and 36 of 4 take two waves); and smaller while a CTA then has at most 8 warps' tokens,
+    or 16 where the CTAs would take more than half of the SMs, which the next launch's CTAs start on (500 tokens of 8 pairs 10.2, 8.9
+    and 9.1 us with 2, 4 and 8, of 32 pairs 10.1 and 11.6 with 2 and 4).  ``grows``: the length goes up from call to call; one C
+    for all of them, as each is a kernel of its own.
+    A captured layer (K3V3, 4 query heads per KV head but where noted), one sequence of 8 KV heads, in two launches and so: 100 tokens
+    11.1 and 8.7 us, 500: 12.1 and 8.9, 2000: 12.2 and 10.4, 4000: 12.7 and 12.9, 6000: 14.0 and 15.0 (not taken); 2 KV heads x 8 at 500
+    tokens 10.0 and 8.7; 4 sequences x 8 heads x 3: 500: 14.7 and 10.1, 4099: 22.1 and 20.0, 8500: 31.9 and 30.2 (x 4); 8 sequences: 500: 16.1 and
+    13.1, 3000: 27.7 and 24.1, 4300: 32.0 and 30.9."""
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    sms, pairs = _sm_count(index), n_batch * n_kv
+    c = next((c for c, most in ((8, 14), (4, 32), (2, 72)) if pairs <= most * sms // 148), 0)
+    if c == 0 or n_tokens * (sms - pairs * c) > 330 * sms * c:
+        return 0
+    while not grows and c > 2 and 2 * n_tokens <= (256 if 2 * pairs * c > sms else 128) * c:
+        c //= 2
+    return _lib.DEC_NARROW | c << _lib.DEC_CLUSTER_SHIFT
 
 
 _PREFILL_WORKSPACE = 2 << 30        # bytes of dequantised operand tiles per launch

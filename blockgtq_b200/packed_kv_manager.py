@@ -23,8 +23,8 @@ import torch
 
 from . import _lib
 from .calib import packed_v_bytes
-from .layer import (HD, LayerTables, attend, buffer_attn, combine, decode, decode_grid_size, decode_partition, default_splits,
-                    encode, rotate_q, step_prepare, tile_flags, _no_tcgen05)
+from .layer import (HD, LayerTables, attend, buffer_attn, cluster_flags, combine, decode, decode_grid_size, decode_partition, default_splits,
+                    encode, merges, rotate_q, step_prepare, tile_flags, _no_tcgen05)
 from .quantizer import BlockGTQQuantizer, build_batched_encode_args
 
 __all__ = ["BlockGTQKVManager", "decode_step"]
@@ -71,6 +71,7 @@ class BlockGTQKVManager:
         self._exchange = None                 # sequence sharding: see sharding.SequenceShard
         self._enc_flags = (_lib.ENC_K_MIXED if k_mixed else 0) | (_lib.ENC_V_NIBBLE if v_nibble else 0)
         self._dec_flags = (_lib.DEC_K_MIXED if k_mixed else 0) | (_lib.DEC_V_NIBBLE if v_nibble else 0)
+        self._cluster_flags = 0               # of layer steps and attend: see layer.cluster_flags
         # single-token decode steps take the position from the device and keep their arrays, so that they can be
         # captured (the reference graphs only its T=1 encode, packed_kv_manager.py:182-257); with fp16 regions that
         # needs one-token blocks, the policy's default
@@ -158,6 +159,8 @@ class BlockGTQKVManager:
                         lt.set_early_fetch(1)
         if dev.type == "cuda":      # by capacity: one kernel for the cache's whole life, captured graphs included
             self._dec_flags |= tile_flags(self.B, self.n_kv, self.max_T, dev)
+            if not self._buffered and self._exchange is None:
+                self._cluster_flags = cluster_flags(self.B, self.n_kv, self.max_T, dev)
         self._prepare_decode_plans()
         self._q_rot = torch.empty(self.B, self.n_q, self.hd, dtype=torch.float16, device=dev)
         self._part_o = torch.empty(self.B, self.n_q, self._n_splits, self.hd, dtype=torch.float32, device=dev)
@@ -187,7 +190,8 @@ class BlockGTQKVManager:
         from concurrent.futures import ThreadPoolExecutor
         layers = [lt for lt in self._layers if lt is not None]
         pd = _lib.DEC_PROGRAMMATIC
-        flag_sets = {self._dec_flags, self._dec_flags | pd}
+        flags = self._dec_flags | self._cluster_flags
+        flag_sets = {flags, flags | pd}
         with ThreadPoolExecutor(max_workers=min(16, os.cpu_count() or 1)) as ex:     # one layer per job: its flag
             list(ex.map(lambda lt: [lt.plan(f) for f in sorted(flag_sets)], layers))  # variants share one kernel
 
@@ -353,7 +357,7 @@ class BlockGTQKVManager:
         if s is not None and s.key == (lt, baked, pd):
             return s
         kp, kn, vp, vn = self._k_packed[li], self._k_norms[li], self._v_packed[li], self._v_norms[li]
-        plan = lt.plan(self._dec_flags | (_lib.DEC_PROGRAMMATIC if pd else 0))
+        plan = lt.plan(self._dec_flags | self._cluster_flags | (_lib.DEC_PROGRAMMATIC if pd else 0))
         s = _lib.LayerStep(
             plan=C.addressof(plan), desc=lt.desc_dev.data_ptr(), rot_k=lt.rot_k.data_ptr(), rot_v=lt.rot_v.data_ptr(),
             v_rot=lt.v_rot.data_ptr(), q_rot=self._q_rot.data_ptr(), part_o=self._part_o.data_ptr(),
@@ -371,7 +375,7 @@ class BlockGTQKVManager:
             kb, vb = self._k_buf[li], self._v_buf[li]
             s.k_buf, s.v_buf, s.kb_sb, s.kb_sh = kb.data_ptr(), vb.data_ptr(), kb.stride(0), kb.stride(1)
             s.buf_o, s.buf_lse, s.n_sink, s.window = self._buf_o.data_ptr(), self._buf_lse.data_ptr(), self.n_sink, self.recent_window
-        s.key, s.addr, s.n_launch = (lt, baked, pd), C.addressof(s), 4 if self._buffered else 3
+        s.key, s.addr, s.n_launch = (lt, baked, pd), C.addressof(s), 4 if self._buffered else 3 - merges(plan)
         self._steps[li] = s
         return s
 
@@ -547,7 +551,7 @@ class BlockGTQKVManager:
         if self._buffered and with_buffers:
             buf_o, buf_lse = self._buffer_partial(li, q, n_sink_tok, n_packed, n_recent)
         return attend(lt, q, self._k_packed[li], self._k_norms[li], self._v_packed[li], self._v_norms[li], lo, hi, rotate=not baked,
-                      n_splits=n_splits, scale=self.scale, flags=self._dec_flags, v_rot=lt.v_rot, buf_o=buf_o, buf_lse=buf_lse,
+                      n_splits=n_splits, scale=self.scale, flags=self._dec_flags | self._cluster_flags, v_rot=lt.v_rot, buf_o=buf_o, buf_lse=buf_lse,
                       want_f32=want_partial, want_lse=want_partial, status=self._status)
 
     def _buffer_partial(self, li, q, n_sink_tok, n_packed, n_recent):

@@ -236,6 +236,12 @@ int bgtq_step_prepare_ring(const BgtqHeadDesc* desc, const float* rot_k, const f
 #define BGTQ_DEC_NARROW 32        /* 16 tokens per warp instead of 32: shorter chains while a CTA gets at most 256 tokens
                                    * (n_batch * n_kv * tokens <= 256 * SMs), less work per load beyond; same results up to
                                    * the order of sums */
+#define BGTQ_DEC_CLUSTER_SHIFT 8  /* n << 8, n = 1, 2, 4, 8 or 16, with BGTQ_DEC_NARROW: bgtq_layer_step and bgtq_attend decode
+                                   * with a cluster of n CTAs per (batch, KV head) pair, which merge their shares and write the
+                                   * output rows themselves: no merge launch.  The plan's specialised kernel is the one for that;
+                                   * bgtq_decode with such a plan takes the general kernel.  bgtq_decode_plan drops the bits
+                                   * where the form does not fit shared memory; fp16 regions (buf_o) take the split form. */
+#define BGTQ_DEC_CLUSTER_MASK 0x1F00
 
 /* Opaque launch plan of the decode kernel for the KV heads of one layer (host
  * memory, plain bytes, copyable).  Built once per layer from the HOST copy of
@@ -291,6 +297,9 @@ int bgtq_jit_set_nvrtc_path(const char* path_host);
  * one of them may be the preceding launch.  bgtq_attend, which may well be called there, never fetches early.
  * No counterpart in the reference. */
 int bgtq_decode_plan_set_early_fetch(BgtqDecodePlan* plan_host, int32_t fresh_rows);
+
+/* CTAs per (batch, KV head) pair of the plan's specialised kernel (BGTQ_DEC_CLUSTER_SHIFT), 0: the split form. */
+int bgtq_decode_plan_cluster(const BgtqDecodePlan* plan_host);
 
 /* Optional item-range table of a launch.  bgtq_decode cuts every (batch, KV head) pair into items and hands
  * each of its CTAs a contiguous range of them; by default every CTA gets the same number.  A CTA whose range

@@ -1,0 +1,96 @@
+"""Decodes whose clusters merge their shares in the launch, against the split form with its merge launch.
+
+Both round p * norm to fp16 relative to running maxima that other groups of tokens give: each weight may differ by 2^-11 of itself
+on either side, so a row by 2^-10 of its largest value; the log-sum-exp sums fp32 weights."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _manager(batch, n_kv, gqa, cap, gen, **kw):
+    from blockgtq_b200 import BlockGTQKVManager
+    from helpers import HD, synth_head
+    mgr = BlockGTQKVManager(1, n_kv * gqa, n_kv, HD, max_seq_len=cap, batch_size=batch, device=DEV, **kw)
+    cal = [synth_head(gen, 256, gqa) for _ in range(n_kv)]
+    mgr.calibrate(0, torch.stack([c[0] for c in cal]).float(), torch.stack([c[1] for c in cal]).float())
+    return mgr
+
+
+def _rand(gen, *shape):
+    return torch.randn(*shape, generator=gen).half().to(DEV)
+
+
+# clusters of 8, 4 and 2; query groups of one, an odd number and eight; both cache layouts
+@pytest.mark.parametrize("batch,n_kv,gqa,cap,k_bits,v_bits,mixed,c", [
+    (1, 2, 4, 2100, 3.0, 3, False, 8), (2, 7, 1, 1100, 2.0, 2, False, 8), (1, 8, 7, 510, 4.0, 4, False, 4), (4, 8, 3, 1030, 3.0, 1, False, 4),
+    (9, 8, 8, 300, 2.5, 3, False, 2), (1, 4, 5, 90, 3.5, 2, False, 2), (3, 8, 2, 1500, 4.0, 3, True, 4)])
+def test_merged_in_the_launch(batch, n_kv, gqa, cap, k_bits, v_bits, mixed, c):
+    from blockgtq_b200 import _lib
+    from blockgtq_b200.layer import attend, merges
+    gen = torch.Generator().manual_seed(cap)
+    mgr = _manager(batch, n_kv, gqa, cap, gen, k_avg_bits=k_bits, v_bits=v_bits, k_mixed=mixed, v_nibble=mixed)
+    mgr.init_from_cache([tuple(_rand(gen, batch, n_kv, cap, 128) for _ in range(2))])
+    assert mgr._cluster_flags >> _lib.DEC_CLUSTER_SHIFT == c
+    lt, cache = mgr._layers[0], (mgr._k_packed[0], mgr._k_norms[0], mgr._v_packed[0], mgr._v_norms[0])
+    plain, flags = mgr._dec_flags, mgr._dec_flags | mgr._cluster_flags
+    assert merges(lt.plan(flags | _lib.DEC_PROGRAMMATIC)) and not merges(lt.plan(plain | _lib.DEC_PROGRAMMATIC))
+    q = _rand(gen, batch, n_kv * gqa, 128)
+    odd = torch.empty(lt.v_rot.numel() + 1, device=DEV)[1:].view_as(lt.v_rot).copy_(lt.v_rot)       # off its 16-byte boundary
+    top = float((mgr._v_norms[0].float().max() * max(t.centroids.abs().max() for t in lt.v_tables)).item())
+    tile = 256 * c
+    for lo, hi, rot in ((0, 0, lt.v_rot), (0, 1, lt.v_rot), (0, 15, None), (0, 16, odd), (0, 17, lt.v_rot), (16, 16 * c + 1, lt.v_rot),
+                        (0, min(cap, tile), None), (0, min(cap, tile + 1), odd), (64, cap, lt.v_rot), (0, cap, lt.v_rot)):
+        args = dict(rotate=True, v_rot=rot, want_f32=True, want_lse=True, status=mgr._status)
+        out, o32, lse = attend(lt, q, *cache, lo, hi, flags=flags, **args)
+        want, w32, wlse = attend(lt, q, *cache, lo, hi, flags=plain, **args)
+        assert torch.equal(out, o32.half()), (lo, hi)
+        norm = 1.0 if rot is None else 128 ** 0.5           # a rotation may gather a row's whole difference in one dim
+        assert (o32 - w32).abs().max().item() <= 2.0 ** -10 * top * norm, (lo, hi)
+        if lo == hi:
+            assert not o32.any() and torch.equal(lse, wlse) and torch.isinf(lse).all()
+        else:
+            assert (lse - wlse).abs().max().item() <= 1e-5 * max(1.0, wlse.abs().max().item()), (lo, hi)
+    mgr.check_status()
+
+
+@pytest.mark.parametrize("batch,n_kv,gqa,start,cap", [(1, 8, 4, 0, 40), (2, 2, 8, 254, 600), (4, 8, 3, 1020, 1030)])
+def test_layer_steps(batch, n_kv, gqa, start, cap):
+    """A layer's steps call by call and replayed: the same cache bytes as the split form, rows within the bound."""
+    gen = torch.Generator().manual_seed(start)
+    from blockgtq_b200 import BlockGTQKVManager
+    a = _manager(batch, n_kv, gqa, cap, gen)
+    b = BlockGTQKVManager(1, n_kv * gqa, n_kv, 128, max_seq_len=cap, batch_size=batch, device=DEV)
+    b.set_quantizers(0, a.quantizers[0])
+    for m in (a, b):
+        m._ensure_storage()
+    assert a._cluster_flags
+    b._cluster_flags = 0
+    if start:
+        kv = tuple(_rand(gen, batch, n_kv, start, 128) for _ in range(2))
+        for m in (a, b):
+            m.init_from_cache([kv])
+    graph = None
+    for step in range(6):
+        q, k, v = (_rand(gen, batch, n, 1, 128) for n in (n_kv * gqa, n_kv, n_kv))
+        want = b.append_and_attend(0, q, k, v).float()
+        if step < 3:
+            got = a.append_and_attend(0, q, k, v).float()
+        else:
+            for dst, src in zip(a.static_inputs(0), (q, k, v)):
+                dst.copy_(src)
+            if graph is None:
+                a._sync_pos()
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph):
+                    a.layer_step(0)
+            graph.replay()
+            got = a.static_outputs()[0].unsqueeze(2).float()
+        for m in (a, b):
+            m.increment_seq_len()
+        top = float(a._v_norms[0].float().max() * max(t.centroids.abs().max() for t in a._layers[0].v_tables)) * 128 ** 0.5
+        assert (got - want).abs().max().item() <= 2.0 ** -10 * top + 2.0 ** -11 * want.abs().max().item()
+        for x, y in zip((a._k_packed, a._k_norms, a._v_packed, a._v_norms), (b._k_packed, b._k_norms, b._v_packed, b._v_norms)):
+            assert torch.equal(x, y)
+    a.check_status()
