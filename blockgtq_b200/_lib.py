@@ -8,6 +8,7 @@ stream provider.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import importlib.machinery
 import importlib.util
 import os
@@ -188,7 +189,7 @@ def lib():
                            "(python -m blockgtq_b200.build --force)")
     module.bind(*[C.cast(getattr(handle, name), C.c_void_p).value for name in (
         "bgtq_layer_step", "bgtq_layer_encode", "bgtq_attend", "bgtq_decode_default_splits", "bgtq_encode", "bgtq_rotate_q_rows",
-        "bgtq_prefill", "bgtq_prefill_workspace_bytes")])
+        "bgtq_prefill", "bgtq_prefill_workspace_bytes", "bgtq_decode_plan_cluster")])
     native = module
     _lib = handle
     return _lib
@@ -212,6 +213,20 @@ def done(result, what: str, n: int = 1):
 def check(code: int, what: str):
     if code != OK:
         raise RuntimeError(f"{what} failed: {lib().bgtq_error_string(code).decode()} ({code})")
+
+
+def no_grad(fn):
+    """``torch.no_grad()`` around a function that is called often: the decorator's objects cost 2.5 us of each call."""
+    @functools.wraps(fn)
+    def call(*args, **kwargs):
+        if not torch.is_grad_enabled():
+            return fn(*args, **kwargs)
+        torch._C._set_grad_enabled(False)
+        try:
+            return fn(*args, **kwargs)
+        finally:
+            torch._C._set_grad_enabled(True)
+    return call
 
 
 def ptr(t):

@@ -44,6 +44,7 @@ class _AdHocLayer:
                 d.v_lut[i] = int(x)
         self.desc_dev = torch.from_numpy(np.frombuffer(self.desc_host, dtype=np.uint8).copy()).to(device)
         self._plans = {}
+        self._handles = {}
 
     def plan(self, flags=0):
         p = self._plans.get(flags)
@@ -96,7 +97,7 @@ def _layer_for(segments, codebook_flat, v_lut, v_bits, n_kv, device):
     return lt
 
 
-@torch.no_grad()
+@_lib.no_grad
 def fused_blockgtq_decode_attention(
         q, k_packed, k_norms, codebook_flat, lut_offset, norm_group, segments,
         v_codes, v_norms, v_lut, scale=None, block_t=64, block_m=16, t_splits=32,

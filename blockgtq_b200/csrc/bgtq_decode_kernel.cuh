@@ -47,6 +47,8 @@
 #ifndef BGTQ_JIT
 #include "bgtq_common.cuh"
 #include "bgtq_plan.h"
+#include <atomic>
+
 #include "bgtq_decode_params.cuh"
 #include "bgtq_decode_cluster.cuh"
 #endif
@@ -1041,11 +1043,32 @@ inline uint32_t decode_jit_quad_bytes(const DecPlanDev& pl) {
     return decode_smem(pl.lut_bytes, stage) + kQuadBytes <= 227 * 1024 ? kQuadBytes : 0u;
 }
 
+// The kernel may use all of an SM's shared memory on this device: asked for on the first launch there (the driver takes about
+// half a microsecond each time).  A table that is full, or a device past 64, means asking again.
+inline cudaError_t allow_smem(const void* fn, bool clusters) {
+    struct Entry { std::atomic<const void*> fn{nullptr}; std::atomic<uint64_t> done{0}; };
+    static Entry table[1024];
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    Entry* mine = nullptr;
+    const size_t at = (reinterpret_cast<uintptr_t>(fn) >> 4) * 0x9E3779B97F4A7C15ull >> 54;
+    for (size_t i = 0; i < 8 && dev < 64 && !mine; ++i) {
+        Entry& t = table[(at + i) & 1023u];
+        const void* is = t.fn.load(std::memory_order_acquire);
+        if (is == fn || (!is && (t.fn.compare_exchange_strong(is, fn) || is == fn))) mine = &t;
+    }
+    if (mine && mine->done.load(std::memory_order_acquire) >> dev & 1u) return cudaSuccess;
+    cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (r == cudaSuccess && clusters) r = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (r == cudaSuccess && mine) mine->done.fetch_or(1ull << dev, std::memory_order_release);
+    return r;
+}
+
 // Launch one of the kernels; cluster > 0: in clusters of that many CTAs.
 inline cudaError_t launch_decode_fn(const void* fn, const DecParams& P, dim3 grid, size_t smem, cudaStream_t stream, bool programmatic,
                                     int cluster) {
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaError_t e = allow_smem(fn, cluster > 8);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;

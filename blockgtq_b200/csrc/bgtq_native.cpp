@@ -30,6 +30,7 @@ struct Fns {
     decltype(&bgtq_rotate_q_rows) rotate_rows;
     decltype(&bgtq_prefill) prefill;
     decltype(&bgtq_prefill_workspace_bytes) prefill_workspace;
+    decltype(&bgtq_decode_plan_cluster) plan_cluster;
 } F;
 
 PyObject* none() { Py_RETURN_NONE; }
@@ -231,20 +232,26 @@ PyObject* attend(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     const int64_t B = q->size(0), n_q = q->size(1);
     if (kp->size(0) < B || kp->size(1) != n_kv || t1 > kp->size(2)) return none();
     if (ns == 0) ns = F.default_splits((int)B, n_kv, t1 - t0);
-    at::Tensor scratch = empty({B * n_q * (ns * (kHD + 1) + kHD / 2)}, at::kFloat, *q);
-    at::Tensor out = four ? empty({B, n_q, 1, kHD}, at::kHalf, *q) : empty({B, n_q, kHD}, at::kHalf, *q);
+    at::Tensor scratch, out = four ? empty({B, n_q, 1, kHD}, at::kHalf, *q) : empty({B, n_q, kHD}, at::kHalf, *q);
     at::Tensor o32, lse;
     if (want32) o32 = empty({B, n_q, kHD}, at::kFloat, *q);
     if (want_lse) lse = empty({B, n_q}, at::kFloat, *q);
     void* const st = stream_of(*q);
     int rc;
+    bool bare = !rot_k && !bo && F.plan_cluster(plan) > 0;      // a decode that merges its shares and rotates nothing needs no scratch ...
+again:
+    if (!bare) scratch = empty({B * n_q * (ns * (kHD + 1) + kHD / 2)}, at::kFloat, *q);
     Py_BEGIN_ALLOW_THREADS
     rc = F.attend(plan, desc, rot_k, q->data_ptr(), q->stride(0), q->stride(1), kp->data_ptr<uint8_t>(), kp->stride(0), kp->stride(1), kp->stride(2),
                   kn->data_ptr(), kn->stride(0), kn->stride(1), kn->stride(2), vp->data_ptr<uint8_t>(), vp->stride(0), vp->stride(1), vp->stride(2),
                   vn->data_ptr(), vn->stride(0), vn->stride(1), vn->stride(2), (int)B, (int)n_q, n_kv, t0, t1, ns, scale, v_rot,
-                  bo ? bo->data_ptr<float>() : nullptr, bl ? bl->data_ptr<float>() : nullptr, scratch.data_ptr(), out.data_ptr(),
+                  bo ? bo->data_ptr<float>() : nullptr, bl ? bl->data_ptr<float>() : nullptr, bare ? nullptr : scratch.data_ptr(), out.data_ptr(),
                   want32 ? o32.data_ptr<float>() : nullptr, want_lse ? lse.data_ptr<float>() : nullptr, status, st);
     Py_END_ALLOW_THREADS
+    if (bare && rc == BGTQ_E_UNSUPPORTED) {      // ... unless it is left to the split form
+        bare = false;
+        goto again;
+    }
     if (rc != BGTQ_OK) return code(rc);
     return Py_BuildValue("(NNN)", wrap(std::move(out)), want32 ? wrap(std::move(o32)) : none(), want_lse ? wrap(std::move(lse)) : none());
 }

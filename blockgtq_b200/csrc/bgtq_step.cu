@@ -93,7 +93,8 @@ extern "C" __attribute__((visibility("default"))) int bgtq_attend(
     int64_t vn_sh, int64_t vn_st, int32_t n_batch, int32_t n_q, int32_t n_kv, int32_t t_begin, int32_t t_end, int32_t n_splits,
     float scale, const float* v_rot, const float* buf_o, const float* buf_lse, void* scratch, void* out, float* out_f32,
     float* lse_out, int32_t* status, void* stream) {
-    if (!plan || !q || !scratch || !out || n_batch < 1 || n_q < 1 || n_splits < 1) return BGTQ_E_BADARG;
+    if (!plan || !q || !out || n_batch < 1 || n_q < 1 || n_splits < 1) return BGTQ_E_BADARG;
+    if (!scratch && (rot_k || buf_o || !bgtq_decode_plan_cluster(plan))) return BGTQ_E_BADARG;
     if (reinterpret_cast<uintptr_t>(scratch) & 15u) return BGTQ_E_ALIGN;
     const int64_t rows = (int64_t)n_batch * n_q;
     float* const part_o = static_cast<float*>(scratch);
@@ -115,7 +116,7 @@ extern "C" __attribute__((visibility("default"))) int bgtq_attend(
         const int rc = launch_decode_plan(plan, q_dec, k_packed, kp_sb, kp_sh, kp_st, k_norms, kn_sb, kn_sh, kn_st, v_packed, vp_sb, vp_sh,
                                           vp_st, v_norms, vn_sb, vn_sh, vn_st, n_batch, n_q, n_kv, t_begin, t_end, 1, scale, nullptr,
                                           nullptr, status, nullptr, 0, false, &M, stream);
-        if (rc != BGTQ_E_UNSUPPORTED) return rc;
+        if (rc != BGTQ_E_UNSUPPORTED || !scratch) return rc;
     }
     const int rc = launch_decode_plan(plan, q_dec, k_packed, kp_sb, kp_sh, kp_st, k_norms, kn_sb, kn_sh, kn_st, v_packed, vp_sb, vp_sh,
                                       vp_st, v_norms, vn_sb, vn_sh, vn_st, n_batch, n_q, n_kv, t_begin, t_end, n_splits, scale, part_o,

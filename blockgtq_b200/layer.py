@@ -123,6 +123,7 @@ class LayerTables:
         self.head_perm = torch.stack([t.head_perm for t in k_tables]).long().to(self.device)   # (n_kv, 128)
         self.addrs = (self.desc_dev.data_ptr(), self.rot_k.data_ptr(), self.rot_v.data_ptr())
         self._plans = {}
+        self._handles = {}
         self._partition = None
         self._row_strides = {}
         self._early_fresh = 0
@@ -411,20 +412,21 @@ def attend(layer, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, *, ro
            v_rot=None, buf_o=None, buf_lse=None, want_f32=False, want_lse=False, status=None):
     """Query rotation (``rotate``: q is in the original basis), split-KV decode over rows [t_begin, t_end) and combine
     in one library call.  q (B, n_q, [1,] 128) -> (out fp16 of q's shape, f32 copy (B, n_q, 128) | None, LSE | None)."""
-    plan, ptr = layer.plan(flags | _lib.DEC_PROGRAMMATIC), _lib.ptr
+    plan, desc, rot_k, merged = _handle(layer, flags | _lib.DEC_PROGRAMMATIC)
+    if not rotate:
+        rot_k = None
     n_splits = 0 if n_splits is None else n_splits or -1       # (the library's choice; 0 is refused like -1)
-
-    def call():
-        return _lib.host().attend(
-            C.addressof(plan), ptr(layer.desc_dev), ptr(layer.rot_k) if rotate else None, q, k_packed, k_norms, v_packed, v_norms,
-            t_begin, t_end, n_splits, _SCALE if scale is None else scale, None if v_rot is None else ptr(v_rot), buf_o, buf_lse,
-            want_f32, want_lse, None if status is None else ptr(status), layer.n_kv)
-
+    scale = _SCALE if scale is None else scale
+    v_rot = None if v_rot is None else v_rot.data_ptr()
+    status = None if status is None else status.data_ptr()
+    native = _lib.host().attend
     try:
-        r = call()
+        r = native(plan, desc, rot_k, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, n_splits, scale, v_rot, buf_o, buf_lse,
+                   want_f32, want_lse, status, layer.n_kv)
     except TypeError:       # (ranges as whole floats, say)
         t_begin, t_end, n_splits = int(t_begin), int(t_end), int(n_splits)
-        r = call()
+        r = native(plan, desc, rot_k, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, n_splits, scale, v_rot, buf_o, buf_lse,
+                   want_f32, want_lse, status, layer.n_kv)
     if r is None:           # another type or layout, or an argument to complain about
         _lib.require_cuda(q, "q")
         if k_norms.dtype != torch.float16 or v_norms.dtype != torch.float16:
@@ -433,10 +435,11 @@ def attend(layer, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, *, ro
             _strides3(t)
         with torch.cuda.device(q.device):
             q = q.to(torch.float16).contiguous()
-            r = call()
+            r = native(plan, desc, rot_k, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, n_splits, scale, v_rot, buf_o, buf_lse,
+                       want_f32, want_lse, status, layer.n_kv)
         if r is None:
             raise ValueError("query, cache and layer do not match")
-    return _lib.done(r, "bgtq_attend", (3 if rotate else 2) - (buf_o is None and merges(plan)))
+    return _lib.done(r, "bgtq_attend", (3 if rotate else 2) - (merged and buf_o is None))
 
 
 _SCALE = 1.0 / math.sqrt(HD)
@@ -459,9 +462,21 @@ def tile_flags(n_batch: int, n_kv: int, n_tokens: int, device) -> int:
     return _lib.DEC_NARROW if n_batch * n_kv * n_tokens <= 256 * _sm_count(index) else 0
 
 
-def merges(plan) -> bool:
-    """Whether the plan's decode merges its shares itself in layer steps and attentions."""
-    return _lib.lib().bgtq_decode_plan_cluster(C.addressof(plan)) > 0
+def merges(layer, flags: int) -> bool:
+    """Whether the layer's decode with these plan flags merges its shares itself in layer steps and attentions."""
+    return _handle(layer, flags)[3]
+
+
+def _handle(layer, flags: int):
+    """What a call with these plan flags passes on each time: addresses of the plan, the descriptors and K's rotation (their
+    owner keeps all three for its life), and whether the decode merges its shares."""
+    h = layer._handles.get(flags)
+    if h is None:
+        plan = layer.plan(flags)
+        rot = getattr(layer, "rot_k", None)
+        h = layer._handles[flags] = (C.addressof(plan), _lib.ptr(layer.desc_dev), None if rot is None else _lib.ptr(rot),
+                                     _lib.lib().bgtq_decode_plan_cluster(C.addressof(plan)) > 0)
+    return h
 
 
 def cluster_flags(n_batch: int, n_kv: int, n_tokens: int, device, grows: bool = False) -> int:
@@ -479,14 +494,23 @@ def cluster_flags(n_batch: int, n_kv: int, n_tokens: int, device, grows: bool = 
     11.1 and 8.7 us, 500: 12.1 and 8.9, 2000: 12.2 and 10.4, 4000: 12.7 and 12.9, 6000: 14.0 and 15.0 (not taken); 2 KV heads x 8 at 500
     tokens 10.0 and 8.7; 4 sequences x 8 heads x 3: 500: 14.7 and 10.1, 4099: 22.1 and 20.0, 8500: 31.9 and 30.2 (x 4); 8 sequences: 500: 16.1 and
     13.1, 3000: 27.7 and 24.1, 4300: 32.0 and 30.9."""
-    index = device.index if device.index is not None else torch.cuda.current_device()
-    sms, pairs = _sm_count(index), n_batch * n_kv
-    c = next((c for c, most in ((8, 14), (4, 32), (2, 72)) if pairs <= most * sms // 148), 0)
-    if c == 0 or n_tokens * (sms - pairs * c) > 330 * sms * c:
+    pairs = n_batch * n_kv
+    sms = _sm_count(device.index if device.index is not None else torch.cuda.current_device())
+    c, most = _largest_cluster(pairs, sms)
+    if n_tokens > most:
         return 0
     while not grows and c > 2 and 2 * n_tokens <= (256 if 2 * pairs * c > sms else 128) * c:
         c //= 2
     return _lib.DEC_NARROW | c << _lib.DEC_CLUSTER_SHIFT
+
+
+@functools.lru_cache(maxsize=1024)
+def _largest_cluster(pairs: int, sms: int):
+    """(C, the most tokens it is taken for): tokens / C - pairs * tokens / sms <= 330."""
+    for c, most in ((8, 14), (4, 32), (2, 72)):
+        if pairs <= most * sms // 148:
+            return c, 330 * sms * c // (sms - pairs * c) if pairs * c < sms else 1 << 30
+    return 0, -1
 
 
 _PREFILL_WORKSPACE = 2 << 30        # bytes of dequantised operand tiles per launch

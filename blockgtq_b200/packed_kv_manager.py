@@ -56,6 +56,7 @@ class BlockGTQKVManager:
         self._max_k_packed_bytes = 0
         self._max_n_groups = 0
         self._k_packed = self._k_norms = self._v_packed = self._v_norms = None
+        self._rows = (None, None)             # a layer's views of these, see _layer_rows
         self._part_dev = self._part_key = self._part_len = None
         # three-region policy
         self.n_sink, self.recent_window, self.block_size = int(n_sink), int(recent_window), int(block_size)
@@ -178,6 +179,15 @@ class BlockGTQKVManager:
             self._k_buf = torch.zeros(self.n_layers, self.B, self.n_kv, self._buf_cap, self.hd,
                                       dtype=torch.float16, device=dev)
             self._v_buf = torch.zeros_like(self._k_buf)
+
+    def _layer_rows(self, li: int):
+        """Layer ``li``'s packed K, K norms, packed V and V norms (four views cost ten microseconds to make)."""
+        of = (self._k_packed, self._k_norms, self._v_packed, self._v_norms)
+        seen, rows = self._rows
+        if seen is None or any(a is not b for a, b in zip(seen, of)):
+            rows = list(zip(*(t.unbind(0) for t in of)))
+            self._rows = (of, rows)
+        return rows[li]
 
     def _norm_row_groups(self) -> int:
         return self._max_n_groups + (self._max_n_groups & 1)
@@ -375,7 +385,7 @@ class BlockGTQKVManager:
             kb, vb = self._k_buf[li], self._v_buf[li]
             s.k_buf, s.v_buf, s.kb_sb, s.kb_sh = kb.data_ptr(), vb.data_ptr(), kb.stride(0), kb.stride(1)
             s.buf_o, s.buf_lse, s.n_sink, s.window = self._buf_o.data_ptr(), self._buf_lse.data_ptr(), self.n_sink, self.recent_window
-        s.key, s.addr, s.n_launch = (lt, baked, pd), C.addressof(s), 4 if self._buffered else 3 - merges(plan)
+        s.key, s.addr, s.n_launch = (lt, baked, pd), C.addressof(s), 4 if self._buffered else 3 - merges(lt, self._dec_flags | self._cluster_flags | (_lib.DEC_PROGRAMMATIC if pd else 0))
         self._steps[li] = s
         return s
 
@@ -528,7 +538,7 @@ class BlockGTQKVManager:
             self._flush(layer_idx, f0, f1)
         return out.unsqueeze(2)
 
-    @torch.no_grad()
+    @_lib.no_grad
     def attend(self, layer_idx: int, q: torch.Tensor, seq_len: int = None, *, n_splits: int = None,
                token_range=None, want_partial: bool = False, flushed: int = None, with_buffers: bool = True):
         """Attention of q (B, n_q, [1,] hd) over the first ``seq_len`` cached tokens.
@@ -541,8 +551,9 @@ class BlockGTQKVManager:
         seq_len = self.seq_len if seq_len is None else seq_len
         n_sink_tok, n_packed, n_recent = self._region_sizes(seq_len, flushed)
         if q.dim() == 4:
-            q = q[:, :, 0]
-        q = q.to(torch.float16)
+            q = q.select(2, 0)
+        if q.dtype != torch.float16:
+            q = q.to(torch.float16)
         lo, hi = (0, n_packed) if token_range is None else token_range
         lo = max(0, min(lo, n_packed))
         hi = max(lo, min(hi, n_packed))
@@ -550,7 +561,7 @@ class BlockGTQKVManager:
         buf_o = buf_lse = None
         if self._buffered and with_buffers:
             buf_o, buf_lse = self._buffer_partial(li, q, n_sink_tok, n_packed, n_recent)
-        return attend(lt, q, self._k_packed[li], self._k_norms[li], self._v_packed[li], self._v_norms[li], lo, hi, rotate=not baked,
+        return attend(lt, q, *self._layer_rows(li), lo, hi, rotate=not baked,
                       n_splits=n_splits, scale=self.scale, flags=self._dec_flags | self._cluster_flags, v_rot=lt.v_rot, buf_o=buf_o, buf_lse=buf_lse,
                       want_f32=want_partial, want_lse=want_partial, status=self._status)
 

@@ -35,7 +35,7 @@ def test_merged_in_the_launch(batch, n_kv, gqa, cap, k_bits, v_bits, mixed, c):
     assert mgr._cluster_flags >> _lib.DEC_CLUSTER_SHIFT == c
     lt, cache = mgr._layers[0], (mgr._k_packed[0], mgr._k_norms[0], mgr._v_packed[0], mgr._v_norms[0])
     plain, flags = mgr._dec_flags, mgr._dec_flags | mgr._cluster_flags
-    assert merges(lt.plan(flags | _lib.DEC_PROGRAMMATIC)) and not merges(lt.plan(plain | _lib.DEC_PROGRAMMATIC))
+    assert merges(lt, flags | _lib.DEC_PROGRAMMATIC) and not merges(lt, plain | _lib.DEC_PROGRAMMATIC)
     q = _rand(gen, batch, n_kv * gqa, 128)
     odd = torch.empty(lt.v_rot.numel() + 1, device=DEV)[1:].view_as(lt.v_rot).copy_(lt.v_rot)       # off its 16-byte boundary
     top = float((mgr._v_norms[0].float().max() * max(t.centroids.abs().max() for t in lt.v_tables)).item())
@@ -94,3 +94,29 @@ def test_layer_steps(batch, n_kv, gqa, start, cap):
         for x, y in zip((a._k_packed, a._k_norms, a._v_packed, a._v_norms), (b._k_packed, b._k_norms, b._v_packed, b._v_norms)):
             assert torch.equal(x, y)
     a.check_status()
+
+
+def test_rows_too_wide_for_the_merging_form():
+    """Packed rows padded until the stages no longer fit beside the shares: the call is left to the split form."""
+    from blockgtq_b200 import fused_blockgtq_decode_attention
+    from blockgtq_b200.quantizer import BlockGTQQuantizer
+    from helpers import HD, synth_head
+    gen = torch.Generator().manual_seed(5)
+    qz = BlockGTQQuantizer(HD, avg_bits=4.0, device=torch.device(DEV))
+    qc, kc = synth_head(gen, 256, 4)
+    qz.calibrate(qc.float(), kc.float())
+    qz.init_v_quantizer(v_bits=4, seed=42)
+    ka, T = qz.build_kernel_args(), 700
+    kp, kn, _ = qz.compress_packed(_rand(gen, 1, 1, T, HD))
+    vp, vn = qz.compress_v_packed(_rand(gen, 1, 1, T, HD))
+    q = qz.rotate_q_for_packed_kernel(_rand(gen, 1, 4, 1, HD))
+    kw = torch.zeros(1, 1, T + 8, 160, dtype=torch.uint8, device=DEV)[:, :, :T, :kp.shape[3]]
+    kw.copy_(kp)
+
+    def call(k):
+        return fused_blockgtq_decode_attention(q, k, kn.half(), ka["codebook_flat"], ka["lut_offset"], ka["norm_group"], ka["segments_b"],
+                                               vp, vn, qz.v_lut, v_bits=4, v_rotation=qz._v_rot, return_lse=True)
+    (a, al), (b, bl) = call(kp), call(kw)
+    top = float(vn.float().max() * qz.v_lut.float().abs().max()) * HD ** 0.5
+    assert (a.float() - b.float()).abs().max().item() <= 2.0 ** -10 * top + 2.0 ** -11 * b.float().abs().max().item()
+    assert (al - bl).abs().max().item() <= 1e-5 * max(1.0, bl.abs().max().item())
