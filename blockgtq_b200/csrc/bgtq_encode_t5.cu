@@ -1,22 +1,24 @@
-// Bulk (prefill) encoder: rotation on tcgen05, then one pass of a thread over its half of a row.
+// Bulk (prefill) encoder: rotation on tcgen05, then one pass of a thread over its part of a row.
 //
 //   * a CTA of 16 warps works on tiles of 128 rows of one (KV head, K or V); the rotation W is staged once as
 //     hi = fp16(W), lo = fp16((W - hi) * 2^10) in the tensor cores' operand layout;
-//   * the warps form two groups of eight, which run out of phase, each on its own tiles: rows arrive by cp.async a
-//     tile ahead (V: straight into the operand's swizzled layout; K: and move on into packed order), two warps issue 8
-//     tcgen05.mma each (x . hi and x . lo into 2 x 128 tensor-memory columns), and meanwhile all warps sum the rows' group
-//     norms;
-//   * then thread (row, half) takes its half of the row's columns eight at a time straight from tensor memory (tcgen05.ld of
-//     one lane): the row is the thread's own, so everything that depends on the column (segment, bin grid, code width,
-//     byte position) is uniform over the warp, codes never leave registers, two values share an instruction where they can
-//     (f32x2), and whole 32-bit words of the packed row go to a staging image of the tile that leaves as coalesced words.
+//   * the warps form two groups of eight, which run out of phase, each on its own tiles (a CTA with a single tile: all sixteen
+//     on it): rows arrive by cp.async a tile ahead (V: straight into the operand's swizzled layout; K: and move on into packed
+//     order, the two dims of a RoPE pair as one word), two warps issue 8 tcgen05.mma each (x . hi and x . lo into 2 x 128
+//     tensor-memory columns), and meanwhile all warps sum the rows' group norms;
+//   * then thread (row, half or quarter) takes its part of the row's columns eight at a time straight from tensor memory
+//     (tcgen05.ld of one lane): the row is the thread's own, so everything that depends on the column (segment, bin grid, code
+//     width, byte position) is uniform over the warp and comes ready made from a list (E5Rec), codes never leave registers, two
+//     values share an instruction where they can (f32x2), and whole 32-bit words of the packed row go to a staging image of the
+//     tile that leaves as coalesced words.
 // Bound: instruction issue and its latencies with 16 warps per SM (all registers and shared memory are taken): 1 048 576 K and
-// as many V rows take 452 us (K rows alone 286, V rows 164), where the bytes alone would take 100: 133 warp instructions per
-// row, issue slots and the shared-memory pipe 56 % busy each, tensor pipe 13 %, DRAM 16 %.  K rows cost what V's do not: the
-// move into packed order and a norm per group.  The form before gave a
-// quad of lanes four rows and four columns each, loaded three tables per element and passed the codes through shared memory
-// to a packing pass: 204 warp instructions per row and 753 us.  Tried and slower: rolled loops (smaller code, less overlap
-// of the table lookups: 589 us).
+// as many V rows take 391 us (K rows alone 229, V rows 164), where the bytes alone would take 100.  K rows cost what V's do
+// not: the move into packed order and a norm per group.  Before the list, the norms by whole segments and the moves in pairs
+// K rows took 286 us (both 451): every thread worked out each task's control for itself, a third of the loop.  A launch of
+// one tile per CTA (777 tokens of 8 heads) takes 8.6 us, and took 10.8 with half of the warps idle.  The form before that
+// gave a quad of lanes four rows and four columns each, loaded three tables per element and passed the codes through shared
+// memory to a packing pass: 753 us.  Tried and slower: rolled loops (smaller code, less overlap of the table lookups: 589 us);
+// squares of converted fp16 values instead of mixed-precision multiply-adds (K 277 -> 287, V 164 -> 168).
 // The sums that decide a code (group norms, products) keep the order they had: the packed bytes are bit for bit the same.
 // Every wait is bounded; tensor memory is released on every path out of the kernel.
 #include "bgtq_common.cuh"
@@ -43,8 +45,17 @@ constexpr int kLutLd = BGTQ_N_BINS + 4;
 
 // Up to eight consecutive codes of one segment, at most 32 bits: first column | count << 8 | stored bits << 12 | segment << 16
 // | bytes << 20.
-// A K row's tasks follow each other in its bytes; half 0 of a row takes tasks [0, split), half 1 the rest.  (A V row is
-// cut in the middle.)
+// A K row's tasks follow each other in its bytes; its threads take equal numbers of them.
+// What the packing of a task needs, ready made (read by all lanes at one address).
+struct E5Rec {
+    uint32_t col;       // first column to load | 2 (first column of the task - that) << 8: a last short task loads from column 120
+    uint32_t mask;      // the valid bits of its code word
+    uint32_t lut;       // shared address of its segment's code table - 0x4B000000 (see bin_addr2)
+    uint32_t part;      // byte offset of its segment's row factors
+    float off, scale;   // bin = (y + off) * scale, in units of 256 bins
+    uint32_t mul;       // 2^(stored bits)
+    uint32_t ctl;       // bit position in its first word | 256 where it completes that word | byte offset of the word in the row << 16
+};
 struct E5Smem {
     __align__(128) uint8_t w_hi[kTile];
     __align__(128) uint8_t w_lo[kTile];
@@ -59,9 +70,10 @@ struct E5Smem {
     float kcent[512];
     uint8_t code_lut[kSeg][kLutLd];                 // entry 256 = entry 255; V: [0] = boundaries below the bin
     float2 grid[kSeg];                              // in units of 256 bins.  K: {offset, 1 / range}; V: [0] = {1 / range, offset / range}
-    __align__(16) uint8_t norm_ctl[2][16];          // K, per half and 16-byte chunk: pairs to sum (bits 0..3), segments that end behind a pair (4..7)
     uint32_t tasks[kMaxTasks];
-    int32_t n_tasks, split, split_byte, row_bytes, data_bytes, n_seg, v_search, v_sb, v_nb;
+    E5Rec rec[kMaxTasks];
+    int32_t cut[5], cut_byte[5];                    // K: first task of each quarter of the tasks, and its first byte
+    int32_t row_bytes, n_seg, paired, v_search, v_sb, v_nb;
     int32_t seg_start[kSeg], seg_len[kSeg], seg_bw[kSeg], seg_lut_off[kSeg];
     __align__(16) uint16_t to[kHD];                 // K: operand offset (row 0) of an input column, its packed position's place
     __align__(8) uint64_t mma_bar[2];
@@ -112,7 +124,7 @@ __device__ __forceinline__ uint32_t squeeze8(const uint32_t (&c)[8], uint32_t m)
 struct ByteStream {
     uint32_t addr;      // shared address of the word being filled
     uint32_t acc, pos;  // its bits so far
-    uint32_t skip;      // bits of the first word that belong to the row's other half
+    uint32_t skip;      // bits of the first word that belong to the part before
     __device__ __forceinline__ void open(uint32_t row_addr, uint32_t byte) {
         addr = row_addr + (byte & ~3u);
         pos = skip = (byte & 3u) * 8u;
@@ -138,6 +150,25 @@ struct ByteStream {
             pos -= 32u;
         }
     }
+    // a task's code word (see E5Rec::ctl)
+    __device__ __forceinline__ void word(uint32_t w, uint32_t ctl, uint32_t row_addr) {
+        const uint32_t at = ctl & 31u;
+        acc |= w << at;
+        if (ctl & 256u) {
+            addr = row_addr + (ctl >> 16);
+            if (skip) {
+                bytes(skip, 32u);
+                skip = 0u;
+            } else {
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(acc) : "memory");
+            }
+            acc = __funnelshift_rc(w, 0u, 32u - at);       // what did not fit (position 0: nothing)
+        }
+    }
+    __device__ __forceinline__ void end_at(uint32_t row_addr, uint32_t byte) {
+        addr = row_addr + (byte & ~3u);
+        pos = (byte & 3u) * 8u;
+    }
     __device__ __forceinline__ void close() { bytes(skip, pos); }
 };
 
@@ -157,7 +188,7 @@ __device__ void e5_setup(E5Smem& S, const EncParams& P, const BgtqHeadDesc& d, b
         S.v_sb = (P.flags & BGTQ_ENC_V_NIBBLE) ? 4 : d.v_bits;
         S.v_nb = (1 << d.v_bits) - 1;
     }
-    if (tid < kHD) S.to[d.head_perm[tid]] = (uint16_t)((tid >> 6) * 16384 + ((tid >> 3) & 7) * 16 + (tid & 7) * 2);
+    if (tid < kHD) S.to[d.head_perm[tid] & (kHD - 1)] = (uint16_t)((tid >> 6) * 16384 + ((tid >> 3) & 7) * 16 + (tid & 7) * 2);
     if (is_v) {
         S.vbound[tid >> 5][tid & 31] = d.v_bounds[tid >> 5];
         S.vcent[tid >> 5][tid & 31] = d.v_cents[tid >> 5];
@@ -181,7 +212,9 @@ __device__ void e5_setup(E5Smem& S, const EncParams& P, const BgtqHeadDesc& d, b
         *reinterpret_cast<uint4*>(S.w_hi + o) = *reinterpret_cast<uint4*>(hi);
         *reinterpret_cast<uint4*>(S.w_lo + o) = *reinterpret_cast<uint4*>(lo);
     }
-    __syncthreads();
+    // RoPE pairs (dims i, i + 64) side by side in packed order, as the reference's calibration lays every head out
+    const bool pair = tid >= kHD / 2 || (d.head_perm[2 * tid] < kHD / 2 && d.head_perm[2 * tid + 1] == d.head_perm[2 * tid] + kHD / 2);
+    const int paired = __syncthreads_and(is_v || pair);
     if (is_v) {
         // V codes count the boundaries below a value.  A monotonic grid of 256 bins finds all but one of them: the table
         // holds the boundaries in earlier bins, and one comparison with the next boundary settles the rest, as long as no
@@ -213,80 +246,107 @@ __device__ void e5_setup(E5Smem& S, const EncParams& P, const BgtqHeadDesc& d, b
             const int st = live ? S.seg_start[lane] : 0, len = live ? S.seg_len[lane] : 0, bw = live ? S.seg_bw[lane] : 1;
             const int sb = (P.flags & BGTQ_ENC_K_MIXED) ? (bw <= 4 ? 4 : 8) : (bw <= 4 ? bw : 8), per = sb == 8 ? 4 : 8;
             auto n_bytes = [&](int n) { return sb == 3 ? 3 : (n * sb + 7) >> 3; };
-            const int nt = (len + per - 1) / per, bytes = nt > 0 ? (nt - 1) * n_bytes(per) + n_bytes(len - (nt - 1) * per) : 0;
-            int t_at = nt, b_at = bytes;
+            const int nt = (len + per - 1) / per;
+            int t_at = nt;
 #pragma unroll
             for (int o = 1; o < 8; o <<= 1) {
-                const int tu = __shfl_up_sync(0xffffffffu, t_at, o), bu = __shfl_up_sync(0xffffffffu, b_at, o);
-                if (lane >= o) {
-                    t_at += tu;
-                    b_at += bu;
-                }
+                const int tu = __shfl_up_sync(0xffffffffu, t_at, o);
+                if (lane >= o) t_at += tu;
             }
-            if (lane == n_seg - 1) {
-                S.n_tasks = S.split = t_at;
-                S.data_bytes = S.split_byte = b_at;
-            }
-            __syncwarp();
+            const int n_tasks = __shfl_sync(0xffffffffu, t_at, n_seg - 1);
             t_at -= nt;
-            b_at -= bytes;
 #pragma unroll 1
             for (int c = 0; c < nt; ++c) {
                 const int first = st + per * c, n = min(per, len - per * c);
                 S.tasks[t_at + c] = (uint32_t)first | (uint32_t)n << 8 | (uint32_t)sb << 12 | (uint32_t)lane << 16 | (uint32_t)n_bytes(n) << 20;
-                // the row is cut before its first task in the upper half of the columns
-                if (first >= kHD / 2 && first - (c > 0 ? per : (st > 0 ? 1 : kHD)) < kHD / 2) {
-                    S.split = t_at + c;
-                    S.split_byte = b_at + c * n_bytes(per);
-                }
             }
-            if (lane == 0) S.row_bytes = P.kp_row_bytes;
-        } else if (warp == 1) {        // lane = (half, chunk): which of the chunk's pairs the half sums, where segments end
-            const int hf = lane >> 4, c = lane & 15;
-            uint32_t ctl = 0u;
+            __syncwarp();
+            int at = 0;
 #pragma unroll 1
-            for (int s = 0; s < n_seg; ++s) {
-                const int p0 = S.seg_start[s] >> 1, p1 = p0 + (S.seg_len[s] >> 1);
-                for (int j = 0; j < 4; ++j) {
-                    const int p = 4 * c + j;
-                    if (p >= p0 && p < p1 && ((p - p0) & 1) == hf) ctl |= 1u << j;
-                    if (p == p1 - 1) ctl |= 16u << j;
+            for (int base = 0; base < n_tasks; base += 32) {        // lane = task
+                const int t = base + lane;
+                const uint32_t task = t < n_tasks ? S.tasks[t] : 0u;
+                const int nb = (int)(task >> 20);
+                int end = nb;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int x = __shfl_up_sync(0xffffffffu, end, o);
+                    if (lane >= o) end += x;
+                }
+                const int byte = at + end - nb;
+                at += __shfl_sync(0xffffffffu, end, 31);
+                if (t < n_tasks) {
+                    const int first = task & 0xFF, bits = (int)((task >> 8) & 15u) * (int)((task >> 12) & 15u), seg = (task >> 16) & 15u;
+                    const int col = min(first, kHD - 8), pos = 8 * (byte & 3);
+                    E5Rec r;
+                    r.col = (uint32_t)col | (uint32_t)(first - col) << 8;
+                    r.mask = bits >= 32 ? ~0u : (1u << bits) - 1u;
+                    r.lut = smem_u32(S.code_lut[seg]) - 0x4B000000u;
+                    r.part = (uint32_t)(seg * kTileRows * 4);
+                    r.off = -S.grid[seg].x;
+                    r.scale = S.grid[seg].y;
+                    r.mul = 1u << ((task >> 12) & 15u);
+                    r.ctl = (uint32_t)pos | (pos + 8 * nb >= 32 ? 256u : 0u) | (uint32_t)(byte & ~3) << 16;
+                    S.rec[t] = r;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (t == (n_tasks * k + 2) / 4) {
+                            S.cut[k] = t;
+                            S.cut_byte[k] = byte;
+                        }
                 }
             }
-            S.norm_ctl[hf][c] = (uint8_t)ctl;
+            if (lane == 0) {
+                S.cut[4] = n_tasks;
+                S.cut_byte[4] = at;
+                S.row_bytes = P.kp_row_bytes;
+                S.paired = paired;
+#pragma unroll 1
+                for (int k = 1; k < 4; ++k)         // (fewer than two tasks: empty quarters)
+                    if ((n_tasks * k + 2) / 4 >= n_tasks) {
+                        S.cut[k] = n_tasks;
+                        S.cut_byte[k] = at;
+                    }
+            }
         }
     }
 }
-
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
     return v;
 }
 
-// Half a V row: 64 columns of one thread's tensor-memory lane -> its bytes in the staged row; returns the sum of the squared
-// levels.  SEARCH: boundaries by halving (see e5_setup).
-template <bool SEARCH, bool CODES>
-__device__ __forceinline__ float e5_half_v(E5Smem& S, uint32_t lane_base, int hf, float r, uint32_t row_addr, uint8_t* codes) {
+// acc + x0^2 + x1^2 of two fp16 values, in that order (fp16 -> fp32 is exact: the same bits as converting first)
+__device__ __forceinline__ float square2(float acc, uint32_t w) {
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tfma.rn.f32.f16 %0, l, l, %0;\n\tfma.rn.f32.f16 %0, h, h, %0;\n\t}" : "+f"(acc) : "r"(w));
+    return acc;
+}
+
+// Columns [first, first + 8 N) of a V row, of one thread's tensor-memory lane -> its bytes in the staged row; returns the sum
+// of the squared levels (added up quarter by quarter).  SEARCH: boundaries by halving (see e5_setup).
+template <bool SEARCH, bool CODES, int N>
+__device__ __forceinline__ float e5_cols_v(E5Smem& S, uint32_t lane_base, int first, float r, uint32_t row_addr, uint8_t* codes) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lut = smem_u32(S.code_lut[0]) - 0x4B000000u, vb = smem_u32(&S.vbound[0][lane]);
     constexpr uint32_t kCent = sizeof(S.vbound);          // vcent lies behind vbound
     const float2 g = S.grid[0];
     const uint32_t sb = (uint32_t)S.v_sb, mul = 1u << sb;
-    const uint32_t col = lane_base + 64u * hf;
+    const uint32_t col = lane_base + (uint32_t)first;
     const uint64_t r2 = pack_f2(r, r), scale2 = pack_f2(1.0f / kLoScale, 1.0f / kLoScale);
-    uint32_t addr = row_addr + 8u * sb * hf, acc = 0u, pos = 0u;
+    uint32_t addr = row_addr + sb * (uint32_t)first / 8u, acc = 0u, pos = 0u;
     uint64_t csq2 = 0ull;
+    float csq = 0.f;
     float hi[2][8], lo[2][8];
     tmem_ld8(col, hi[0]);
     tmem_ld8(col + kHD, lo[0]);
 #pragma unroll
-    for (int t2 = 0; t2 < 8; t2 += 2) {
+    for (int t2 = 0; t2 < N; t2 += 2) {
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             const int ti = t2 + u;
             tmem_ld_wait();
-            if (ti + 1 < 8) {       // the next columns come while these are worked on
+            if (ti + 1 < N) {       // the next columns come while these are worked on
                 tmem_ld8(col + 8u * (ti + 1), hi[u ^ 1]);
                 tmem_ld8(col + kHD + 8u * (ti + 1), lo[u ^ 1]);
             }
@@ -315,7 +375,7 @@ __device__ __forceinline__ float e5_half_v(E5Smem& S, uint32_t lane_base, int hf
             }
             if (CODES && codes) {
 #pragma unroll
-                for (int e = 0; e < 8; ++e) codes[64 * hf + 8 * ti + e] = (uint8_t)c[e];
+                for (int e = 0; e < 8; ++e) codes[first + 8 * ti + e] = (uint8_t)c[e];
             }
             const uint32_t w = squeeze8(c, mul);
             acc |= w << pos;
@@ -326,10 +386,50 @@ __device__ __forceinline__ float e5_half_v(E5Smem& S, uint32_t lane_base, int hf
             }
             pos = (pos + 8u * sb) & 31u;
         }
+        if ((t2 & 3) == 2) {        // a quarter ends
+            float s0, s1;
+            unpack_f2(csq2, s0, s1);
+            csq += s0 + s1;
+            csq2 = 0ull;
+        }
     }
-    float s0, s1;
-    unpack_f2(csq2, s0, s1);
-    return s0 + s1;
+    return csq;
+}
+
+// Sums of squares of segments first, first + step, .. of a K row: of its pairs 0, 2, .. and of its pairs 1, 3, .., each in
+// order.  A 16-byte load brings four pairs, even and odd positions into a sum of their own; what belongs to a neighbour in a
+// segment's first and last chunk counts as zero.  (Bits that said per chunk what to do with each pair took three times the
+// instructions: 4 x 32768 tokens x 8 heads of K rows alone 286 us with them and the tasks' control worked out by every
+// thread, 232 with this and E5Rec.)
+__device__ __forceinline__ void e5_norms_k(E5Smem& S, int grp, uint32_t tile, int row, int first, int step) {
+    const uint32_t xr = tile + (uint32_t)row * 128u, sw = (uint32_t)(row & 7) << 4;
+    const int n_seg = S.n_seg;
+#pragma unroll 1
+    for (int s = first; s < n_seg; s += step) {
+        const int p0 = S.seg_start[s] >> 1, p1 = p0 + (S.seg_len[s] >> 1), c0 = p0 >> 2, c1 = (p1 - 1) >> 2;
+        auto chunk = [&](int c) { return lds128(xr + (uint32_t)(c >> 3) * 16384u + (((uint32_t)(c & 7) << 4) ^ sw)); };
+        float even = 0.f, odd = 0.f;        // of positions
+        auto add = [&](const uint4& v) {
+            even = square2(even, v.x);
+            odd = square2(odd, v.y);
+            even = square2(even, v.z);
+            odd = square2(odd, v.w);
+        };
+        auto cut = [&](uint4 v, int c) {
+            const uint32_t lo = (uint32_t)(p0 - 4 * c), n = (uint32_t)(p1 - p0);
+            v.x = 0u - lo < n ? v.x : 0u;
+            v.y = 1u - lo < n ? v.y : 0u;
+            v.z = 2u - lo < n ? v.z : 0u;
+            v.w = 3u - lo < n ? v.w : 0u;
+            return v;
+        };
+        add(cut(chunk(c0), c0));
+#pragma unroll 4
+        for (int c = c0 + 1; c < c1; ++c) add(chunk(c));
+        if (c1 > c0) add(cut(chunk(c1), c1));
+        S.part[grp][0][s][row] = p0 & 1 ? odd : even;
+        S.part[grp][1][s][row] = p0 & 1 ? even : odd;
+    }
 }
 
 // operand descriptor of a tile in the 128-byte-swizzle layout; k-step ks of 16: see tile_step
@@ -337,21 +437,17 @@ __device__ __forceinline__ uint64_t tile_desc(uint32_t smem_addr) {
     return (1ull << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61) | (uint64_t)(smem_addr >> 4);
 }
 __device__ __forceinline__ uint32_t tile_step(int ks) { return (uint32_t)(ks >> 2) * (16384u >> 4) + (uint32_t)(ks & 3) * 2u; }
-// acc + x0^2 + x1^2 of two fp16 values, in that order (fp16 -> fp32 is exact: the same bits as converting first)
-__device__ __forceinline__ float square2(float acc, uint32_t w) {
-    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tfma.rn.f32.f16 %0, l, l, %0;\n\tfma.rn.f32.f16 %0, h, h, %0;\n\t}" : "+f"(acc) : "r"(w));
-    return acc;
-}
-
 // Tiles [lo, hi) of one (head, K or V).  `n_mma`: products this thread's group has issued so far (the barrier's phase).
-// ONE: the CTA's only tile.  Its time is that of one pass over code that no instruction cache holds yet, so the code is kept
-// short where nothing is lost by it: no next tile's loads, the two row groups of the column move in a loop (777 tokens of a
-// layer: 12.0 -> 10.8 us; in the many-tile form the loop costs 1 %, and shorter loops in the epilogue cost 20 % in either).
+// ONE: the CTA's only tile, on which all sixteen warps work, a thread on a quarter of its row (a second group would have
+// nothing to do, and the launch takes as long as one tile).
 template <bool IS_V, bool MIXED, bool CODES, bool ONE>
-__device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int h, const int lo_tile, const int hi_tile, int& n_mma) {
+__device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int h, const int lo_tile, const int hi_tile, int& n_mma,
+                                        bool& waited) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int grp = tid >> 8, gt = tid & (kGroup - 1);
-    const int hf = (warp >> 2) & 1, row = (warp & 3) * 32 + lane;      // (a warp reads tensor-memory lanes 32 (warp % 4) .. + 31)
+    constexpr int kThr = ONE ? kThreads : kGroup, kWrp = kThr / 32;
+    const int grp = ONE ? 0 : tid >> 8, gt = ONE ? tid : tid & (kGroup - 1);
+    constexpr int kParts = kThr / kTileRows;                 // threads of a row: 2 or 4
+    const int qf = (warp >> 2) & (kParts - 1), hf = qf & 1, row = (warp & 3) * 32 + lane;      // (a warp reads tensor-memory lanes 32 (warp % 4) .. + 31)
     const int n_rows = P.n_batch * P.n_tok;                  // the launcher checks that this fits
     const int t0 = P.pos_dev ? *P.pos_dev : P.t0;
     const uint32_t acc_hi = S.tmem_base + 256u * grp;
@@ -366,26 +462,30 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
     const int64_t o_sb = IS_V ? P.vp_sb : P.kp_sb, o_st = IS_V ? P.vp_st : P.kp_st;
     const uint32_t magic = ((1u << 24) + (uint32_t)rb - 1u) / (uint32_t)rb;      // x / rb = x * magic >> 24 below 128 rows
     const int stage_ld = 4 * (((rb + 3) >> 2) | 1);       // bytes between staged rows: an odd number of words
-    const int task_lo = hf ? S.split : 0, task_hi = hf ? S.n_tasks : S.split;
+    const int q_lo = qf * (4 / kParts);                      // this thread's first quarter
+    const int task_lo = S.cut[q_lo], task_hi = S.cut[q_lo + 4 / kParts], task_mid = S.cut[q_lo + 1];
+    auto tile_sync = [&]() {
+        if (ONE) __syncthreads();
+        else group_sync(grp);
+    };
     uint8_t* const codes_out = IS_V ? P.v_codes : P.k_codes;
 
-    // K: where the elements of the chunks that this lane moves into the operand go (chunks 4 j + lane / 8 of rows = lane mod 8:
-    // eight rows and four chunks per access keep the scattered 2-byte stores two to a bank instead of six)
-    uint32_t koff[IS_V ? 1 : 4][8];
-    uint4 nctl = make_uint4(0u, 0u, 0u, 0u);
+    // K: where the pairs of the chunks that this lane moves into the operand go (dims 8 (4 j + lane / 8) .. + 7 and 64 above, of
+    // rows = lane mod 8: eight rows and four chunks per access keep the scattered stores few to a bank)
+    uint32_t koff[IS_V ? 1 : 2][8];
     if constexpr (!IS_V) {
-        nctl = *reinterpret_cast<const uint4*>(S.norm_ctl[hf]);
-        const uint32_t rows = smem_u32(S.buf[grp][1]) + ((gt >> 5) * 16 + (lane & 7)) * 128;
+        const uint32_t rows = smem_u32(S.buf[grp][1]) + ((gt >> 5) * (kTileRows / kWrp) + (lane & 7)) * 128;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < 2; ++j) {
             const uint4 o = *reinterpret_cast<const uint4*>(&S.to[(4 * j + (lane >> 3)) * 8]);
             const uint32_t w[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
             for (int e = 0; e < 8; ++e) koff[j][e] = rows + (((w[e >> 1] >> (16 * (e & 1))) & 0xFFFFu) ^ ((uint32_t)(lane & 7) << 4));
         }
     }
-    // Rows of a tile -> a buffer, asynchronously: thread -> chunk (gt & 15) of rows (gt >> 4) + 16 q; rows past the end are
+    // Rows of a tile -> a buffer, asynchronously: thread -> chunk (gt & 15) of rows (gt >> 4) + kStep q; rows past the end are
     // zero-filled.
+    constexpr int kStep = kThr / 16, kRowsEach = kTileRows / kStep;
     const int fr = gt >> 4, fc = gt & 15;
     const uint32_t fetch_off = (uint32_t)((fc >> 3) * 16384 + fr * 128 + (((fc & 7) ^ (fr & 7)) << 4));
     auto prefetch = [&](int tl, int b0, int s0, uint8_t* to) {
@@ -395,24 +495,28 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
         };
         if (s0 + kTileRows <= P.n_tok && (tl + 1) * kTileRows <= n_rows) {
             const __half* src = src_base + b0 * s_sb + (s0 + fr) * s_ss + fc * 8;
-            const int64_t inc = 16 * s_ss;
+            const int64_t inc = kStep * s_ss;
 #pragma unroll
-            for (int q = 0; q < 8; ++q, src += inc) copy(dst + q * 2048u, src, 16);
+            for (int q = 0; q < kRowsEach; ++q, src += inc) copy(dst + q * (128u * kStep), src, 16);
             return;
         }
         int b = b0, s = s0 + fr;
 #pragma unroll 1
-        for (int q = 0; q < 8; ++q) {
+        for (int q = 0; q < kRowsEach; ++q) {
             while (s >= P.n_tok) { s -= P.n_tok; ++b; }
-            const bool valid = tl * kTileRows + fr + 16 * q < n_rows;
-            copy(dst + q * 2048u, valid ? src_base + b * s_sb + s * s_ss + fc * 8 : src_base, valid ? 16 : 0);
-            s += 16;
+            const bool valid = tl * kTileRows + fr + kStep * q < n_rows;
+            copy(dst + q * (128u * kStep), valid ? src_base + b * s_sb + s * s_ss + fc * 8 : src_base, valid ? 16 : 0);
+            s += kStep;
         }
     };
     // (b0, s0) = first row of tile tl
     const int step_b = (int)((uint32_t)(2 * kTileRows) / (uint32_t)P.n_tok), step_s = 2 * kTileRows - step_b * P.n_tok;
     int tl = lo_tile + grp;
     int b0 = (int)((uint32_t)(tl * kTileRows) / (uint32_t)P.n_tok), s0 = tl * kTileRows - b0 * P.n_tok;
+    if (ONE && !waited) {
+        grid_dependency_wait();
+        waited = true;
+    }
     if (tl < hi_tile) prefetch(tl, b0, s0, S.buf[grp][0]);
     for (int it = 0, nb0, ns0; tl < hi_tile; tl += 2, ++it, b0 = nb0, s0 = ns0) {
         const int n0 = tl * kTileRows, n_valid = n_rows - n0 < kTileRows ? n_rows - n0 : kTileRows;
@@ -420,30 +524,46 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
         ns0 = s0 + step_s;
         if (ns0 >= P.n_tok) { ns0 -= P.n_tok; ++nb0; }
         uint8_t* const a = S.buf[grp][IS_V ? it & 1 : 1];       // the operand tile
-        // sums of squared levels per (half, segment, row), behind the staged rows in the (by then dead) operand tile
-        auto level = [&](int half, int s, int r) -> float& { return reinterpret_cast<float*>(a + kLevelOff)[(half * kSeg + s) * kTileRows + r]; };
+        // sums of squared levels per (part, segment, row), behind the staged rows in the (by then dead) operand tile, or in the
+        // other group's buffer
+        auto level = [&](int part, int s, int r) -> float& {
+            return reinterpret_cast<float*>(ONE ? S.buf[1][0] : a + kLevelOff)[(part * kSeg + s) * kTileRows + r];
+        };
         // ---- the prefetched rows; K: their columns into packed order ----
         asm volatile("cp.async.wait_all;" ::: "memory");
         if constexpr (!IS_V) {
-            group_sync(grp);
+            tile_sync();
             const uint32_t raw = smem_u32(S.buf[grp][0]);
-#pragma unroll (ONE ? 1 : 2)
-            for (int rg = 0; rg < 2; ++rg)
+            if (S.paired) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int chunk = 4 * j + (lane >> 3), r = (gt >> 5) * 16 + 8 * rg + (lane & 7);
-                    const uint4 v = lds128(raw + (uint32_t)((chunk >> 3) * 16384 + r * 128 + (((chunk & 7) ^ (lane & 7)) << 4)));
-                    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+                for (int rg = 0; rg < kTileRows / kWrp / 8; ++rg)
 #pragma unroll
-                    for (int c = 0; c < 8; ++c)
-                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(koff[j][c] + rg * 1024u), "h"((unsigned short)(w[c >> 1] >> (16 * (c & 1)))) : "memory");
+                    for (int j = 0; j < 2; ++j) {
+                        const int chunk = 4 * j + (lane >> 3), r = (gt >> 5) * (kTileRows / kWrp) + 8 * rg + (lane & 7);
+                        const uint32_t from = raw + (uint32_t)(r * 128 + ((chunk ^ (lane & 7)) << 4));
+                        const uint4 v = lds128(from), v2 = lds128(from + 16384u);
+                        const uint32_t w[4] = {v.x, v.y, v.z, v.w}, w2[4] = {v2.x, v2.y, v2.z, v2.w};
+#pragma unroll
+                        for (int c = 0; c < 8; ++c)
+                            asm volatile("st.shared.u32 [%0], %1;" ::"r"(koff[j][c] + rg * 1024u), "r"(__byte_perm(w[c >> 1], w2[c >> 1], c & 1 ? 0x7632 : 0x5410)) : "memory");
+                    }
+            } else {            // any other order, element by element
+                const uint32_t op = smem_u32(a);
+#pragma unroll 1
+                for (int i = gt; i < kTileRows * kHD / 2; i += kThr) {
+                    const int r = i >> 6, c2 = (i & 63) * 2;
+                    const uint32_t sw = (uint32_t)(r & 7) << 4, v = lds32(raw + (uint32_t)((c2 >> 6) * 16384 + r * 128) + (((uint32_t)(c2 & 63) * 2u) ^ sw));
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(op + (uint32_t)(r * 128) + (S.to[c2 + e] ^ sw)), "h"((unsigned short)(v >> (16 * e))) : "memory");
                 }
+            }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // these rows -> tensor-core reads
         tc_fence_before_sync();     // also orders this thread's tensor-memory reads of the previous tile
-        group_sync(grp);
+        tile_sync();
         // ---- product: one warp issues x . hi, another x . lo ----
-        if ((warp & 7) < 2) {
+        if (ONE ? warp < 2 : (warp & 7) < 2) {
             tc_fence_after_sync();
             const uint32_t lead = elect_one();
             const uint32_t which = warp & 1;
@@ -455,99 +575,92 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
             __syncwarp();
         }
         if (!ONE && tl + 2 < hi_tile) prefetch(tl + 2, nb0, ns0, S.buf[grp][IS_V ? (it + 1) & 1 : 0]);     // arrives during this tile's work
-        // ---- group norms: the row's two threads take alternate element pairs of each segment ----
-        {
+        // ---- group norms.  K: a thread per segment; V: two threads take alternate element pairs ----
+        if constexpr (!IS_V) {
+            e5_norms_k(S, grp, smem_u32(a), row, qf, kParts);
+        } else if (qf < 2) {
             const uint32_t xr = smem_u32(a) + (uint32_t)row * 128u, sw = (uint32_t)(row & 7) << 4;
             float acc = 0.f;
-            float* part = &S.part[grp][hf][0][row];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {       // four chunks requested together
                 uint4 w[4];
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
                     w[c] = lds128(xr + (uint32_t)(q >> 1) * 16384u + (((uint32_t)(4 * (q & 1) + c) << 4) ^ sw));
-                const uint32_t ctl = IS_V ? (hf ? 0x0A0A0A0Au : 0x05050505u) : q == 0 ? nctl.x : q == 1 ? nctl.y : q == 2 ? nctl.z : nctl.w;
-                if (ctl == 0x05050505u) {
+                if (hf == 0) {
 #pragma unroll
                     for (int c = 0; c < 4; ++c) acc = square2(square2(acc, w[c].x), w[c].z);
-                } else if (IS_V || ctl == 0x0A0A0A0Au) {
+                } else {
 #pragma unroll
                     for (int c = 0; c < 4; ++c) acc = square2(square2(acc, w[c].y), w[c].w);
-                } else {
-                    auto pair = [&](uint32_t bit, uint32_t v) {
-                        if (ctl & bit) acc = square2(acc, v);
-                        if (ctl & (bit << 4)) {
-                            *part = acc;
-                            part += kTileRows;
-                            acc = 0.f;
-                        }
-                    };
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        pair(1u << (8 * c), w[c].x);
-                        pair(2u << (8 * c), w[c].y);
-                        pair(4u << (8 * c), w[c].z);
-                        pair(8u << (8 * c), w[c].w);
-                    }
                 }
             }
-            if (IS_V) *part = acc;
+            S.part[grp][hf][0][row] = acc;
         }
         const int n = n0 + row;
         int b = b0, t = s0 + row;                   // this thread's row
         while (t >= P.n_tok) { t -= P.n_tok; ++b; }
-        group_sync(grp);
-        // half hf finishes segments 2 hf, 2 hf + 1, 2 hf + 4, 2 hf + 5 (norm rows are written two values at a time)
+        tile_sync();
+        // part q finishes segments 2 q, 2 q + 1 and, of two, 2 q + 4, 2 q + 5 (norm rows are written two values at a time)
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int s = 2 * hf + (u & 1) + 4 * (u >> 1);
+        for (int u = 0; u < 8 / kParts; ++u) {
+            const int s = 2 * qf + (u & 1) + 4 * (u >> 1);
             if (s >= n_seg) continue;
             const float nr = sqrtf((S.part[grp][0][s][row] + S.part[grp][1][s][row]) + 1e-30f);
             S.part[grp][0][s][row] = nr;
             S.part[grp][1][s][row] = nr > (IS_V ? 1e-8f : 1e-10f) ? 1.0f / nr : 1.0f;
         }
-        if (!bar_and(3 + grp, kGroup, mbar_wait_bounded(bar, n_mma++ & 1))) {      // same verdict for the whole group
+        if (!bar_and(3 + grp, kThr, mbar_wait_bounded(bar, n_mma++ & 1))) {      // same verdict for the whole group
             if (gt == 0) atomicExch(&g_enc5_status, kStatusWaitTimeout);
             asm volatile("cp.async.wait_all;" ::: "memory");
             return false;
         }
         tc_fence_after_sync();
-        // ---- quantise and pack this thread's half of its row ----
+        // ---- quantise and pack this thread's part of its row ----
         const uint32_t row_addr = smem_u32(a) + (uint32_t)(row * stage_ld);
         uint8_t* const cd = CODES && codes_out && n < n_rows ? codes_out + (((size_t)b * P.n_kv + h) * P.n_tok + t) * kHD : nullptr;
         float csq = 0.f;
         ByteStream out;
         if (IS_V) {
+            constexpr int kCols = kHD / kParts;
             const float r = S.part[grp][1][0][row];
-            csq = S.v_search ? e5_half_v<true, CODES>(S, lane_base, hf, r, row_addr, cd) : e5_half_v<false, CODES>(S, lane_base, hf, r, row_addr, cd);
-            level(hf, 0, row) = csq;
+            csq = S.v_search ? e5_cols_v<true, CODES, kCols / 8>(S, lane_base, kCols * qf, r, row_addr, cd)
+                             : e5_cols_v<false, CODES, kCols / 8>(S, lane_base, kCols * qf, r, row_addr, cd);
+            level(qf, 0, row) = csq;
         } else {
-            out.open(row_addr, hf ? (uint32_t)S.split_byte : 0u);
-            // (a last short task near column 128 loads from column 120: no read past the accumulators)
-            auto load_of = [](uint32_t task) { return min(task & 0xFFu, (uint32_t)kHD - 8u); };
+            out.open(row_addr, (uint32_t)S.cut_byte[q_lo]);
+            if (mixed) {                // (a part without tasks of a segment adds nothing)
+                for (int s = 0; s < n_seg; ++s) level(qf, s, row) = 0.f;
+            }
+            float before = 0.f;         // the segment's sum in this thread's first quarter
             int seg_now = -1;
-            const uint32_t lut0 = smem_u32(S.code_lut[0]) - 0x4B000000u;
             const uint64_t scale2 = pack_f2(1.0f / kLoScale, 1.0f / kLoScale);
+            const uint32_t factors = smem_u32(&S.part[grp][1][0][row]), recs = smem_u32(S.rec);
             // Two tasks at a time: their table lookups overlap.  An odd count repeats the last task and packs it once.
             float hi[2][8], lo[2][8];
-            auto fetch = [&](int ti, int u, uint32_t& tk) {
-                tk = S.tasks[min(ti, task_hi - 1)];
-                tmem_ld8(lane_base + load_of(tk), hi[u]);
-                tmem_ld8(lane_base + kHD + load_of(tk), lo[u]);
+            auto fetch = [&](int ti, int u) {
+                const uint32_t col = lane_base + (lds32(recs + (uint32_t)min(ti, task_hi - 1) * (uint32_t)sizeof(E5Rec)) & 0xFFu);
+                tmem_ld8(col, hi[u]);
+                tmem_ld8(col + kHD, lo[u]);
             };
-            uint32_t next[2] = {0u, 0u};
             if (task_lo < task_hi) {
-                fetch(task_lo, 0, next[0]);
-                fetch(task_lo + 1, 1, next[1]);
+                fetch(task_lo, 0);
+                fetch(task_lo + 1, 1);
             }
             for (int ti = task_lo; ti < task_hi; ti += 2) {
-                const uint32_t cur[2] = {next[0], next[1]};
                 uint32_t c[2][8];
+                uint4 ra[2], rb[2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const uint32_t at = recs + (uint32_t)min(ti + u, task_hi - 1) * (uint32_t)sizeof(E5Rec);
+                    ra[u] = lds128(at);
+                    rb[u] = lds128(at + 16);
+                }
                 __syncwarp();
                 tmem_ld_wait();
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
-                    const uint32_t off = (cur[u] & 0xFFu) - load_of(cur[u]);      // 0, 2, 4 or 6
+                    const uint32_t off = ra[u].x >> 8;      // 0, 2, 4 or 6
                     if (off) {
                         if (off & 2u) {
 #pragma unroll
@@ -561,83 +674,83 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
                 }
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
-                    const int seg = (cur[u] >> 16) & 0xF;
-                    const float r = S.part[grp][1][seg][row];
-                    const float2 g = S.grid[seg];
-                    const uint32_t lut = lut0 + (uint32_t)(seg * kLutLd);
-                    const uint64_t r2 = pack_f2(r, r), off2 = pack_f2(-g.x, -g.x);
+                    const float r = lds_f(factors + ra[u].w), g = __uint_as_float(rb[u].y), o = __uint_as_float(rb[u].x);
+                    const uint64_t r2 = pack_f2(r, r), off2 = pack_f2(o, o);
 #pragma unroll
                     for (int e = 0; e < 8; e += 2) {
                         const uint64_t x2 = fma_f2(pack_f2(lo[u][e], lo[u][e + 1]), scale2, pack_f2(hi[u][e], hi[u][e + 1]));
                         float y0, y1;
                         unpack_f2(fma_f2(x2, r2, off2), y0, y1);
                         uint32_t a0, a1;
-                        bin_addr2(__saturatef(y0 * g.y), __saturatef(y1 * g.y), lut, a0, a1);
+                        bin_addr2(__saturatef(y0 * g), __saturatef(y1 * g), ra[u].z, a0, a1);
                         c[u][e] = lds8(a0);
                         c[u][e + 1] = lds8(a1);
                     }
                 }
                 if (ti + 2 < task_hi) {       // the next tasks' columns come while this pair is packed
-                    fetch(ti + 2, 0, next[0]);
-                    fetch(ti + 3, 1, next[1]);
+                    fetch(ti + 2, 0);
+                    fetch(ti + 3, 1);
                 }
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
-                    const int cnt = (cur[u] >> 8) & 0xF, sb = (cur[u] >> 12) & 0xF, seg = (cur[u] >> 16) & 0xF, nb = (cur[u] >> 20) & 0xF;
                     if (ti + u >= task_hi) break;
-                    if (cnt < 8) {
+                    if (mixed || CODES) {
+                        const uint32_t task = S.tasks[ti + u];
+                        const int cnt = (task >> 8) & 0xF, seg = (task >> 16) & 0xF;
+                        if (mixed) {        // squared norm of the chosen levels, per segment
+                            if (seg != seg_now) {
+                                if (seg_now >= 0) level(qf, seg_now, row) = before + csq;
+                                csq = before = 0.f;
+                                seg_now = seg;
+                            } else if (!ONE && ti + u == task_mid) {
+                                before = csq;
+                                csq = 0.f;
+                            }
+                            const uint32_t cent = smem_u32(S.kcent + S.seg_lut_off[seg]);
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) c[u][e] = e < cnt ? c[u][e] : 0u;
-                    }
-                    if (mixed) {        // squared norm of the chosen levels, per segment
-                        if (seg != seg_now) {
-                            if (seg_now >= 0) level(hf, seg_now, row) = csq;
-                            csq = 0.f;
-                            seg_now = seg;
+                            for (int e = 0; e < 8; ++e) {
+                                const float cv = e < cnt ? lds_f(cent + 4u * c[u][e]) : 0.f;
+                                csq = fmaf(cv, cv, csq);
+                            }
                         }
-                        const uint32_t cent = smem_u32(S.kcent + S.seg_lut_off[seg]);
+                        if (CODES && cd) {
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            const float cv = e < cnt ? lds_f(cent + 4u * c[u][e]) : 0.f;
-                            csq = fmaf(cv, cv, csq);
+                            for (int e = 0; e < 8; ++e)
+                                if (e < cnt) cd[(task & 0xFFu) + e] = (uint8_t)c[u][e];
                         }
                     }
-                    if (CODES && cd) {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            if (e < cnt) cd[(cur[u] & 0xFFu) + e] = (uint8_t)c[u][e];
-                    }
-                    out.put(squeeze8(c[u], 1u << sb), 8u * nb);
+                    out.word(squeeze8(c[u], rb[u].z) & ra[u].y, rb[u].w, row_addr);
                 }
             }
-            if (mixed && seg_now >= 0) level(hf, seg_now, row) = csq;
-            if (hf)
+            out.end_at(row_addr, (uint32_t)S.cut_byte[q_lo + 4 / kParts]);
+            if (mixed && seg_now >= 0) level(qf, seg_now, row) = before + csq;
+            if (qf == kParts - 1)
 #pragma unroll 1
-                for (int p = S.data_bytes; p < rb; p += 4) out.put(0u, 8u * min(4, rb - p));      // rows of a head with fewer bytes than the widest
+                for (int p = S.cut_byte[4]; p < rb; p += 4) out.put(0u, 8u * min(4, rb - p));      // rows of a head with fewer bytes than the widest
             out.close();
         }
         tc_fence_before_sync();
-        group_sync(grp);
+        tile_sync();
         // ---- norms out ----
         if (n < n_rows) {
             if (!IS_V) {
                 const size_t o = b * P.kn_sb + h * P.kn_sh + (size_t)(t0 + t) * P.kn_st;
-                const int mid = S.split < S.n_tasks ? (int)(S.tasks[S.split] & 0xFFu) : kHD;
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int s = 2 * hf + (u & 1) + 4 * (u >> 1);
+                for (int u = 0; u < 8 / kParts; ++u) {
+                    const int s = 2 * qf + (u & 1) + 4 * (u >> 1);
                     if (s >= P.kn_count) continue;
                     float val = s < n_seg ? S.part[grp][0][s][row] : 0.f;
-                    if (mixed && s < n_seg) {       // (a segment on both sides of the split has two sums)
-                        const float q = (S.seg_start[s] < mid ? level(0, s, row) : 0.f) +
-                                        (S.seg_start[s] + S.seg_len[s] > mid ? level(1, s, row) : 0.f);
+                    if (mixed && s < n_seg) {       // (a segment on both sides of a cut has several sums)
+                        const float q = ONE ? (level(0, s, row) + level(1, s, row)) + (level(2, s, row) + level(3, s, row))
+                                            : level(0, s, row) + level(1, s, row);
                         val = val / fmaxf(sqrtf(q), 1e-10f);
                     }
                     if (f16n) static_cast<__half*>(P.kn)[o + s] = __float2half_rn(val);
                     else static_cast<float*>(P.kn)[o + s] = val;
                 }
-            } else if (hf == 0) {
-                const float cnorm = sqrtf((level(0, 0, row) + level(1, 0, row)) + 1e-20f);
+            } else if (qf == 0) {
+                const float sum = ONE ? (level(0, 0, row) + level(1, 0, row)) + (level(2, 0, row) + level(3, 0, row)) : level(0, 0, row) + level(1, 0, row);
+                const float cnorm = sqrtf(sum + 1e-20f);
                 P.vn[b * P.vn_sb + h * P.vn_sh + (size_t)(t0 + t) * P.vn_st] =
                     __float2half_rn(S.part[grp][0][0][row] / (cnorm > 1e-10f ? cnorm : 1.0f));
             }
@@ -650,7 +763,8 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
             const uint32_t stage = smem_u32(a);
             auto row_of = [&](int x) { return (int)(((uint32_t)x * magic) >> 24); };     // x / rb, exact below 128 rows
             if (head == 0 && (rb & 3) == 0) {
-                for (int i = gt; i < words; i += kGroup) {
+#pragma unroll 4
+                for (int i = gt; i < words; i += kThr) {
                     const int r = row_of(4 * i);
                     *reinterpret_cast<uint32_t*>(dst0 + 4 * i) = lds32(stage + (uint32_t)(r * (stage_ld - rb) + 4 * i));
                 }
@@ -661,7 +775,7 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
                 const int x = total - tail + gt, r = row_of(x);
                 dst0[x] = a[r * stage_ld + x - r * rb];
             }
-            for (int i = gt; i < words; i += kGroup) {
+            for (int i = gt; i < words; i += kThr) {
                 const int x = head + 4 * i, r = row_of(x), p = x - r * rb;
                 const uint32_t at = stage + (uint32_t)(r * stage_ld + (p & ~3));
                 uint32_t w = lds32(at);
@@ -671,7 +785,7 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
                 *reinterpret_cast<uint32_t*>(dst0 + x) = w;
             }
         } else {
-            for (int i = gt; i < n_valid * rb; i += kGroup) {
+            for (int i = gt; i < n_valid * rb; i += kThr) {
                 const int r = i / rb, p = i - r * rb;
                 const int nn = n0 + r, bb = (int)((uint32_t)nn / (uint32_t)P.n_tok), tt = nn - bb * P.n_tok;
                 out_base[bb * o_sb + (int64_t)(t0 + tt) * o_st + p] = a[r * stage_ld + p];
@@ -682,9 +796,9 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
 }
 
 // One CTA per SM.  The tiles of all (KV head, K or V) form one list, a K tile kUnitsK units long and a V tile kUnitsV (what
-// they take: a K row's columns move into packed order first); CTA i works on the tiles that begin in its share of the units,
+// they take: 229 and 164 us for a million rows; 13 to 7, as it was, 458 us for both, 10 to 7 393, so 391); CTA i works on the tiles that begin in its share of the units,
 // and loads the tables again where its share crosses into the next (head, role).
-constexpr int kUnitsK = 13, kUnitsV = 7;
+constexpr int kUnitsK = 11, kUnitsV = 8;
 template <bool MIXED, bool CODES, bool ONE>
 __global__ void __launch_bounds__(kThreads, 1) encode_t5_kernel(const EncParams P, const int units_k, const int units_v) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -711,8 +825,10 @@ __global__ void __launch_bounds__(kThreads, 1) encode_t5_kernel(const EncParams 
         u = end;
         if (lo >= hi) continue;
         e5_setup(S, P, P.desc[h], is_v, h);
-        if (!waited) {
-            grid_dependency_wait();       // the rows, and what this launch overwrites, belong to earlier work in the stream
+        // The rows, and what this launch overwrites, belong to earlier work in the stream.  (The one-tile form waits where it
+        // asks for its rows; with many tiles that costs the loop registers.)
+        if (!waited && (!ONE || P.pos_dev)) {
+            grid_dependency_wait();
             waited = true;
             if (P.pos_dev) in_range = enc_range_ok(P, *P.pos_dev, P.n_tok);      // (uniform over the launch: else nothing is stored)
         }
@@ -721,7 +837,7 @@ __global__ void __launch_bounds__(kThreads, 1) encode_t5_kernel(const EncParams 
         __syncthreads();
         tc_fence_after_sync();
         if (!in_range) break;
-        const bool ok = is_v ? e5_role<true, MIXED, CODES, ONE>(S, P, h, lo, hi, n_mma) : e5_role<false, MIXED, CODES, ONE>(S, P, h, lo, hi, n_mma);
+        const bool ok = is_v ? e5_role<true, MIXED, CODES, ONE>(S, P, h, lo, hi, n_mma, waited) : e5_role<false, MIXED, CODES, ONE>(S, P, h, lo, hi, n_mma, waited);
         if (!__syncthreads_and(ok ? 1 : 0) || ONE) break;      // (also: everyone is done with this range's tables)
     }
     if (!waited) grid_dependency_wait();

@@ -24,7 +24,7 @@ import torch
 from . import _lib
 from .calib import packed_v_bytes
 from .layer import (HD, LayerTables, attend, buffer_attn, cluster_flags, combine, decode, decode_grid_size, decode_partition, default_splits,
-                    encode, merges, rotate_q, step_prepare, tile_flags, _no_tcgen05)
+                    encode, rotate_q, step_prepare, tile_flags, _no_tcgen05)
 from .quantizer import BlockGTQQuantizer, build_batched_encode_args
 
 __all__ = ["BlockGTQKVManager", "decode_step"]
@@ -385,7 +385,8 @@ class BlockGTQKVManager:
             kb, vb = self._k_buf[li], self._v_buf[li]
             s.k_buf, s.v_buf, s.kb_sb, s.kb_sh = kb.data_ptr(), vb.data_ptr(), kb.stride(0), kb.stride(1)
             s.buf_o, s.buf_lse, s.n_sink, s.window = self._buf_o.data_ptr(), self._buf_lse.data_ptr(), self.n_sink, self.recent_window
-        s.key, s.addr, s.n_launch = (lt, baked, pd), C.addressof(s), 4 if self._buffered else 3 - merges(lt, self._dec_flags | self._cluster_flags | (_lib.DEC_PROGRAMMATIC if pd else 0))
+        s.key, s.addr, s.n_launch = (lt, baked, pd), C.addressof(s), \
+            4 if self._buffered else 3 - (self._cluster_flags > 0 and _lib.lib().bgtq_decode_plan_cluster(s.plan) > 0)
         self._steps[li] = s
         return s
 

@@ -72,3 +72,35 @@ def test_one_tile_per_cta_and_more(case, mixed):
     for a, b in zip(run([(0, n)]), run([(0, n - 1), (n - 200, n)])):
         assert torch.equal(a, b)
     assert _lib.lib().bgtq_encode_tcgen05_status() == 0
+
+
+@pytest.mark.parametrize("n", [129, 130 * 148])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_any_order_of_dims(n, mixed):
+    """Heads whose packed order does not keep RoPE pairs side by side take the bulk encoder's other way into packed order: the
+    same bytes as the reference's order gives for inputs whose dims are exchanged accordingly."""
+    import copy
+    from blockgtq_b200 import _lib
+    from blockgtq_b200.layer import LayerTables, encode
+    from helpers import HD, tables_for
+    kt, vt = tables_for("a3_1to8", 0)
+    gen = torch.Generator().manual_seed(n)
+    order = torch.randperm(HD, generator=gen)
+    other = copy.copy(kt)
+    other.head_perm = order[kt.head_perm]
+    k, v = (torch.randn(1, 1, n, HD, generator=gen).half().to(DEV) for _ in range(2))
+    k2 = torch.empty_like(k)
+    k2[..., order.to(DEV)] = k
+    flags = _lib.ENC_K_MIXED | _lib.ENC_V_NIBBLE if mixed else 0
+
+    def run(table, keys):
+        lt = LayerTables([table], [vt], DEV)
+        kb, vb = (lt.max_mixed_bytes, HD // 2) if mixed else (lt.max_tpb, lt.vpb)
+        out = [torch.zeros(1, 1, n, w, dtype=torch.uint8, device=DEV) for w in (kb, vb)]
+        out += [torch.zeros(1, 1, n, lt.max_ng, dtype=torch.float16, device=DEV), torch.zeros(1, 1, n, dtype=torch.float16, device=DEV)]
+        encode(lt, keys, v, 0, out[0], out[2], out[1], out[3], flags=flags)
+        return out
+
+    for a, b in zip(run(kt, k), run(other, k2)):
+        assert torch.equal(a, b)
+    assert _lib.lib().bgtq_encode_tcgen05_status() == 0
