@@ -12,15 +12,17 @@
 //     values share an instruction where they can (f32x2), and whole 32-bit words of the packed row go to a staging image of the
 //     tile that leaves as coalesced words.
 // Bound: instruction issue and its latencies with 16 warps per SM (all registers and shared memory are taken): 1 048 576 K and
-// as many V rows take 391 us (K rows alone 229, V rows 164), where the bytes alone would take 100.  K rows cost what V's do
+// as many V rows take 374 us (K rows alone 219, V rows 162), where the bytes alone would take 100.  K rows cost what V's do
 // not: the move into packed order and a norm per group.  Before the list, the norms by whole segments and the moves in pairs
 // K rows took 286 us (both 451): every thread worked out each task's control for itself, a third of the loop.  A launch of
-// one tile per CTA (777 tokens of 8 heads) takes 8.6 us, and took 10.8 with half of the warps idle.  The form before that
+// one tile per CTA (777 tokens of 8 heads) takes 8.5 us, and took 10.8 with half of the warps idle.  The form before that
 // gave a quad of lanes four rows and four columns each, loaded three tables per element and passed the codes through shared
 // memory to a packing pass: 753 us.  Tried and slower: rolled loops (smaller code, less overlap of the table lookups: 589 us);
 // squares of converted fp16 values instead of mixed-precision multiply-adds (K 277 -> 287, V 164 -> 168).
 // The sums that decide a code (group norms, products) keep the order they had: the packed bytes are bit for bit the same.
 // Every wait is bounded; tensor memory is released on every path out of the kernel.
+#include <type_traits>
+
 #include "bgtq_common.cuh"
 #include "bgtq_encode_params.cuh"
 #include "bgtq_tcgen05.cuh"
@@ -50,7 +52,7 @@ constexpr int kLutLd = BGTQ_N_BINS + 4;
 struct E5Rec {
     uint32_t col;       // first column to load | 2 (first column of the task - that) << 8: a last short task loads from column 120
     uint32_t mask;      // the valid bits of its code word
-    uint32_t lut;       // shared address of its segment's code table - 0x4B000000 (see bin_addr2)
+    uint32_t lut;       // shared address of its segment's code table
     uint32_t part;      // byte offset of its segment's row factors
     float off, scale;   // bin = (y + off) * scale, in units of 256 bins
     uint32_t mul;       // 2^(stored bits)
@@ -66,14 +68,14 @@ struct E5Smem {
     // per group: the two partial sums of squares of a (segment, row), replaced by its group norm and by 1 / norm (or 1
     // where the norm is below the floor)
     float part[2][2][kSeg][kTileRows];
-    float vbound[16][32], vcent[16][32];            // one copy per lane: conflict-free lookups
+    float vtab[32];                                 // V: boundaries, levels (sixteen neighbouring words: lookups never collide)
     float kcent[512];
-    uint8_t code_lut[kSeg][kLutLd];                 // entry 256 = entry 255; V: [0] = boundaries below the bin
-    float2 grid[kSeg];                              // in units of 256 bins.  K: {offset, 1 / range}; V: [0] = {1 / range, offset / range}
+    uint8_t code_lut[kSeg][kLutLd];                 // K: entry 256 = entry 255
+    float2 grid[kSeg];                              // K, in units of 256 bins: {offset, 1 / range}
     uint32_t tasks[kMaxTasks];
     E5Rec rec[kMaxTasks];
     int32_t cut[5], cut_byte[5];                    // K: first task of each quarter of the tasks, and its first byte
-    int32_t row_bytes, n_seg, paired, v_search, v_sb, v_nb;
+    int32_t row_bytes, n_seg, paired, v_sb, v_bits;
     int32_t seg_start[kSeg], seg_len[kSeg], seg_bw[kSeg], seg_lut_off[kSeg];
     __align__(16) uint16_t to[kHD];                 // K: operand offset (row 0) of an input column, its packed position's place
     __align__(8) uint64_t mma_bar[2];
@@ -81,16 +83,16 @@ struct E5Smem {
 };
 static_assert(sizeof(E5Smem) > 114 * 1024 && sizeof(E5Smem) <= 227 * 1024, "exactly one CTA per SM (it takes all tensor memory)");
 
-// Entries trunc(clamp(256 v, 0, 255)) of a byte table for two values already saturated to [0, 1]: adding 2^23 with rounding
-// toward zero leaves the truncated bin in the low bits.  `table` = the table's shared address - 0x4B000000 (the bits of
-// 2^23).  v = 1 reads entry 256, a copy of entry 255.
+// Shared addresses of entries trunc(256 v) of a byte table at `table`, for two values already saturated to [0, 1].  An
+// address is an integer, and as the bits of a float a multiple of the smallest subnormal: 256 v added to it in those units and
+// rounded toward zero is the entry's address.  v = 1 reads entry 256, a copy of entry 255.
 __device__ __forceinline__ void bin_addr2(float v0, float v1, uint32_t table, uint32_t& a0, uint32_t& a1) {
+    const float t = __uint_as_float(table), step = __uint_as_float(256u);
     float b0, b1;
-    unpack_f2(fma_rz_f2(pack_f2(v0, v1), pack_f2(256.0f, 256.0f), pack_f2(8388608.0f, 8388608.0f)), b0, b1);
-    a0 = __float_as_uint(b0) + table;
-    a1 = __float_as_uint(b1) + table;
+    unpack_f2(fma_rz_f2(pack_f2(v0, v1), pack_f2(step, step), pack_f2(t, t)), b0, b1);
+    a0 = __float_as_uint(b0);
+    a1 = __float_as_uint(b1);
 }
-__device__ __forceinline__ uint32_t bin_of(float v) { return min(__float_as_uint(__fmaf_rz(v, 256.0f, 8388608.0f)) - 0x4B000000u, 255u); }
 __device__ __forceinline__ uint32_t lds8(uint32_t addr) {
     uint32_t v;
     asm("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(addr));
@@ -117,6 +119,14 @@ __device__ __forceinline__ uint32_t squeeze8(const uint32_t (&c)[8], uint32_t m)
 #pragma unroll
     for (int e = 6; e >= 0; --e) w = w * m + c[e];
     return w;
+}
+
+// The same of 4 x the codes (stored bits at most 4).
+__device__ __forceinline__ uint32_t squeeze8_4(const uint32_t (&c)[8], uint32_t m) {
+    uint32_t w = c[7];
+#pragma unroll
+    for (int e = 6; e >= 1; --e) w = w * m + c[e];
+    return (w >> 2) * m + (c[0] >> 2);
 }
 
 // A thread's part of a packed row on its way into the staging image: bytes are appended, whole words stored.  Staged rows
@@ -186,12 +196,11 @@ __device__ void e5_setup(E5Smem& S, const EncParams& P, const BgtqHeadDesc& d, b
     if (tid == 32) {
         S.n_seg = is_v ? 1 : d.n_seg;
         S.v_sb = (P.flags & BGTQ_ENC_V_NIBBLE) ? 4 : d.v_bits;
-        S.v_nb = (1 << d.v_bits) - 1;
+        S.v_bits = d.v_bits;
     }
     if (tid < kHD) S.to[d.head_perm[tid] & (kHD - 1)] = (uint16_t)((tid >> 6) * 16384 + ((tid >> 3) & 7) * 16 + (tid & 7) * 2);
     if (is_v) {
-        S.vbound[tid >> 5][tid & 31] = d.v_bounds[tid >> 5];
-        S.vcent[tid >> 5][tid & 31] = d.v_cents[tid >> 5];
+        if (tid < 32) S.vtab[tid] = tid < 16 ? d.v_bounds[tid] : d.v_cents[tid - 16];
     } else {
         *reinterpret_cast<uint32_t*>(&S.code_lut[tid >> 6][4 * (tid & 63)]) = reinterpret_cast<const uint32_t*>(&d.code_lut[0][0])[tid];
         S.kcent[tid] = d.k_cents[tid];
@@ -216,28 +225,7 @@ __device__ void e5_setup(E5Smem& S, const EncParams& P, const BgtqHeadDesc& d, b
     const bool pair = tid >= kHD / 2 || (d.head_perm[2 * tid] < kHD / 2 && d.head_perm[2 * tid + 1] == d.head_perm[2 * tid] + kHD / 2);
     const int paired = __syncthreads_and(is_v || pair);
     if (is_v) {
-        // V codes count the boundaries below a value.  A monotonic grid of 256 bins finds all but one of them: the table
-        // holds the boundaries in earlier bins, and one comparison with the next boundary settles the rest, as long as no
-        // bin holds two of them (else a halving search does).
-        const int nb = S.v_nb;
-        const float b0 = S.vbound[0][lane], b1 = S.vbound[nb - 1][lane];
-        const float per = (b1 > b0 ? 250.0f / (b1 - b0) : 1.0f) * (1.0f / 256.0f), off = 3.0f / 256.0f - b0 * per;
-        auto v_bin = [&](float y) { return bin_of(__saturatef(fmaf(y, per, off))); };
-        if (tid <= BGTQ_N_BINS) {
-            int below = 0;
-#pragma unroll 1
-            for (int i = 0; i < nb; ++i) below += v_bin(S.vbound[i][lane]) < (uint32_t)min(tid, BGTQ_N_BINS - 1) ? 1 : 0;
-            S.code_lut[0][tid] = (uint8_t)below;
-        }
-        if (warp == 15) {
-            const bool two = lane + 1 < nb && v_bin(S.vbound[lane & 15][lane]) >= v_bin(S.vbound[(lane + 1) & 15][lane]);
-            const bool any = __any_sync(0xffffffffu, two);
-            if (lane == 0) {
-                S.v_search = any ? 1 : 0;
-                S.grid[0] = make_float2(per, off);
-                S.row_bytes = seg_storage_bytes(S.v_sb, kHD);
-            }
-        }
+        if (tid == 0) S.row_bytes = seg_storage_bytes(S.v_sb, kHD);
     } else {
         if (tid < kSeg) S.code_lut[tid][BGTQ_N_BINS] = S.code_lut[tid][BGTQ_N_BINS - 1];
         const int n_seg = S.n_seg;
@@ -281,7 +269,7 @@ __device__ void e5_setup(E5Smem& S, const EncParams& P, const BgtqHeadDesc& d, b
                     E5Rec r;
                     r.col = (uint32_t)col | (uint32_t)(first - col) << 8;
                     r.mask = bits >= 32 ? ~0u : (1u << bits) - 1u;
-                    r.lut = smem_u32(S.code_lut[seg]) - 0x4B000000u;
+                    r.lut = smem_u32(S.code_lut[seg]);
                     r.part = (uint32_t)(seg * kTileRows * 4);
                     r.off = -S.grid[seg].x;
                     r.scale = S.grid[seg].y;
@@ -324,17 +312,21 @@ __device__ __forceinline__ float square2(float acc, uint32_t w) {
 }
 
 // Columns [first, first + 8 N) of a V row, of one thread's tensor-memory lane -> its bytes in the staged row; returns the sum
-// of the squared levels (added up quarter by quarter).  SEARCH: boundaries by halving (see e5_setup).
-template <bool SEARCH, bool CODES, int N>
+// of the squared levels (added up quarter by quarter).  A code counts the boundaries below a value: the upper halvings of
+// the search are compares with boundaries in registers, the last one (of 4 bits: two) looks its boundary up.  (With a table of
+// 256 bins for all but the last compare V rows alone take as long, K and V rows together 380 us instead of 374: its lookups
+// collide, three wavefronts each, and the other group's K tile shares the pipe.  Compares as saturated multiply-adds, off the
+// integer pipe: 182 us for V rows instead of 162.)
+template <int BITS, bool CODES, int N>
 __device__ __forceinline__ float e5_cols_v(E5Smem& S, uint32_t lane_base, int first, float r, uint32_t row_addr, uint8_t* codes) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t lut = smem_u32(S.code_lut[0]) - 0x4B000000u, vb = smem_u32(&S.vbound[0][lane]);
-    constexpr uint32_t kCent = sizeof(S.vbound);          // vcent lies behind vbound
-    const float2 g = S.grid[0];
+    const char* const vt = reinterpret_cast<const char*>(S.vtab);       // byte 4 c: boundary c, 64 + 4 c: level c
+    auto entry = [&](uint32_t at) { return *reinterpret_cast<const float*>(vt + at); };
+    constexpr int kMid = (1 << (BITS - 1)) - 1;
+    const float mid = S.vtab[kMid], low = BITS > 2 ? S.vtab[kMid / 2] : 0.f, high = BITS > 2 ? S.vtab[kMid + 1 + kMid / 2] : 0.f;
     const uint32_t sb = (uint32_t)S.v_sb, mul = 1u << sb;
     const uint32_t col = lane_base + (uint32_t)first;
-    const uint64_t r2 = pack_f2(r, r), scale2 = pack_f2(1.0f / kLoScale, 1.0f / kLoScale);
     uint32_t addr = row_addr + sb * (uint32_t)first / 8u, acc = 0u, pos = 0u;
+    const uint64_t r2 = pack_f2(r, r), scale2 = pack_f2(1.0f / kLoScale, 1.0f / kLoScale);
     uint64_t csq2 = 0ull;
     float csq = 0.f;
     float hi[2][8], lo[2][8];
@@ -350,34 +342,29 @@ __device__ __forceinline__ float e5_cols_v(E5Smem& S, uint32_t lane_base, int fi
                 tmem_ld8(col + 8u * (ti + 1), hi[u ^ 1]);
                 tmem_ld8(col + kHD + 8u * (ti + 1), lo[u ^ 1]);
             }
-            uint32_t c[8];
+            uint32_t c[8];          // 4 x codes
 #pragma unroll
             for (int e = 0; e < 8; e += 2) {
                 float y[2], cv[2];
-                uint32_t at[2];
                 unpack_f2(mul_f2(fma_f2(pack_f2(lo[u][e], lo[u][e + 1]), scale2, pack_f2(hi[u][e], hi[u][e + 1])), r2), y[0], y[1]);
-                if (!SEARCH) bin_addr2(__saturatef(fmaf(y[0], g.x, g.y)), __saturatef(fmaf(y[1], g.x, g.y)), lut, at[0], at[1]);
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
-                    uint32_t cc = 0u;
-                    if (!SEARCH) {
-                        cc = lds8(at[k]);
-                        cc += y[k] > lds_f(vb + 128u * cc) ? 1u : 0u;
-                    } else {
-#pragma unroll
-                        for (int st = 3; st >= 0; --st) cc += y[k] > lds_f(vb + 128u * (cc + (1u << st) - 1u)) ? (1u << st) : 0u;
-                    }
+                    const bool up = y[k] > mid;
+                    uint32_t cc = up ? 4u << (BITS - 1) : 0u;
+                    if (BITS > 2 && y[k] > (up ? high : low)) cc += 2u << (BITS - 1);
+                    if (BITS > 3 && y[k] > entry(cc + 4u)) cc += 8u;
+                    if (BITS > 1 && y[k] > entry(cc)) cc += 4u;
                     c[e + k] = cc;
-                    cv[k] = lds_f(vb + kCent + 128u * cc);
+                    cv[k] = entry(64u + cc);
                 }
                 const uint64_t cv2 = pack_f2(cv[0], cv[1]);
                 csq2 = fma_f2(cv2, cv2, csq2);
             }
             if (CODES && codes) {
 #pragma unroll
-                for (int e = 0; e < 8; ++e) codes[first + 8 * ti + e] = (uint8_t)c[e];
+                for (int e = 0; e < 8; ++e) codes[first + 8 * ti + e] = (uint8_t)(c[e] >> 2);
             }
-            const uint32_t w = squeeze8(c, mul);
+            const uint32_t w = squeeze8_4(c, mul);
             acc |= w << pos;
             if (pos + 8u * sb >= 32u) {
                 asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(acc) : "memory");
@@ -400,7 +387,7 @@ __device__ __forceinline__ float e5_cols_v(E5Smem& S, uint32_t lane_base, int fi
 // order.  A 16-byte load brings four pairs, even and odd positions into a sum of their own; what belongs to a neighbour in a
 // segment's first and last chunk counts as zero.  (Bits that said per chunk what to do with each pair took three times the
 // instructions: 4 x 32768 tokens x 8 heads of K rows alone 286 us with them and the tasks' control worked out by every
-// thread, 232 with this and E5Rec.)
+// thread, 229 with this and E5Rec.)
 __device__ __forceinline__ void e5_norms_k(E5Smem& S, int grp, uint32_t tile, int row, int first, int step) {
     const uint32_t xr = tile + (uint32_t)row * 128u, sw = (uint32_t)(row & 7) << 4;
     const int n_seg = S.n_seg;
@@ -624,8 +611,13 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
         if (IS_V) {
             constexpr int kCols = kHD / kParts;
             const float r = S.part[grp][1][0][row];
-            csq = S.v_search ? e5_cols_v<true, CODES, kCols / 8>(S, lane_base, kCols * qf, r, row_addr, cd)
-                             : e5_cols_v<false, CODES, kCols / 8>(S, lane_base, kCols * qf, r, row_addr, cd);
+            auto cols = [&](auto bits) { return e5_cols_v<decltype(bits)::value, CODES, kCols / 8>(S, lane_base, kCols * qf, r, row_addr, cd); };
+            switch (S.v_bits) {
+                case 1: csq = cols(std::integral_constant<int, 1>{}); break;
+                case 2: csq = cols(std::integral_constant<int, 2>{}); break;
+                case 3: csq = cols(std::integral_constant<int, 3>{}); break;
+                default: csq = cols(std::integral_constant<int, 4>{}); break;
+            }
             level(qf, 0, row) = csq;
         } else {
             out.open(row_addr, (uint32_t)S.cut_byte[q_lo]);
@@ -770,6 +762,8 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
                 }
                 continue;
             }
+            // (Sixteen lanes to a row's words, which spares finding a word's row, took K rows from 219 to 231 us: stores of half
+            // a line.)
             if (gt < head) dst0[gt] = a[gt];                                                   // (inside row 0: rb >= 4)
             if (gt < tail) {
                 const int x = total - tail + gt, r = row_of(x);
@@ -796,7 +790,7 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
 }
 
 // One CTA per SM.  The tiles of all (KV head, K or V) form one list, a K tile kUnitsK units long and a V tile kUnitsV (what
-// they take: 229 and 164 us for a million rows; 13 to 7, as it was, 458 us for both, 10 to 7 393, so 391); CTA i works on the tiles that begin in its share of the units,
+// they take, 219 and 162 us for a million rows: 374 us for both so; with 13 to 7, made for slower K rows, a sixth more); CTA i works on the tiles that begin in its share of the units,
 // and loads the tables again where its share crosses into the next (head, role).
 constexpr int kUnitsK = 11, kUnitsV = 8;
 template <bool MIXED, bool CODES, bool ONE>
