@@ -189,7 +189,7 @@ def lib():
                            "(python -m blockgtq_b200.build --force)")
     module.bind(*[C.cast(getattr(handle, name), C.c_void_p).value for name in (
         "bgtq_layer_step", "bgtq_layer_encode", "bgtq_attend", "bgtq_decode_default_splits", "bgtq_encode", "bgtq_rotate_q_rows",
-        "bgtq_prefill", "bgtq_prefill_workspace_bytes", "bgtq_decode_plan_cluster")])
+        "bgtq_prefill", "bgtq_prefill_workspace_bytes")])
     native = module
     _lib = handle
     return _lib

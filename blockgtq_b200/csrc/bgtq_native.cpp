@@ -30,7 +30,6 @@ struct Fns {
     decltype(&bgtq_rotate_q_rows) rotate_rows;
     decltype(&bgtq_prefill) prefill;
     decltype(&bgtq_prefill_workspace_bytes) prefill_workspace;
-    decltype(&bgtq_decode_plan_cluster) plan_cluster;
 } F;
 
 PyObject* none() { Py_RETURN_NONE; }
@@ -238,7 +237,7 @@ PyObject* attend(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     if (want_lse) lse = empty({B, n_q}, at::kFloat, *q);
     void* const st = stream_of(*q);
     int rc;
-    bool bare = !rot_k && !bo && F.plan_cluster(plan) > 0;      // a decode that merges its shares and rotates nothing needs no scratch ...
+    bool bare = !rot_k && !bo;      // a decode that merges its shares and rotates nothing needs no scratch ...
 again:
     if (!bare) scratch = empty({B * n_q * (ns * (kHD + 1) + kHD / 2)}, at::kFloat, *q);
     Py_BEGIN_ALLOW_THREADS
@@ -248,7 +247,7 @@ again:
                   bo ? bo->data_ptr<float>() : nullptr, bl ? bl->data_ptr<float>() : nullptr, bare ? nullptr : scratch.data_ptr(), out.data_ptr(),
                   want32 ? o32.data_ptr<float>() : nullptr, want_lse ? lse.data_ptr<float>() : nullptr, status, st);
     Py_END_ALLOW_THREADS
-    if (bare && rc == BGTQ_E_UNSUPPORTED) {      // ... unless it is left to the split form
+    if (bare && rc == BGTQ_E_UNSUPPORTED) {      // ... any other does, and says so before it launches anything
         bare = false;
         goto again;
     }

@@ -94,7 +94,7 @@ extern "C" __attribute__((visibility("default"))) int bgtq_attend(
     float scale, const float* v_rot, const float* buf_o, const float* buf_lse, void* scratch, void* out, float* out_f32,
     float* lse_out, int32_t* status, void* stream) {
     if (!plan || !q || !out || n_batch < 1 || n_q < 1 || n_splits < 1) return BGTQ_E_BADARG;
-    if (!scratch && (rot_k || buf_o || !bgtq_decode_plan_cluster(plan))) return BGTQ_E_BADARG;
+    if (!scratch && (rot_k || buf_o || !bgtq_decode_plan_cluster(plan))) return BGTQ_E_UNSUPPORTED;
     if (reinterpret_cast<uintptr_t>(scratch) & 15u) return BGTQ_E_ALIGN;
     const int64_t rows = (int64_t)n_batch * n_q;
     float* const part_o = static_cast<float*>(scratch);

@@ -73,6 +73,7 @@ class BlockGTQKVManager:
         self._enc_flags = (_lib.ENC_K_MIXED if k_mixed else 0) | (_lib.ENC_V_NIBBLE if v_nibble else 0)
         self._dec_flags = (_lib.DEC_K_MIXED if k_mixed else 0) | (_lib.DEC_V_NIBBLE if v_nibble else 0)
         self._cluster_flags = 0               # of layer steps and attend: see layer.cluster_flags
+        self._merging = set()                 # layers whose decode merges its shares (one launch less)
         # single-token decode steps take the position from the device and keep their arrays, so that they can be
         # captured (the reference graphs only its T=1 encode, packed_kv_manager.py:182-257); with fp16 regions that
         # needs one-token blocks, the policy's default
@@ -204,6 +205,7 @@ class BlockGTQKVManager:
         flag_sets = {flags, flags | pd}
         with ThreadPoolExecutor(max_workers=min(16, os.cpu_count() or 1)) as ex:     # one layer per job: its flag
             list(ex.map(lambda lt: [lt.plan(f) for f in sorted(flag_sets)], layers))  # variants share one kernel
+        self._merging = {lt for lt in layers if self._cluster_flags and _lib.lib().bgtq_decode_plan_cluster(C.byref(lt.plan(flags))) > 0}
 
     # -- encode --------------------------------------------------------------------------
     def _encode_kv(self, layer_idx: int, k: torch.Tensor, v: torch.Tensor, t_start: int, t_end: int):
@@ -385,8 +387,7 @@ class BlockGTQKVManager:
             kb, vb = self._k_buf[li], self._v_buf[li]
             s.k_buf, s.v_buf, s.kb_sb, s.kb_sh = kb.data_ptr(), vb.data_ptr(), kb.stride(0), kb.stride(1)
             s.buf_o, s.buf_lse, s.n_sink, s.window = self._buf_o.data_ptr(), self._buf_lse.data_ptr(), self.n_sink, self.recent_window
-        s.key, s.addr, s.n_launch = (lt, baked, pd), C.addressof(s), \
-            4 if self._buffered else 3 - (self._cluster_flags > 0 and _lib.lib().bgtq_decode_plan_cluster(s.plan) > 0)
+        s.key, s.addr, s.n_launch = (lt, baked, pd), C.addressof(s), 4 if self._buffered else 3 - (lt in self._merging)
         self._steps[li] = s
         return s
 

@@ -465,9 +465,9 @@ int bgtq_layer_encode(const BgtqLayerStep* step, const void* k, int64_t k_sb, in
  * (rot_k may be NULL: q is in the packed-K basis and contiguous) -> bgtq_decode -> bgtq_combine into the
  * contiguous out (n_batch, n_q, 128) fp16 and the optional out_f32 / lse_out.  The decode starts without the plan's
  * early fetch: the rows may come from the work right in front of the call.  scratch: device memory of
- * bgtq_attend_scratch_bytes(n_batch, n_q, n_splits) bytes, 16-byte aligned; it may be NULL where the plan's decode merges
- * its shares (bgtq_decode_plan_cluster), nothing is rotated and buf_o is NULL: BGTQ_E_UNSUPPORTED then says that this
- * call (wider rows than the plan was made for) needs it after all. */
+ * bgtq_attend_scratch_bytes(n_batch, n_q, n_splits) bytes, 16-byte aligned.  It may be NULL: a decode that merges its
+ * shares (bgtq_decode_plan_cluster) with nothing to rotate and no buf_o needs none, any other call returns
+ * BGTQ_E_UNSUPPORTED before it launches anything. */
 int64_t bgtq_attend_scratch_bytes(int32_t n_batch, int32_t n_q, int32_t n_splits);
 int bgtq_attend(const BgtqDecodePlan* plan, const BgtqHeadDesc* desc, const float* rot_k,
                 const void* q, int64_t q_sb, int64_t q_sh,
