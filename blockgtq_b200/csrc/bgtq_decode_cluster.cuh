@@ -119,6 +119,13 @@ __device__ __forceinline__ void merge_finish(const DecParams& P, uint8_t* smem, 
     const MergeParams& F = P.m;
     const int tid = threadIdx.x;
     const int dl = tid % kWidth, pt = tid / kWidth;             // output dim of the slice, kPer rows of the rotation
+    // this thread's value of the other partial, requested ahead
+    const int64_t row0 = (int64_t)b * P.n_q + h * P.gqa;
+    float bo = 0.f, bl = -BGTQ_INF;
+    if (F.buf_o && tid < P.gqa * kWidth) {
+        bo = F.buf_o[(row0 + tid / kWidth) * kHD + rank * kWidth + dl];
+        bl = F.buf_lse[row0 + tid / kWidth];
+    }
     if (F.v_rot) asm volatile("cp.async.wait_all;" ::: "memory");
     cluster_sync();
     const uint8_t* shares = smem + F.share_off;
@@ -189,10 +196,23 @@ __device__ __forceinline__ void merge_finish(const DecParams& P, uint8_t* smem, 
         } else {
             y = merged[q * kHD + dim];
         }
-        const int64_t row = (int64_t)b * P.n_q + hq;
+        const int64_t row = row0 + q;
+        float tot = lse[q];
+        if (F.buf_o) {
+            if (i != tid) {
+                bo = F.buf_o[row * kHD + dim];
+                bl = F.buf_lse[row];
+            }
+            const float m2 = fmaxf(tot, bl);
+            if (m2 > -BGTQ_INF) {
+                const float wp = tot == -BGTQ_INF ? 0.f : expf(tot - m2), wb = bl == -BGTQ_INF ? 0.f : expf(bl - m2);
+                y = (wp * y + wb * bo) / (wp + wb);
+                tot = m2 + logf(wp + wb);
+            }
+        }
         F.out[b * F.o_sb + hq * F.o_sh + dim] = f16_bits(y);
         if (F.out_f32) F.out_f32[row * kHD + dim] = y;
-        if (F.lse_out && dim == 0) F.lse_out[row] = lse[q];
+        if (F.lse_out && dim == 0) F.lse_out[row] = tot;
     }
 }
 

@@ -43,6 +43,8 @@ struct MergeParams {
     int64_t o_sb, o_sh;
     float* out_f32;                 // optional, (n_batch, n_q, 128)
     float* lse_out;                 // optional, (n_batch, n_q)
+    const float* buf_o;             // optional: another partial of every row, (n_batch, n_q, 128) with its log-sum-exp
+    const float* buf_lse;
     uint32_t share_off, rot_off;    // shared memory: the cluster's shares, the CTA's slice of the rotation
 };
 

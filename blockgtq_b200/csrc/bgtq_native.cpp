@@ -237,7 +237,7 @@ PyObject* attend(PyObject*, PyObject* const* argv, Py_ssize_t n) {
     if (want_lse) lse = empty({B, n_q}, at::kFloat, *q);
     void* const st = stream_of(*q);
     int rc;
-    bool bare = !rot_k && !bo;      // a decode that merges its shares and rotates nothing needs no scratch ...
+    bool bare = !rot_k;      // a decode that merges its shares and rotates nothing needs no scratch ...
 again:
     if (!bare) scratch = empty({B * n_q * (ns * (kHD + 1) + kHD / 2)}, at::kFloat, *q);
     Py_BEGIN_ALLOW_THREADS

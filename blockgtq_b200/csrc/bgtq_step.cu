@@ -49,8 +49,20 @@ extern "C" __attribute__((visibility("default"))) int bgtq_layer_step(
                                s->kn_sb, s->kn_sh, s->kn_st, s->kn_count, s->v_packed, s->vp_sb, s->vp_sh, s->vp_st, s->v_norms,
                                s->vn_sb, s->vn_sh, s->vn_st, s->enc_flags, s->pos_dev, s->t_capacity, s->status, stream);
     if (rc != BGTQ_OK) return rc;
-    if (!ring && bgtq_decode_plan_cluster(s->plan)) {
-        const MergeParams M = {s->v_rot, static_cast<uint16_t*>(s->out), s->o_sb, s->o_sh, nullptr, nullptr, 0, 0};
+    auto regions = [&]() {      // the fp16 sink and window
+        return bgtq_buffer_attn_pos(q, q_sb, q_sh, s->k_buf, s->v_buf, s->kb_sb, s->kb_sh, 0, 0, s->n_sink, 0, s->window + 1, s->n_batch,
+                                    s->n_q, s->n_kv, s->scale, s->buf_o, s->buf_lse, s->pos_dev, stream);
+    };
+    bool regions_done = false;
+    if (bgtq_decode_plan_cluster(s->plan)) {
+        if (ring) {     // its partial comes first here: the decode merges it too.  (The decode's early fetch stays sound: the append
+                        // lets its dependents start behind its own wait, and so this one the decode.)
+            rc = regions();
+            if (rc != BGTQ_OK) return rc;
+            regions_done = true;
+        }
+        const MergeParams M = {s->v_rot, static_cast<uint16_t*>(s->out), s->o_sb, s->o_sh, nullptr, nullptr, ring ? s->buf_o : nullptr,
+                               ring ? s->buf_lse : nullptr, 0, 0};
         rc = launch_decode_plan(s->plan, q_dec, s->k_packed, s->kp_sb, s->kp_sh, s->kp_st, s->k_norms, s->kn_sb, s->kn_sh, s->kn_st,
                                 s->v_packed, s->vp_sb, s->vp_sh, s->vp_st, s->v_norms, s->vn_sb, s->vn_sh, s->vn_st, s->n_batch, s->n_q,
                                 s->n_kv, 0, s->t_capacity, 1, s->scale, nullptr, nullptr, s->status, s->pos_dev, s->pos_add, true, &M,
@@ -61,9 +73,8 @@ extern "C" __attribute__((visibility("default"))) int bgtq_layer_step(
                      s->v_packed, s->vp_sb, s->vp_sh, s->vp_st, s->v_norms, s->vn_sb, s->vn_sh, s->vn_st, s->n_batch, s->n_q, s->n_kv,
                      0, s->t_capacity, s->n_splits, s->scale, s->part_o, s->part_lse, s->status, s->pos_dev, s->pos_add, stream);
     if (rc != BGTQ_OK) return rc;
-    if (ring) {
-        rc = bgtq_buffer_attn_pos(q, q_sb, q_sh, s->k_buf, s->v_buf, s->kb_sb, s->kb_sh, 0, 0, s->n_sink, 0, s->window + 1, s->n_batch,
-                                  s->n_q, s->n_kv, s->scale, s->buf_o, s->buf_lse, s->pos_dev, stream);
+    if (ring && !regions_done) {
+        rc = regions();
         if (rc != BGTQ_OK) return rc;
     }
     return bgtq_combine(s->part_o, s->part_lse, s->n_splits, s->v_rot, ring ? s->buf_o : nullptr, ring ? s->buf_lse : nullptr,
@@ -94,7 +105,7 @@ extern "C" __attribute__((visibility("default"))) int bgtq_attend(
     float scale, const float* v_rot, const float* buf_o, const float* buf_lse, void* scratch, void* out, float* out_f32,
     float* lse_out, int32_t* status, void* stream) {
     if (!plan || !q || !out || n_batch < 1 || n_q < 1 || n_splits < 1) return BGTQ_E_BADARG;
-    if (!scratch && (rot_k || buf_o || !bgtq_decode_plan_cluster(plan))) return BGTQ_E_UNSUPPORTED;
+    if (!scratch && (rot_k || !bgtq_decode_plan_cluster(plan))) return BGTQ_E_UNSUPPORTED;
     if (reinterpret_cast<uintptr_t>(scratch) & 15u) return BGTQ_E_ALIGN;
     const int64_t rows = (int64_t)n_batch * n_q;
     float* const part_o = static_cast<float*>(scratch);
@@ -111,8 +122,8 @@ extern "C" __attribute__((visibility("default"))) int bgtq_attend(
     // No early fetch here, whatever the plan says: what is in front of this call may be a bulk encode of the very rows
     // that are attended, and it lets its dependents start while it runs.  (A layer step is different: there the launch in
     // front of the decode is its own append.)
-    if (!buf_o && bgtq_decode_plan_cluster(plan)) {
-        const MergeParams M = {v_rot, static_cast<uint16_t*>(out), (int64_t)n_q * kHD, kHD, out_f32, lse_out, 0, 0};
+    if ((buf_o == nullptr) == (buf_lse == nullptr) && bgtq_decode_plan_cluster(plan)) {
+        const MergeParams M = {v_rot, static_cast<uint16_t*>(out), (int64_t)n_q * kHD, kHD, out_f32, lse_out, buf_o, buf_lse, 0, 0};
         const int rc = launch_decode_plan(plan, q_dec, k_packed, kp_sb, kp_sh, kp_st, k_norms, kn_sb, kn_sh, kn_st, v_packed, vp_sb, vp_sh,
                                           vp_st, v_norms, vn_sb, vn_sh, vn_st, n_batch, n_q, n_kv, t_begin, t_end, 1, scale, nullptr,
                                           nullptr, status, nullptr, 0, false, &M, stream);

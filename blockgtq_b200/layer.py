@@ -439,7 +439,7 @@ def attend(layer, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, *, ro
                        want_f32, want_lse, status, layer.n_kv)
         if r is None:
             raise ValueError("query, cache and layer do not match")
-    return _lib.done(r, "bgtq_attend", (3 if rotate else 2) - (merged and buf_o is None))
+    return _lib.done(r, "bgtq_attend", (3 if rotate else 2) - merged)
 
 
 _SCALE = 1.0 / math.sqrt(HD)

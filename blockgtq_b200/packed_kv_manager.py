@@ -161,7 +161,7 @@ class BlockGTQKVManager:
                         lt.set_early_fetch(1)
         if dev.type == "cuda":      # by capacity: one kernel for the cache's whole life, captured graphs included
             self._dec_flags |= tile_flags(self.B, self.n_kv, self.max_T, dev)
-            if not self._buffered and self._exchange is None:
+            if self._exchange is None:
                 self._cluster_flags = cluster_flags(self.B, self.n_kv, self.max_T, dev)
         self._prepare_decode_plans()
         self._q_rot = torch.empty(self.B, self.n_q, self.hd, dtype=torch.float16, device=dev)
@@ -387,7 +387,7 @@ class BlockGTQKVManager:
             kb, vb = self._k_buf[li], self._v_buf[li]
             s.k_buf, s.v_buf, s.kb_sb, s.kb_sh = kb.data_ptr(), vb.data_ptr(), kb.stride(0), kb.stride(1)
             s.buf_o, s.buf_lse, s.n_sink, s.window = self._buf_o.data_ptr(), self._buf_lse.data_ptr(), self.n_sink, self.recent_window
-        s.key, s.addr, s.n_launch = (lt, baked, pd), C.addressof(s), 4 if self._buffered else 3 - (lt in self._merging)
+        s.key, s.addr, s.n_launch = (lt, baked, pd), C.addressof(s), 3 + self._buffered - (lt in self._merging)
         self._steps[li] = s
         return s
 

@@ -240,7 +240,7 @@ int bgtq_step_prepare_ring(const BgtqHeadDesc* desc, const float* rot_k, const f
                                    * with a cluster of n CTAs per (batch, KV head) pair, which merge their shares and write the
                                    * output rows themselves: no merge launch.  The plan's specialised kernel is the one for that;
                                    * bgtq_decode with such a plan takes the general kernel.  bgtq_decode_plan drops the bits
-                                   * where the form does not fit shared memory; fp16 regions (buf_o) take the split form. */
+                                   * where the form does not fit shared memory. */
 #define BGTQ_DEC_CLUSTER_MASK 0x1F00
 
 /* Opaque launch plan of the decode kernel for the KV heads of one layer (host
@@ -466,7 +466,7 @@ int bgtq_layer_encode(const BgtqLayerStep* step, const void* k, int64_t k_sb, in
  * contiguous out (n_batch, n_q, 128) fp16 and the optional out_f32 / lse_out.  The decode starts without the plan's
  * early fetch: the rows may come from the work right in front of the call.  scratch: device memory of
  * bgtq_attend_scratch_bytes(n_batch, n_q, n_splits) bytes, 16-byte aligned.  It may be NULL: a decode that merges its
- * shares (bgtq_decode_plan_cluster) with nothing to rotate and no buf_o needs none, any other call returns
+ * shares (bgtq_decode_plan_cluster) with nothing to rotate needs none, any other call returns
  * BGTQ_E_UNSUPPORTED before it launches anything. */
 int64_t bgtq_attend_scratch_bytes(int32_t n_batch, int32_t n_q, int32_t n_splits);
 int bgtq_attend(const BgtqDecodePlan* plan, const BgtqHeadDesc* desc, const float* rot_k,

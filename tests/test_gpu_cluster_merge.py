@@ -55,13 +55,16 @@ def test_merged_in_the_launch(batch, n_kv, gqa, cap, k_bits, v_bits, mixed, c):
     mgr.check_status()
 
 
-@pytest.mark.parametrize("batch,n_kv,gqa,start,cap", [(1, 8, 4, 0, 40), (2, 2, 8, 254, 600), (4, 8, 3, 1020, 1030)])
-def test_layer_steps(batch, n_kv, gqa, start, cap):
-    """A layer's steps call by call and replayed: the same cache bytes as the split form, rows within the bound."""
+@pytest.mark.parametrize("batch,n_kv,gqa,start,cap,sink,window", [
+    (1, 8, 4, 0, 40, 0, 0), (2, 2, 8, 254, 600, 0, 0), (4, 8, 3, 1020, 1030, 0, 0), (1, 8, 4, 3, 40, 2, 4), (2, 4, 4, 700, 720, 4, 128), (9, 8, 1, 260, 300, 0, 9)])
+def test_layer_steps(batch, n_kv, gqa, start, cap, sink, window):
+    """A layer's steps call by call and replayed, with and without fp16 regions (a packed region that is still empty among them):
+    the same cache bytes as the split form, rows within the bound."""
     gen = torch.Generator().manual_seed(start)
     from blockgtq_b200 import BlockGTQKVManager
-    a = _manager(batch, n_kv, gqa, cap, gen)
-    b = BlockGTQKVManager(1, n_kv * gqa, n_kv, 128, max_seq_len=cap, batch_size=batch, device=DEV)
+    regions = dict(n_sink=sink, recent_window=window)
+    a = _manager(batch, n_kv, gqa, cap, gen, **regions)
+    b = BlockGTQKVManager(1, n_kv * gqa, n_kv, 128, max_seq_len=cap, batch_size=batch, device=DEV, **regions)
     b.set_quantizers(0, a.quantizers[0])
     for m in (a, b):
         m._ensure_storage()
@@ -89,10 +92,15 @@ def test_layer_steps(batch, n_kv, gqa, start, cap):
             got = a.static_outputs()[0].unsqueeze(2).float()
         for m in (a, b):
             m.increment_seq_len()
-        top = float(a._v_norms[0].float().max() * max(t.centroids.abs().max() for t in a._layers[0].v_tables)) * 128 ** 0.5
+        # (an fp16 region's values are at most as large as their norm, which the packed rows' is within a factor of)
+        top = max(float(a._v_norms[0].float().max() * max(t.centroids.abs().max() for t in a._layers[0].v_tables)), 2.0) * 128 ** 0.5
         assert (got - want).abs().max().item() <= 2.0 ** -10 * top + 2.0 ** -11 * want.abs().max().item()
-        for x, y in zip((a._k_packed, a._k_norms, a._v_packed, a._v_norms), (b._k_packed, b._k_norms, b._v_packed, b._v_norms)):
-            assert torch.equal(x, y)
+        for x, y in zip((a._k_packed, a._k_norms, a._v_packed, a._v_norms, a._k_buf, a._v_buf), (b._k_packed, b._k_norms, b._v_packed, b._v_norms, b._k_buf, b._v_buf)):
+            assert x is y is None or torch.equal(x, y)
+    # several calls' worth of attention over what is there, with the regions' partial
+    out, o32, lse = a.attend(0, q, want_partial=True)
+    want, w32, wlse = b.attend(0, q, want_partial=True)
+    assert (o32 - w32).abs().max().item() <= 2.0 ** -10 * top and (lse - wlse).abs().max().item() <= 1e-5 * max(1.0, wlse.abs().max().item())
     a.check_status()
 
 
