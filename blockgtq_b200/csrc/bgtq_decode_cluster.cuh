@@ -110,6 +110,21 @@ __device__ __forceinline__ void merge_share(const DecParams& P, uint8_t* smem, u
     }
 }
 
+// merge_finish of shares that are all empty: this CTA's slice of the other partial, or zeros.
+__device__ __forceinline__ void merge_none(const DecParams& P, int h, int b, int rank) {
+    constexpr int kWidth = kHD / kClusterN;
+    const MergeParams& F = P.m;
+    for (int i = threadIdx.x; i < P.gqa * kWidth; i += kDecThreads) {
+        const int q = i / kWidth, dim = rank * kWidth + i % kWidth, hq = h * P.gqa + q;
+        const int64_t row = (int64_t)b * P.n_q + hq;
+        const float lse = F.buf_o ? fmaxf(F.buf_lse[row], -BGTQ_INF) : -BGTQ_INF;      // (not a number: nothing)
+        const float y = lse == -BGTQ_INF ? 0.f : F.buf_o[row * kHD + dim];
+        F.out[b * F.o_sb + hq * F.o_sh + dim] = f16_bits(y);
+        if (F.out_f32) F.out_f32[row * kHD + dim] = y;
+        if (F.lse_out && dim == 0) F.lse_out[row] = lse;
+    }
+}
+
 // The cluster's shares -> this CTA's slice of the pair's output rows.  `buf`: shared memory that this CTA no longer uses (21 KB).
 // Called by all threads of the cluster, their shares on their way.
 __device__ __forceinline__ void merge_finish(const DecParams& P, uint8_t* smem, uint8_t* buf, int h, int b, int rank) {

@@ -31,6 +31,8 @@
 //     trip count); the segment list of the head drives which bodies run;
 //   * softmax state is fp32 and per warp; warps are merged at the end of a run
 //     through the (then idle) stage buffers.
+//   * with kMerges (specialised builds only) a cluster of CTAs serves one pair,
+//     a share of its tokens each, and merges in the launch: bgtq_decode_cluster.cuh.
 //   * rounding points follow the reference kernel
 //     (blockgtq/kernels/fused_packed_attention.py:770-873): fp32 logits,
 //     p rounded to fp16 for the PV product while the denominator uses fp32 p,
@@ -551,6 +553,15 @@ extern "C" __global__ void __launch_bounds__(kDecThreads, 1) bgtq_decode_jit(con
             P.part_lse[i] = -BGTQ_INF;
         if (tables_pending) wait_tables();
         return;
+    }
+    if constexpr (kMerges) {
+        if (n_tok == 0) {       // nothing packed yet: the rows are the other partial's
+            if (!dep_waited) grid_dependency_wait();
+            merge_none(P, c_pair / P.n_batch, c_pair % P.n_batch, c_rank);
+            cluster_all_started();
+            wait_tables();
+            return;
+        }
     }
     // Equal item counts, unless the caller's table was made for exactly this launch (the same items per pair,
     // pairs, CTAs and units per item: every CTA sees the same four words, so all take the same branch)

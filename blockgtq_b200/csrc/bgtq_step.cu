@@ -1,7 +1,7 @@
 // One call for the launches of a layer's decode step, and one for those of an attention over cached tokens.
 //
-// A decode step of a short sequence is bounded by the host: the three (four with fp16 regions) launches of a layer
-// take the GPU about 15 us, and passing their forty-odd arguments one launch at a time, or staging the step's inputs
+// A decode step of a short sequence is bounded by the host: the two or three (one more with fp16 regions) launches of a
+// layer take the GPU 9 to 15 us, and passing their forty-odd arguments one launch at a time, or staging the step's inputs
 // for a captured graph (three copies and a graph launch per layer), took the host 36 us.  Everything that does not
 // change from step to step is filled in once (BgtqLayerStep); a step then costs one call, and the kernels read the
 // caller's query, key and value rows where they lie.
