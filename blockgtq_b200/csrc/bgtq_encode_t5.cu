@@ -790,9 +790,10 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
 }
 
 // One CTA per SM.  The tiles of all (KV head, K or V) form one list, a K tile kUnitsK units long and a V tile kUnitsV (what
-// they take, 219 and 162 us for a million rows: 374 us for both so; with 13 to 7, made for slower K rows, a sixth more); CTA i works on the tiles that begin in its share of the units,
-// and loads the tables again where its share crosses into the next (head, role).
-constexpr int kUnitsK = 11, kUnitsV = 8;
+// they take, 219 and 162 us for a million rows: 374 us for both so; with 13 to 7 a sixth more); CTA i works on the tiles that begin in its share of the units,
+// and loads the tables again where its share crosses into the next (head, role).  With few tiles per CTA whole tiles count, not
+// units: see slowest_share.
+constexpr int kUnitsK = 11, kUnitsV = 8, kUnitsK2 = 13, kUnitsV2 = 7;
 template <bool MIXED, bool CODES, bool ONE>
 __global__ void __launch_bounds__(kThreads, 1) encode_t5_kernel(const EncParams P, const int units_k, const int units_v) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -842,6 +843,27 @@ __global__ void __launch_bounds__(kThreads, 1) encode_t5_kernel(const EncParams 
 
 }  // namespace
 
+// The slowest CTA's time, in tenths of a unit, for K and V tiles that count uk and uv: the two row groups of a CTA work side by
+// side, so an odd tile takes about 1.3 of its units instead of half a pair's two, and a (head, role) begun takes four.
+static int slowest_share(int n_tiles, int n_kv, int uk, int uv, int sms) {
+    const int len_k = uk * n_tiles, len = len_k + uv * n_tiles, all = len * n_kv;
+    int worst = 0;
+    for (int i = 0; i < sms; ++i) {
+        const int u1 = all * (i + 1) / sms;
+        int t = 0;
+        for (int u = all * i / sms; u < u1;) {
+            const int at = u / len * len, base = u - at >= len_k ? at + len_k : at;
+            const bool is_v = base != at;
+            const int end = is_v ? at + len : at + len_k, w = is_v ? uv : uk, top = u1 < end ? u1 : end;
+            const int n = (top - base + w - 1) / w - (u - base + w - 1) / w;
+            if (n > 0) t += (n / 2 * 20 + n % 2 * 13) * (is_v ? kUnitsV : kUnitsK) + 40;
+            u = end;
+        }
+        worst = t > worst ? t : worst;
+    }
+    return worst;
+}
+
 // The launcher's caller checks: every input row 16-byte aligned and n_tok >= 16 (as for the warp-MMA bulk path).
 int launch_encode_t5(const EncParams& P, cudaStream_t stream) {
     const int64_t n_rows = (int64_t)P.n_batch * P.n_tok;
@@ -853,7 +875,14 @@ int launch_encode_t5(const EncParams& P, cudaStream_t stream) {
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t all = (int64_t)n_tiles * P.n_kv * ((do_k ? 1 : 0) + (do_v ? 1 : 0));
     const bool few = all <= sms;                // one tile per CTA (the code written out for it: ONE)
-    const int units_k = do_k ? (few ? 1 : kUnitsK) : 0, units_v = do_v ? (few ? 1 : kUnitsV) : 0;
+    int units_k = do_k ? (few ? 1 : kUnitsK) : 0, units_v = do_v ? (few ? 1 : kUnitsV) : 0;
+    // With up to eight tiles per CTA the better of two weightings (2.5 us of host time, beside a kernel of 16 and more):
+    // 4 KV heads at 6144 tokens 28 and 22 us with 11 : 8 and 13 : 7, at 5120 19 and 22, at 10000 (11 : 8) 29 and 33.
+    if (do_k && do_v && !few && all <= 8 * sms &&
+        slowest_share(n_tiles, P.n_kv, kUnitsK2, kUnitsV2, sms) < slowest_share(n_tiles, P.n_kv, kUnitsK, kUnitsV, sms)) {
+        units_k = kUnitsK2;
+        units_v = kUnitsV2;
+    }
     const int smem = (int)sizeof(E5Smem);
     const bool mixed = P.flags & BGTQ_ENC_K_MIXED, codes = P.k_codes != nullptr || P.v_codes != nullptr;
     auto kern = mixed ? (codes ? encode_t5_kernel<true, true, false> : few ? encode_t5_kernel<true, false, true> : encode_t5_kernel<true, false, false>)
