@@ -417,16 +417,17 @@ def attend(layer, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, *, ro
         rot_k = None
     n_splits = 0 if n_splits is None else n_splits or -1       # (the library's choice; 0 is refused like -1)
     scale = _SCALE if scale is None else scale
-    v_rot = None if v_rot is None else v_rot.data_ptr()
-    status = None if status is None else status.data_ptr()
+    # (names of their own: the parameters may be the only references to these tensors, and the library takes addresses)
+    rot_addr = None if v_rot is None else v_rot.data_ptr()
+    status_addr = None if status is None else status.data_ptr()
     native = _lib.host().attend
     try:
-        r = native(plan, desc, rot_k, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, n_splits, scale, v_rot, buf_o, buf_lse,
-                   want_f32, want_lse, status, layer.n_kv)
+        r = native(plan, desc, rot_k, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, n_splits, scale, rot_addr, buf_o, buf_lse,
+                   want_f32, want_lse, status_addr, layer.n_kv)
     except TypeError:       # (ranges as whole floats, say)
         t_begin, t_end, n_splits = int(t_begin), int(t_end), int(n_splits)
-        r = native(plan, desc, rot_k, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, n_splits, scale, v_rot, buf_o, buf_lse,
-                   want_f32, want_lse, status, layer.n_kv)
+        r = native(plan, desc, rot_k, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, n_splits, scale, rot_addr, buf_o, buf_lse,
+                   want_f32, want_lse, status_addr, layer.n_kv)
     if r is None:           # another type or layout, or an argument to complain about
         _lib.require_cuda(q, "q")
         if k_norms.dtype != torch.float16 or v_norms.dtype != torch.float16:
@@ -435,8 +436,8 @@ def attend(layer, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, *, ro
             _strides3(t)
         with torch.cuda.device(q.device):
             q = q.to(torch.float16).contiguous()
-            r = native(plan, desc, rot_k, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, n_splits, scale, v_rot, buf_o, buf_lse,
-                       want_f32, want_lse, status, layer.n_kv)
+            r = native(plan, desc, rot_k, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, n_splits, scale, rot_addr, buf_o, buf_lse,
+                       want_f32, want_lse, status_addr, layer.n_kv)
         if r is None:
             raise ValueError("query, cache and layer do not match")
     return _lib.done(r, "bgtq_attend", (3 if rotate else 2) - merged)
