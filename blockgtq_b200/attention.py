@@ -16,14 +16,14 @@ import numpy as np
 import torch
 
 from . import _lib
-from .layer import HD, attend, cluster_flags, make_decode_plan, tile_flags
+from .layer import HD, DecodePlans, attend, cluster_flags, make_decode_plan, tile_flags
 
 _tables = {}          # tables by contents
 _cache = {}           # the same by the full description of the tensors they were made of, with these tensors
 _recent = {}          # the latest tensors seen at an address, with their tables
 
 
-class _AdHocLayer:
+class _AdHocLayer(DecodePlans):
     """Minimal stand-in for LayerTables built from operator arguments."""
 
     def __init__(self, segments, cb, vl, v_bits, n_kv, nopack, device):
@@ -44,14 +44,9 @@ class _AdHocLayer:
                 d.v_lut[i] = int(x)
         self.desc_dev = torch.from_numpy(np.frombuffer(self.desc_host, dtype=np.uint8).copy()).to(device)
         self._plans = {}
-        self._handles = {}
 
-    def plan(self, flags=0):
-        p = self._plans.get(flags)
-        if p is None:
-            p = make_decode_plan(self.desc_host, self.n_kv, flags, self.device)
-            self._plans[flags] = p
-        return p[0]
+    def _make_plan(self, flags):
+        return make_decode_plan(self.desc_host, self.n_kv, flags, self.device)
 
 
 def _version(t):

@@ -100,7 +100,24 @@ def _specialize(plan):
         raise RuntimeError("specialising the decode kernel failed:\n" + log.value.decode(errors="replace"))
 
 
-class LayerTables:
+class DecodePlans:
+    """The decode plans of a layer's KV heads, made by ``_make_plan(flags)`` on first use and kept for the layer's life:
+    calls pass a plan's address on, and its image is device memory that launches read."""
+
+    def plan_entry(self, flags: int):
+        """(plan, image, whether the plan's decode merges its shares).  Threads may make a plan side by side (the compiler
+        runs without the interpreter's lock): the first to finish is the one all of them get."""
+        e = self._plans.get(flags)
+        if e is None:
+            p, image = self._make_plan(flags)
+            e = self._plans.setdefault(flags, (p, image, _lib.lib().bgtq_decode_plan_cluster(C.byref(p)) > 0))
+        return e
+
+    def plan(self, flags: int = 0) -> _lib.DecodePlan:
+        return self.plan_entry(flags)[0]
+
+
+class LayerTables(DecodePlans):
     """Device-resident static tables for the KV heads of one layer."""
 
     def __init__(self, k_tables, v_tables, device):
@@ -123,24 +140,20 @@ class LayerTables:
         self.head_perm = torch.stack([t.head_perm for t in k_tables]).long().to(self.device)   # (n_kv, 128)
         self.addrs = (self.desc_dev.data_ptr(), self.rot_k.data_ptr(), self.rot_v.data_ptr())
         self._plans = {}
-        self._handles = {}
         self._partition = None
         self._row_strides = {}
         self._early_fresh = 0
 
-    def plan(self, flags: int = 0) -> _lib.DecodePlan:
-        p = self._plans.get(flags)
-        if p is None:
-            p = make_decode_plan(self.desc_host, self.n_kv, flags, self.device,
-                                 row_strides=self._row_strides.get(bool(flags & _lib.DEC_K_MIXED)))
-            if self._partition is not None:
-                _lib.check(_lib.lib().bgtq_decode_plan_set_partition(C.byref(p[0]), self._partition.data_ptr()),
-                           "bgtq_decode_plan_set_partition")
-            if self._early_fresh:
-                _lib.check(_lib.lib().bgtq_decode_plan_set_early_fetch(C.byref(p[0]), self._early_fresh),
-                           "bgtq_decode_plan_set_early_fetch")
-            self._plans[flags] = p
-        return p[0]
+    def _make_plan(self, flags):
+        p, image = make_decode_plan(self.desc_host, self.n_kv, flags, self.device,
+                                    row_strides=self._row_strides.get(bool(flags & _lib.DEC_K_MIXED)))
+        if self._partition is not None:
+            _lib.check(_lib.lib().bgtq_decode_plan_set_partition(C.byref(p), self._partition.data_ptr()),
+                       "bgtq_decode_plan_set_partition")
+        if self._early_fresh:
+            _lib.check(_lib.lib().bgtq_decode_plan_set_early_fetch(C.byref(p), self._early_fresh),
+                       "bgtq_decode_plan_set_early_fetch")
+        return p, image
 
     def set_row_strides(self, kp_st: int, kn_st: int, vp_st: int, vn_st: int, mixed: bool = False) -> None:
         """Row strides (packed-K bytes, K-norm values, packed-V bytes, V-norm values per token) of the cache
@@ -412,9 +425,8 @@ def attend(layer, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, *, ro
            v_rot=None, buf_o=None, buf_lse=None, want_f32=False, want_lse=False, status=None):
     """Query rotation (``rotate``: q is in the original basis), split-KV decode over rows [t_begin, t_end) and combine
     in one library call.  q (B, n_q, [1,] 128) -> (out fp16 of q's shape, f32 copy (B, n_q, 128) | None, LSE | None)."""
-    plan, desc, rot_k, merged = _handle(layer, flags | _lib.DEC_PROGRAMMATIC)
-    if not rotate:
-        rot_k = None
+    plan, _image, merged = layer.plan_entry(flags | _lib.DEC_PROGRAMMATIC)
+    plan, desc, rot_k = C.addressof(plan), layer.desc_dev.data_ptr(), layer.rot_k.data_ptr() if rotate else None
     n_splits = 0 if n_splits is None else n_splits or -1       # (the library's choice; 0 is refused like -1)
     scale = _SCALE if scale is None else scale
     # (names of their own: the parameters may be the only references to these tensors, and the library takes addresses)
@@ -465,19 +477,7 @@ def tile_flags(n_batch: int, n_kv: int, n_tokens: int, device) -> int:
 
 def merges(layer, flags: int) -> bool:
     """Whether the layer's decode with these plan flags merges its shares itself in layer steps and attentions."""
-    return _handle(layer, flags)[3]
-
-
-def _handle(layer, flags: int):
-    """What a call with these plan flags passes on each time: addresses of the plan, the descriptors and K's rotation (their
-    owner keeps all three for its life), and whether the decode merges its shares."""
-    h = layer._handles.get(flags)
-    if h is None:
-        plan = layer.plan(flags)
-        rot = getattr(layer, "rot_k", None)
-        h = layer._handles[flags] = (C.addressof(plan), _lib.ptr(layer.desc_dev), None if rot is None else _lib.ptr(rot),
-                                     _lib.lib().bgtq_decode_plan_cluster(C.addressof(plan)) > 0)
-    return h
+    return layer.plan_entry(flags)[2]
 
 
 def cluster_flags(n_batch: int, n_kv: int, n_tokens: int, device, grows: bool = False) -> int:

@@ -24,7 +24,7 @@ import torch
 from . import _lib
 from .calib import packed_v_bytes
 from .layer import (HD, LayerTables, attend, buffer_attn, cluster_flags, combine, decode, decode_grid_size, decode_partition, default_splits,
-                    encode, rotate_q, step_prepare, tile_flags, _no_tcgen05)
+                    encode, merges, rotate_q, step_prepare, tile_flags, _no_tcgen05)
 from .quantizer import BlockGTQQuantizer, build_batched_encode_args
 
 __all__ = ["BlockGTQKVManager", "decode_step"]
@@ -212,7 +212,7 @@ class BlockGTQKVManager:
         flag_sets = {flags, flags | pd}
         with ThreadPoolExecutor(max_workers=min(16, os.cpu_count() or 1)) as ex:     # one layer per job: its flag
             list(ex.map(lambda lt: [lt.plan(f) for f in sorted(flag_sets)], layers))  # variants share one kernel
-        self._merging = {lt for lt in layers if self._cluster_flags and _lib.lib().bgtq_decode_plan_cluster(C.byref(lt.plan(flags))) > 0}
+        self._merging = {lt for lt in layers if self._cluster_flags and merges(lt, flags)}
 
     # -- encode --------------------------------------------------------------------------
     def _encode_kv(self, layer_idx: int, k: torch.Tensor, v: torch.Tensor, t_start: int, t_end: int):
