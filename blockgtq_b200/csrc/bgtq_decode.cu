@@ -65,7 +65,8 @@ int bgtq::launch_decode_plan(
     const int64_t max_items = (int64_t)n_batch * n_kv * n_splits;
     // the kernel cuts the item range among its CTAs in 32-bit arithmetic: (CTA index + 1) * items must fit
     if (max_items * ((int64_t)sms + 1) > 0xFFFFFFFFll) return BGTQ_E_TOOBIG;
-    const int cluster = merge ? decode_cluster(P.plan) : 0;
+    if (merge && n_batch > 65535) return BGTQ_E_TOOBIG;       // (the merge launch's limit, and the split form's number of splits
+    const int cluster = merge ? decode_cluster(P.plan) : 0;   // above, hold for this form too: what one refuses both do)
     dim3 grid((unsigned)(merge ? n_batch * n_kv * cluster : max_items < sms ? max_items : sms));
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool pdl = (P.plan.flags & BGTQ_DEC_PROGRAMMATIC) != 0;

@@ -65,7 +65,7 @@ extern "C" __attribute__((visibility("default"))) int bgtq_layer_step(
                                ring ? s->buf_lse : nullptr, 0, 0};
         rc = launch_decode_plan(s->plan, q_dec, s->k_packed, s->kp_sb, s->kp_sh, s->kp_st, s->k_norms, s->kn_sb, s->kn_sh, s->kn_st,
                                 s->v_packed, s->vp_sb, s->vp_sh, s->vp_st, s->v_norms, s->vn_sb, s->vn_sh, s->vn_st, s->n_batch, s->n_q,
-                                s->n_kv, 0, s->t_capacity, 1, s->scale, nullptr, nullptr, s->status, s->pos_dev, s->pos_add, true, &M,
+                                s->n_kv, 0, s->t_capacity, s->n_splits, s->scale, nullptr, nullptr, s->status, s->pos_dev, s->pos_add, true, &M,
                                 stream);
         if (rc != BGTQ_E_UNSUPPORTED) return rc;
     }
@@ -125,7 +125,7 @@ extern "C" __attribute__((visibility("default"))) int bgtq_attend(
     if ((buf_o == nullptr) == (buf_lse == nullptr) && bgtq_decode_plan_cluster(plan)) {
         const MergeParams M = {v_rot, static_cast<uint16_t*>(out), (int64_t)n_q * kHD, kHD, out_f32, lse_out, buf_o, buf_lse, 0, 0};
         const int rc = launch_decode_plan(plan, q_dec, k_packed, kp_sb, kp_sh, kp_st, k_norms, kn_sb, kn_sh, kn_st, v_packed, vp_sb, vp_sh,
-                                          vp_st, v_norms, vn_sb, vn_sh, vn_st, n_batch, n_q, n_kv, t_begin, t_end, 1, scale, nullptr,
+                                          vp_st, v_norms, vn_sb, vn_sh, vn_st, n_batch, n_q, n_kv, t_begin, t_end, n_splits, scale, nullptr,
                                           nullptr, status, nullptr, 0, false, &M, stream);
         if (rc != BGTQ_E_UNSUPPORTED || !scratch) return rc;
     }

@@ -128,3 +128,22 @@ def test_rows_too_wide_for_the_merging_form():
     top = float(vn.float().max() * qz.v_lut.float().abs().max()) * HD ** 0.5
     assert (a.float() - b.float()).abs().max().item() <= 2.0 ** -10 * top + 2.0 ** -11 * b.float().abs().max().item()
     assert (al - bl).abs().max().item() <= 1e-5 * max(1.0, bl.abs().max().item())
+
+
+def test_numbers_of_splits_that_are_refused():
+    """The merging form has no splits, and takes no number of them that the split form does not take."""
+    from blockgtq_b200 import _lib
+    from blockgtq_b200.layer import attend, merges
+    gen = torch.Generator().manual_seed(4)
+    mgr = _manager(1, 2, 4, 300, gen)
+    mgr.init_from_cache([tuple(_rand(gen, 1, 2, 300, 128) for _ in range(2))])
+    lt, cache = mgr._layers[0], (mgr._k_packed[0], mgr._k_norms[0], mgr._v_packed[0], mgr._v_norms[0])
+    flags = mgr._dec_flags | mgr._cluster_flags
+    assert merges(lt, flags | _lib.DEC_PROGRAMMATIC)
+    q = _rand(gen, 1, 8, 128)
+    for n in (0, -1, (1 << 31) - 1):
+        with pytest.raises(RuntimeError):
+            attend(lt, q, *cache, 0, 300, rotate=False, n_splits=n, flags=flags)
+    with pytest.raises(OverflowError):
+        attend(lt, q, *cache, 0, 300, rotate=False, n_splits=1 << 31, flags=flags)
+    assert torch.equal(*(attend(lt, q, *cache, 0, 300, rotate=False, n_splits=n, flags=flags)[0] for n in (1, 33)))
