@@ -101,12 +101,28 @@ __device__ __forceinline__ void merge_share(const DecParams& P, uint8_t* smem, u
     float L = s.y * a;
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+    L = __shfl_sync(0xffffffffu, L, 0);
+    if (!(L > 0.f)) {       // no tokens, or a score that is no number: nothing, as the split form's partial of such a run
+        M = -BGTQ_INF;
+        L = 0.f;
+        acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     const uint32_t mine = smem_u32(smem + P.m.share_off + rank * kShareBytes);
 #pragma unroll
     for (int k = 0; k < kClusterN; ++k) {
         const uint32_t to = cluster_addr(mine, k);
         st_cluster4(to + 4u * (q * kHD + 4 * c), acc);
         if (c == 0) st_cluster2(to + 8u * kHD * 4u + 8u * q, M, L);
+    }
+}
+
+// A row's value and log-sum-exp with the other partial's, as the merge launch does it (launch_combine).
+__device__ __forceinline__ void merge_other(float& y, float& lse, float other, float other_lse) {
+    const float m = fmaxf(lse, other_lse);
+    if (m > -BGTQ_INF) {
+        const float wy = lse == -BGTQ_INF ? 0.f : expf(lse - m), wo = other_lse == -BGTQ_INF ? 0.f : expf(other_lse - m);
+        y = (wy * y + wo * other) / (wy + wo);
+        lse = m + logf(wy + wo);
     }
 }
 
@@ -117,8 +133,8 @@ __device__ __forceinline__ void merge_none(const DecParams& P, int h, int b, int
     for (int i = threadIdx.x; i < P.gqa * kWidth; i += kDecThreads) {
         const int q = i / kWidth, dim = rank * kWidth + i % kWidth, hq = h * P.gqa + q;
         const int64_t row = (int64_t)b * P.n_q + hq;
-        const float lse = F.buf_o ? fmaxf(F.buf_lse[row], -BGTQ_INF) : -BGTQ_INF;      // (not a number: nothing)
-        const float y = lse == -BGTQ_INF ? 0.f : F.buf_o[row * kHD + dim];
+        float y = 0.f, lse = -BGTQ_INF;
+        if (F.buf_o) merge_other(y, lse, F.buf_o[row * kHD + dim], F.buf_lse[row]);
         F.out[b * F.o_sb + hq * F.o_sh + dim] = f16_bits(y);
         if (F.out_f32) F.out_f32[row * kHD + dim] = y;
         if (F.lse_out && dim == 0) F.lse_out[row] = lse;
@@ -218,12 +234,7 @@ __device__ __forceinline__ void merge_finish(const DecParams& P, uint8_t* smem, 
                 bo = F.buf_o[row * kHD + dim];
                 bl = F.buf_lse[row];
             }
-            const float m2 = fmaxf(tot, bl);
-            if (m2 > -BGTQ_INF) {
-                const float wp = tot == -BGTQ_INF ? 0.f : expf(tot - m2), wb = bl == -BGTQ_INF ? 0.f : expf(bl - m2);
-                y = (wp * y + wb * bo) / (wp + wb);
-                tot = m2 + logf(wp + wb);
-            }
+            merge_other(y, tot, bo, bl);
         }
         F.out[b * F.o_sb + hq * F.o_sh + dim] = f16_bits(y);
         if (F.out_f32) F.out_f32[row * kHD + dim] = y;

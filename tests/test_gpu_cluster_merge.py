@@ -147,3 +147,63 @@ def test_numbers_of_splits_that_are_refused():
     with pytest.raises(OverflowError):
         attend(lt, q, *cache, 0, 300, rotate=False, n_splits=1 << 31, flags=flags)
     assert torch.equal(*(attend(lt, q, *cache, 0, 300, rotate=False, n_splits=n, flags=flags)[0] for n in (1, 33)))
+
+
+@pytest.mark.parametrize("batch,n_kv,gqa,cap,c", [(1, 2, 4, 2100, 8), (1, 8, 7, 510, 4), (9, 8, 8, 300, 2)])
+def test_scores_that_are_no_numbers(batch, n_kv, gqa, cap, c):
+    """A share with such a score counts as empty, and no other one: what is left is the attention over the other shares' tokens.
+    Values that are infinite, and rows without any share left, come out as from the split form."""
+    from blockgtq_b200.layer import attend
+    gen = torch.Generator().manual_seed(cap + 1)
+    mgr = _manager(batch, n_kv, gqa, cap, gen)
+    mgr.init_from_cache([tuple(_rand(gen, batch, n_kv, cap, 128) for _ in range(2))])
+    lt, cache = mgr._layers[0], (mgr._k_packed[0], mgr._k_norms[0], mgr._v_packed[0], mgr._v_norms[0])
+    plain, flags = mgr._dec_flags, mgr._dec_flags | mgr._cluster_flags
+    q = _rand(gen, batch, n_kv * gqa, 128)
+    top = float((mgr._v_norms[0].float().max() * max(t.centroids.abs().max() for t in lt.v_tables)).item())
+
+    def run(fl, lo=0, hi=cap, **kw):
+        return attend(lt, q, *cache, lo, hi, flags=fl, **dict(dict(rotate=True, want_f32=True, want_lse=True), **kw))
+
+    tiles, share = (cap + 15) // 16, c // 2
+    lo, hi = 16 * (tiles * share // c), min(cap, 16 * (tiles * (share + 1) // c))
+    norms, kept = cache[1], cache[1].clone()
+    norms[:, :, lo + 1] = float("nan")
+    _, got, lse = run(flags)
+    (_, a, la), (_, b, lb) = run(plain, 0, lo), run(plain, hi, cap)
+    want_lse = torch.logaddexp(la, lb)
+    want = a * (la - want_lse).exp()[..., None] + b * (lb - want_lse).exp()[..., None]
+    assert (got - want).abs().max().item() <= 2.0 ** -10 * top and (lse - want_lse).abs().max().item() <= 1e-5 * max(1.0, lse.abs().max().item())
+    norms.copy_(kept)
+    for head in range(n_kv):            # one head without a usable share, the others untouched
+        norms[:, head] = float("nan")
+        (_, got, lse), (_, want, want_lse) = run(flags, v_rot=lt.v_rot), run(plain, v_rot=lt.v_rot)
+        rows = slice(head * gqa, (head + 1) * gqa)
+        assert not got[:, rows].any() and not want[:, rows].any() and torch.isneginf(lse[:, rows]).all() and torch.isneginf(want_lse[:, rows]).all()
+        assert (got - want).abs().max().item() <= 2.0 ** -10 * top * 128 ** 0.5
+        norms.copy_(kept)
+    cache[3][:, :, 0] = float("inf")    # (of a token that no share leaves out)
+    for rot in (None, lt.v_rot):
+        (_, got, lse), (_, want, want_lse) = run(flags, v_rot=rot), run(plain, v_rot=rot)
+        assert not got.isfinite().any() and not want.isfinite().any()
+        assert (lse - want_lse).abs().max().item() <= 1e-5 * max(1.0, lse.abs().max().item())
+
+
+def test_the_other_partial_beside_an_empty_range():
+    """Partials of any kind, infinities and NaN among them, with no packed tokens: the same rows as from the split form."""
+    from blockgtq_b200.layer import attend
+    gen = torch.Generator().manual_seed(3)
+    mgr = _manager(2, 2, 4, 600, gen)
+    mgr.init_from_cache([tuple(_rand(gen, 2, 2, 600, 128) for _ in range(2))])
+    lt, cache = mgr._layers[0], (mgr._k_packed[0], mgr._k_norms[0], mgr._v_packed[0], mgr._v_norms[0])
+    q, other = _rand(gen, 2, 8, 128), torch.randn(2, 8, 128, generator=gen).to(DEV)
+    inf, nan = float("inf"), float("nan")
+    lse = torch.tensor([[0.0, 3.5, -200.0, 90.0, -inf, inf, nan, 1.0]] * 2, device=DEV)
+    other[0, 7, 5], other[1, 7, 6], other[1, 4, 3] = nan, inf, nan
+    for hi in (0, 40):
+        got, want = (attend(lt, q, *cache, 0, hi, rotate=True, v_rot=lt.v_rot, buf_o=other, buf_lse=lse, want_f32=True, want_lse=True,
+                            flags=mgr._dec_flags | f) for f in (mgr._cluster_flags, 0))
+        for g, w in zip(got, want):
+            assert torch.equal(g.isnan(), w.isnan()) and torch.equal(g.isinf(), w.isinf())
+            if hi == 0:
+                assert torch.equal(g.nan_to_num(), w.nan_to_num())
