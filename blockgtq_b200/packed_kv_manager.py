@@ -124,7 +124,8 @@ class BlockGTQKVManager:
         self._batched_args[layer_idx] = build_batched_encode_args(quantizers, device=self.device)
         self._layers[layer_idx] = self._batched_args[layer_idx]["_layer"]
 
-    def _ensure_storage(self):
+    def _ensure_storage(self, merging: bool = True):
+        """``merging=False``: for a manager that is about to be sharded, whose steps decode in the split form."""
         if self._k_packed is not None:
             return
         vpb = self.hd // 2 if self.v_nibble else packed_v_bytes(self.hd, self.v_bits)
@@ -161,7 +162,7 @@ class BlockGTQKVManager:
                         lt.set_early_fetch(1)
         if dev.type == "cuda":      # by capacity: one kernel for the cache's whole life, captured graphs included
             self._dec_flags |= tile_flags(self.B, self.n_kv, self.max_T, dev)
-            if self._exchange is None:
+            if merging:
                 # (with fp16 regions where their attention, in front of the decode then, leaves SMs to it: a decode's CTA takes all
                 # registers of one.  A layer of 8 sequences x 4 KV heads, window 128, 4 query heads per KV head, 32 CTAs: 24.5 and
                 # 21.2 us; 4 x 8 x 3, 96: 29.3 and 20.5; window 600, 8 x 4 x 1, 32: 30.8 and 28.8, x 4, 128: 38 and 39.7, x 7, 224:
@@ -187,6 +188,13 @@ class BlockGTQKVManager:
             self._k_buf = torch.zeros(self.n_layers, self.B, self.n_kv, self._buf_cap, self.hd,
                                       dtype=torch.float16, device=dev)
             self._v_buf = torch.zeros_like(self._k_buf)
+
+    def _attach(self, exchange):
+        """Sequence sharding: from here on a step leaves its partials to the exchange, so its decode is the split form."""
+        self._exchange = exchange
+        if self._cluster_flags:
+            self._cluster_flags = 0
+            self._prepare_decode_plans()
 
     def _layer_rows(self, li: int):
         """Layer ``li``'s packed K, K norms, packed V and V norms (four views cost ten microseconds to make)."""

@@ -102,7 +102,7 @@ class SequenceShard:
         self.world = dist.get_world_size(group)
         self.rank = dist.get_rank(group)
         self.is_owner = self.rank == (self.world - 1 if owner is None else owner)
-        mgr._ensure_storage()
+        mgr._ensure_storage(merging=False)
         self.B, self.n_q = mgr.B, mgr.n_q
         rows = mgr.B * mgr.n_q
         dev = mgr.device
@@ -134,7 +134,7 @@ class SequenceShard:
             self.gathered = torch.zeros(self.world, self.stride, dtype=torch.float32, device=dev)
             self.all_gather()                            # communicator set-up outside any graph capture
             torch.cuda.synchronize(dev) if dev.type == "cuda" else None
-        mgr._exchange = self
+        mgr._attach(self)
 
     def combine_publish(self, part_o, part_lse, n_kv, v_rot, programmatic=False):
         """Peer-memory transport: merge this rank's split partials and store the result straight into every

@@ -75,3 +75,29 @@ def test_sequence_chunk_exchange_gloo_world2():
     port = 29500 + (os.getpid() % 2000)
     mp.spawn(_worker, args=(world, port, ret), nprocs=world, join=True)
     assert len(ret) == world and max(ret.values()) < 1e-5, dict(ret)
+
+
+@pytest.mark.parametrize("stored", [False, True])
+def test_a_sharded_manager_has_the_plans_of_its_steps(monkeypatch, stored):
+    """A sharded step decodes in the split form: its plans are made when the shard is attached, not at the first step (which may
+    be under capture), whatever form the manager had before."""
+    from blockgtq_b200 import BlockGTQKVManager
+    from blockgtq_b200.sharding import SequenceShard
+    made = []
+
+    class Manager(BlockGTQKVManager):
+        def _prepare_decode_plans(self):
+            made.append(self._dec_flags | self._cluster_flags)
+
+    mgr = Manager(1, 8, 2, HD, max_seq_len=64, device="cpu")
+    mgr._max_k_packed_bytes, mgr._max_n_groups = 48, 2
+    if stored:                      # (on a GPU: by the rule on sizes)
+        mgr._cluster_flags = 8 << 8
+        mgr._ensure_storage()
+    dist.init_process_group("gloo", store=dist.HashStore(), rank=0, world_size=1)
+    try:
+        SequenceShard(mgr)
+    finally:
+        dist.destroy_process_group()
+    assert mgr._exchange is not None and mgr._cluster_flags == 0
+    assert made[-1] == mgr._dec_flags and len(made) == 1 + stored
