@@ -21,6 +21,7 @@
 // squares of converted fp16 values instead of mixed-precision multiply-adds (K 277 -> 287, V 164 -> 168).
 // The sums that decide a code (group norms, products) keep the order they had: the packed bytes are bit for bit the same.
 // Every wait is bounded; tensor memory is released on every path out of the kernel.
+#include <cstddef>
 #include <type_traits>
 
 #include "bgtq_common.cuh"
@@ -45,11 +46,8 @@ constexpr uint32_t kTmemCols = 512;             // per group: hi accumulator 128
 constexpr int kSeg = BGTQ_MAX_SEGMENTS;
 constexpr int kLutLd = BGTQ_N_BINS + 4;
 
-// Up to eight consecutive codes of one segment, at most 32 bits: first column | count << 8 | stored bits << 12 | segment << 16
-// | bytes << 20.
-// A K row's tasks follow each other in its bytes; its threads take equal numbers of them.
-// What the packing of a task needs, ready made (read by all lanes at one address).
-struct E5Rec {
+// What the packing of a task (E5Smem::tasks) needs, ready made: read by all lanes at one address, in two 16-byte loads.
+struct __align__(16) E5Rec {
     uint32_t col;       // first column to load | 2 (first column of the task - that) << 8: a last short task loads from column 120
     uint32_t mask;      // the valid bits of its code word
     uint32_t lut;       // shared address of its segment's code table
@@ -72,6 +70,8 @@ struct E5Smem {
     float kcent[512];
     uint8_t code_lut[kSeg][kLutLd];                 // K: entry 256 = entry 255
     float2 grid[kSeg];                              // K, in units of 256 bins: {offset, 1 / range}
+    // Up to eight consecutive codes of one segment, at most 32 bits: first column | count << 8 | stored bits << 12 | segment << 16
+    // | bytes << 20.  A K row's tasks follow each other in its bytes; its threads take equal numbers of them.
     uint32_t tasks[kMaxTasks];
     E5Rec rec[kMaxTasks];
     int32_t cut[5], cut_byte[5];                    // K: first task of each quarter of the tasks, and its first byte
@@ -81,6 +81,7 @@ struct E5Smem {
     __align__(8) uint64_t mma_bar[2];
     uint32_t tmem_base;
 };
+static_assert(sizeof(E5Rec) == 32 && offsetof(E5Smem, rec) % 16 == 0 && offsetof(E5Smem, to) % 16 == 0, "loaded 16 bytes at a time");
 static_assert(sizeof(E5Smem) > 114 * 1024 && sizeof(E5Smem) <= 227 * 1024, "exactly one CTA per SM (it takes all tensor memory)");
 
 // Shared addresses of entries trunc(256 v) of a byte table at `table`, for two values already saturated to [0, 1].  An
