@@ -103,7 +103,7 @@ int bgtq::launch_decode_plan(
     }
     if (e != cudaSuccess) {
         cudaGetLastError();
-        return BGTQ_E_LAUNCH;
+        return merge ? BGTQ_E_UNSUPPORTED : BGTQ_E_LAUNCH;       // (a device that cannot place such clusters: the split form's turn)
     }
     return BGTQ_OK;
 }

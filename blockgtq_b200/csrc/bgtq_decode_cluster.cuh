@@ -145,6 +145,7 @@ __device__ __forceinline__ void merge_none(const DecParams& P, int h, int b, int
 // Called by all threads of the cluster, their shares on their way.
 __device__ __forceinline__ void merge_finish(const DecParams& P, uint8_t* smem, uint8_t* buf, int h, int b, int rank) {
     constexpr int kWidth = kHD / kClusterN, kParts = kDecThreads / kWidth, kPer = kHD / kParts;
+    static_assert(!kMerges || (kPer % 4 == 0 && 8 * kWidth <= kDecThreads), "clusters of 2, 4 and 8");
     constexpr int kShare = kWidth < 32 ? 32 / kWidth : 1;       // parts in a warp
     constexpr int kSums = kParts / kShare;
     const MergeParams& F = P.m;
@@ -198,15 +199,10 @@ __device__ __forceinline__ void merge_finish(const DecParams& P, uint8_t* smem, 
 #pragma unroll 2
         for (int g = 0; g < P.gqa; ++g, m += kHD, to += kSums * kWidth) {
             float acc = 0.f;
-            if constexpr (kPer % 4 == 0) {
 #pragma unroll
-                for (int i = 0; i < kPer; i += 4) {
-                    const float4 v = *reinterpret_cast<const float4*>(m + i);
-                    acc = fmaf(v.x, r[i], acc); acc = fmaf(v.y, r[i + 1], acc); acc = fmaf(v.z, r[i + 2], acc); acc = fmaf(v.w, r[i + 3], acc);
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < kPer; ++i) acc = fmaf(m[i], r[i], acc);
+            for (int i = 0; i < kPer; i += 4) {
+                const float4 v = *reinterpret_cast<const float4*>(m + i);
+                acc = fmaf(v.x, r[i], acc); acc = fmaf(v.y, r[i + 1], acc); acc = fmaf(v.z, r[i + 2], acc); acc = fmaf(v.w, r[i + 3], acc);
             }
 #pragma unroll
             for (int o = kWidth; o < 32; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -214,12 +210,11 @@ __device__ __forceinline__ void merge_finish(const DecParams& P, uint8_t* smem, 
         }
         __syncthreads();
     }
-#pragma unroll 1
-    for (int i = tid; i < P.gqa * kWidth; i += kDecThreads) {
-        const int q = i / kWidth, dim = rank * kWidth + i % kWidth, hq = h * P.gqa + q;
+    if (tid < P.gqa * kWidth) {
+        const int q = tid / kWidth, dim = rank * kWidth + dl, hq = h * P.gqa + q;
         float y;
         if (F.v_rot) {
-            const float* from = red + q * kSums * kWidth + i % kWidth;
+            const float* from = red + q * kSums * kWidth + dl;
             float s4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int s = 0; s < kSums; ++s) s4[s & 3] += from[s * kWidth];
@@ -229,13 +224,7 @@ __device__ __forceinline__ void merge_finish(const DecParams& P, uint8_t* smem, 
         }
         const int64_t row = row0 + q;
         float tot = lse[q];
-        if (F.buf_o) {
-            if (i != tid) {
-                bo = F.buf_o[row * kHD + dim];
-                bl = F.buf_lse[row];
-            }
-            merge_other(y, tot, bo, bl);
-        }
+        if (F.buf_o) merge_other(y, tot, bo, bl);
         F.out[b * F.o_sb + hq * F.o_sh + dim] = f16_bits(y);
         if (F.out_f32) F.out_f32[row * kHD + dim] = y;
         if (F.lse_out && dim == 0) F.lse_out[row] = tot;

@@ -1056,7 +1056,7 @@ inline uint32_t decode_jit_quad_bytes(const DecPlanDev& pl) {
 
 // The kernel may use all of an SM's shared memory on this device: asked for on the first launch there (the driver takes about
 // half a microsecond each time).  A table that is full, or a device past 64, means asking again.
-inline cudaError_t allow_smem(const void* fn, bool clusters) {
+inline cudaError_t allow_smem(const void* fn) {
     struct Entry { std::atomic<const void*> fn{nullptr}; std::atomic<uint64_t> done{0}; };
     static Entry table[1024];
     int dev = 0;
@@ -1070,8 +1070,7 @@ inline cudaError_t allow_smem(const void* fn, bool clusters) {
         if (is == fn || (!is && (t.fn.compare_exchange_strong(is, fn) || is == fn))) mine = &t;
     }
     if (mine && mine->done.load(std::memory_order_acquire) >> dev & 1u) return cudaSuccess;
-    cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (r == cudaSuccess && clusters) r = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    const cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (r == cudaSuccess && mine) mine->done.fetch_or(1ull << dev, std::memory_order_release);
     return r;
 }
@@ -1079,7 +1078,7 @@ inline cudaError_t allow_smem(const void* fn, bool clusters) {
 // Launch one of the kernels; cluster > 0: in clusters of that many CTAs.
 inline cudaError_t launch_decode_fn(const void* fn, const DecParams& P, dim3 grid, size_t smem, cudaStream_t stream, bool programmatic,
                                     int cluster) {
-    cudaError_t e = allow_smem(fn, cluster > 8);
+    cudaError_t e = allow_smem(fn);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;

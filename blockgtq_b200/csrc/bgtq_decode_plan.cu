@@ -124,7 +124,7 @@ extern "C" __attribute__((visibility("default"))) int bgtq_decode_plan(const Bgt
     pl.lut_bytes = (lut_bytes + 127u) / 128u * 128u;
     if (const int n = decode_cluster(pl)) {      // shares merged in the launch: only where they fit besides tables and stages
         const uint32_t stages = 2u * (256u * row_bytes + 4u * 64u + 128u);
-        if (n > 16 || (n & (n - 1)) ||
+        if ((n != 2 && n != 4 && n != 8) ||
             kOffStagesMin + pl.lut_bytes + (stages > kMergeRowsBytes ? stages : kMergeRowsBytes) + n * kShareBytes + kHD * kHD * 4u / n > 227u * 1024u)
             pl.flags &= ~BGTQ_DEC_CLUSTER_MASK;
     }

@@ -236,11 +236,11 @@ int bgtq_step_prepare_ring(const BgtqHeadDesc* desc, const float* rot_k, const f
 #define BGTQ_DEC_NARROW 32        /* 16 tokens per warp instead of 32: shorter chains while a CTA gets at most 256 tokens
                                    * (n_batch * n_kv * tokens <= 256 * SMs), less work per load beyond; same results up to
                                    * the order of sums */
-#define BGTQ_DEC_CLUSTER_SHIFT 8  /* n << 8, n = 1, 2, 4, 8 or 16, with BGTQ_DEC_NARROW: bgtq_layer_step and bgtq_attend decode
+#define BGTQ_DEC_CLUSTER_SHIFT 8  /* n << 8, n = 2, 4 or 8, with BGTQ_DEC_NARROW: bgtq_layer_step and bgtq_attend decode
                                    * with a cluster of n CTAs per (batch, KV head) pair, which merge their shares and write the
                                    * output rows themselves: no merge launch.  The plan's specialised kernel is the one for that;
                                    * bgtq_decode with such a plan takes the general kernel.  bgtq_decode_plan drops the bits
-                                   * where the form does not fit shared memory. */
+                                   * for any other n and where the form does not fit shared memory. */
 #define BGTQ_DEC_CLUSTER_MASK 0x1F00
 
 /* Opaque launch plan of the decode kernel for the KV heads of one layer (host

@@ -242,3 +242,12 @@ def test_specialised_kernel_source_compiles_for_sm100a(case, flags):
     assert " error" not in log.value.decode(errors="replace")
     plan = Plan.from_buffer_copy(bytes(raw.opaque)[:C.sizeof(Plan)])
     assert L.bgtq_decode_plan_specialize(None, 1, None, 0) == -1
+
+
+def test_cluster_sizes():
+    """The merging form comes in clusters of 2, 4 and 8; any other request is a plan of the split form."""
+    descs = (_lib.HeadDesc * 1)()
+    _fill_desc(descs[0], *tables_for("a3_1to8", 0))
+    for n in range(32):
+        plan, _ = _plan_and_image(descs, 1, _lib.DEC_NARROW | n << _lib.DEC_CLUSTER_SHIFT)
+        assert plan.flags == _lib.DEC_NARROW | (n << _lib.DEC_CLUSTER_SHIFT if n in (2, 4, 8) else 0)
