@@ -131,6 +131,7 @@ _SIGNATURES = {
                                                _vp, _i64, _i64, _i64, _vp, _i64, _i64, _i64,
                                                _i32, _i32, _i32, _i32, _i32, _i32, _f32,
                                                _vp, _vp, _i64, _i64, _vp, _vp, _vp]),
+    "bgtq_buffer_attn_ctas": (C.c_int, [_i32] * 5),
     "bgtq_buffer_attn_pos": (C.c_int, [_vp, _i64, _i64, _vp, _vp, _i64, _i64, _i32, _i32, _i32, _i32, _i32,
                                    _i32, _i32, _i32, _f32,
                                    _vp, _vp, _vp, _vp]),

@@ -563,6 +563,20 @@ __global__ void __launch_bounds__(kBufThreads) buffer_attn_group_kernel(const __
     }
 }
 
+// The form of a buffer attention over up to n_tok tokens: one CTA per KV head whose query heads share the staged rows
+// (groups of 2, 4 and 8, while the rows fit), else one per query head.  (Groups of 3 and 7 staged too, in front of a decode
+// in clusters: one sequence of 4 KV heads x 7 at 105 tokens went from 14 to 17.5 us per layer, 16 sequences of 8 x 3 from 59.5 to 53.)
+struct BufferShape { bool grouped; int sc_cap, cap_rows; size_t smem; };
+BufferShape buffer_shape(int n_rep, int n_tok, int sink_cap, int ring_size) {
+    BufferShape S;
+    S.sc_cap = (n_tok + 3) & ~3;       // keeps the query block 16-byte aligned
+    S.cap_rows = sink_cap + (ring_size > 0 ? ring_size : 1);      // buffer slots a live token can sit in
+    const size_t scores = (size_t)(S.sc_cap + 16 + 4 * kHD) * sizeof(float), staged = 2 * (size_t)S.cap_rows * kBufRowLd + n_rep * scores;
+    S.grouped = (n_rep == 2 || n_rep == 4 || n_rep == 8) && n_tok > 0 && staged <= 200 * 1024;
+    S.smem = S.grouped ? staged : scores;
+    return S;
+}
+
 // The combine variant for a launch of n_q x n_batch rows: one row per CTA with its rotation entries in registers
 // while all CTAs fit the GPU at once; beyond that four rows of one KV head per CTA where the head grouping
 // allows it, else the lean one-row variant.
@@ -651,6 +665,12 @@ extern "C" __attribute__((visibility("default"))) int bgtq_combine_ranks(const f
                ? BGTQ_OK : BGTQ_E_LAUNCH;
 }
 
+extern "C" __attribute__((visibility("default"))) int bgtq_buffer_attn_ctas(int32_t sink_cap, int32_t ring_size, int32_t n_batch, int32_t n_q,
+                                                                            int32_t n_kv) {
+    if (sink_cap < 0 || ring_size < 0 || n_batch < 1 || n_kv < 1 || n_q < n_kv || n_q % n_kv) return BGTQ_E_BADARG;
+    return n_batch * (buffer_shape(n_q / n_kv, sink_cap + ring_size, sink_cap, ring_size).grouped ? n_kv : n_q);
+}
+
 extern "C" int bgtq_buffer_attn_pos(const void* q, int64_t q_sb, int64_t q_sh, const void* k_buf, const void* v_buf,
                                 int64_t kb_sb, int64_t kb_sh, int32_t n_sink_tokens, int32_t n_ring_tokens,
                                 int32_t sink_cap, int32_t ring_first, int32_t ring_size, int32_t n_batch, int32_t n_q,
@@ -682,27 +702,24 @@ extern "C" __attribute__((visibility("default"))) int bgtq_buffer_attn_pos(const
     if (n_buf_tokens > 0 && ((reinterpret_cast<uintptr_t>(k_buf) & 15u) || (reinterpret_cast<uintptr_t>(v_buf) & 15u) ||
                              (kb_sb & 7) || (kb_sh & 7) || (reinterpret_cast<uintptr_t>(buf_o) & 7u)))
         return BGTQ_E_ALIGN;
-    const int sc_cap = (n_buf_tokens + 3) & ~3;       // keeps the query block 16-byte aligned
     const int n_rep = n_q / n_kv;
-    const int cap_rows = sink_cap + (ring_size > 0 ? ring_size : 1);      // buffer slots a live token can sit in
-    const size_t smem_group = 2 * (size_t)cap_rows * kBufRowLd + (size_t)n_rep * (sc_cap + 16 + 4 * kHD) * sizeof(float);
-    if ((n_rep == 2 || n_rep == 4 || n_rep == 8) && n_buf_tokens > 0 && smem_group <= 200 * 1024) {
-        // grouped heads with the rows staged in shared memory: one CTA per KV head.  (Groups of 3 and 7 so, in front of a decode in
-        // clusters: one sequence of 4 KV heads x 7 at 105 tokens went from 14 to 17.5 us per layer, 16 sequences of 8 x 3 from 59.5 to 53.)
+    const BufferShape S = buffer_shape(n_rep, n_buf_tokens, sink_cap, ring_size);
+    const int sc_cap = S.sc_cap, cap_rows = S.cap_rows;
+    if (S.grouped) {
+        // grouped heads with the rows staged in shared memory: one CTA per KV head
         auto kern = n_rep == 2 ? buffer_attn_group_kernel<2> : n_rep == 4 ? buffer_attn_group_kernel<4> : buffer_attn_group_kernel<8>;
         // the attribute is per device: set it on every launch (cheap, and legal under stream capture)
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess) {
             cudaGetLastError();
             return BGTQ_E_LAUNCH;
         }
-        return launch_kernel(kern, dim3(n_kv, n_batch), dim3(kBufThreads), smem_group, static_cast<cudaStream_t>(stream), true,
+        return launch_kernel(kern, dim3(n_kv, n_batch), dim3(kBufThreads), S.smem, static_cast<cudaStream_t>(stream), true,
                              static_cast<const __half*>(q), q_sb, q_sh, static_cast<const __half*>(k_buf),
                              static_cast<const __half*>(v_buf), kb_sb, kb_sh, n_sink_tokens, n_ring_tokens, sink_cap, ring_first,
                              ring_size > 0 ? ring_size : 1, n_q, scale, buf_o, buf_lse, pos_dev, sc_cap, cap_rows) == cudaSuccess
                    ? BGTQ_OK : BGTQ_E_LAUNCH;
     }
-    const size_t smem = (size_t)(sc_cap + 16 + 4 * kHD) * sizeof(float);
-    return launch_kernel(buffer_attn_kernel, dim3(n_q, n_batch), dim3(kBufThreads), smem, static_cast<cudaStream_t>(stream), true,
+    return launch_kernel(buffer_attn_kernel, dim3(n_q, n_batch), dim3(kBufThreads), S.smem, static_cast<cudaStream_t>(stream), true,
                          static_cast<const __half*>(q), q_sb, q_sh, static_cast<const __half*>(k_buf), static_cast<const __half*>(v_buf),
                          kb_sb, kb_sh, n_sink_tokens, n_ring_tokens, sink_cap, ring_first, ring_size > 0 ? ring_size : 1, n_q, n_kv, scale,
                          buf_o, buf_lse, pos_dev, sc_cap) == cudaSuccess ? BGTQ_OK : BGTQ_E_LAUNCH;

@@ -163,13 +163,10 @@ class BlockGTQKVManager:
         if dev.type == "cuda":      # by capacity: one kernel for the cache's whole life, captured graphs included
             self._dec_flags |= tile_flags(self.B, self.n_kv, self.max_T, dev)
             if merging:
-                # (with fp16 regions where their attention, in front of the decode then, leaves SMs to it: a decode's CTA takes all
-                # registers of one.  A layer of 8 sequences x 4 KV heads, window 128, 4 query heads per KV head, 32 CTAs: 24.5 and
-                # 21.2 us; 4 x 8 x 3, 96: 29.3 and 20.5; window 600, 8 x 4 x 1, 32: 30.8 and 28.8, x 4, 128: 38 and 39.7, x 7, 224:
-                # 50 and 71.6, window 128: 25.7 and 26.7)
-                n_rep, cap = self.n_q // self.n_kv, self.n_sink + self.recent_window + 1
-                grouped = n_rep in (2, 4, 8) and 2 * 272 * cap + n_rep * 4 * (cap + 531) <= 200 * 1024
-                if not self._buffered or 3 * self.B * (self.n_kv if grouped else self.n_q) <= 2 * torch.cuda.get_device_properties(dev).multi_processor_count:
+                # With fp16 regions their attention runs in front of the decode, whose CTAs take all registers of an SM each: the
+                # merging form pays where that launch leaves a third of the SMs to it.
+                L, sms = _lib.lib(), torch.cuda.get_device_properties(dev).multi_processor_count
+                if not self._buffered or 3 * L.bgtq_buffer_attn_ctas(self.n_sink, self.recent_window + 1, self.B, self.n_q, self.n_kv) <= 2 * sms:
                     self._cluster_flags = cluster_flags(self.B, self.n_kv, self.max_T, dev)
         self._prepare_decode_plans()
         self._q_rot = torch.empty(self.B, self.n_q, self.hd, dtype=torch.float16, device=dev)

@@ -399,6 +399,9 @@ int bgtq_buffer_attn_pos(const void* q, int64_t q_sb, int64_t q_sh,
                      int32_t n_batch, int32_t n_q, int32_t n_kv,
                      float scale, float* buf_o, float* buf_lse, const int32_t* pos_dev, void* stream);
 
+/* CTAs of that launch with a device-side position: what it leaves of the SMs to a launch beside it. */
+int bgtq_buffer_attn_ctas(int32_t sink_cap, int32_t ring_size, int32_t n_batch, int32_t n_q, int32_t n_kv);
+
 /* Merge split partials, undo V's rotation, fold in the fp16-buffer partial.
  *
  * Replaces _split_t_merge_kernel (blockgtq/kernels/fused_packed_attention.py:59-103),

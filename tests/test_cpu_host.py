@@ -328,3 +328,17 @@ def test_decode_plan_option_setters_check_their_arguments():
     assert L.bgtq_decode_plan_set_partition(C.byref(raw), None) == 0 and not view().partition
     assert L.bgtq_decode_grid_size(8, 2, 64) == 148 and L.bgtq_decode_grid_size(1, 2, 4) == 8
     assert L.bgtq_decode_grid_size(0, 2, 4) == -1
+
+
+def test_buffer_attention_ctas():
+    """One CTA per KV head for the groups whose rows are staged and fit, else one per query head."""
+    from blockgtq_b200 import _lib
+    ctas = _lib.lib().bgtq_buffer_attn_ctas
+    for n_rep in range(1, 9):
+        staged = [ctas(4, w + 1, 3, 2 * n_rep, 2) == 3 * 2 for w in range(0, 2000, 7)]
+        if n_rep in (2, 4, 8):          # while the key and value rows (272 bytes each) fit 200 KB
+            last = max(i for i, x in enumerate(staged) if x)
+            assert all(staged[:last + 1]) and 2 * 272 * (7 * last + 5) <= 200 * 1024 < 2 * 272 * (7 * (last + 1) + 5) + n_rep * 4 * (7 * (last + 1) + 540)
+        assert n_rep in (1, 2, 4, 8) or not any(staged)
+        assert all(ctas(4, w + 1, 3, 2 * n_rep, 2) == 6 * n_rep for w in (500, 1999))
+    assert ctas(4, 5, 0, 4, 2) == ctas(4, 5, 1, 3, 2) == ctas(-1, 5, 1, 4, 2) == -1
