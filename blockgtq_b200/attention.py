@@ -9,8 +9,8 @@ CUDA decode + combine kernels.  Callers that hold a whole layer should use
 """
 from __future__ import annotations
 
-import ctypes as C
 import math
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import torch
@@ -128,12 +128,41 @@ def fused_blockgtq_decode_attention(
     if k_norms.dtype != torch.float16:
         k_norms = k_norms.to(torch.float16)
     lt = _layer_for(segments, codebook_flat, v_lut, vb_codebook, n_kv, q.device)
-    flags = (_lib.DEC_K_MIXED if k_nibble else 0) | (_lib.DEC_V_NIBBLE if v_nibble else 0) | \
-        (cluster_flags(B, n_kv, T, q.device, grows=True) or tile_flags(B, n_kv, T, q.device))
+    flags = (_lib.DEC_K_MIXED if k_nibble else 0) | (_lib.DEC_V_NIBBLE if v_nibble else 0)
+    form = k_packed.stride(2) + v_codes.stride(2) <= _MERGING_ROW and cluster_flags(B, n_kv, T, q.device, grows=True) or \
+        tile_flags(B, n_kv, T, q.device)
+    if form and flags | form | _lib.DEC_PROGRAMMATIC not in lt._plans:
+        form = _make_plans(lt, flags, form, tile_flags(B, n_kv, T, q.device), cluster_flags(B, n_kv, 1, q.device, grows=True))
+    flags |= form
     out, _o32, lse = attend(lt, q, k_packed, k_norms, v_codes, v_norms, 0, T, rotate=False,
                             n_splits=max(1, int(t_splits)), scale=scale, flags=flags, v_rot=_rotation(v_rotation, n_kv),
                             want_lse=return_lse)
     return (out, lse) if return_lse else out
+
+
+_MERGING_ROW = 192          # bytes a token's packed K and V rows may be apart: the widest there are (padded ones leave the shares no room)
+
+
+def _capturing(lt) -> bool:
+    return lt.device.type == "cuda" and torch.cuda.is_current_stream_capturing()
+
+
+def _make_plans(lt, flags, form, split, merging):
+    """A short context's decode has two forms, each a kernel that takes a second or two to compile: the one that merges its shares
+    in the launch, and the split one that takes over as the context grows.  Both are made when the first call needs either,
+    side by side, so that a later call, or its capture, finds them.  Returns the form for this call: ``form``, or under a capture
+    that it was not made before, the split one."""
+    if _capturing(lt):
+        return split
+    stream = torch.cuda.current_stream(lt.device) if lt.device.type == "cuda" else None
+
+    def make(f):
+        with torch.cuda.stream(stream):         # (the caller's: what the plan's image lies in returns to that stream's pool)
+            lt.plan(flags | f | _lib.DEC_PROGRAMMATIC)
+
+    with ThreadPoolExecutor(max_workers=2) as ex:
+        list(ex.map(make, {split, merging or split}))
+    return form
 
 
 def _rotation(v_rotation, n_kv):
