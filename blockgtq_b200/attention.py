@@ -127,12 +127,14 @@ def fused_blockgtq_decode_attention(
         v_norms = v_norms[..., 0]
     if k_norms.dtype != torch.float16:
         k_norms = k_norms.to(torch.float16)
-    lt = _layer_for(segments, codebook_flat, v_lut, vb_codebook, n_kv, q.device)
+    dev, stored = q.device, 4 if v_nibble else vb_codebook
+    lt = _layer_for(segments, codebook_flat, v_lut, vb_codebook, n_kv, dev)
     flags = (_lib.DEC_K_MIXED if k_nibble else 0) | (_lib.DEC_V_NIBBLE if v_nibble else 0)
-    form = k_packed.stride(2) + v_codes.stride(2) <= _MERGING_ROW and cluster_flags(B, n_kv, T, q.device, grows=True) or \
-        tile_flags(B, n_kv, T, q.device)
+    form = cluster_flags(B, n_kv, T, dev, n_q // n_kv, stored, True)
+    if not form or not (k_packed.is_contiguous() and v_codes.is_contiguous()) and k_packed.stride(-2) + v_codes.stride(-2) > _MERGING_ROW:
+        form = tile_flags(B, n_kv, T, dev)
     if form and flags | form | _lib.DEC_PROGRAMMATIC not in lt._plans:
-        form = _make_plans(lt, flags, form, tile_flags(B, n_kv, T, q.device), cluster_flags(B, n_kv, 1, q.device, grows=True))
+        form = _make_plans(lt, flags, form, tile_flags(B, n_kv, T, dev), cluster_flags(B, n_kv, 1, dev, n_q // n_kv, stored, True))
     flags |= form
     out, _o32, lse = attend(lt, q, k_packed, k_norms, v_codes, v_norms, 0, T, rotate=False,
                             n_splits=max(1, int(t_splits)), scale=scale, flags=flags, v_rot=_rotation(v_rotation, n_kv),

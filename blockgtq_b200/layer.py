@@ -426,7 +426,8 @@ def attend(layer, q, k_packed, k_norms, v_packed, v_norms, t_begin, t_end, *, ro
     """Query rotation (``rotate``: q is in the original basis), split-KV decode over rows [t_begin, t_end) and combine
     in one library call.  q (B, n_q, [1,] 128) -> (out fp16 of q's shape, f32 copy (B, n_q, 128) | None, LSE | None)."""
     plan, _image, merged = layer.plan_entry(flags | _lib.DEC_PROGRAMMATIC)
-    plan, desc, rot_k = C.addressof(plan), layer.desc_dev.data_ptr(), layer.rot_k.data_ptr() if rotate else None
+    plan = C.addressof(plan)
+    desc, rot_k = (layer.desc_dev.data_ptr(), layer.rot_k.data_ptr()) if rotate else (None, None)      # (of the query rotation)
     n_splits = 0 if n_splits is None else n_splits or -1       # (the library's choice; 0 is refused like -1)
     scale = _SCALE if scale is None else scale
     # (names of their own: the parameters may be the only references to these tensors, and the library takes addresses)
@@ -480,24 +481,22 @@ def merges(layer, flags: int) -> bool:
     return layer.plan_entry(flags)[2]
 
 
-def cluster_flags(n_batch: int, n_kv: int, n_tokens: int, device, grows: bool = False) -> int:
+def cluster_flags(n_batch: int, n_kv: int, n_tokens: int, device, gqa: int, v_bits: int, grows: bool = False) -> int:
     """Plan flags of the form that merges a pair's shares inside the decode launch (``DEC_CLUSTER_SHIFT``; the narrow tile), for
     layer steps and attentions over up to ``n_tokens`` rows, or 0 where the decode over all SMs and its merge launch are faster.
+    ``v_bits``: as stored (nibbles: 4).
 
-    A cluster of C CTAs per (batch, KV head) pair saves the second launch and the partials' way through memory, about 3 us.
-    Against that, pairs * C CTAs share the work instead of one per SM: it is taken while that costs a CTA at most 330 tokens
-    (9 ns each) more than an SM's even share.  C is the largest of 8, 4 and 2 whose clusters all run at once: 14 clusters
-    of 8, 32 of 4 and 72 of 2 do (16 of 8 and 36 of 4 take two waves); and smaller while a CTA then has at most 8 warps' tokens,
-    or 16 where the CTAs would take more than half of the SMs, which the next launch's CTAs start on (500 tokens of 8 pairs 10.2, 8.9
-    and 9.1 us with 2, 4 and 8, of 32 pairs 10.1 and 11.6 with 2 and 4).  ``grows``: the length goes up from call to call; one C
-    for all of them, as each is a kernel of its own.
-    A captured layer (K3V3, 4 query heads per KV head but where noted), one sequence of 8 KV heads, in two launches and so: 100 tokens
-    11.1 and 8.7 us, 500: 12.1 and 8.9, 2000: 12.2 and 10.4, 4000: 12.7 and 12.9, 6000: 14.0 and 15.0 (not taken); 2 KV heads x 8 at 500
-    tokens 10.0 and 8.7; 4 sequences x 8 heads x 3: 500: 14.7 and 10.1, 4099: 22.1 and 20.0, 8500: 31.9 and 30.2 (x 4); 8 sequences: 500: 16.1 and
-    13.1, 3000: 27.7 and 24.1, 4300: 32.0 and 30.9."""
+    A cluster of C CTAs per (batch, KV head) pair saves the second launch and the partials' way through memory, 2 to 4 us (one
+    sequence of 8 KV heads, K3V3, 500 tokens: 12.6 -> 10.9 us per layer; 4 sequences at 4000 tokens: 23.1 -> 19.8).  How far that
+    carries: see ``_merging_limit``.  C is the largest of 8, 4 and 2 whose clusters all run at once: 14 clusters of 8, 32 of 4 and
+    72 of 2 do (16 of 8 and 36 of 4 take two waves); and smaller while a CTA then has at most 8 warps' tokens, or 16 where the CTAs
+    would take more than half of the SMs, which the next launch's CTAs start on.  ``grows``: the length goes up from call to call;
+    one C for all of them, as each is a kernel of its own."""
     pairs = n_batch * n_kv
+    if pairs < 1 or v_bits not in _TOKEN_NS:        # (a call to complain about)
+        return 0
     sms = _sm_count(device.index if device.index is not None else torch.cuda.current_device())
-    c, most = _largest_cluster(pairs, sms)
+    c, most = _merging_limit(pairs, sms, gqa > 4, v_bits)
     if n_tokens > most:
         return 0
     while not grows and c > 2 and 2 * n_tokens <= (256 if 2 * pairs * c > sms else 128) * c:
@@ -505,12 +504,31 @@ def cluster_flags(n_batch: int, n_kv: int, n_tokens: int, device, grows: bool = 
     return _lib.DEC_NARROW | c << _lib.DEC_CLUSTER_SHIFT
 
 
+_TOKEN_NS = {1: (8.2, 6.3), 2: (8.2, 6.3), 3: (9.4, 7.9), 4: (11.9, 11.5)}      # of a CTA, narrow and wide tile, by V's bits
+
+
 @functools.lru_cache(maxsize=1024)
-def _largest_cluster(pairs: int, sms: int):
-    """(C, the most tokens it is taken for): tokens / C - pairs * tokens / sms <= 330."""
+def _merging_limit(pairs: int, sms: int, wide_groups: bool, v_bits: int):
+    """(C, the most tokens its clusters are taken for).  A CTA of a cluster gets tokens / C of them instead of an SM's even share,
+    in the narrow tile, where the split form takes the wide one past 256 tokens per SM (see ``tile_flags``).  Limits on both,
+    from layers of 1 to 72 pairs, 1 to 8 query heads per KV head and every V width timed both ways:
+      * about 300 tokens more than the even share (3 us; with wider V codes fewer), 110 fewer where eight CTAs exchange the rows of
+        more than four query heads; up to 60 more with few pairs, whose rows leave many partials to a merge launch;
+      * beside the wide tile, 3.8 us more time (nibbles, whose wide tile gains little: 4.6).  Without this limit 72 pairs
+        lost 17 % (K3V3, 24000 tokens: 106.9 -> 124.7 us) and 24 % (K2V2); as it is, 32 pairs go from 24.1 to 22.0 us at 5000
+        tokens and take the split form from 6000 on, where the two are even."""
+    narrow, wide = _TOKEN_NS[v_bits]
     for c, most in ((8, 14), (4, 32), (2, 72)):
         if pairs <= most * sms // 148:
-            return c, 330 * sms * c // (sms - pairs * c) if pairs * c < sms else 1 << 30
+            even = min(pairs / sms, 1 / c - 1e-6)
+            apart = {1: 330, 2: 330, 3: 280, 4: 270}[v_bits] - (110 if c == 8 and wide_groups else 0)
+            if pairs <= 4:
+                apart = min(apart + 60, 330)
+            limit = apart / (1 / c - even)
+            slower = narrow / c - wide * even           # ns per token of the context
+            if slower > 0:
+                limit = min(limit, max(256 / even, (4600 if v_bits == 4 else 3800) / slower))
+            return c, int(limit)
     return 0, -1
 
 

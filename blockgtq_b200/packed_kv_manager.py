@@ -167,7 +167,8 @@ class BlockGTQKVManager:
                 # merging form pays where that launch leaves a third of the SMs to it.
                 L, sms = _lib.lib(), torch.cuda.get_device_properties(dev).multi_processor_count
                 if not self._buffered or 3 * L.bgtq_buffer_attn_ctas(self.n_sink, self.recent_window + 1, self.B, self.n_q, self.n_kv) <= 2 * sms:
-                    self._cluster_flags = cluster_flags(self.B, self.n_kv, self.max_T, dev)
+                    self._cluster_flags = cluster_flags(self.B, self.n_kv, self.max_T, dev, gqa=self.n_q // self.n_kv,
+                                                        v_bits=4 if self.v_nibble else self.v_bits)
         self._prepare_decode_plans()
         self._q_rot = torch.empty(self.B, self.n_q, self.hd, dtype=torch.float16, device=dev)
         self._part_o = torch.empty(self.B, self.n_q, self._n_splits, self.hd, dtype=torch.float32, device=dev)
