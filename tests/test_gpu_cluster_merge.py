@@ -2,6 +2,8 @@
 
 Both round p * norm to fp16 relative to running maxima that other groups of tokens give: each weight may differ by 2^-11 of itself
 on either side, so a row by 2^-10 of its largest value; the log-sum-exp sums fp32 weights."""
+import random
+
 import pytest
 import torch
 
@@ -207,3 +209,106 @@ def test_the_other_partial_beside_an_empty_range():
             assert torch.equal(g.isnan(), w.isnan()) and torch.equal(g.isinf(), w.isinf())
             if hi == 0:
                 assert torch.equal(g.nan_to_num(), w.nan_to_num())
+
+
+def _regions(mgr, n_tok):
+    """Sink and packed tokens of a step's attention (a token that leaves the window is packed behind it)."""
+    from oracle import bgtq_oracle as O
+    return O.three_region_plan(n_tok - 1, mgr.n_sink, mgr.recent_window)[:2] if mgr._buffered else (0, n_tok)
+
+
+def _step_reference(mgr, q, ks, vs, b, hq, n_tok):
+    """A query head's attention in 64 bits over the dequantised packed rows and the fp16 rows: weights and values of all tokens in
+    order (packed values in V's rotated space), and V's rotation."""
+    import numpy as np
+    from helpers import oracle_meta
+    from oracle import bgtq_oracle as O
+    n_sink, n_packed = _regions(mgr, n_tok)
+    h = hq // (mgr.n_q // mgr.n_kv)
+    qz = mgr.quantizers[0][h]
+    meta = oracle_meta(qz._tables, qz._v_tables)
+    q64, k, v = (x.cpu().numpy().astype(np.float64) for x in (q[b, hq, 0], ks[b, h, :n_tok], vs[b, h, :n_tok]))
+    lo, hi = n_sink, n_sink + n_packed
+    row = lambda t: t[0, b, h, :n_packed].cpu().numpy()
+    s = k @ q64
+    s[lo:hi] = O.dequant_k(row(mgr._k_packed)[:, :qz._total_packed_bytes], row(mgr._k_norms), meta) @ \
+        O.rotate_q(q[b, hq].cpu().numpy(), meta)[0].astype(np.float64)
+    v[lo:hi] = O.dequant_v(row(mgr._v_packed), row(mgr._v_norms), meta, f16_product=False)
+    return s * mgr.scale, v, slice(lo, hi), meta["v_rot"].astype(np.float64)
+
+
+def _attend_reference(s, v, packed, rot):
+    """Output, and the size of what rounds: each packed weight to fp16 relative to two running maxima, 2^-10 of itself, which the
+    rotation may gather in one dim."""
+    import numpy as np
+    w = np.exp(s - s.max())
+    w /= w.sum()
+    p = w[packed] @ v[packed]
+    rest = np.concatenate([w[:packed.start], w[packed.stop:]]) @ np.concatenate([v[:packed.start], v[packed.stop:]])
+    return p @ rot + rest, np.linalg.norm(w[packed] @ np.abs(v[packed]))
+
+
+@pytest.mark.parametrize("batch,n_kv,gqa,start,cap,sink,window", [
+    (1, 8, 4, 0, 40, 0, 0), (2, 2, 8, 254, 600, 0, 0), (4, 8, 3, 1020, 1030, 0, 0), (1, 8, 4, 3, 40, 2, 4), (2, 4, 4, 700, 720, 4, 128), (9, 8, 1, 260, 300, 0, 9)])
+def test_layer_steps_weigh_single_rows(batch, n_kv, gqa, start, cap, sink, window):
+    """Queries that single rows decide: the one just appended, the first and last of a CTA's share, the oldest, one of the fp16 window,
+    and two such rows against each other.  Without the row, or with its weight a few percent off, the output is off by many
+    times the bound; the reference says so itself."""
+    import numpy as np
+    from blockgtq_b200 import _lib
+    gen = torch.Generator().manual_seed(start + 1)
+    mgr = _manager(batch, n_kv, gqa, cap, gen, n_sink=sink, recent_window=window)
+    mgr._ensure_storage()
+    c = mgr._cluster_flags >> _lib.DEC_CLUSTER_SHIFT
+    assert c
+    ks, vs = (torch.randn(batch, n_kv, cap, 128, generator=gen).half() for _ in range(2))
+    if start:
+        mgr.init_from_cache([(ks[:, :, :start].to(DEV), vs[:, :, :start].to(DEV))])
+    graph, single, shared, rng = None, 0, 0, random.Random(start)
+    for step in range(6):
+        n_tok = start + step + 1
+        packed0, n_packed = _regions(mgr, n_tok)
+        tiles = (n_packed + 15) // 16
+        cuts = [16 * (tiles * r // c) for r in range(1, c)]
+        rows = [n_tok - 1] + ([packed0 + n_packed - 1, packed0] if n_packed else []) + ([n_tok - window, n_tok - window // 2 - 1] if window else [])
+        rows += [packed0 + t for cut in cuts for t in (cut - 1, cut) if 0 <= t < n_packed]
+        rows = sorted(set(rows))
+        q = torch.empty(batch, n_kv * gqa, 1, 128, dtype=torch.float16)
+        decisive = {}
+        for b in range(batch):
+            for hq in range(n_kv * gqa):
+                pick = rng.sample(rows, min(len(rows), rng.randint(1, 2)))
+                decisive[b, hq] = pick
+                q[b, hq, 0] = sum(14.0 * 128 ** 0.5 * ks[b, hq // gqa, t].float() / ks[b, hq // gqa, t].float().square().sum() for t in pick).half()
+        args = [q.to(DEV)] + [x[:, :, n_tok - 1:n_tok].to(DEV) for x in (ks, vs)]
+        if step < 3:
+            got = mgr.append_and_attend(0, *args)
+        else:
+            for dst, src in zip(mgr.static_inputs(0), args):
+                dst.copy_(src)
+            if graph is None:
+                mgr._sync_pos()
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph):
+                    mgr.layer_step(0)
+            graph.replay()
+            got = mgr.static_outputs()[0].unsqueeze(2)
+        mgr.increment_seq_len()
+        mgr.check_status()
+        got = got.double().cpu().numpy()
+        for i, ((b, hq), pick) in enumerate(decisive.items()):
+            if len(decisive) > 40 and (i + step) % (len(decisive) // 40):
+                continue
+            s, v, packed, rot = _step_reference(mgr, args[0], ks, vs, b, hq, n_tok)
+            want, size = _attend_reference(s, v, packed, rot)
+            # (2^-10 again: a score is off by as much where the library rounds an element of the rotated query the other way)
+            bound = 2.0 ** -9 * size + 2.0 ** -10 * np.abs(want).max()
+            assert np.abs(got[b, hq, 0] - want).max() <= bound, (step, b, hq, pick)
+            if n_tok > 1:
+                def off(row, by):
+                    moved = s.copy()
+                    moved[row] += by
+                    return np.abs(_attend_reference(moved, v, packed, rot)[0] - want).max() / bound
+                single += sum(off(t, -np.inf) > 10 for t in pick)
+                shared += len(pick) == 2 and off(pick[0], 0.1) > 2
+    assert single >= 20 and shared >= 5
