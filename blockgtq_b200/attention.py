@@ -16,7 +16,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .layer import HD, DecodePlans, attend, cluster_flags, make_decode_plan, tile_flags
+from .layer import HD, DecodePlans, attend, growing_forms, make_decode_plan
 
 _tables = {}          # tables by contents
 _cache = {}           # the same by the full description of the tensors they were made of, with these tensors
@@ -130,11 +130,11 @@ def fused_blockgtq_decode_attention(
     dev, stored = q.device, 4 if v_nibble else vb_codebook
     lt = _layer_for(segments, codebook_flat, v_lut, vb_codebook, n_kv, dev)
     flags = (_lib.DEC_K_MIXED if k_nibble else 0) | (_lib.DEC_V_NIBBLE if v_nibble else 0)
-    form = cluster_flags(B, n_kv, T, dev, n_q // n_kv, stored, True)
-    if not form or not (k_packed.is_contiguous() and v_codes.is_contiguous()) and k_packed.stride(-2) + v_codes.stride(-2) > _MERGING_ROW:
-        form = tile_flags(B, n_kv, T, dev)
+    form, split, short = growing_forms(B, n_kv, T, dev.index, n_q // n_kv, stored)
+    if form != split and not (k_packed.is_contiguous() and v_codes.is_contiguous()) and k_packed.stride(-2) + v_codes.stride(-2) > _MERGING_ROW:
+        form = split
     if form and flags | form | _lib.DEC_PROGRAMMATIC not in lt._plans:
-        form = _make_plans(lt, flags, form, tile_flags(B, n_kv, T, dev), cluster_flags(B, n_kv, 1, dev, n_q // n_kv, stored, True))
+        form = _make_plans(lt, flags, form, split, short)
     flags |= form
     out, _o32, lse = attend(lt, q, k_packed, k_norms, v_codes, v_norms, 0, T, rotate=False,
                             n_splits=max(1, int(t_splits)), scale=scale, flags=flags, v_rot=_rotation(v_rotation, n_kv),

@@ -12,13 +12,8 @@
 //     values share an instruction where they can (f32x2), and whole 32-bit words of the packed row go to a staging image of the
 //     tile that leaves as coalesced words.
 // Bound: instruction issue and its latencies with 16 warps per SM (all registers and shared memory are taken): 1 048 576 K and
-// as many V rows take 374 us (K rows alone 219, V rows 162), where the bytes alone would take 100.  K rows cost what V's do
-// not: the move into packed order and a norm per group.  Before the list, the norms by whole segments and the moves in pairs
-// K rows took 286 us (both 451): every thread worked out each task's control for itself, a third of the loop.  A launch of
-// one tile per CTA (777 tokens of 8 heads) takes 8.5 us, and took 10.8 with half of the warps idle.  The form before that
-// gave a quad of lanes four rows and four columns each, loaded three tables per element and passed the codes through shared
-// memory to a packing pass: 753 us.  Tried and slower: rolled loops (smaller code, less overlap of the table lookups: 589 us);
-// squares of converted fp16 values instead of mixed-precision multiply-adds (K 277 -> 287, V 164 -> 168).
+// as many V rows take 374 us (451 with every thread working out each task's control; K rows alone 219 and 286, V rows 162 and
+// 164), where the bytes alone would take 100; 777 tokens of 8 heads, a tile per CTA, 8.5 us (10.8 with half of the warps on it).
 // The sums that decide a code (group norms, products) keep the order they had: the packed bytes are bit for bit the same.
 // Every wait is bounded; tensor memory is released on every path out of the kernel.
 #include <cstddef>
@@ -314,10 +309,8 @@ __device__ __forceinline__ float square2(float acc, uint32_t w) {
 
 // Columns [first, first + 8 N) of a V row, of one thread's tensor-memory lane -> its bytes in the staged row; returns the sum
 // of the squared levels (added up quarter by quarter).  A code counts the boundaries below a value: the upper halvings of
-// the search are compares with boundaries in registers, the last one (of 4 bits: two) looks its boundary up.  (With a table of
-// 256 bins for all but the last compare V rows alone take as long, K and V rows together 380 us instead of 374: its lookups
-// collide, three wavefronts each, and the other group's K tile shares the pipe.  Compares as saturated multiply-adds, off the
-// integer pipe: 182 us for V rows instead of 162.)
+// the search are compares with boundaries in registers, the last one (of 4 bits: two) looks its boundary up: few lookups, as the
+// other group's K tile shares their pipe (with a table of 256 bins K and V rows together take 380 us, so 374).
 template <int BITS, bool CODES, int N>
 __device__ __forceinline__ float e5_cols_v(E5Smem& S, uint32_t lane_base, int first, float r, uint32_t row_addr, uint8_t* codes) {
     const char* const vt = reinterpret_cast<const char*>(S.vtab);       // byte 4 c: boundary c, 64 + 4 c: level c
@@ -386,9 +379,7 @@ __device__ __forceinline__ float e5_cols_v(E5Smem& S, uint32_t lane_base, int fi
 
 // Sums of squares of segments first, first + step, .. of a K row: of its pairs 0, 2, .. and of its pairs 1, 3, .., each in
 // order.  A 16-byte load brings four pairs, even and odd positions into a sum of their own; what belongs to a neighbour in a
-// segment's first and last chunk counts as zero.  (Bits that said per chunk what to do with each pair took three times the
-// instructions: 4 x 32768 tokens x 8 heads of K rows alone 286 us with them and the tasks' control worked out by every
-// thread, 229 with this and E5Rec.)
+// segment's first and last chunk counts as zero.  (4 x 32768 tokens x 8 heads of K rows: with E5Rec 286 -> 229 us.)
 __device__ __forceinline__ void e5_norms_k(E5Smem& S, int grp, uint32_t tile, int row, int first, int step) {
     const uint32_t xr = tile + (uint32_t)row * 128u, sw = (uint32_t)(row & 7) << 4;
     const int n_seg = S.n_seg;
@@ -763,8 +754,6 @@ __device__ __forceinline__ bool e5_role(E5Smem& S, const EncParams& P, const int
                 }
                 continue;
             }
-            // (Sixteen lanes to a row's words, which spares finding a word's row, took K rows from 219 to 231 us: stores of half
-            // a line.)
             if (gt < head) dst0[gt] = a[gt];                                                   // (inside row 0: rb >= 4)
             if (gt < tail) {
                 const int x = total - tail + gt, r = row_of(x);

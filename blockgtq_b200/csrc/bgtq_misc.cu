@@ -564,8 +564,7 @@ __global__ void __launch_bounds__(kBufThreads) buffer_attn_group_kernel(const __
 }
 
 // The form of a buffer attention over up to n_tok tokens: one CTA per KV head whose query heads share the staged rows
-// (groups of 2, 4 and 8, while the rows fit), else one per query head.  (Groups of 3 and 7 staged too, in front of a decode
-// in clusters: one sequence of 4 KV heads x 7 at 105 tokens went from 14 to 17.5 us per layer, 16 sequences of 8 x 3 from 59.5 to 53.)
+// (groups of 2, 4 and 8, while the rows fit), else one per query head.
 struct BufferShape { bool grouped; int sc_cap, cap_rows; size_t smem; };
 BufferShape buffer_shape(int n_rep, int n_tok, int sink_cap, int ring_size) {
     BufferShape S;

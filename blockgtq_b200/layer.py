@@ -467,11 +467,9 @@ def _sm_count(index: int) -> int:
 def tile_flags(n_batch: int, n_kv: int, n_tokens: int, device) -> int:
     """``DEC_NARROW`` while every SM's share of the tokens fits one narrow tile (16 warps x 16 tokens): twice the warps
     work on half the chain each.  Beyond, the wide tile loads each query fragment for twice the tokens.  A captured layer of
-    one sequence with 8 KV heads (K3V3), wide and narrow tile, by tokens per SM: 27: 14.6 and 12.3 us, 64: 14.0 and 12.5,
-    128: 13.6 and 12.3, 192: 14.8 and 13.2, 224: 14.8 and 14.0, 240: 14.9 and 14.4, 250: 15.1 and 15.5, 254: 14.5 and 14.1,
-    past 256: 14.8 and 15.2, 320: 14.5 and 14.6, 512: 16.6 and 16.9 (K2V2 alike).  Eight sequences with 2 heads gain less (192: 14.6 and 14.5)
-    and lose 3 % at 250 to 320.  ``n_tokens`` is what the kernel is chosen for: a manager passes its capacity, so that one
-    kernel serves the cache's whole life; a short sequence in a large cache runs the wide tile."""
+    one sequence with 8 KV heads (K3V3), wide and narrow tile, by tokens per SM: 64: 14.0 and 12.5 us, 192: 14.8 and 13.2, 254: 14.5 and
+    14.1, past 256: 14.8 and 15.2, 512: 16.6 and 16.9 (K2V2 alike).  ``n_tokens`` is what the kernel is chosen for: a manager passes its
+    capacity, so that one kernel serves the cache's whole life; a short sequence in a large cache runs the wide tile."""
     index = device.index if device.index is not None else torch.cuda.current_device()
     return _lib.DEC_NARROW if n_batch * n_kv * n_tokens <= 256 * _sm_count(index) else 0
 
@@ -530,6 +528,16 @@ def _merging_limit(pairs: int, sms: int, wide_groups: bool, v_bits: int):
                 limit = min(limit, max(256 / even, (4600 if v_bits == 4 else 3800) / slower))
             return c, int(limit)
     return 0, -1
+
+
+@functools.lru_cache(maxsize=4096)
+def growing_forms(n_batch: int, n_kv: int, n_tokens: int, index, gqa: int, v_bits: int):
+    """Plan flags of a call on device ``index`` whose context grows from call to call: of its form, of the split form beside it and of
+    the merging form that its shape takes while it is short (0: none).  (A microsecond of arithmetic, asked for per head and layer.)"""
+    device = torch.device("cuda" if index is None else f"cuda:{index}")
+    split = tile_flags(n_batch, n_kv, n_tokens, device)
+    merging, short = (cluster_flags(n_batch, n_kv, n, device, gqa, v_bits, True) for n in (n_tokens, 1))
+    return merging or split, split, short
 
 
 _PREFILL_WORKSPACE = 2 << 30        # bytes of dequantised operand tiles per launch

@@ -156,8 +156,9 @@ class BlockGTQKVManager:
                     # the cache rows every decode launch of this manager reads (16-byte aligned slices: the
                     # token capacity is a multiple of 64)
                     lt.set_row_strides(self._max_k_packed_bytes, self._norm_row_groups(), vpb, 1, mixed=self.k_mixed)
-                    # In a layer step the launch before the decode is the append (one new row + the rotated
-                    # query), and the position is advanced between steps: the decode may start streaming early.
+                    # In a layer step only the append (one new row + the rotated query), and with fp16 regions their
+                    # attention, can still run when the decode starts, and the position is advanced between steps: the
+                    # decode may start streaming early.
                     if not os.environ.get("BGTQ_DEC_NO_EARLY_FETCH"):
                         lt.set_early_fetch(1)
         if dev.type == "cuda":      # by capacity: one kernel for the cache's whole life, captured graphs included

@@ -295,6 +295,8 @@ int bgtq_jit_set_nvrtc_path(const char* path_host);
  * launch whatever is in front of them: they let the decode start only when all work before them is complete.  The other
  * programmatic dependents listed above do not: behind bgtq_encode of rows that the decode reads, neither that encode nor
  * one of them may be the preceding launch.  bgtq_attend, which may well be called there, never fetches early.
+ * (Inside bgtq_layer_step a merging decode follows the attention over the fp16 regions: that launch starts behind the append's
+ * wait, and so does the decode, with nothing but the append itself still running.)
  * No counterpart in the reference. */
 int bgtq_decode_plan_set_early_fetch(BgtqDecodePlan* plan_host, int32_t fresh_rows);
 
@@ -425,7 +427,8 @@ int bgtq_combine(const float* part_o, const float* part_lse, int32_t n_splits,
 /* ---- whole steps ------------------------------------------------------------
  * The launches of one layer's decode step in one call: bgtq_step_prepare (its ring form when k_buf is set, its
  * rotary form when rope tables are passed) -> bgtq_decode over rows [0, *pos_dev + pos_add) -> with k_buf
- * bgtq_buffer_attn_pos -> bgtq_combine.  Replaces the body of append_and_attend
+ * bgtq_buffer_attn_pos -> bgtq_combine; with a plan whose decode merges its shares (bgtq_decode_plan_cluster)
+ * bgtq_step_prepare -> with k_buf bgtq_buffer_attn_pos -> that decode.  Replaces the body of append_and_attend
  * (blockgtq/packed_kv_manager.py:268-348) for a step whose arrays stay where they are: everything constant over
  * the steps is filled in once (host memory, plain values; the plan and every pointer must outlive its use), and
  * a call passes only the step's rows.  Arguments as for those functions.  No allocation, no synchronisation. */

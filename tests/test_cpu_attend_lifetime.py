@@ -46,8 +46,7 @@ def test_a_converted_rotation_outlives_the_call(monkeypatch, shape, dtype, step)
 
     host = _Host(made)
     monkeypatch.setattr(attention, "_rotation", watch)
-    monkeypatch.setattr(attention, "cluster_flags", lambda *a, **k: 0)
-    monkeypatch.setattr(attention, "tile_flags", lambda *a: 0)
+    monkeypatch.setattr(attention, "growing_forms", lambda *shape: (0, 0, 0))
     monkeypatch.setattr(_lib, "host", lambda: host)
     rot = torch.ones(*shape[:-1], shape[-1] * step, dtype=dtype)[..., ::step]
     attention.fused_blockgtq_decode_attention(*_args(), v_bits=3, v_rotation=rot)

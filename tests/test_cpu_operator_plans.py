@@ -27,8 +27,11 @@ def operator(monkeypatch):
             return None, None, None
 
     monkeypatch.setattr(attention, "make_decode_plan", make_plan)
-    monkeypatch.setattr(attention, "cluster_flags", lambda B, n_kv, T, *a, **k: MERGING if T <= 3000 else 0)
-    monkeypatch.setattr(attention, "tile_flags", lambda B, n_kv, T, *a: NARROW if T <= 9000 else 0)
+    def forms(B, n_kv, T, *shape):
+        split = NARROW if T <= 9000 else 0
+        return MERGING if T <= 3000 else split, split, MERGING
+
+    monkeypatch.setattr(attention, "growing_forms", forms)
     monkeypatch.setattr(_lib, "host", lambda: Host())
 
     def call(T, lut, row=48):
