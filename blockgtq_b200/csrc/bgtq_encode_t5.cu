@@ -797,6 +797,12 @@ __global__ void __launch_bounds__(kThreads, 1) encode_t5_kernel(const EncParams 
     }
     if (tid < 32) tmem_alloc(&S.tmem_base, kTmemCols);
     const int n_tiles = (P.n_batch * P.n_tok + kTileRows - 1) / kTileRows;
+    // What follows may start once every CTA is at its last (head, role).  From the start of the launch, its CTAs (and those of
+    // the launch behind it) all settle on the first SMs to be free, while this launch holds the others, and share them to the
+    // end: encode, rotation and prefill of 5192 tokens of 4 KV heads x 2 took 187.3 us, 182.7 so (10000 x 1: 293.6, 288.1).  With
+    // more than 32 tiles per CTA the few that begin their last range late would hold up the next launch's tables more than
+    // that costs (1 048 576 K and as many V rows, again and again: 373.7 us from the start, 375.0 so).
+    if (!ONE && n_tiles * P.n_kv > 16 * (int)gridDim.x) grid_launch_dependents();
     const int64_t len_k = (int64_t)units_k * n_tiles, len_v = (int64_t)units_v * n_tiles, len = len_k + len_v, all = len * P.n_kv;
     const int64_t u0 = all * blockIdx.x / gridDim.x, u1 = all * (blockIdx.x + 1) / gridDim.x;
     bool waited = false, in_range = true;
@@ -808,9 +814,6 @@ __global__ void __launch_bounds__(kThreads, 1) encode_t5_kernel(const EncParams 
         const int w = is_v ? units_v : units_k;
         const int lo = (int)((u - base + w - 1) / w), hi = (int)((min(u1, end) - base + w - 1) / w);
         u = end;
-        // What follows may start once every CTA is at its last (head, role).  From the start of the launch, its CTAs (and those of
-        // the launch behind it) all settled on the first SMs to be free, while this launch held the others, and shared them to
-        // the end: encode, rotation and prefill of 5192 tokens of 4 KV heads x 2 took 187.3 us, 182.7 so (10000 x 1: 293.6, 288.1).
         if (u >= u1) grid_launch_dependents();
         if (lo >= hi) continue;
         e5_setup(S, P, P.desc[h], is_v, h);
