@@ -34,17 +34,17 @@ sys.path.insert(0, os.path.join(ROOT, "tests"))
 HD = 128
 
 WORKLOADS = {
-    # BASELINE.json configs[1]: Qwen2.5-3B shape, K3V3 packed cache, batch 8 per GPU, context 32768
+    # Qwen2.5-3B shape, K3V3 packed cache, batch 8 per GPU, context 32768
     "qwen2.5-3b_k3v3_b8_t32768": dict(layers=36, n_q=16, n_kv=2, batch=8, ctx=32768, k_bits=3.0, v_bits=3,
                                       theta=1e6, n_sink=0, window=0),
-    # BASELINE.json configs[2]: Llama-3.1-8B shape, K2V2, batch 32, context 16384, fp16 sink 4 + window 128
+    # Llama-3.1-8B shape, K2V2, batch 32, context 16384, fp16 sink 4 + window 128
     "llama3.1-8b_k2v2_b32_t16384_sink4_win128": dict(layers=32, n_q=32, n_kv=8, batch=32, ctx=16384, k_bits=2.0,
                                                      v_bits=2, theta=5e5, n_sink=4, window=128),
-    # BASELINE.json configs[3]: one 131072-token sequence, Llama-3.1-8B shape, K2V2, sequence chunks across
+    # one 131072-token sequence, Llama-3.1-8B shape, K2V2, sequence chunks across
     # GPUs with one all-gather of (O, LSE) per layer (strong scaling: the total context is fixed)
     "llama3.1-8b_k2v2_b1_t131072_seqshard": dict(layers=32, n_q=32, n_kv=8, batch=1, ctx=131072, k_bits=2.0,
                                                  v_bits=2, theta=5e5, n_sink=0, window=0, mode="seq"),
-    # BASELINE.json configs[4]: bulk (prefill) encode, Mistral-Nemo-12B shape, 4 x 32768 tokens per layer into the
+    # bulk (prefill) encode, Mistral-Nemo-12B shape, 4 x 32768 tokens per layer into the
     # BlockGTQKVManager layout, then single-token appends; two layers with separate inputs stand for the 40
     "mistral-nemo-12b_k3v3_encode_b4_t32768": dict(layers=2, n_q=32, n_kv=8, batch=4, ctx=32768, k_bits=3.0,
                                                    v_bits=3, theta=1e6, n_sink=0, window=0, mode="encode"),
@@ -52,10 +52,10 @@ WORKLOADS = {
     # 16384-token prompt, K3V3; a step = bulk encode + causal prefill attention of one layer
     "llama3.1-8b_k3v3_prefill_t16384": dict(layers=1, n_q=32, n_kv=8, batch=1, ctx=16384, k_bits=3.0, v_bits=3,
                                             theta=5e5, n_sink=0, window=0, mode="prefill"),
-    # small variant of configs[2] for quick runs and profiler captures
+    # small variant of the Llama-3.1-8B batch workload for quick runs and profiler captures
     "llama3.1-8b_k2v2_b32_t16384_sink4_win128_4layers": dict(layers=4, n_q=32, n_kv=8, batch=32, ctx=16384,
                                                              k_bits=2.0, v_bits=2, theta=5e5, n_sink=4, window=128),
-    # small variant of configs[1] for quick runs and profiler captures
+    # small variant of the default workload for quick runs and profiler captures
     "qwen2.5-3b_k3v3_b8_t32768_4layers": dict(layers=4, n_q=16, n_kv=2, batch=8, ctx=32768, k_bits=3.0, v_bits=3,
                                               theta=1e6, n_sink=0, window=0),
 }
@@ -63,7 +63,8 @@ DEFAULT = "qwen2.5-3b_k3v3_b8_t32768"
 REF_DIR = os.path.join(ROOT, "baseline", "_ref")
 
 
-TRAFFIC_SOURCES = ["blockgtq_b200/csrc/bgtq_decode_kernel.cuh", "blockgtq_b200/csrc/bgtq_decode_plan.cu",
+TRAFFIC_SOURCES = ["blockgtq_b200/csrc/bgtq_decode_kernel.cuh", "blockgtq_b200/csrc/bgtq_decode_params.cuh",
+                   "blockgtq_b200/csrc/bgtq_decode_cluster.cuh", "blockgtq_b200/csrc/bgtq_decode_plan.cu",
                    "blockgtq_b200/csrc/bgtq_plan.h", "blockgtq_b200/csrc/bgtq_decode.cu",
                    "blockgtq_b200/csrc/bgtq_decode_jit.cu", "blockgtq_b200/csrc/bgtq_common.cuh"]
 
