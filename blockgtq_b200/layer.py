@@ -479,22 +479,22 @@ def merges(layer, flags: int) -> bool:
     return layer.plan_entry(flags)[2]
 
 
-def cluster_flags(n_batch: int, n_kv: int, n_tokens: int, device, gqa: int, v_bits: int, grows: bool = False) -> int:
+def cluster_flags(n_batch: int, n_kv: int, n_tokens: int, device, gqa: int, v_bits: int, grows: bool = False, eager: bool = False) -> int:
     """Plan flags of the form that merges a pair's shares inside the decode launch (``DEC_CLUSTER_SHIFT``; the narrow tile), for
     layer steps and attentions over up to ``n_tokens`` rows, or 0 where the decode over all SMs and its merge launch are faster.
     ``v_bits``: as stored (nibbles: 4).
 
     A cluster of C CTAs per (batch, KV head) pair saves the second launch and the partials' way through memory, 2 to 4 us (one
-    sequence of 8 KV heads, K3V3, 500 tokens: 12.6 -> 10.9 us per layer; 4 sequences at 4000 tokens: 23.1 -> 19.8).  How far that
+    sequence of 8 KV heads, K3V3, 500 tokens: 12.6 -> 10.9 us per layer; 4 sequences at 4000 tokens: 23.1 -> 20.6).  How far that
     carries: see ``_merging_limit``.  C is the largest of 8, 4 and 2 whose clusters all run at once: 14 clusters of 8, 32 of 4 and
     72 of 2 do (16 of 8 and 36 of 4 take two waves); and smaller while a CTA then has at most 8 warps' tokens, or 16 where the CTAs
     would take more than half of the SMs, which the next launch's CTAs start on.  ``grows``: the length goes up from call to call;
-    one C for all of them, as each is a kernel of its own."""
+    one C for all of them, as each is a kernel of its own.  ``eager``: never captured, so that a launch costs the host's time too."""
     pairs = n_batch * n_kv
-    if pairs < 1 or v_bits not in _TOKEN_NS:        # (a call to complain about)
+    if pairs < 1 or v_bits not in _MOST_SHARE:      # (a call to complain about)
         return 0
     sms = _sm_count(device.index if device.index is not None else torch.cuda.current_device())
-    c, most = _merging_limit(pairs, sms, gqa > 4, v_bits)
+    c, most = _merging_limit(pairs, sms, gqa > 4, v_bits, eager)
     if n_tokens > most:
         return 0
     while not grows and c > 2 and 2 * n_tokens <= (256 if 2 * pairs * c > sms else 128) * c:
@@ -502,31 +502,32 @@ def cluster_flags(n_batch: int, n_kv: int, n_tokens: int, device, gqa: int, v_bi
     return _lib.DEC_NARROW | c << _lib.DEC_CLUSTER_SHIFT
 
 
-_TOKEN_NS = {1: (8.2, 6.3), 2: (8.2, 6.3), 3: (9.4, 7.9), 4: (11.9, 11.5)}      # of a CTA, narrow and wide tile, by V's bits
+_MOST_SHARE = {1: 2200, 2: 2200, 3: 2500, 4: 6000}      # tokens of a CTA of a cluster, by V's bits: see _merging_limit
 
 
 @functools.lru_cache(maxsize=1024)
-def _merging_limit(pairs: int, sms: int, wide_groups: bool, v_bits: int):
-    """(C, the most tokens its clusters are taken for).  A CTA of a cluster gets tokens / C of them instead of an SM's even share,
-    in the narrow tile, where the split form takes the wide one past 256 tokens per SM (see ``tile_flags``).  Limits on both,
-    from layers of 1 to 72 pairs, 1 to 8 query heads per KV head and every V width timed both ways:
-      * about 300 tokens more than the even share (3 us; with wider V codes fewer), 110 fewer where eight CTAs exchange the rows of
-        more than four query heads; up to 60 more with few pairs, whose rows leave many partials to a merge launch;
-      * beside the wide tile, 3.8 us more time (nibbles, whose wide tile gains little: 4.6).  Without this limit 72 pairs
-        lost 17 % (K3V3, 24000 tokens: 106.9 -> 124.7 us) and 24 % (K2V2); as it is, 32 pairs go from 24.1 to 22.0 us at 5000
-        tokens and take the split form from 6000 on, where the two are even."""
-    narrow, wide = _TOKEN_NS[v_bits]
+def _merging_limit(pairs: int, sms: int, wide_groups: bool, v_bits: int, eager: bool):
+    """(C, the most tokens its clusters are taken for), from layers of 2 to 72 pairs, 4 and 8 query heads per KV head and V of 2 to 4
+    bits timed in both forms at up to eight lengths each, captured and called one by one:
+      * a CTA gets tokens / C of them instead of an SM's even share: up to 330 more (3 us) are made up for.  Fewer of a captured
+        layer with few pairs, whose split form runs the narrow tile too: 270 with 4-bit values and up to 16 pairs (one sequence of 8 heads,
+        4600 tokens: 16.6 -> 17.5 us), 110 less where eight CTAs exchange the rows of more than four query heads (4600 tokens: 16.5 ->
+        17.5, K3V3).  Called one by one the second launch costs the host 2.5 us, which carries that far (attention 18.0, 15.6);
+      * beside the wide tile clusters fall behind with every token, the more the narrower V is: to 2200, 2500 and 6000 tokens of a
+        CTA with 2, 3 and 4 bits (two layers, K3V3, clusters and split form: of 2 CTAs, 72 pairs, 4500 tokens 66.6 and 69.8 us, 5500 75.9
+        both, 9000 108.7 and 100.1; of 4, 32 pairs, 8900: 63.9 and 65.6, 9700: 69.0 and 67.0; K2V2, 72 pairs, 4200: 61.5 both,
+        7000: 84.3 and 76.4), and to 1050 in clusters of 8 (14 pairs, 7600: 37.7 and 39.0, 8900: 41.0 and 39.4)."""
     for c, most in ((8, 14), (4, 32), (2, 72)):
         if pairs <= most * sms // 148:
-            even = min(pairs / sms, 1 / c - 1e-6)
-            apart = {1: 330, 2: 330, 3: 280, 4: 270}[v_bits] - (110 if c == 8 and wide_groups else 0)
-            if pairs <= 4:
-                apart = min(apart + 60, 330)
-            limit = apart / (1 / c - even)
-            slower = narrow / c - wide * even           # ns per token of the context
-            if slower > 0:
-                limit = min(limit, max(256 / even, (4600 if v_bits == 4 else 3800) / slower))
-            return c, int(limit)
+            apart = 330
+            if not eager:
+                wide = c == 8 and wide_groups
+                if v_bits == 4 and 4 * (1 if wide else 2) <= pairs <= 16:
+                    apart = 270
+                if wide and pairs > 4:
+                    apart -= 110
+            limit = apart * sms * c // (sms - pairs * c) if pairs * c < sms else 1 << 30
+            return c, min(limit, c * (1050 if c == 8 else _MOST_SHARE[v_bits]))
     return 0, -1
 
 
@@ -536,7 +537,7 @@ def growing_forms(n_batch: int, n_kv: int, n_tokens: int, index, gqa: int, v_bit
     the merging form that its shape takes while it is short (0: none).  (A microsecond of arithmetic, asked for per head and layer.)"""
     device = torch.device("cuda" if index is None else f"cuda:{index}")
     split = tile_flags(n_batch, n_kv, n_tokens, device)
-    merging, short = (cluster_flags(n_batch, n_kv, n, device, gqa, v_bits, True) for n in (n_tokens, 1))
+    merging, short = (cluster_flags(n_batch, n_kv, n, device, gqa, v_bits, grows=True, eager=True) for n in (n_tokens, 1))
     return merging or split, split, short
 
 

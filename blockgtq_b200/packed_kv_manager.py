@@ -73,6 +73,7 @@ class BlockGTQKVManager:
         self._enc_flags = (_lib.ENC_K_MIXED if k_mixed else 0) | (_lib.ENC_V_NIBBLE if v_nibble else 0)
         self._dec_flags = (_lib.DEC_K_MIXED if k_mixed else 0) | (_lib.DEC_V_NIBBLE if v_nibble else 0)
         self._cluster_flags = 0               # of layer steps and attend: see layer.cluster_flags
+        self._attend_flags = 0                # of attend alone, where a captured layer is past them (0: as the steps)
         self._merging = set()                 # layers whose decode merges its shares (one launch less)
         # single-token decode steps take the position from the device and keep their arrays, so that they can be
         # captured (the reference graphs only its T=1 encode, packed_kv_manager.py:182-257); with fp16 regions that
@@ -168,8 +169,9 @@ class BlockGTQKVManager:
                 # merging form pays where that launch leaves a third of the SMs to it.
                 L, sms = _lib.lib(), torch.cuda.get_device_properties(dev).multi_processor_count
                 if not self._buffered or 3 * L.bgtq_buffer_attn_ctas(self.n_sink, self.recent_window + 1, self.B, self.n_q, self.n_kv) <= 2 * sms:
-                    self._cluster_flags = cluster_flags(self.B, self.n_kv, self.max_T, dev, gqa=self.n_q // self.n_kv,
-                                                        v_bits=4 if self.v_nibble else self.v_bits)
+                    shape = (self.B, self.n_kv, self.max_T, dev, self.n_q // self.n_kv, 4 if self.v_nibble else self.v_bits)
+                    self._cluster_flags = cluster_flags(*shape)
+                    self._attend_flags = 0 if self._cluster_flags else cluster_flags(*shape, eager=True)
         self._prepare_decode_plans()
         self._q_rot = torch.empty(self.B, self.n_q, self.hd, dtype=torch.float16, device=dev)
         self._part_o = torch.empty(self.B, self.n_q, self._n_splits, self.hd, dtype=torch.float32, device=dev)
@@ -191,8 +193,8 @@ class BlockGTQKVManager:
     def _attach(self, exchange):
         """Sequence sharding: from here on a step leaves its partials to the exchange, so its decode is the split form."""
         self._exchange = exchange
-        if self._cluster_flags:
-            self._cluster_flags = 0
+        if self._cluster_flags or self._attend_flags:
+            self._cluster_flags = self._attend_flags = 0
             self._prepare_decode_plans()
 
     def _layer_rows(self, li: int):
@@ -217,6 +219,8 @@ class BlockGTQKVManager:
         pd = _lib.DEC_PROGRAMMATIC
         flags = self._dec_flags | self._cluster_flags
         flag_sets = {flags, flags | pd}
+        if self._attend_flags:
+            flag_sets.add(self._dec_flags | self._attend_flags | pd)
         with ThreadPoolExecutor(max_workers=min(16, os.cpu_count() or 1)) as ex:     # one layer per job: its flag
             list(ex.map(lambda lt: [lt.plan(f) for f in sorted(flag_sets)], layers))  # variants share one kernel
         self._merging = {lt for lt in layers if self._cluster_flags and merges(lt, flags)}
@@ -578,7 +582,7 @@ class BlockGTQKVManager:
         if self._buffered and with_buffers:
             buf_o, buf_lse = self._buffer_partial(li, q, n_sink_tok, n_packed, n_recent)
         return attend(lt, q, *self._layer_rows(li), lo, hi, rotate=not baked,
-                      n_splits=n_splits, scale=self.scale, flags=self._dec_flags | self._cluster_flags, v_rot=lt.v_rot, buf_o=buf_o, buf_lse=buf_lse,
+                      n_splits=n_splits, scale=self.scale, flags=self._dec_flags | (self._cluster_flags or self._attend_flags), v_rot=lt.v_rot, buf_o=buf_o, buf_lse=buf_lse,
                       want_f32=want_partial, want_lse=want_partial, status=self._status)
 
     def _buffer_partial(self, li, q, n_sink_tok, n_packed, n_recent):

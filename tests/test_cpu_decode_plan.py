@@ -256,23 +256,24 @@ def test_cluster_sizes():
 @pytest.mark.parametrize("sms", [148, 132, 74])
 def test_limits_of_the_merging_form(monkeypatch, sms):
     """Taken for every shape while it is short, up to one length, and for no longer contexts: more than an SM's share of them goes to
-    each CTA, in the tile that is the slower one for long runs."""
+    each CTA, in the tile that is the slower one for long runs.  Calls one by one are taken as far as captured ones or further."""
     from blockgtq_b200 import layer
     monkeypatch.setattr(layer, "_sm_count", lambda index: sms)
     dev = torch.device("cuda:0")
     for v_bits in (1, 2, 3, 4):
         for gqa in (1, 4, 8):
             for pairs in range(1, 73 * sms // 148 + 2):
-                flags = [layer.cluster_flags(pairs, 1, n, dev, gqa=gqa, v_bits=v_bits, grows=True) for n in range(1, 30001, 311)]
-                taken = sum(map(bool, flags))
-                assert all(flags[:taken]) and not any(flags[taken:]) and len(set(flags[:taken])) <= 1
-                assert (taken > 0) == (pairs <= 72 * sms // 148)
-                c = (flags[0] or 8 << 8) >> 8
-                assert pairs * c <= sms or not taken
-                if taken:           # tokens of a CTA: no more than 330 above the even share, nor 3.8 us (4.6) of the wide tile's time
-                    n = 311 * (taken - 1) + 1
-                    assert n / c - n * pairs / sms <= 331
-                    if n * pairs > 257 * sms:
-                        narrow, wide = {1: (8.2, 6.3), 2: (8.2, 6.3), 3: (9.4, 7.9), 4: (11.9, 11.5)}[v_bits]
-                        assert narrow * n / c - wide * n * pairs / sms <= (4601 if v_bits == 4 else 3801)
+                kept = 0
+                for eager in (False, True):
+                    flags = [layer.cluster_flags(pairs, 1, n, dev, gqa=gqa, v_bits=v_bits, grows=True, eager=eager) for n in range(1, 30001, 311)]
+                    taken = sum(map(bool, flags))
+                    assert all(flags[:taken]) and not any(flags[taken:]) and len(set(flags[:taken])) <= 1
+                    assert (taken > 0) == (pairs <= 72 * sms // 148) and taken >= kept
+                    kept = taken
+                    c = (flags[0] or 8 << 8) >> 8
+                    assert pairs * c <= sms or not taken
+                    if taken:           # tokens of a CTA: no more than 330 above the even share, nor than clusters keep up with
+                        n = 311 * (taken - 1) + 1
+                        assert n / c - n * pairs / sms <= 331
+                        assert n <= c * (1050 if c == 8 else {1: 2200, 2: 2200, 3: 2500, 4: 6000}[v_bits])
     assert layer.cluster_flags(0, 8, 100, dev, gqa=4, v_bits=3) == layer.cluster_flags(1, 8, 100, dev, gqa=4, v_bits=5) == 0

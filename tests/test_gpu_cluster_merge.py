@@ -211,6 +211,30 @@ def test_the_other_partial_beside_an_empty_range():
                 assert torch.equal(g.nan_to_num(), w.nan_to_num())
 
 
+@pytest.mark.parametrize("batch,n_kv,gqa,v_bits,cap", [(1, 8, 8, 3, 3200), (2, 4, 4, 4, 3900)])
+def test_attention_past_the_steps_limit(batch, n_kv, gqa, v_bits, cap):
+    """A capacity past which captured layers take the split form and attentions, called one by one, still merge: the same rows."""
+    from blockgtq_b200 import _lib
+    from blockgtq_b200.layer import attend
+    gen = torch.Generator().manual_seed(8)
+    mgr = _manager(batch, n_kv, gqa, cap, gen, v_bits=v_bits)
+    n = cap - 7
+    mgr.init_from_cache([tuple(_rand(gen, batch, n_kv, n, 128) for _ in range(2))])
+    assert not mgr._cluster_flags and mgr._attend_flags >> _lib.DEC_CLUSTER_SHIFT == 8
+    q = _rand(gen, batch, n_kv * gqa, 128)
+    lt, cache = mgr._layers[0], (mgr._k_packed[0], mgr._k_norms[0], mgr._v_packed[0], mgr._v_norms[0])
+    top = float((mgr._v_norms[0].float().max() * max(t.centroids.abs().max() for t in lt.v_tables)).item())
+    for lo, hi in ((0, n), (5, 1700), (40, 40)):
+        out, o32, lse = mgr.attend(0, q, token_range=(lo, hi), want_partial=True)
+        _, want, want_lse = attend(lt, q, *cache, lo, hi, rotate=True, v_rot=lt.v_rot, want_f32=True, want_lse=True, flags=mgr._dec_flags)
+        if hi > lo:
+            assert (lse - want_lse).abs().max().item() <= 1e-5 * max(1.0, want_lse.abs().max().item())
+        else:
+            assert torch.equal(lse, want_lse)
+        assert (o32 - want).abs().max().item() <= 2.0 ** -10 * top * 128 ** 0.5
+        assert torch.equal(out, o32.half())
+
+
 def _regions(mgr, n_tok):
     """Sink and packed tokens of a step's attention (a token that leaves the window is packed behind it)."""
     from oracle import bgtq_oracle as O
