@@ -801,8 +801,9 @@ __global__ void __launch_bounds__(kThreads, 1) encode_t5_kernel(const EncParams 
     // the launch behind it) all settle on the first SMs to be free, while this launch holds the others, and share them to the
     // end: encode, rotation and prefill of 5192 tokens of 4 KV heads x 2 took 187.3 us, 182.7 so (10000 x 1: 293.6, 288.1).  With
     // more than 32 tiles per CTA the few that begin their last range late would hold up the next launch's tables more than
-    // that costs (1 048 576 K and as many V rows, again and again: 373.7 us from the start, 375.0 so).
-    if (!ONE && n_tiles * P.n_kv > 16 * (int)gridDim.x) grid_launch_dependents();
+    // that costs (1 048 576 K and as many V rows, again and again: 373.7 us from the start, 375.0 so); with one tile each all end
+    // together (K, then V, of 2000 rows of 8 heads: 18.5, 19.1).
+    if (ONE || n_tiles * P.n_kv > 16 * (int)gridDim.x) grid_launch_dependents();
     const int64_t len_k = (int64_t)units_k * n_tiles, len_v = (int64_t)units_v * n_tiles, len = len_k + len_v, all = len * P.n_kv;
     const int64_t u0 = all * blockIdx.x / gridDim.x, u1 = all * (blockIdx.x + 1) / gridDim.x;
     bool waited = false, in_range = true;
@@ -814,7 +815,7 @@ __global__ void __launch_bounds__(kThreads, 1) encode_t5_kernel(const EncParams 
         const int w = is_v ? units_v : units_k;
         const int lo = (int)((u - base + w - 1) / w), hi = (int)((min(u1, end) - base + w - 1) / w);
         u = end;
-        if (u >= u1) grid_launch_dependents();
+        if (!ONE && u >= u1) grid_launch_dependents();
         if (lo >= hi) continue;
         e5_setup(S, P, P.desc[h], is_v, h);
         // The rows, and what this launch overwrites, belong to earlier work in the stream.  (The one-tile form waits where it
